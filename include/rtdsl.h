@@ -59,10 +59,13 @@ typedef enum rtd_radius_heuristic {
     RTD_RADIUS_SAMPLED_PERCENTILE = 1,  /* k_nn! default: param = percentile P, x1.1 */
     RTD_RADIUS_FIXED = 2,               /* param = radius */
     RTD_RADIUS_SAMPLED_MAX = 3,         /* percentile 1.0 */
-    RTD_RADIUS_MORTON_WINDOW = 4        /* no radius rounds: each query's list starts with the
-                                           4k points around it in the index's Morton order and
-                                           one unbounded round follows (thread-per-query search;
-                                           elsewhere as RTD_RADIUS_SAMPLED_NN with param) */
+    RTD_RADIUS_MORTON_WINDOW = 4        /* no radius rounds: each query starts from the points
+                                           around it in the index's Morton order and one
+                                           unbounded round follows.  Exact searches
+                                           (partial_results = 0) with min(k, n) <= 2048 run
+                                           this way whatever the heuristic, since their result
+                                           does not depend on it; where rounds do run, as
+                                           RTD_RADIUS_SAMPLED_NN with param */
 } rtd_radius_heuristic;
 
 /* gprt-ir Schedule (gprt-ir/src/lib.rs:58-89) re-expressed for the kernels
@@ -79,7 +82,8 @@ typedef struct rtd_schedule {
     uint32_t use_morton_lbv;      /* process queries in Morton order (k_nn! lib.rs:456-460) */
     uint32_t leaf_size;           /* LBVH leaf size: subtrees of <= leaf_size points collapse */
     uint32_t block_size;          /* threads per block of the search kernel (0 = auto) */
-    uint32_t lanes_per_query;     /* 1 = thread per query, 32 = warp per query (0 = auto) */
+    uint32_t lanes_per_query;     /* 1 = thread per query, 32 = warp per query (0 = auto: by k
+                                     and the number of queries) */
     uint32_t morton_bits;         /* 30 (u32 keys, the reference layout) or 33..63 in steps
                                      of 3 (u64 keys, bits/3 per axis); 0 = auto */
     uint32_t partial_results;     /* 0 (default): exact; the last allowed round is unbounded.
@@ -195,9 +199,9 @@ void rtd_limits_get(rtd_limits *l);
  * d2 != NULL).  Slots beyond the number of points hold 0xFFFFFFFF / +inf.
  * Any k >= 1, as the reference's 2K-slot per-query slab
  * (gprt-macros/src/lib.rs:300-310): k <= 16 keeps a thread's list in
- * registers, k <= 256 a warp's list striped over its registers, and larger
- * k a warp's sorted list in shared memory (min(k, n) <= 2048) or in a
- * device slab the index keeps (grown on demand, at most 1 GiB).
+ * registers, larger k (and small calls) collect a warp's candidates in
+ * shared memory (min(k, n) <= 2048), and the largest k keep a warp's sorted
+ * list in a device slab of the index (grown on demand, at most 1 GiB).
  * ------------------------------------------------------------------- */
 rtd_status rtd_knn(rtd_index *idx, const float *d_queries, uint64_t nq, uint32_t k,
                    const rtd_schedule *sched, uint32_t *d_ids, float *d_d2, rtd_stream stream);

@@ -6,6 +6,7 @@
 // (knn_traverse.cuh).
 #include <atomic>
 
+#include "knn_collect.cuh"
 #include "knn_traverse.cuh"
 
 namespace rtd {
@@ -29,6 +30,7 @@ struct KnnArgs {
     int key64;
     float scale;
     const uint32_t *wpos;   // optional: each query's position, by processing order
+    const float4 *pyr;      // box pyramid over the sorted points
 };
 
 // Position of a query among the points' sorted Morton keys (lower bound),
@@ -61,6 +63,23 @@ __device__ __forceinline__ uint32_t morton_position(const IndexHeader *h, const 
         }
     }
     return lo;
+}
+
+// The same by a whole warp.
+__device__ __forceinline__ uint32_t morton_position_warp(const IndexHeader *h, const void *skeys, uint32_t n,
+                                                         int key64, float scale, float qx, float qy, float qz) {
+    if (key64) {
+        const SceneNorm s = scene_norm_cubic(h);
+        return warp_lower_bound<uint64_t>(static_cast<const uint64_t *>(skeys), 0u, n,
+                                          morton63(quantize(qx, s.lo[0], s.ext[0], scale),
+                                                   quantize(qy, s.lo[1], s.ext[1], scale),
+                                                   quantize(qz, s.lo[2], s.ext[2], scale)));
+    }
+    const SceneNorm s = scene_norm(h);
+    return warp_lower_bound<uint32_t>(static_cast<const uint32_t *>(skeys), 0u, n,
+                                      morton30(quantize(qx, s.lo[0], s.ext[0], 1023.0f),
+                                               quantize(qy, s.lo[1], s.ext[1], 1023.0f),
+                                               quantize(qz, s.lo[2], s.ext[2], 1023.0f)));
 }
 
 // Every query's position, in processing order, ahead of the search (so the
@@ -150,6 +169,32 @@ __global__ void __launch_bounds__(BLOCK, KC <= 5 ? 1280 / BLOCK : 0) knn_thread_
                 if (p.d2) p.d2[ob + j - (KC - kk)] = bk[j];
             }
         }
+    }
+}
+
+// One warp per query that collects and selects (knn_collect.cuh); kk =
+// min(k, points) <= COLLECT_MAX_K.
+constexpr int COLLECT_WARPS = 4;
+__global__ void __launch_bounds__(COLLECT_WARPS * 32, 10) knn_collect_kernel(const KnnArgs p, uint32_t kk) {
+    chain_wait();
+    extern __shared__ uint2 s_dyn[];
+    __shared__ uint32_t s_off[12];
+    const uint32_t n = (uint32_t)p.ix.n;
+    if (threadIdx.x == 0) collect_offsets(n, s_off);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5;
+    const CollectScratch s = collect_scratch(
+        reinterpret_cast<char *>(s_dyn) + (size_t)warp * collect_warp_bytes(kk, n), kk, n);
+    const CollectTree tree{p.ix.pts, p.pyr, s_off, 0u, n};
+    for (uint64_t t = (uint64_t)blockIdx.x * COLLECT_WARPS + warp; t < p.nq;
+         t += (uint64_t)gridDim.x * COLLECT_WARPS) {
+        const uint64_t qi = p.perm ? p.perm[t] : t;
+        const float qx = p.q[3 * qi], qy = p.q[3 * qi + 1], qz = p.q[3 * qi + 2];
+        const uint32_t pos = p.wpos ? p.wpos[t]
+                                    : morton_position_warp(p.ix.hdr, p.skeys, n, p.key64, p.scale, qx, qy, qz);
+        Collected c = collect_query(tree, s, qx, qy, qz, kk, pos);
+        const uint64_t ob = qi * (uint64_t)p.k;
+        collect_store(s, c, kk, p.k, p.ids + ob, p.d2 ? p.d2 + ob : nullptr);
     }
 }
 
@@ -360,6 +405,17 @@ rtd_status launch_wide(rtd_index *idx, const KnnArgs &a, cudaStream_t st) {
     return RTD_OK;
 }
 
+rtd_status launch_collect(rtd_index *idx, const KnnArgs &a, cudaStream_t st) {
+    const uint32_t kk = (uint32_t)(a.k < a.ix.n ? a.k : a.ix.n);
+    const size_t smem = COLLECT_WARPS * collect_warp_bytes(kk, a.ix.n);
+    if (smem > 48 * 1024)
+        RTD_CUDA(cudaFuncSetAttribute(knn_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(COLLECT_WARPS * collect_warp_bytes(COLLECT_MAX_K, 1ull << 30))));
+    RTD_LAUNCH_CHAINED(knn_collect_kernel, dim3(grid_for(a.nq, COLLECT_WARPS, 1 << 20)), dim3(COLLECT_WARPS * 32),
+                       smem, st, a, kk);
+    return RTD_OK;
+}
+
 // Moves the query-ordering error flags into the index's.
 __global__ void fold_errors_kernel(IndexHeader *into, IndexHeader *from) {
     if (from->err) {
@@ -401,29 +457,54 @@ rtd_status knn_search(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t k,
     return knn_search_ex(idx, d_q, nq, k, sched, d_ids, d_d2, st, false, nullptr, nullptr);
 }
 
-// Whether a search with this schedule runs the Morton-window seed (the
-// thread-per-query kernel with RTD_RADIUS_MORTON_WINDOW).
-static bool uses_window(const rtd_index *idx, const rtd_schedule &s, uint32_t k) {
+// How a search runs.  Exact searches (partial_results = 0) start from the
+// points around each query in Morton order and need no radius rounds: their
+// result is the same for every starting radius.
+enum class Search { thread_window, collect, rounds };
+// lanes_per_query = 0 (auto): a warp per query for k > 16 and, in exact
+// searches, for few queries.  A thread's search is a serial chain that takes
+// about as long for 1,000 queries as for 100,000, while the warp's grows
+// with their number: measured, 100,000 uniform points, thread / warp, us:
+// k = 5: 10,000 queries 141 / 41, 100,000 156 / 290; k = 16: 331 / 52 and
+// 397 / 373; the two cross near 8,000 k queries.
+constexpr uint64_t WARP_QUERIES_PER_K = 8000;
+static uint32_t search_lanes(const rtd_schedule &s, uint64_t nq, uint32_t k) {
     uint32_t lanes = s.lanes_per_query;
-    if (lanes == 0) lanes = k <= 16 ? 1 : 32;
+    if (lanes == 0) lanes = k <= 16 && (s.partial_results || nq > WARP_QUERIES_PER_K * k) ? 1 : 32;
     if (lanes == 1 && k > 32) lanes = 32;
-    return lanes == 1 && !s.partial_results && s.radius_heuristic == RTD_RADIUS_MORTON_WINDOW &&
-           idx->n > 1 && idx->skeys != nullptr;
+    return lanes;
+}
+// (n: points of the index, whose sorted keys every build of n > 0 keeps)
+static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
+    if (s.partial_results || n < 2) return Search::rounds;
+    const uint32_t lanes = search_lanes(s, nq, k);
+    if (lanes == 1) return Search::thread_window;
+    const uint64_t kk = k < n ? k : n;
+    return lanes == 32 && kk <= COLLECT_MAX_K ? Search::collect : Search::rounds;
+}
+// Whether the queries are put in Morton order first.  The warp search gains
+// little from neighbours running together (40,000 queries, k = 300: 1.16 ms
+// without, 1.18 ms with; 100,000: 2.30 and 2.21), so below this many queries
+// it does without the dozen launches of the ordering, about 40 us.
+constexpr uint64_t COLLECT_ORDER_MIN = 49152;
+static bool wants_order(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
+    return s.use_morton_lbv && !(nq < COLLECT_ORDER_MIN && search_mode(n, s, nq, k) == Search::collect);
 }
 
-// Launches the search kernel the schedule selects for the queries of a.
-static rtd_status launch_search(rtd_index *idx, const rtd_schedule &s, uint32_t k, KnnArgs a,
+// Launches the search kernel the schedule selects for the queries of a
+// (nq: of the whole search, of which a may hold a chunk).
+static rtd_status launch_search(rtd_index *idx, const rtd_schedule &s, uint64_t nq, uint32_t k, KnnArgs a,
                                 cudaStream_t st) {
-    uint32_t lanes = s.lanes_per_query;
-    if (lanes == 0) lanes = k <= 16 ? 1 : 32;
-    if (lanes == 1 && k > 32) lanes = 32;
+    const uint32_t lanes = search_lanes(s, nq, k);
     const uint32_t block = s.block_size;
+    const Search mode = search_mode(idx->n, s, nq, k);
     rtd_status r;
-    if (lanes == 1) {
-        // The Morton-window seed runs in the thread-per-query kernel; the
-        // other launch modes treat the heuristic as RTD_RADIUS_SAMPLED_NN.
-        if (uses_window(idx, s, k)) a.skeys = idx->skeys;
-        else a.wpos = nullptr;
+    if (mode != Search::rounds) a.skeys = idx->skeys;
+    else a.wpos = nullptr;
+    if (mode == Search::collect) {
+        a.pyr = idx->pyramid.as<float4>();
+        r = launch_collect(idx, a, st);
+    } else if (lanes == 1) {
         if (k <= 1) r = launch_thread<1>(a, block, st);
         else if (k <= 2) r = launch_thread<2>(a, block, st);
         else if (k <= 4) r = launch_thread<4>(a, block, st);
@@ -463,11 +544,11 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
         return fail(RTD_ERR_INVALID_ARGUMENT, "fixed radius must be > 0");
     for (int e = EV_SEARCH0; e <= EV_SEARCH1; ++e) idx->ev_set[e] = false;
     idx->mark(EV_SEARCH0, st);
-    // the Morton-window search runs one unbounded round: no initial radius
-    if (!uses_window(idx, s, k)) RTD_TRY(seed_radius(idx, d_q, nq, k, s, st));
+    // (only the radius rounds need an initial radius)
+    if (search_mode(idx->n, s, nq, k) == Search::rounds) RTD_TRY(seed_radius(idx, d_q, nq, k, s, st));
     idx->mark(EV_SEEDED, st);
     const uint32_t *perm = given_perm;
-    if (!have_perm) RTD_TRY(order_queries(idx, d_q, nq, s.use_morton_lbv != 0, &perm, st));
+    if (!have_perm) RTD_TRY(order_queries(idx, d_q, nq, wants_order(idx->n, s, nq, k), &perm, st));
     idx->mark(EV_ORDERED, st);
     KnnArgs a;
     a.ix = view_of(idx);
@@ -484,11 +565,12 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
     a.err = &idx->hdr.as<IndexHeader>()->err;
     a.skeys = nullptr;
     a.wpos = wpos;
+    a.pyr = nullptr;
     a.key64 = idx->morton_bits != 30;
     a.scale = idx->morton_bits == 30 ? 1023.0f : (float)((1u << (idx->morton_bits / 3)) - 1u);
     rtd_status r = RTD_OK;
     if (!hc || hc->chunks <= 1) {
-        r = launch_search(idx, s, k, a, st);
+        r = launch_search(idx, s, nq, k, a, st);
         if (r == RTD_OK && hc) {   // one chunk: copy every row out
             RTD_CUDA(cudaMemcpyAsync(hc->h_ids, d_ids, nq * (uint64_t)k * 4, cudaMemcpyDeviceToHost, st));
             if (d_d2 && hc->h_d2)
@@ -515,7 +597,7 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
                     if (a.d2) ac.d2 = a.d2 + b * k;
                 }
                 if (a.wpos) ac.wpos = a.wpos + b;
-                r = launch_search(idx, s, k, ac, cs);
+                r = launch_search(idx, s, nq, k, ac, cs);
                 if (r == RTD_OK) {
                     RTD_CUDA(cudaMemcpyAsync(hc->h_ids + b * k, d_ids + b * k, (e - b) * k * 4,
                                              cudaMemcpyDeviceToHost, cs));
@@ -545,21 +627,25 @@ rtd_status k_nn_device(rtd_index *idx, const float *d_points, uint64_t n, const 
     rtd_schedule_default(&def);
     const rtd_schedule &s = sched ? *sched : def;
     const uint32_t chunks = hc ? hc->chunks : 1u;
+    const bool order = nq >= 2 && k > 0 && wants_order(n, s, nq, k);
+    // With the thread-per-query window search, the queries' positions among
+    // the sorted keys are found on the side stream as soon as the keys are
+    // sorted, while the tree is built (a warp finds its own).
+    const bool window = nq && k > 0 && search_mode(n, s, nq, k) == Search::thread_window;
+    const bool fork = order || window || hc;   // (a host call copies its queries in on the side stream)
     RTD_TRY(ensure_side_stream(idx));
     cudaStream_t side = idx->side_stream;
-    RTD_CUDA(cudaEventRecord(idx->ev_fork, st));   // the queries' producers come first
-    RTD_CUDA(cudaStreamWaitEvent(side, idx->ev_fork, 0));
     const uint32_t *perm = nullptr;
     rtd_status ord = RTD_OK;
-    if (s.use_morton_lbv && nq >= 2 && k > 0)
-        ord = order_queries_own(idx->qorder, d_q, nq, &perm, side, chunks);
-    RTD_CUDA(cudaEventRecord(idx->ev_join, side));
+    if (fork) {
+        RTD_CUDA(cudaEventRecord(idx->ev_fork, st));   // the queries' producers come first
+        RTD_CUDA(cudaStreamWaitEvent(side, idx->ev_fork, 0));
+        if (order) ord = order_queries_own(idx->qorder, d_q, nq, &perm, side, chunks);
+        RTD_CUDA(cudaEventRecord(idx->ev_join, side));
+    }
     rtd_status r = index_build(idx, d_points, n, &s, st);
-    // With the Morton-window seed, the queries' positions among the sorted
-    // keys are found on the side stream as soon as the keys are sorted,
-    // while the tree is built.
     const uint32_t *wpos = nullptr;
-    if (r == RTD_OK && ord == RTD_OK && nq && uses_window(idx, s, k)) {
+    if (r == RTD_OK && ord == RTD_OK && window) {
         r = idx->wpos.reserve(nq * sizeof(uint32_t));
         if (r == RTD_OK) {
             RTD_CUDA(cudaStreamWaitEvent(side, idx->ev_sorted, 0));
@@ -573,7 +659,7 @@ rtd_status k_nn_device(rtd_index *idx, const float *d_points, uint64_t n, const 
             wpos = idx->wpos.as<uint32_t>();
         }
     }
-    RTD_CUDA(cudaStreamWaitEvent(st, idx->ev_join, 0));   // also on the error paths
+    if (fork) RTD_CUDA(cudaStreamWaitEvent(st, idx->ev_join, 0));   // also on the error paths
     RTD_TRY(ord);
     RTD_TRY(r);
     if (perm && !wpos) {   // (window_pos_kernel has folded them otherwise)
