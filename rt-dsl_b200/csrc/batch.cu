@@ -5,18 +5,22 @@
 // cloud's points together in Morton order, and one Karras tree over the
 // whole key array is a forest whose node covering a cloud's key range is
 // that cloud's LBVH (keys sharing the cloud prefix form a subtree of a
-// binary radix tree).  Search: one persistent launch.  Work items of <= 32
-// Morton-ordered queries of one cloud, each carrying its k class, are taken
-// from one device counter by every warp of the grid; an item runs the
-// thread-per-query register list (k <= 16), the warp-per-query striped
-// register list (k <= 256) or the warp-per-query memory list (any larger k)
-// of knn_traverse.cuh against its cloud's root.  Items are queued heaviest
-// class first, so the long warp-per-query items start early and the short
-// ones fill the tail.  The whole pass is launch-only (no host
+// binary radix tree).  Search: work items of <= 32 Morton-ordered queries of
+// one cloud, taken from device counters by two persistent launches.  Lists
+// of more than 8 are collected by a warp per query (knn_collect.cuh) on a
+// side stream, longest first; shorter lists run a thread per query from the
+// query's Morton neighbours (knn_traverse.cuh) in the second launch, whose
+// blocks take the SMs as the first one's leave.  The second launch also
+// holds the warp-per-query lists of passes with partial_results and the
+// memory lists of more than 512 entries.  256 clouds, 9M points, 2.2M
+// queries, k from {1, 5, 16, 64}: 25.0 ms with radius rounds and merged
+// warp lists, now 7.1 ms; bound by instruction issue (0.85 of the slots).  The whole pass is launch-only (no host
 // synchronisation), so it can be captured as one CUDA graph and replayed.
+#include <algorithm>
 #include <new>
 #include <vector>
 
+#include "knn_collect.cuh"
 #include "knn_traverse.cuh"
 
 struct rtd_batch;
@@ -196,9 +200,26 @@ struct BatchArgs {
     uint32_t max_rounds;
     uint32_t partial;   // the reference's round cap (rtd_schedule.partial_results)
     uint32_t *err;
-    uint2 *wide;        // per-warp list slabs of the k > 256 class
+    uint2 *wide;        // per-warp list slabs of the widest class
     uint32_t wide_kk;   // entries per slab: the largest min(k, points) of that class
+    // exact passes: the sorted keys of the points and of the queries (in item
+    // order), and the box pyramid over the sorted points
+    const uint64_t *skeys, *qskeys;
+    const float4 *pyr;
+    uint32_t n_points;
+    uint32_t collect_kk, collect_n;   // largest min(k, points) and points of the collecting clouds
 };
+
+// Position of the queries of an item among their cloud's sorted keys.
+__device__ __forceinline__ uint32_t cloud_position(const BatchArgs &a, const CloudDesc &c, uint64_t key) {
+    uint32_t lo = c.pt_begin, hi = c.pt_begin + c.n_pts;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(&a.skeys[mid]) < key) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
 
 template <int KC>
 __device__ __forceinline__ void item_thread(const BatchArgs &a, const TreeRef &t,
@@ -211,7 +232,25 @@ __device__ __forceinline__ void item_thread(const BatchArgs &a, const TreeRef &t
     const int kk = (int)c.k;
     float bk[KC];
     uint32_t bi[KC];
-    knn_query_thread<KC>(t, rs, qx, qy, qz, kk, s_col, 32, l_stack, a.err, bk, bi);
+    if (a.skeys) {
+        // one unbounded round from the 4k points around the query in the
+        // cloud's Morton order
+        list_init<KC>(bk, bi, kk);
+        const uint32_t pos = cloud_position(a, c, a.qskeys[w.start + lane]);
+        const uint32_t n = 4u * (uint32_t)kk < c.n_pts ? 4u * (uint32_t)kk : c.n_pts;
+        uint32_t w0 = pos - c.pt_begin > n / 2u ? pos - n / 2u : c.pt_begin;
+        if (w0 + n > c.pt_begin + c.n_pts) w0 = c.pt_begin + c.n_pts - n;
+        for (uint32_t j = w0; j < w0 + n; ++j) {
+            const float4 pt = __ldg(&t.pts[j]);
+            const float key = exact_key(qx, qy, qz, pt.x, pt.y, pt.z);
+            const uint32_t id = __float_as_uint(pt.w);
+            if (key_less(key, id, bk[KC - 1], bi[KC - 1])) list_insert<KC>(bk, bi, key, id);
+        }
+        const RoundSpec one{rs.r0sq, rs.mult2, 1u, 0u};
+        knn_query_thread<KC, true>(t, one, qx, qy, qz, kk, s_col, 32, l_stack, a.err, bk, bi, w0, w0 + n);
+    } else {
+        knn_query_thread<KC>(t, rs, qx, qy, qz, kk, s_col, 32, l_stack, a.err, bk, bi);
+    }
     const uint64_t ob = c.out_off + (uint64_t)(qi - c.q_begin) * kk;
 #pragma unroll
     for (int j = 0; j < KC; ++j)
@@ -261,12 +300,21 @@ __device__ __forceinline__ void item_wide(const BatchArgs &a, const TreeRef &t, 
     }
 }
 
-// k classes of the search: register list of 8 or 16 slots (thread per
-// query), warp list of 32, 64 or 256 slots (warp per query), memory list
-// (warp per query, k > 256).
-constexpr int N_CLASSES = 6;
-__host__ __device__ constexpr int k_class(uint32_t k) {
-    return k <= 8 ? 0 : k <= 16 ? 1 : k <= 32 ? 2 : k <= 64 ? 3 : k <= 256 ? 4 : 5;
+// k classes of the search: register lists (thread per query), warp lists
+// of 32, 64 or 256 slots (warp per query; passes with partial_results),
+// memory list (warp per query), and collected lists (knn_collect.cuh, warp
+// per query, in a launch of their own).
+enum : uint32_t { CLS_T1, CLS_T5, CLS_T8, CLS_T16, CLS_W32, CLS_W64, CLS_W256, CLS_WIDE, CLS_COLLECT, N_CLASSES };
+// Lists above this are collected: all 256 clouds of 1,000 to 200,000 points
+// with k = 16, a thread / a warp per query: 11.1 / 10.2 ms, of up to 8,000
+// points 1.20 / 0.93 ms; with k = 5 the thread's list is far shorter.
+constexpr uint32_t COLLECT_ABOVE = 8;
+constexpr uint32_t BATCH_COLLECT_MAX = 512;     // entries: 11 KB of shared memory a warp
+inline uint32_t k_class(uint32_t k, uint32_t n, bool exact, bool warp) {
+    const uint32_t kk = k < n ? k : n;
+    if (exact && (k > COLLECT_ABOVE || warp) && kk <= BATCH_COLLECT_MAX) return CLS_COLLECT;
+    if (k <= 16 && !warp) return k <= 1 ? CLS_T1 : k <= 5 ? CLS_T5 : k <= 8 ? CLS_T8 : CLS_T16;
+    return k <= 32 ? CLS_W32 : k <= 64 ? CLS_W64 : k <= 256 ? CLS_W256 : CLS_WIDE;
 }
 
 // Shared memory of one warp, reused by whichever class its current item
@@ -295,14 +343,49 @@ __global__ void __launch_bounds__(SWARPS * 32) batch_knn_kernel(const BatchArgs 
         const TreeRef t{a.pts, a.nodes, nullptr, c.root, c.root_count, visit_cap};
         const RoundSpec rs{c.r0sq, a.mult2, a.max_rounds, a.partial};
         switch (w.cls) {
-        case 0: item_thread<8>(a, t, rs, c, w, sw + lane, l_stack); break;
-        case 1: item_thread<16>(a, t, rs, c, w, sw + lane, l_stack); break;
-        case 2: item_warp<1>(a, t, rs, c, w, stk, ls); break;
-        case 3: item_warp<2>(a, t, rs, c, w, stk, ls); break;
-        case 4: item_warp<8>(a, t, rs, c, w, stk, ls); break;
+        case CLS_T1: item_thread<1>(a, t, rs, c, w, sw + lane, l_stack); break;
+        case CLS_T5: item_thread<5>(a, t, rs, c, w, sw + lane, l_stack); break;
+        case CLS_T8: item_thread<8>(a, t, rs, c, w, sw + lane, l_stack); break;
+        case CLS_T16: item_thread<16>(a, t, rs, c, w, sw + lane, l_stack); break;
+        case CLS_W32: item_warp<1>(a, t, rs, c, w, stk, ls); break;
+        case CLS_W64: item_warp<2>(a, t, rs, c, w, stk, ls); break;
+        case CLS_W256: item_warp<8>(a, t, rs, c, w, stk, ls); break;
         default: item_wide(a, t, rs, c, w, stk, s_r, slab); break;
         }
         __syncwarp();
+    }
+}
+
+// The collected lists: a persistent launch over their items, a quarter of
+// an item (8 queries) at a time, so that the last ones end close together.
+constexpr uint32_t COLLECT_PART = 8;
+__global__ void __launch_bounds__(SWARPS * 32, 10) batch_collect_kernel(const BatchArgs a) {
+    extern __shared__ uint2 s_dyn[];
+    __shared__ uint32_t s_off[12];
+    if (threadIdx.x == 0) collect_offsets(a.n_points, s_off);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    char *base = reinterpret_cast<char *>(s_dyn) + (size_t)warp * collect_warp_bytes(a.collect_kk, a.collect_n);
+    while (true) {
+        uint32_t it = 0;
+        if (lane == 0) it = atomicAdd(a.counter, 1u);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it / (32 / COLLECT_PART) >= a.n_items) break;
+        const WorkItem w = a.items[it / (32 / COLLECT_PART)];
+        const CloudDesc c = a.cd[w.cloud];
+        const uint32_t kk = c.k < c.n_pts ? c.k : (c.n_pts ? c.n_pts : 1u);
+        const CollectScratch s = collect_scratch(base, kk, c.n_pts);
+        const CollectTree tree{a.pts, a.pyr, s_off, c.pt_begin, c.pt_begin + c.n_pts};
+        const uint32_t j0 = it % (32 / COLLECT_PART) * COLLECT_PART;
+        for (uint32_t j = j0; j < w.count && j < j0 + COLLECT_PART; ++j) {
+            const uint32_t qi = a.qperm[w.start + j];
+            const float qx = a.q[3 * (uint64_t)qi], qy = a.q[3 * (uint64_t)qi + 1], qz = a.q[3 * (uint64_t)qi + 2];
+            const uint32_t pos = warp_lower_bound<uint64_t>(a.skeys, c.pt_begin, c.pt_begin + c.n_pts,
+                                                            a.qskeys[w.start + j]);
+            const Collected got = collect_query(tree, s, qx, qy, qz, kk, pos);
+            const uint64_t ob = c.out_off + (uint64_t)(qi - c.q_begin) * c.k;
+            collect_store(s, got, kk, c.k, a.ids + ob, a.d2 ? a.d2 + ob : nullptr);
+        }
     }
 }
 
@@ -343,7 +426,9 @@ using namespace rtd;
 struct rtd_batch {
     std::vector<rtd_cloud> clouds;
     uint32_t n_clouds = 0, n_items = 0;
-    int blocks = 0;             // grid of the persistent search
+    uint32_t n_collect = 0;     // items of the collected lists, ahead of the others
+    uint32_t collect_kk = 0, collect_n = 0;
+    int blocks = 0, collect_blocks = 0;   // grids of the persistent searches
     uint32_t wide_kk = 0;       // list slab entries per warp (0: no k > 256 cloud)
     uint64_t n_points = 0, n_queries = 0;
     int cbits = 0, bpa = 21;
@@ -376,7 +461,7 @@ static rtd_status batch_pass(rtd_batch *b, const float *d_pts, const float *d_q,
     CloudDesc *cd = b->cd.as<CloudDesc>();
     IndexHeader *h = f.hdr.as<IndexHeader>();
     RTD_CUDA(cudaMemsetAsync(h, 0, sizeof(IndexHeader), st));
-    RTD_CUDA(cudaMemsetAsync(b->counter.ptr, 0, sizeof(uint32_t), st));
+    RTD_CUDA(cudaMemsetAsync(b->counter.ptr, 0, 2 * sizeof(uint32_t), st));
     batch_reset_kernel<<<grid_for(b->n_clouds, 128, 1024), 128, 0, st>>>(cd, b->n_clouds);
     RTD_LAUNCH_CHECK();
     batch_cloud_of_kernel<<<b->n_clouds, 256, 0, st>>>(cd, b->pcloud.as<uint32_t>(),
@@ -392,6 +477,7 @@ static rtd_status batch_pass(rtd_batch *b, const float *d_pts, const float *d_q,
         b->sched.radius_param);
     RTD_LAUNCH_CHECK();
     const int kbits = 3 * b->bpa + b->cbits;
+    const uint64_t *skeys = nullptr;
     if (n) {
         batch_keys_kernel<<<g, BLOCK, 0, st>>>(d_pts, n, b->pcloud.as<uint32_t>(), cd, b->bpa,
                                               f.keys.as<uint64_t>());
@@ -401,6 +487,7 @@ static rtd_status batch_pass(rtd_batch *b, const float *d_pts, const float *d_q,
                                            f.vals.as<uint32_t>(), f.vals_alt.as<uint32_t>(), true, n,
                                            0, kbits, f.sort, &h->err, st, &alt));
         const uint64_t *sk = alt ? f.keys_alt.as<uint64_t>() : f.keys.as<uint64_t>();
+        skeys = sk;
         const uint32_t *perm = alt ? f.vals_alt.as<uint32_t>() : f.vals.as<uint32_t>();
         batch_gather_kernel<<<g, BLOCK, 0, st>>>(d_pts, perm, b->pcloud.as<uint32_t>(), cd, n,
                                                  f.pts.as<float4>());
@@ -438,15 +525,48 @@ static rtd_status batch_pass(rtd_batch *b, const float *d_pts, const float *d_q,
         a.max_rounds = b->sched.max_rounds;
         a.partial = b->sched.partial_results ? 1u : 0u;
         a.err = &h->err;
-        a.items = b->items.as<WorkItem>();
-        a.n_items = b->n_items;
-        a.counter = b->counter.as<uint32_t>();
         a.wide = b->wide_kk ? b->wide.as<uint2>() : nullptr;
         a.wide_kk = b->wide_kk;
-        if (b->n_items) {
-            batch_knn_kernel<<<b->blocks, SWARPS * 32, 0, st>>>(a);
-            RTD_LAUNCH_CHECK();
+        // (without points no key is read: every window is empty)
+        a.skeys = a.partial ? nullptr : n ? skeys : b->qkeys.as<uint64_t>();
+        a.qskeys = alt ? b->qkeys_alt.as<uint64_t>() : b->qkeys.as<uint64_t>();
+        a.pyr = f.pyramid.as<float4>();
+        a.n_points = (uint32_t)n;
+        a.collect_kk = b->collect_kk;
+        a.collect_n = b->collect_n;
+        // The collected lists run on the side stream; the other classes'
+        // blocks take the SMs as theirs leave.
+        const bool both = b->n_collect && b->n_items;
+        cudaStream_t cs = st;
+        if (both) {
+            RTD_TRY(ensure_side_stream(&f));
+            cs = f.side_stream;
+            RTD_CUDA(cudaEventRecord(f.ev_fork, st));
+            RTD_CUDA(cudaStreamWaitEvent(cs, f.ev_fork, 0));
         }
+        cudaError_t ce = cudaSuccess;
+        if (b->n_collect) {
+            a.items = b->items.as<WorkItem>();
+            a.n_items = b->n_collect;
+            a.counter = b->counter.as<uint32_t>() + 1;
+            batch_collect_kernel<<<b->collect_blocks, SWARPS * 32,
+                                   SWARPS * collect_warp_bytes(b->collect_kk, b->collect_n), cs>>>(a);
+            note_launch();
+            ce = cudaGetLastError();
+        }
+        if (both) RTD_CUDA(cudaEventRecord(f.ev_join, cs));
+        cudaError_t te = cudaSuccess;
+        if (b->n_items) {
+            a.items = b->items.as<WorkItem>() + b->n_collect;
+            a.n_items = b->n_items;
+            a.counter = b->counter.as<uint32_t>();
+            batch_knn_kernel<<<b->blocks, SWARPS * 32, 0, st>>>(a);
+            note_launch();
+            te = cudaGetLastError();
+        }
+        if (both) RTD_CUDA(cudaStreamWaitEvent(st, f.ev_join, 0));   // also on the error paths
+        if (ce != cudaSuccess) return cuda_fail(ce, "batch_collect_kernel launch");
+        if (te != cudaSuccess) return cuda_fail(te, "batch_knn_kernel launch");
     }
     return RTD_OK;
 }
@@ -484,7 +604,7 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
     if (s.max_rounds < 1) return fail(RTD_ERR_INVALID_ARGUMENT, "max_rounds must be >= 1");
     if (s.leaf_size < 1 || s.leaf_size > 64) return fail(RTD_ERR_INVALID_ARGUMENT, "leaf_size must be in [1, 64]");
     uint64_t np = 0, nq = 0;
-    uint32_t wide_kk = 0;
+    uint32_t wide_kk = 0, collect_kk = 0, collect_n = 0;
     std::vector<CloudDesc> cd(n_clouds);
     std::vector<WorkItem> cls_items[N_CLASSES];
     for (uint32_t c = 0; c < n_clouds; ++c) {
@@ -494,20 +614,24 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
         if (x.k < 1) return fail(RTD_ERR_INVALID_ARGUMENT, "k must be >= 1");
         cd[c] = CloudDesc{(uint32_t)np, x.n_points, (uint32_t)nq, x.n_queries, x.k, 0u, 0u, {}, 0.f,
                           x.out_offset};
-        const int cls = s.lanes_per_query == 32 && x.k <= 32 ? 2 : k_class(x.k);
-        if (cls == 5 && x.n_queries) {
-            const uint32_t kk = x.k < x.n_points ? x.k : (x.n_points ? x.n_points : 1u);
-            if (kk > wide_kk) wide_kk = kk;
+        const uint32_t cls = k_class(x.k, x.n_points, !s.partial_results, s.lanes_per_query == 32);
+        const uint32_t kk = x.k < x.n_points ? x.k : (x.n_points ? x.n_points : 1u);
+        if (cls == CLS_WIDE && x.n_queries && kk > wide_kk) wide_kk = kk;
+        if (cls == CLS_COLLECT && x.n_queries) {
+            if (kk > collect_kk) collect_kk = kk;
+            if (x.n_points > collect_n) collect_n = x.n_points;
         }
         for (uint32_t s0 = 0; s0 < x.n_queries; s0 += 32)
             cls_items[cls].push_back(WorkItem{c, (uint32_t)nq + s0,
-                                              x.n_queries - s0 < 32u ? x.n_queries - s0 : 32u,
-                                              (uint32_t)cls});
+                                              x.n_queries - s0 < 32u ? x.n_queries - s0 : 32u, cls});
         np += x.n_points;
         nq += x.n_queries;
     }
     if (np >= (1ull << 30) - 1 || nq >= (1ull << 30)) return fail(RTD_ERR_INVALID_ARGUMENT, "batch too large");
-    // one queue, heaviest class first
+    // the collected lists' queue, longest lists first, then the others',
+    // heaviest class first
+    std::stable_sort(cls_items[CLS_COLLECT].begin(), cls_items[CLS_COLLECT].end(),
+                     [&](const WorkItem &x, const WorkItem &y) { return clouds[x.cloud].k > clouds[y.cloud].k; });
     std::vector<WorkItem> items;
     for (int c = N_CLASSES - 1; c >= 0; --c) items.insert(items.end(), cls_items[c].begin(), cls_items[c].end());
     b->drop_graph();
@@ -515,7 +639,10 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
     b->n_clouds = n_clouds;
     b->n_points = np;
     b->n_queries = nq;
-    b->n_items = (uint32_t)items.size();
+    b->n_collect = (uint32_t)cls_items[CLS_COLLECT].size();
+    b->n_items = (uint32_t)items.size() - b->n_collect;
+    b->collect_kk = collect_kk;
+    b->collect_n = collect_n;
     b->wide_kk = wide_kk;
     b->sched = s;
     int cb = 0;
@@ -546,7 +673,7 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
     RTD_TRY(b->qkeys_alt.reserve(nq * 8 + 8));
     RTD_TRY(b->qvals.reserve(nq * 4 + 4));
     RTD_TRY(b->qvals_alt.reserve(nq * 4 + 4));
-    RTD_TRY(b->counter.reserve(sizeof(uint32_t)));
+    RTD_TRY(b->counter.reserve(2 * sizeof(uint32_t)));
     if (n_clouds)
         RTD_CUDA(cudaMemcpy(b->cd.ptr, cd.data(), n_clouds * sizeof(CloudDesc), cudaMemcpyHostToDevice));
     if (!items.empty())
@@ -559,7 +686,7 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
     RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_knn_kernel, SWARPS * 32, 0));
     if (per_sm < 1) per_sm = 1;
     uint64_t blocks = (uint64_t)sms * per_sm;
-    const uint64_t need = ((uint64_t)items.size() + SWARPS - 1) / SWARPS;
+    const uint64_t need = ((uint64_t)b->n_items + SWARPS - 1) / SWARPS;
     if (blocks > need) blocks = need ? need : 1;
     if (wide_kk) {
         const uint64_t per_block = (uint64_t)SWARPS * wide_kk * sizeof(uint2);
@@ -568,6 +695,16 @@ rtd_status rtd_batch_plan(rtd_batch *b, const rtd_cloud *clouds, uint32_t n_clou
         RTD_TRY(b->wide.reserve(blocks * per_block));
     }
     b->blocks = (int)blocks;
+    if (b->n_collect) {
+        const size_t smem = SWARPS * collect_warp_bytes(collect_kk, collect_n);
+        RTD_CUDA(cudaFuncSetAttribute(batch_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(SWARPS * collect_warp_bytes(BATCH_COLLECT_MAX, 1ull << 30))));
+        RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_collect_kernel, SWARPS * 32, smem));
+        if (per_sm < 1) per_sm = 1;
+        const uint64_t most = ((uint64_t)b->n_collect * (32 / COLLECT_PART) + SWARPS - 1) / SWARPS;
+        blocks = (uint64_t)sms * per_sm;
+        b->collect_blocks = (int)(blocks < most ? blocks : most);
+    }
     return RTD_OK;
 }
 

@@ -80,12 +80,11 @@ template <typename K>
 __device__ __forceinline__ uint32_t warp_lower_bound(const K *__restrict__ sk, uint32_t lo, uint32_t hi, K key) {
     const int lane = threadIdx.x & 31;
     while (hi - lo > 32) {
-        const uint32_t len = hi - lo;
-        const uint32_t at = lo + (uint32_t)(((uint64_t)len * (lane + 1)) / 33);
-        const uint32_t less = __popc(__ballot_sync(0xffffffffu, __ldg(&sk[at]) < key));
-        const uint32_t base = lo;
-        if (less) lo = base + (uint32_t)(((uint64_t)len * less) / 33) + 1;
-        if (less < 32) hi = base + (uint32_t)(((uint64_t)len * (less + 1)) / 33);
+        const uint32_t step = (hi - lo) / 33 + 1, at = lo + (lane + 1) * step - 1;
+        const uint32_t less = __popc(__ballot_sync(0xffffffffu, at < hi && __ldg(&sk[at]) < key));
+        const uint32_t next = lo + (less + 1) * step - 1;   // the first probe not below the key
+        lo += less * step;
+        if (less < 32 && next < hi) hi = next;
     }
     return lo + __popc(__ballot_sync(0xffffffffu, lo + lane < hi && __ldg(&sk[lo + lane]) < key));
 }
@@ -104,7 +103,7 @@ struct Collected {
 // the keys differ (keys are >= +0, so their bits order as they do), stopping
 // at the first threshold that keeps few enough.
 // (Not inlined: its four call sites would not fit the instruction cache.)
-__device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, Collected c, uint32_t kk, uint32_t slack) {
+static __device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, Collected c, uint32_t kk, uint32_t slack) {
     const int lane = threadIdx.x & 31;
     const uint32_t *kb = reinterpret_cast<const uint32_t *>(key);
     __syncwarp();
@@ -226,12 +225,12 @@ __device__ __forceinline__ Collected collect_query(const CollectTree &t, const C
         const bool near = bk * 16.0f <= c.tk;
         const uint32_t mo = __ballot_sync(0xffffffffu, ok), ml = mo & __ballot_sync(0xffffffffu, level == 1);
         const uint32_t mnear = __ballot_sync(0xffffffffu, near);
-        const uint32_t same = level == 1 ? ml : mo & ~ml, far = same & ~mnear;
-        const uint32_t at = near ? __popc(far) + __popc(same & mnear & lt) : __popc(far & lt);
-        const uint2 entry = make_uint2(level << 28 | e, __float_as_uint(bk));
-        if (ok) *(level == 1 ? s.leaf + lq + at : s.stack + sp + at) = entry;
-        lq += __popc(ml);
-        sp += __popc(mo & ~ml);
+        const uint32_t same = level == 1 ? ml : mo & ~ml, nl = __popc(ml), nn = __popc(mo & ~ml);
+        const uint32_t at = __popc(same & (near ? mnear : ~mnear) & lt);
+        uint2 *to = level == 1 ? s.leaf + lq : s.stack + sp;
+        if (ok) to[near ? (level == 1 ? nl : nn) - 1 - at : at] = make_uint2(level << 28 | e, __float_as_uint(bk));
+        lq += nl;
+        sp += nn;
         __syncwarp();
     };
     uint32_t top = 1;
@@ -308,7 +307,7 @@ __device__ __forceinline__ void collect_lane_exchange(float (&key)[E], uint32_t 
 // and more go through shared memory, the others through shuffles, two runs
 // at a time; everything loops (sorts unrolled in registers, E = 12 for k =
 // 300, spent more time on instruction fetches than on anything else).
-__device__ __noinline__ void collect_sort_store(float *key, uint32_t *id, uint32_t cnt, uint32_t k, uint32_t *ids,
+static __device__ __noinline__ void collect_sort_store(float *key, uint32_t *id, uint32_t cnt, uint32_t k, uint32_t *ids,
                                                 float *d2) {
     const int lane = threadIdx.x & 31;
     const uint32_t runs = cnt ? (cnt + 31) / 32 : 1u, n = runs * 32;
