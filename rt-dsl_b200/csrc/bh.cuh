@@ -18,7 +18,7 @@ namespace rtd {
 
 constexpr uint32_t BH_LEAF_BIT = 0x80000000u;
 constexpr int BH_MAX_LEVEL = 21;            // octant digits held by a 63-bit path key
-constexpr int BH_GROUP = 32;                // bodies per warp-coherent group
+constexpr int BH_GROUP = 32;                // bodies per warp-coherent group: a run of the flat order
 
 struct BhHeader {
     float root_min[3], root_max[3];
@@ -30,7 +30,6 @@ struct BhHeader {
     uint32_t err;
     uint32_t level_count[BH_MAX_LEVEL + 2];
     uint32_t level_off[BH_MAX_LEVEL + 3];
-    uint32_t n_groups;        // warp groups of the Plummer walks
     uint32_t max_stack;       // deepest traversal stack seen by a walk
     uint32_t group_counter;   // work queue of the walks (next group to take)
     uint32_t ilog_used;       // interaction-log pages taken by the last logging forward
@@ -47,7 +46,7 @@ constexpr uint32_t ILOG_PAGE = 16;
 constexpr uint32_t ILOG_NONE = 0xFFFFFFFFu;
 struct IlogView {
     uint2 *entries;     // pages * ILOG_PAGE * 32
-    uint8_t *counts;    // pages * ILOG_PAGE: entries | 0x80 for a body tile
+    uint8_t *counts;    // pages * ILOG_PAGE: entries | kind of the tile << 6
     uint32_t *next;     // pages: the group's next page
     uint2 *group;       // per warp group; nullptr = no log (forward) / walk (adjoint)
     uint32_t pages;     // pool capacity
@@ -67,7 +66,7 @@ struct rtd_bh {
     uint32_t bucket = 128;
     float min_width = 1e-5f;
     bool built = false;
-    bool plummer_ready = false;   // child table and groups built (Plummer-law walks)
+    bool plummer_ready = false;   // child table built (Plummer-law walks)
     bool has_quad = false;        // quadrupoles computed
     rtd::DevBuf hdr;
     // build scratch
@@ -82,8 +81,8 @@ struct rtd_bh {
     rtd::DevBuf order;        // flat order: original index of the i-th body
     rtd::DevBuf fbody;        // float4 (pos, mass) in flat order
     rtd::DevBuf node_a, node_b, node_q;
-    // walk structures: child table (8 per node), leaf list, warp groups
-    rtd::DevBuf child8, leaf_node, groups, stack;
+    // walk structures: child table (8 per node), traversal stacks
+    rtd::DevBuf child8, stack;
     uint64_t stack_warps = 0;
     // adjoint scratch
     rtd::DevBuf cell_grad, prefix, gpos_flat, gmass_flat;
@@ -118,13 +117,12 @@ struct BhView {
     const BhHeader *hdr;
     uint64_t n;
     const uint4 *child8;       // 2 uint4 per node: up to 8 children, 0xFFFFFFFF pads
-    const uint2 *groups;       // (first flat body, count <= 32)
 };
 
 inline BhView bh_view(const rtd_bh *b) {
     return BhView{b->node_a.as<float4>(), b->node_b.as<uint4>(), b->node_q.as<float4>(),
                   b->fbody.as<float4>(), b->order.as<uint32_t>(), b->hdr.as<BhHeader>(), b->n,
-                  b->child8.as<uint4>(), b->groups.as<uint2>()};
+                  b->child8.as<uint4>()};
 }
 
 rtd_status bh_build(rtd_bh *b, const float *d_pos, const float *d_mass, uint64_t n,

@@ -87,8 +87,8 @@ rtd_status rtd_bh_release(rtd_bh *b) {
                       &b->pvals, &b->pvals_alt, &b->lcp, &b->wmin, &b->lam, &b->nn, &b->base,
                       &b->heads, &b->leaf_head, &b->leaf_of, &b->fkeys, &b->fkeys_alt, &b->fvals,
                       &b->fvals_alt, &b->node_start, &b->node_level, &b->level_nodes, &b->order,
-                      &b->fbody, &b->node_a, &b->node_b, &b->node_q, &b->child8, &b->leaf_node,
-                      &b->groups, &b->stack, &b->cell_grad, &b->prefix, &b->gpos_flat,
+                      &b->fbody, &b->node_a, &b->node_b, &b->node_q, &b->child8,
+                      &b->stack, &b->cell_grad, &b->prefix, &b->gpos_flat,
                       &b->gmass_flat})
         d->release();
     for (DevBuf *d : {&b->ilog_entries, &b->ilog_counts, &b->ilog_next, &b->ilog_group})

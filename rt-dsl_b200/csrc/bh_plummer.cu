@@ -7,18 +7,26 @@
 // CPU oracle makes identical decisions); rejected leaves are summed
 // directly, rejected internal cells opened.
 //
-// Execution: a warp takes a group of <= 32 bodies (packed sibling leaves,
+// Execution: a warp takes a group of 32 bodies (consecutive in flat order,
 // so spatially compact) and walks the tree once for all of them.  Stack
-// entries carry the mask of lanes that still need the node; per step up to
-// 32 entries are loaded in parallel and each is tested by every lane in its
-// mask.  Accepted cells and the bodies of rejected leaves go to per-warp
-// lists with their lane masks; every 32 entries form a tile staged in
-// shared memory and evaluated by all lanes from broadcast reads.
+// entries carry the mask of lanes that still need the node; up to 32 are
+// taken per step, one per lane, and each lane decides its node for the whole
+// group from the group's box where the box settles it (every operation of
+// the per-body test is monotone in the distance, so a box decision equals
+// every body's); only nodes it leaves open are tested body by body.
+// Accepted cells and the bodies of rejected leaves go to four per-warp
+// lists: those every body of the group interacts with, and those with a lane
+// mask.  32 entries of a list form a tile, staged in shared memory as pairs
+// and evaluated by all lanes (lane = body) two interactions at a time in
+// packed FP32 (f32x2), which halves the instructions issued.
 //
-// Adjoint (dL/dx, dL/dm for upstream dL/da, dL/dphi): per tile, pass 1
-// (lane = body) adds d/dx_i of the body's interactions; pass 2 (lane =
-// source) sums the source-side derivatives over the group's bodies and
-// issues one vector atomic per source.  Cell derivatives (COM, mass,
+// Adjoint (dL/dx, dL/dm for upstream dL/da, dL/dphi): lane = body evaluates
+// each (body, source) pair once, adds the body's derivative up and leaves
+// three to five coefficients in shared memory; then lane = source sums the
+// source's derivative over the bodies from the coefficients (replayed from
+// the log at 1M bodies: 20.2 ms; a table of the derivatives themselves,
+// summed row by row: 33.8 ms) and adds it with one vector atomic per source
+// and part.  Cell derivatives (COM, mass,
 // quadrupole) are then pushed to the bodies by a top-down pass: with Q
 // about the COM the first moment vanishes, so for a cell C holding body j
 //     dL/dx_j += m_j (g_c/M - 2 B c + 2 B x_j)
@@ -34,63 +42,67 @@ namespace {
 
 constexpr int WW = 4;   // warps per block
 
-// Adjoint: source-side derivatives of RED_CELLS cells (3 float4 each) or
-// RED_BODIES bodies (1 float4 each) per chunk, one row per lane.
-
-constexpr int RED_CELLS = 3;
-constexpr int RED_BODIES = 9;
+// Lists of a warp, and the kinds of its tiles: what every body of the group
+// takes, and what only the lanes of a mask take.
+enum : int { L_CELLS = 0, L_CELLS_MASKED = 1, L_BODIES = 2, L_BODIES_MASKED = 3 };
 
 struct WarpTile {
-    float4 cell[32][3];   // (com, M), (Qxx Qyy Qzz Qxy), (Qxz Qyz 0 0)
-    uint32_t cmask_t[32];
-    float4 body[32];      // (x, y, z, m)
-    uint32_t bid[32];
-    uint32_t bmask_t[32];
-    uint32_t clist[32], cmask[32];
-    uint32_t blist[64], bmask[64];
+    float4 pair[16][5];   // sources 2p, 2p + 1 interleaved: (-x -x -y -y) (-z -z -M -M)
+                          // (xx xx yy yy) (zz zz xy xy) (xz xz yz yz)
+    uint32_t mask[32];
+    uint2 list[4][64];    // (cell or body, lane mask)
+    uint4 leaf[32];       // rejected leaves not yet listed: first body, bodies, lane mask
 };
 
-// The adjoint's per-chunk table: red[j][lane] = lane's share of source j.
-struct WarpRed {
-    float4 red[RED_CELLS * 3][32];
+// Adjoint: what the bodies' side of an interaction leaves for the source's
+// side, for up to ADJ_SOURCES sources at a time: the coefficients of each
+// (body, source) pair, a row a body (18 words apart: both sides read and
+// write 64-bit pairs without bank conflicts), and the bodies' positions and
+// upstream gradients, each value twice.
+constexpr int ADJ_SOURCES = 16;
+struct WarpAdj {
+    float coef[5][32][ADJ_SOURCES + 2];
+    float4 body[32][3];   // (x x y y) (z z vx vx) (vy vy vz vz)
 };
-static_assert(RED_BODIES <= RED_CELLS * 3, "body chunk fits the cell chunk's table");
 
-// Sum of each of `rows` table rows over its 32 entries, L lanes per row:
-// lane l takes row l / L and the entries seg, seg + L, seg + 2L, ... of
-// it (seg = l % L), rotated by the row so that the lanes of one load phase
-// read different banks; the row's lanes then add up by shuffles.  On
-// return `owner` marks the row's first lane, which holds the sum.
-template <int L>
-__device__ __forceinline__ float4 table_row_sum(const WarpRed &R, int rows, int lane, int &row,
-                                                bool &owner) {
-    constexpr int T = (32 + L - 1) / L;
-    row = lane / L;
-    const int seg = lane - row * L;
-    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row < rows) {
-#pragma unroll
-        for (int i = 0; i < T; ++i) {
-            int ii = i + row;
-            if (ii >= T) ii -= T;
-            const int j = seg + L * ii;
-            if (j < 32) {
-                const float4 e = R.red[row][j];
-                t.x += e.x; t.y += e.y; t.z += e.z; t.w += e.w;
-            }
-        }
-    }
-    const float4 t0 = t;
-#pragma unroll
-    for (int d = 1; d < L; ++d) {
-        t.x += __shfl_down_sync(0xffffffffu, t0.x, d);
-        t.y += __shfl_down_sync(0xffffffffu, t0.y, d);
-        t.z += __shfl_down_sync(0xffffffffu, t0.z, d);
-        t.w += __shfl_down_sync(0xffffffffu, t0.w, d);
-    }
-    owner = row < rows && seg == 0;
-    return t;
+// ------------------------------------------------------- packed FP32 pairs
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pk(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
 }
+__device__ __forceinline__ f2 pk(float a) { return pk(a, a); }
+__device__ __forceinline__ float lo(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x;
+}
+__device__ __forceinline__ float hi(f2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return y;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 rsqrt2(f2 a) { return pk(rsqrtf(lo(a)), rsqrtf(hi(a))); }
+// The halves that are wanted, else 0.
+__device__ __forceinline__ f2 keep2(f2 a, bool k0, bool k1) { return pk(k0 ? lo(a) : 0.f, k1 ? hi(a) : 0.f); }
+__device__ __forceinline__ f2 xy(const float4 &v) { return pk(v.x, v.y); }
+__device__ __forceinline__ f2 zw(const float4 &v) { return pk(v.z, v.w); }
 
 __device__ __forceinline__ float dot3_rn(float x, float y, float z) {
     float s = __fmul_rn(x, x);
@@ -112,416 +124,586 @@ __device__ __forceinline__ uint32_t lane_lt() {
     return m;
 }
 
-// Forward interaction of field point r = x - c with a cell (G omitted).
+// Forward interaction of a field point with a pair of cells (r = x - c, G
+// omitted, nM = -M): what it adds to phi and a.
 template <bool QUAD>
-__device__ __forceinline__ void cell_fwd(float rx, float ry, float rz, const float4 &c,
-                                         const float4 &q0, const float4 &q1, float eps2,
-                                         float &ax, float &ay, float &az, float &phi) {
-    const float s = rx * rx + ry * ry + rz * rz + eps2;
-    const float i1 = rsqrtf(s), i2 = i1 * i1, i3 = i1 * i2;
-    phi -= c.w * i1;
-    ax -= c.w * rx * i3;
-    ay -= c.w * ry * i3;
-    az -= c.w * rz * i3;
-    if (QUAD) {
-        const float qx = q0.x * rx + q0.w * ry + q1.x * rz;
-        const float qy = q0.w * rx + q0.y * ry + q1.y * rz;
-        const float qz = q1.x * rx + q1.y * ry + q0.z * rz;
-        const float q = rx * qx + ry * qy + rz * qz;
-        const float i5 = i3 * i2, i7 = i5 * i2;
-        phi -= 0.5f * q * i5;
-        ax += qx * i5 - 2.5f * q * rx * i7;
-        ay += qy * i5 - 2.5f * q * ry * i7;
-        az += qz * i5 - 2.5f * q * rz * i7;
+__device__ __forceinline__ void cells_fwd(const float4 *c, f2 x, f2 y, f2 z, f2 eps2, f2 &phi, f2 &ax, f2 &ay, f2 &az) {
+    const float4 c0 = c[0], c1 = c[1];
+    const f2 rx = add2(x, xy(c0)), ry = add2(y, zw(c0)), rz = add2(z, xy(c1)), nM = zw(c1);
+    const f2 i1 = rsqrt2(fma2(rx, rx, fma2(ry, ry, fma2(rz, rz, eps2))));
+    const f2 i2 = mul2(i1, i1), i3 = mul2(i1, i2);
+    phi = fma2(nM, i1, phi);
+    if (!QUAD) {
+        const f2 k = mul2(nM, i3);
+        ax = fma2(k, rx, ax);
+        ay = fma2(k, ry, ay);
+        az = fma2(k, rz, az);
+    } else {
+        const float4 q0 = c[2], q1 = c[3], q2 = c[4];
+        const f2 xx = xy(q0), yy = zw(q0), zz = xy(q1), cxy = zw(q1), cxz = xy(q2), cyz = zw(q2);
+        const f2 qx = fma2(xx, rx, fma2(cxy, ry, mul2(cxz, rz)));
+        const f2 qy = fma2(cxy, rx, fma2(yy, ry, mul2(cyz, rz)));
+        const f2 qz = fma2(cxz, rx, fma2(cyz, ry, mul2(zz, rz)));
+        const f2 i5 = mul2(i3, i2);
+        const f2 t = mul2(fma2(rx, qx, fma2(ry, qy, mul2(rz, qz))), i5);   // r.Q.r / r^5
+        phi = fma2(pk(-0.5f), t, phi);
+        const f2 k = fma2(mul2(pk(-2.5f), t), i2, mul2(nM, i3));
+        ax = fma2(k, rx, fma2(qx, i5, ax));
+        ay = fma2(k, ry, fma2(qy, i5, ay));
+        az = fma2(k, rz, fma2(qz, i5, az));
     }
 }
 
-// Derivatives of u*phi + v.a for one cell interaction (G omitted):
-// g_r = d/dr (r = x - c), gM = d/dM, gq = d/dQ (symmetric part, 6 comps).
+// Body side of the derivatives of L = u*phi + v.a for a pair of sources (r =
+// x - c, G omitted): d/dx added to g, and the coefficients
+//   A, B, H, I, N:  dL/dr = A r + B v + Q (2 H r + I v),  dL/dM = N,
+//                   dL/dQ = sym(r (H r + I v)^T)
+// zeroed for the sources this lane does not take.
+template <bool QUAD, bool MASKED>
+__device__ __forceinline__ void sources_adj(const float4 *c, f2 x, f2 y, f2 z, f2 eps2, f2 u, f2 vx, f2 vy, f2 vz,
+                                            bool k0, bool k1, f2 &gx, f2 &gy, f2 &gz, f2 (&coef)[5]) {
+    const float4 c0 = c[0], c1 = c[1];
+    const f2 rx = add2(x, xy(c0)), ry = add2(y, zw(c0)), rz = add2(z, xy(c1)), nM = zw(c1);
+    const f2 i1 = rsqrt2(fma2(rx, rx, fma2(ry, ry, fma2(rz, rz, eps2))));
+    const f2 i2 = mul2(i1, i1), i3 = mul2(i1, i2), i5 = mul2(i3, i2);
+    const f2 nvr = mul2(pk(-1.f), fma2(vx, rx, fma2(vy, ry, mul2(vz, rz)))), nu = mul2(pk(-1.f), u);
+    f2 N = fma2(nvr, i3, mul2(nu, i1));
+    // monopole: dL/dr = M ((u i3 + 3 vr i5) r - i3 v)
+    f2 A = mul2(nM, fma2(mul2(nvr, pk(3.f)), i5, mul2(nu, i3))), B = mul2(nM, i3);
+    if (!QUAD) {
+        if (MASKED) {
+            A = keep2(A, k0, k1);
+            B = keep2(B, k0, k1);
+            N = keep2(N, k0, k1);
+        }
+        gx = fma2(A, rx, fma2(B, vx, gx));
+        gy = fma2(A, ry, fma2(B, vy, gy));
+        gz = fma2(A, rz, fma2(B, vz, gz));
+    } else {
+        const float4 q0 = c[2], q1 = c[3], q2 = c[4];
+        const f2 xx = xy(q0), yy = zw(q0), zz = xy(q1), cxy = zw(q1), cxz = xy(q2), cyz = zw(q2);
+        const f2 qrx = fma2(xx, rx, fma2(cxy, ry, mul2(cxz, rz)));
+        const f2 qry = fma2(cxy, rx, fma2(yy, ry, mul2(cyz, rz)));
+        const f2 qrz = fma2(cxz, rx, fma2(cyz, ry, mul2(zz, rz)));
+        const f2 i7 = mul2(i5, i2);
+        const f2 nk1 = mul2(mul2(fma2(rx, qrx, fma2(ry, qry, mul2(rz, qrz))), pk(-2.5f)), i7);   // -2.5 rQr i7
+        const f2 vqr = fma2(vx, qrx, fma2(vy, qry, mul2(vz, qrz)));
+        // u phi_Q + v.a_Q adds (u k1 - 5 vQr i7 + 7 k1 vr i2) r - k1 v
+        // - (u i5 + 5 vr i7) Qr + i5 Qv
+        const f2 n5i7 = mul2(pk(-5.f), i7);
+        A = fma2(nu, nk1, fma2(vqr, n5i7, fma2(mul2(nk1, pk(7.f)), mul2(nvr, i2), A)));
+        B = add2(B, nk1);
+        f2 H = mul2(pk(0.5f), fma2(nu, i5, mul2(nvr, mul2(pk(5.f), i7)))), I = i5;
+        if (MASKED) {
+            A = keep2(A, k0, k1);
+            B = keep2(B, k0, k1);
+            H = keep2(H, k0, k1);
+            I = keep2(I, k0, k1);
+            N = keep2(N, k0, k1);
+        }
+        const f2 C = add2(H, H);
+        // Q (C r + I v): Q applied to one vector
+        const f2 tx = fma2(C, rx, mul2(I, vx)), ty = fma2(C, ry, mul2(I, vy)), tz = fma2(C, rz, mul2(I, vz));
+        gx = fma2(xx, tx, fma2(cxy, ty, fma2(cxz, tz, fma2(A, rx, fma2(B, vx, gx)))));
+        gy = fma2(cxy, tx, fma2(yy, ty, fma2(cyz, tz, fma2(A, ry, fma2(B, vy, gy)))));
+        gz = fma2(cxz, tx, fma2(cyz, ty, fma2(zz, tz, fma2(A, rz, fma2(B, vz, gz)))));
+        coef[3] = H;
+        coef[4] = I;
+    }
+    coef[0] = A;
+    coef[1] = B;
+    coef[2] = N;
+}
+
+// Sum of a pair over the lanes whose numbers differ in bits 3 and 4.
+__device__ __forceinline__ f2 quarter_sum(f2 a) {
+#pragma unroll
+    for (int o = 8; o <= 16; o <<= 1)
+        a = add2(a, pk(__shfl_xor_sync(0xffffffffu, lo(a), o), __shfl_xor_sync(0xffffffffu, hi(a), o)));
+    return a;
+}
+
+// Source side: lane l + 8 h takes the pair of sources l of a chunk of 8 and
+// every 4th body from h on, and adds up dL/dc (= -dL/dr), dL/dM and dL/dQ
+// from the coefficients; the four lanes of a pair then add theirs, and two
+// of them write one source each.
 template <bool QUAD>
-__device__ __forceinline__ void cell_adj(float rx, float ry, float rz, const float4 &c,
-                                         const float4 &q0, const float4 &q1, float eps2, float u,
-                                         float vx, float vy, float vz, float &grx, float &gry,
-                                         float &grz, float &gM, float gq[6]) {
-    const float s = rx * rx + ry * ry + rz * rz + eps2;
-    const float i1 = rsqrtf(s), i2 = i1 * i1, i3 = i1 * i2, i5 = i3 * i2;
-    const float M = c.w;
-    const float vr = vx * rx + vy * ry + vz * rz;
-    grx = u * M * rx * i3 - M * (vx * i3 - 3.f * vr * rx * i5);
-    gry = u * M * ry * i3 - M * (vy * i3 - 3.f * vr * ry * i5);
-    grz = u * M * rz * i3 - M * (vz * i3 - 3.f * vr * rz * i5);
-    gM = -u * i1 - vr * i3;
+__device__ __forceinline__ void sources_sum(const WarpAdj &J, const float4 *c, uint32_t rows, bool have0, bool have1,
+                                            uint32_t id0, uint32_t id1, bool cells, float G, float4 *cell_grad,
+                                            float4 *body_grad) {
+    const int lane = threadIdx.x & 31, l = lane & 7, h = lane >> 3;
+    const f2 z = pk(0.f);
+    const float4 c0 = c[0], c1 = c[1];
+    const f2 nx = xy(c0), ny = zw(c0), nz = xy(c1);
+    f2 sx = z, sy = z, sz = z, N = z, tx = z, ty = z, tz = z, gq[6] = {z, z, z, z, z, z};
+    auto coef = [&](int k, uint32_t i) { return *reinterpret_cast<const f2 *>(&J.coef[k][i][2 * l]); };
+#pragma unroll 1
+    for (uint32_t i = h; i < rows; i += 4) {
+        const float4 b0 = J.body[i][0], b1 = J.body[i][1], b2 = J.body[i][2];
+        const f2 rx = add2(xy(b0), nx), ry = add2(zw(b0), ny), rz = add2(xy(b1), nz);
+        const f2 vx = zw(b1), vy = xy(b2), vz = zw(b2);
+        const f2 A = coef(0, i), B = coef(1, i);
+        N = add2(N, coef(2, i));
+        sx = fma2(A, rx, fma2(B, vx, sx));
+        sy = fma2(A, ry, fma2(B, vy, sy));
+        sz = fma2(A, rz, fma2(B, vz, sz));
+        if (QUAD) {
+            const f2 H = coef(3, i), I = coef(4, i);
+            const f2 hx = mul2(H, rx), hy = mul2(H, ry), hz = mul2(H, rz);
+            const f2 wx = fma2(I, vx, hx), wy = fma2(I, vy, hy), wz = fma2(I, vz, hz);
+            tx = add2(tx, add2(wx, hx));
+            ty = add2(ty, add2(wy, hy));
+            tz = add2(tz, add2(wz, hz));
+            gq[0] = fma2(rx, wx, gq[0]);
+            gq[1] = fma2(ry, wy, gq[1]);
+            gq[2] = fma2(rz, wz, gq[2]);
+            gq[3] = fma2(rx, wy, fma2(ry, wx, gq[3]));
+            gq[4] = fma2(rx, wz, fma2(rz, wx, gq[4]));
+            gq[5] = fma2(ry, wz, fma2(rz, wy, gq[5]));
+        }
+    }
     if (QUAD) {
-        const float Qxx = q0.x, Qyy = q0.y, Qzz = q0.z, Qxy = q0.w, Qxz = q1.x, Qyz = q1.y;
-        const float qrx = Qxx * rx + Qxy * ry + Qxz * rz;
-        const float qry = Qxy * rx + Qyy * ry + Qyz * rz;
-        const float qrz = Qxz * rx + Qyz * ry + Qzz * rz;
-        const float qvx = Qxx * vx + Qxy * vy + Qxz * vz;
-        const float qvy = Qxy * vx + Qyy * vy + Qyz * vz;
-        const float qvz = Qxz * vx + Qyz * vy + Qzz * vz;
-        const float q = rx * qrx + ry * qry + rz * qrz;
-        const float vqr = vx * qrx + vy * qry + vz * qrz;
-        const float i7 = i5 * i2, i9 = i7 * i2;
-        // phi_Q = -q i5 / 2, a_Q = Qr i5 - 2.5 q r i7: u dphi_Q/dr = -u a_Q
-        const float k1 = 2.5f * q * i7;
-        grx -= u * (qrx * i5 - k1 * rx);
-        gry -= u * (qry * i5 - k1 * ry);
-        grz -= u * (qrz * i5 - k1 * rz);
-        // d(v.a_Q)/dr = Qv i5 - 5 vQr i7 r - 5 vr i7 Qr - 2.5 q i7 v + 17.5 q vr i9 r
-        const float kr = -5.f * vqr * i7 + 17.5f * q * vr * i9;
-        const float kq = -5.f * vr * i7;
-        const float kv = -2.5f * q * i7;
-        grx += qvx * i5 + kr * rx + kq * qrx + kv * vx;
-        gry += qvy * i5 + kr * ry + kq * qry + kv * vy;
-        grz += qvz * i5 + kr * rz + kq * qrz + kv * vz;
-        // dL/dQ: -u i5 rr^T / 2 + i5 sym(v r^T) - 2.5 vr i7 rr^T
-        const float cr = -0.5f * u * i5 - 2.5f * vr * i7;
-        gq[0] = cr * rx * rx + i5 * vx * rx;
-        gq[1] = cr * ry * ry + i5 * vy * ry;
-        gq[2] = cr * rz * rz + i5 * vz * rz;
-        gq[3] = cr * rx * ry + 0.5f * i5 * (vx * ry + vy * rx);
-        gq[4] = cr * rx * rz + 0.5f * i5 * (vx * rz + vz * rx);
-        gq[5] = cr * ry * rz + 0.5f * i5 * (vy * rz + vz * ry);
+        const float4 q0 = c[2], q1 = c[3], q2 = c[4];
+        sx = fma2(xy(q0), tx, fma2(zw(q1), ty, fma2(xy(q2), tz, sx)));
+        sy = fma2(zw(q1), tx, fma2(zw(q0), ty, fma2(zw(q2), tz, sy)));
+        sz = fma2(xy(q2), tx, fma2(zw(q2), ty, fma2(xy(q1), tz, sz)));
+    }
+    sx = quarter_sum(sx);
+    sy = quarter_sum(sy);
+    sz = quarter_sum(sz);
+    N = quarter_sum(N);
+    if (QUAD)
+#pragma unroll
+        for (int k = 0; k < 6; ++k) gq[k] = quarter_sum(gq[k]);
+    if (h == 0 ? have0 : h == 1 && have1) {
+        auto half = [&](f2 a) { return G * (h ? hi(a) : lo(a)); };
+        const uint32_t id = h ? id1 : id0;
+        float4 *to = cells ? &cell_grad[3 * (uint64_t)id] : &body_grad[id];
+        atomicAdd(to, make_float4(-half(sx), -half(sy), -half(sz), half(N)));
+        if (QUAD) {
+            atomicAdd(to + 1, make_float4(half(gq[0]), half(gq[1]), half(gq[2]), 0.5f * half(gq[3])));
+            atomicAdd(reinterpret_cast<float2 *>(to + 2), make_float2(0.5f * half(gq[4]), 0.5f * half(gq[5])));
+        }
     }
 }
 
-// Derivatives of u*phi + v.a for one body-body interaction (G omitted),
-// r = x_target - x_source, source mass m: g_r and d/dm.
-__device__ __forceinline__ void body_adj(float rx, float ry, float rz, float m, float eps2, float u,
-                                         float vx, float vy, float vz, float &grx, float &gry,
-                                         float &grz, float &gm) {
-    const float s = rx * rx + ry * ry + rz * rz + eps2;
-    const float i1 = rsqrtf(s), i2 = i1 * i1, i3 = i1 * i2, i5 = i3 * i2;
-    const float vr = vx * rx + vy * ry + vz * rz;
-    grx = u * m * rx * i3 - m * (vx * i3 - 3.f * vr * rx * i5);
-    gry = u * m * ry * i3 - m * (vy * i3 - 3.f * vr * ry * i5);
-    grz = u * m * rz * i3 - m * (vz * i3 - 3.f * vr * rz * i5);
-    gm = -u * i1 - vr * i3;
-}
+template <bool V>
+struct Flag {
+    static constexpr bool value = V;
+};
 
-// The adjoint walk holds more state: bounded to 6 blocks of 4 warps per SM
-// (79 registers, no spills) instead of the 5 its unbounded 93 registers give.
-template <bool QUAD, bool ADJ>
-__global__ void __launch_bounds__(WW * 32, ADJ ? 6 : 0) bh_walk_kernel(
+// The adjoint holds more state, and its coefficients leave room for 3 blocks
+// of 4 warps per SM.
+// SPLIT = 1: a warp per group.  SPLIT = WW: the warps of a block share a
+// group, each the subtrees of every WW-th entry of the stack once it holds
+// SPLIT_AT of them.
+constexpr int SPLIT_AT = 64;
+template <bool QUAD, bool ADJ, int SPLIT>
+__global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 7) bh_walk_kernel(
     const BhView v, float theta2, float eps2, float G, const float *__restrict__ g_acc,
     const float *__restrict__ g_phi, float *__restrict__ acc_out, float *__restrict__ phi_out,
     float4 *__restrict__ cell_grad, float4 *__restrict__ body_grad, uint2 *__restrict__ stack,
     uint32_t stack_entries, const IlogView lg, BhHeader *hm) {
     __shared__ WarpTile tiles[WW];
-    __shared__ WarpRed reds[ADJ ? WW : 1];
+    extern __shared__ WarpAdj adjs[];   // the adjoint's: one a warp
+    __shared__ uint32_t s_group;        // SPLIT: the block's group
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     WarpTile &T = tiles[warp];
-    WarpRed &R = reds[ADJ ? warp : 0];
+    WarpAdj &J = adjs[ADJ ? warp : 0];
     const uint64_t gw = (uint64_t)blockIdx.x * WW + warp;
     uint2 *stk = stack + gw * BH_STACK_CAP_MAX;   // this warp's slice
-    const uint32_t ngroups = v.hdr->n_groups, n_nodes = v.hdr->n_nodes;
-    const uint32_t lt = lane_lt();
-    const uint32_t *child = reinterpret_cast<const uint32_t *>(v.child8);
+    const uint32_t ngroups = (uint32_t)((v.n + BH_GROUP - 1) / BH_GROUP), n_nodes = v.hdr->n_nodes;
+    const uint32_t lt = lane_lt(), mine = 1u << lane;
+    const f2 e2 = pk(eps2);
     uint32_t max_sp = 0;
     while (true) {
         uint32_t g = 0;
-        if (lane == 0) g = atomicAdd(&hm->group_counter, 1u);
-        g = __shfl_sync(0xffffffffu, g, 0);
+        if (SPLIT == 1) {
+            if (lane == 0) g = atomicAdd(&hm->group_counter, 1u);
+            g = __shfl_sync(0xffffffffu, g, 0);
+        } else {
+            if (threadIdx.x == 0) s_group = atomicAdd(&hm->group_counter, 1u);
+            __syncthreads();
+            g = s_group;
+        }
         if (g >= ngroups) break;
-        const uint2 gr = v.groups[g];
-        const uint32_t gs = gr.x, gc = gr.y;
+        const uint32_t part = SPLIT == 1 ? 0u : (uint32_t)warp, slot_g = g * SPLIT + part;   // the log's entry
+        bool shared = SPLIT > 1;   // still the part of the walk that every warp makes
+        const uint32_t gs = g * BH_GROUP, gc = (uint32_t)(v.n - gs < BH_GROUP ? v.n - gs : BH_GROUP);
         const uint32_t i = gs + lane;
         const bool valid = (uint32_t)lane < gc;
-        const float4 me = valid ? v.fbody[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-        float ax = 0.f, ay = 0.f, az = 0.f, phi = 0.f;   // forward sums / adjoint d/dx_i
-        float vx = 0.f, vy = 0.f, vz = 0.f, u = 0.f;
-        if (ADJ) {
-            if (valid) {
-                const uint32_t o = v.order[i];
-                vx = g_acc[3 * (uint64_t)o];
-                vy = g_acc[3 * (uint64_t)o + 1];
-                vz = g_acc[3 * (uint64_t)o + 2];
-                u = g_phi ? g_phi[o] : 0.f;
-            }
+        // spare lanes stand at the first body, with no upstream gradient
+        const float4 me = v.fbody[valid ? i : gs];
+        const f2 px = pk(me.x), py = pk(me.y), pz = pk(me.z);
+        f2 ax = pk(0.f), ay = pk(0.f), az = pk(0.f), phi = pk(0.f);   // forward sums / adjoint d/dx_i
+        f2 vx = pk(0.f), vy = pk(0.f), vz = pk(0.f), u = pk(0.f);
+        if (ADJ && valid) {
+            const uint32_t o = v.order[i];
+            vx = pk(g_acc[3 * (uint64_t)o]);
+            vy = pk(g_acc[3 * (uint64_t)o + 1]);
+            vz = pk(g_acc[3 * (uint64_t)o + 2]);
+            u = pk(g_phi ? g_phi[o] : 0.f);
         }
-        int cn = 0, bn = 0, sp = 0;
+        if (ADJ) {
+            J.body[lane][0] = make_float4(me.x, me.x, me.y, me.y);
+            J.body[lane][1] = make_float4(me.z, me.z, lo(vx), lo(vx));
+            J.body[lane][2] = make_float4(lo(vy), lo(vy), lo(vz), lo(vz));
+        }
         const uint32_t all = __ballot_sync(0xffffffffu, valid);
+        // the group's box; a body with a NaN coordinate accepts no cell, so
+        // no box speaks for it
+        float blo[3] = {me.x, me.y, me.z}, bhi[3] = {me.x, me.y, me.z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                blo[a] = fminf(blo[a], __shfl_xor_sync(0xffffffffu, blo[a], o));
+                bhi[a] = fmaxf(bhi[a], __shfl_xor_sync(0xffffffffu, bhi[a], o));
+            }
+        const bool boxed = !__any_sync(0xffffffffu, isnan(me.x) || isnan(me.y) || isnan(me.z));
+        int n_list[4] = {0, 0, 0, 0};   // (constant indices only)
+        int n_leaf = 0, sp = 0;
         // The adjoint replays the group's tiles from the forward's log when
         // the log holds them all; otherwise it walks the tree.
-        const uint2 lgg = (ADJ && lg.group) ? lg.group[g] : make_uint2(ILOG_NONE, ILOG_NONE);
-        const uint32_t logged = lgg.y;
-        if (n_nodes > 0 && logged == ILOG_NONE) {
+        const uint2 lgg = (ADJ && lg.group) ? lg.group[slot_g] : make_uint2(ILOG_NONE, ILOG_NONE);
+        const bool replay = ADJ && lgg.y != ILOG_NONE;
+        const uint32_t logged = replay ? lgg.y : 0u;
+        if (n_nodes > 0 && !replay) {
             if (lane == 0) stk[0] = make_uint2(0u, all);
             sp = 1;
         }
         __syncwarp();
-        // forward: every evaluated tile (cnt entries of clist/cmask or
-        // blist/bmask) appended to the group's chain of log pages, while the
-        // pool has pages (all warp-uniform)
+        // replay: a page's tile counts come in one load (lane l: tile l) with
+        // the next page's id, and each tile's entries are loaded while the
+        // tile before it is evaluated
+        uint32_t rt = 0, rpg = lgg.x, rpg_next = ILOG_NONE, rcounts = 0;
+        uint2 rentry = make_uint2(0u, 0u);
+        if (logged > 0) {
+            rcounts = lane < (int)ILOG_PAGE ? lg.counts[(uint64_t)rpg * ILOG_PAGE + lane] : 0u;
+            rpg_next = logged > ILOG_PAGE ? lg.next[rpg] : ILOG_NONE;
+            rentry = lg.entries[(uint64_t)rpg * ILOG_PAGE * 32 + lane];
+        }
+        // forward: every evaluated tile appended to the group's chain of log
+        // pages, while the pool has pages (all warp-uniform)
         uint32_t nt = 0, page = ILOG_NONE, first = ILOG_NONE;
         bool lok = !ADJ && lg.group != nullptr;
-        auto log_tile = [&](int cnt, bool bodies) {
-            if (ADJ || !lg.group) return;
-            const uint32_t pos = nt % ILOG_PAGE;
-            if (pos == 0 && lok) {
-                uint32_t pg = 0;
-                if (lane == 0) pg = atomicAdd(&hm->ilog_used, 1u);
-                pg = __shfl_sync(0xffffffffu, pg, 0);
-                if (pg >= lg.pages) {
-                    lok = false;
-                } else {
-                    if (page == ILOG_NONE) first = pg;
-                    else if (lane == 0) lg.next[page] = pg;
-                    page = pg;
-                }
-            }
-            if (lok) {
-                const uint64_t slot = (uint64_t)page * ILOG_PAGE + pos;
-                if (lane < cnt)
-                    lg.entries[slot * 32 + lane] = bodies ? make_uint2(T.blist[lane], T.bmask[lane])
-                                                          : make_uint2(T.clist[lane], T.cmask[lane]);
-                if (lane == 0) lg.counts[slot] = (uint8_t)(cnt | (bodies ? 0x80 : 0));
-            }
-            ++nt;
-        };
 
-        auto eval_cells = [&](int cnt) {
-            log_tile(cnt, false);
-            uint32_t nid = 0, cm = 0;
-            if (lane < cnt) {
-                nid = T.clist[lane];
-                cm = T.cmask[lane];
-                T.cell[lane][0] = __ldg(&v.node_a[nid]);
-                if (QUAD) {
-                    T.cell[lane][1] = __ldg(&v.node_q[2 * nid]);
-                    T.cell[lane][2] = __ldg(&v.node_q[2 * nid + 1]);
-                }
-                T.cmask_t[lane] = cm;
-            }
-            __syncwarp();
-            const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (!ADJ) {
-                for (int k = 0; k < cnt; ++k) {   // lane = body
-                    if (!((T.cmask_t[k] >> lane) & 1u)) continue;
-                    const float4 c = T.cell[k][0];
-                    const float4 q0 = QUAD ? T.cell[k][1] : z4, q1 = QUAD ? T.cell[k][2] : z4;
-                    cell_fwd<QUAD>(me.x - c.x, me.y - c.y, me.z - c.z, c, q0, q1, eps2, ax, ay, az, phi);
-                }
-            } else {
-                // One evaluation per (body, cell) pair, lane = body: the
-                // body's derivative stays in its registers, the cell's (COM,
-                // mass, quadrupole; d/dc = -d/dx) goes to the chunk table, one
-                // row per (cell, part), and each row is summed over the lanes
-                // by a few lanes each (table_row_sum).
-                constexpr int PARTS = QUAD ? 3 : 1;
-                for (int k0 = 0; k0 < cnt; k0 += RED_CELLS) {
-                    const int kn = cnt - k0 < RED_CELLS ? cnt - k0 : RED_CELLS;
-                    for (int kk = 0; kk < kn; ++kk) {
-                        const int k = k0 + kk;
-                        float4 r0 = z4, r1 = z4, r2 = z4;
-                        if ((T.cmask_t[k] >> lane) & 1u) {
-                            const float4 c = T.cell[k][0];
-                            const float4 q0 = QUAD ? T.cell[k][1] : z4, q1 = QUAD ? T.cell[k][2] : z4;
-                            float grx, gry, grz, gM, gq[6];
-                            cell_adj<QUAD>(me.x - c.x, me.y - c.y, me.z - c.z, c, q0, q1, eps2, u,
-                                           vx, vy, vz, grx, gry, grz, gM, gq);
-                            ax += grx; ay += gry; az += grz;
-                            r0 = make_float4(-grx, -gry, -grz, gM);
-                            if (QUAD) {
-                                r1 = make_float4(gq[0], gq[1], gq[2], gq[3]);
-                                r2 = make_float4(gq[4], gq[5], 0.f, 0.f);
-                            }
-                        }
-                        R.red[PARTS * kk][lane] = r0;
-                        if (QUAD) {
-                            R.red[PARTS * kk + 1][lane] = r1;
-                            R.red[PARTS * kk + 2][lane] = r2;
-                        }
-                    }
-                    __syncwarp();
-                    int row;
-                    bool owner;
-                    const float4 t = table_row_sum<32 / (RED_CELLS * PARTS)>(R, kn * PARTS, lane,
-                                                                             row, owner);
-                    if (owner) {
-                        const int kk = row / PARTS, part = row - kk * PARTS;
-                        const uint32_t cid = T.clist[k0 + kk];
-                        atomicAdd(&cell_grad[3 * cid + part], make_float4(G * t.x, G * t.y, G * t.z, G * t.w));
-                    }
-                    __syncwarp();
-                }
-            }
-            __syncwarp();
-        };
-        auto eval_bodies = [&](int cnt) {
-            log_tile(cnt, true);
-            uint32_t bid = 0, bm = 0;
-            if (lane < cnt) {
-                bid = T.blist[lane];
-                bm = T.bmask[lane];
-                T.body[lane] = __ldg(&v.fbody[bid]);
-                T.bid[lane] = bid;
-                T.bmask_t[lane] = bm;
-            }
-            __syncwarp();
-            if (!ADJ) {
-                for (int k = 0; k < cnt; ++k) {   // lane = target
-                    if (!((T.bmask_t[k] >> lane) & 1u) || T.bid[k] == i) continue;
-                    const float4 o = T.body[k];
-                    const float rx = me.x - o.x, ry = me.y - o.y, rz = me.z - o.z;
-                    const float s = rx * rx + ry * ry + rz * rz + eps2;
-                    const float i1 = rsqrtf(s), i3 = i1 * i1 * i1;
-                    phi -= o.w * i1;
-                    ax -= o.w * rx * i3;
-                    ay -= o.w * ry * i3;
-                    az -= o.w * rz * i3;
-                }
-            } else {
-                // as for cells: one evaluation per (target, source) pair,
-                // the source's derivative summed over the lanes
-                const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k0 = 0; k0 < cnt; k0 += RED_BODIES) {
-                    const int kn = cnt - k0 < RED_BODIES ? cnt - k0 : RED_BODIES;
-                    for (int kk = 0; kk < kn; ++kk) {
-                        const int k = k0 + kk;
-                        float4 r = z4;
-                        if (((T.bmask_t[k] >> lane) & 1u) && T.bid[k] != i) {
-                            const float4 o = T.body[k];
-                            float grx, gry, grz, gm;
-                            body_adj(me.x - o.x, me.y - o.y, me.z - o.z, o.w, eps2, u, vx, vy, vz,
-                                     grx, gry, grz, gm);
-                            ax += grx; ay += gry; az += grz;
-                            r = make_float4(-grx, -gry, -grz, gm);
-                        }
-                        R.red[kk][lane] = r;
-                    }
-                    __syncwarp();
-                    int row;
-                    bool owner;
-                    const float4 t = table_row_sum<32 / RED_BODIES>(R, kn, lane, row, owner);
-                    if (owner)
-                        atomicAdd(&body_grad[T.bid[k0 + row]], make_float4(G * t.x, G * t.y, G * t.z, G * t.w));
-                    __syncwarp();
-                }
-            }
-            __syncwarp();
-        };
-
-        if (logged != ILOG_NONE && logged > 0) {
-            // replay: each logged tile back into the lists, evaluated as
-            // the walk evaluated it (same tiles, same order).  A page's
-            // tile counts come in one load (lane l: tile l) with the next
-            // page's id, and each tile's entries are loaded while the tile
-            // before it is evaluated.
-            uint32_t pg = lgg.x;
-            uint32_t c_lane = lane < (int)ILOG_PAGE ? lg.counts[(uint64_t)pg * ILOG_PAGE + lane] : 0u;
-            uint32_t pg_next = logged > ILOG_PAGE ? lg.next[pg] : ILOG_NONE;
-            uint2 e = lg.entries[(uint64_t)pg * ILOG_PAGE * 32 + lane];
-            for (uint32_t t = 0; t < logged; ++t) {
-                const uint32_t pos = t % ILOG_PAGE;
-                if (pos == 0 && t > 0) {
-                    pg = pg_next;
-                    c_lane = lane < (int)ILOG_PAGE ? lg.counts[(uint64_t)pg * ILOG_PAGE + lane] : 0u;
-                    pg_next = t + ILOG_PAGE < logged ? lg.next[pg] : ILOG_NONE;
-                }
-                const uint32_t c = __shfl_sync(0xffffffffu, c_lane, (int)pos);
-                const int cnt = (int)(c & 0x7F);
-                uint2 en = make_uint2(0u, 0u);
-                if (t + 1 < logged) {
-                    const uint32_t pos1 = (t + 1) % ILOG_PAGE;
-                    const uint32_t pg1 = pos1 == 0 ? pg_next : pg;
-                    en = lg.entries[((uint64_t)pg1 * ILOG_PAGE + pos1) * 32 + lane];
-                }
-                if (lane < cnt) {
-                    if (c & 0x80) { T.blist[lane] = e.x; T.bmask[lane] = e.y; }
-                    else { T.clist[lane] = e.x; T.cmask[lane] = e.y; }
-                }
-                __syncwarp();
-                if (c & 0x80) eval_bodies(cnt);
-                else eval_cells(cnt);
-                e = en;
-            }
-        }
-        while (sp > 0) {
+        // One step of the walk: up to 32 stack entries, one a lane.
+        auto step = [&]() {
             const int t = sp < 32 ? sp : 32;
             sp -= t;
             uint2 e = make_uint2(0u, 0u);
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
             uint4 b = make_uint4(0u, 0u, 0u, 0u);
-            if (lane < t) {
+            bool open = lane < t;
+            uint32_t A = 0;
+            if (open) {
                 e = stk[sp + lane];
                 a = __ldg(&v.node_a[e.x]);
                 b = __ldg(&v.node_b[e.x]);
+                // nearest and farthest squared distance from the COM to the
+                // box, rounded as the per-body distance is
+                const float w2 = __fmul_rn(__uint_as_float(b.w), __uint_as_float(b.w));
+                const float c[3] = {a.x, a.y, a.z};
+                float dn[3], df[3];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const float l = __fsub_rn(blo[q], c[q]), h = __fsub_rn(c[q], bhi[q]);
+                    dn[q] = fmaxf(fmaxf(l, h), 0.f);
+                    df[q] = fmaxf(fabsf(l), fabsf(h));
+                }
+                const bool far = w2 < __fmul_rn(theta2, dot3_rn(dn[0], dn[1], dn[2]));
+                const bool near = !(w2 < __fmul_rn(theta2, dot3_rn(df[0], df[1], df[2])));
+                if (boxed && (far || near)) {
+                    if (far) A = e.y;
+                    open = false;
+                }
             }
             __syncwarp();
-            for (int k = 0; k < t; ++k) {
-                const uint32_t nk = __shfl_sync(0xffffffffu, e.x, k);
-                const uint32_t mk = __shfl_sync(0xffffffffu, e.y, k);
+            for (uint32_t m = __ballot_sync(0xffffffffu, open); m; m &= m - 1) {
+                const int k = __ffs(m) - 1;
                 const float cx = __shfl_sync(0xffffffffu, a.x, k);
                 const float cy = __shfl_sync(0xffffffffu, a.y, k);
                 const float cz = __shfl_sync(0xffffffffu, a.z, k);
-                const uint32_t bz = __shfl_sync(0xffffffffu, b.z, k);
-                const uint32_t bw = __shfl_sync(0xffffffffu, b.w, k);
-                const bool in = (mk >> lane) & 1u;
-                const bool acc = in && body_accept(me.x, me.y, me.z, cx, cy, cz, __uint_as_float(bw), theta2);
-                const uint32_t A = __ballot_sync(0xffffffffu, acc);
-                const uint32_t R = mk & ~A;
-                if (A) {
-                    if (lane == 0) { T.clist[cn] = nk; T.cmask[cn] = A; }
-                    ++cn;
-                    __syncwarp();
-                    if (cn == 32) { eval_cells(32); cn = 0; }
-                }
-                if (!R) continue;
-                if (bz & BH_LEAF_BIT) {
-                    const uint32_t bs = __shfl_sync(0xffffffffu, b.y, k);
-                    const uint32_t bc = bz & ~BH_LEAF_BIT;
-                    for (uint32_t off = 0; off < bc; off += 32) {
-                        const uint32_t kk = bc - off < 32u ? bc - off : 32u;
-                        if ((uint32_t)lane < kk) {
-                            T.blist[bn + lane] = bs + off + lane;
-                            T.bmask[bn + lane] = R;
-                        }
-                        bn += (int)kk;
-                        __syncwarp();
-                        if (bn >= 32) {
-                            eval_bodies(32);
-                            if (lane < bn - 32) {
-                                T.blist[lane] = T.blist[32 + lane];
-                                T.bmask[lane] = T.bmask[32 + lane];
-                            }
-                            bn -= 32;
-                            __syncwarp();
-                        }
-                    }
-                } else {
-                    const uint32_t c = lane < 8 ? __ldg(&child[8 * (uint64_t)nk + lane]) : 0xFFFFFFFFu;
-                    const uint32_t pm = __ballot_sync(0xffffffffu, c != 0xFFFFFFFFu);
-                    const int np = __popc(pm);
-                    if ((uint32_t)(sp + np) <= stack_entries) {
-                        if (c != 0xFFFFFFFFu) stk[sp + __popc(pm & lt)] = make_uint2(c, R);
-                        sp += np;
-                    } else if (lane == 0) {
-                        atomicOr(&hm->err, DEVERR_STACK);
-                    }
-                    __syncwarp();
-                }
+                const float w = __uint_as_float(__shfl_sync(0xffffffffu, b.w, k));
+                const uint32_t acc = __ballot_sync(0xffffffffu, body_accept(me.x, me.y, me.z, cx, cy, cz, w, theta2));
+                if (lane == k) A = acc & e.y;
+            }
+            const uint32_t rest = lane < t ? e.y & ~A : 0u;   // lanes that open the node
+            uint32_t m = __ballot_sync(0xffffffffu, A == all);
+            if (A == all) T.list[L_CELLS][n_list[L_CELLS] + __popc(m & lt)] = make_uint2(e.x, A);
+            n_list[L_CELLS] += __popc(m);
+            m = __ballot_sync(0xffffffffu, A != all && A != 0);
+            if (A != all && A != 0) T.list[L_CELLS_MASKED][n_list[L_CELLS_MASKED] + __popc(m & lt)] = make_uint2(e.x, A);
+            n_list[L_CELLS_MASKED] += __popc(m);
+            const bool leaf = b.z & BH_LEAF_BIT;
+            m = __ballot_sync(0xffffffffu, rest && leaf);
+            if (rest && leaf) T.leaf[__popc(m & lt)] = make_uint4(b.y, b.z & ~BH_LEAF_BIT, rest, 0u);
+            n_leaf = __popc(m);
+            // children of the opened cells
+            uint32_t c[8];
+            uint32_t np = 0;
+            if (rest && !leaf) {
+                const uint4 c0 = __ldg(&v.child8[2 * (uint64_t)e.x]), c1 = __ldg(&v.child8[2 * (uint64_t)e.x + 1]);
+                c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w;
+                c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) np += c[q] != 0xFFFFFFFFu;
+            }
+            uint32_t incl = np;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            if ((uint32_t)sp + total <= stack_entries) {
+                uint2 *to = stk + sp + (incl - np);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                    if (q < np) to[q] = make_uint2(c[q], rest);
+                sp += (int)total;
+            } else if (lane == 0) {
+                atomicOr(&hm->err, DEVERR_STACK);
             }
             max_sp = max(max_sp, (uint32_t)sp);
-        }
-        if (cn > 0) eval_cells(cn);
-        if (bn > 0) eval_bodies(bn);
-        if (!ADJ && lg.group && lane == 0) {
-            lg.group[g] = make_uint2(first, lok ? nt : ILOG_NONE);
-            atomicAdd(&hm->ilog_need, (nt + ILOG_PAGE - 1) / ILOG_PAGE);
-        }
-        if (valid) {
-            if (!ADJ) {
-                const uint32_t o = v.order[i];
-                acc_out[3 * (uint64_t)o] = G * ax;
-                acc_out[3 * (uint64_t)o + 1] = G * ay;
-                acc_out[3 * (uint64_t)o + 2] = G * az;
-                if (phi_out) phi_out[o] = G * phi;
+            __syncwarp();
+        };
+        // Keeps this warp's share of the stack.
+        auto share_out = [&]() {
+            const int had = sp;
+            for (int base = 0; base < had; base += 32) {
+                const int j = base + lane;
+                const uint2 e = j < had ? stk[j] : make_uint2(0u, 0u);
+                __syncwarp();
+                if (j < had && j % SPLIT == (int)part) stk[j / SPLIT] = e;
+                __syncwarp();
+            }
+            sp = (had - (int)part + SPLIT - 1) / SPLIT;
+        };
+        // Up to 32 bodies of the last waiting leaf into a list.  A leaf that
+        // holds bodies of the group goes to the masked list, each body
+        // without its own lane.
+        auto list_leaf = [&]() {
+            const uint4 lf = T.leaf[n_leaf - 1];
+            const uint32_t take = lf.y < 32u ? lf.y : 32u, id = lf.x + lane;
+            const bool own = lf.x < gs + gc && lf.x + take > gs, plain = lf.z == all && !own;
+            const int at = plain ? n_list[L_BODIES] : n_list[L_BODIES_MASKED];
+            __syncwarp();
+            if ((uint32_t)lane < take)
+                T.list[plain ? L_BODIES : L_BODIES_MASKED][at + lane] =
+                    make_uint2(id, id - gs < gc ? lf.z & ~(1u << (id - gs)) : lf.z);
+            if (plain) n_list[L_BODIES] += (int)take;
+            else n_list[L_BODIES_MASKED] += (int)take;
+            if (lf.y > 32u) {
+                if (lane == 0) T.leaf[n_leaf - 1] = make_uint4(lf.x + 32, lf.y - 32, lf.z, 0u);
             } else {
-                atomicAdd(&body_grad[i], make_float4(G * ax, G * ay, G * az, 0.f));
+                --n_leaf;
+            }
+            __syncwarp();
+        };
+
+        while (true) {
+            // the next tile: its kind and entries, in list[kind][0 .. cnt)
+            int kind = -1, cnt = 32;
+            if (ADJ && replay) {
+                if (rt >= logged) break;
+                const uint32_t pos = rt % ILOG_PAGE;
+                if (pos == 0 && rt > 0) {
+                    rpg = rpg_next;
+                    rcounts = lane < (int)ILOG_PAGE ? lg.counts[(uint64_t)rpg * ILOG_PAGE + lane] : 0u;
+                    rpg_next = rt + ILOG_PAGE < logged ? lg.next[rpg] : ILOG_NONE;
+                }
+                const uint32_t c = __shfl_sync(0xffffffffu, rcounts, (int)pos);
+                kind = (int)(c >> 6);
+                cnt = (int)(c & 0x3F);
+                if (lane < cnt) T.list[kind][lane] = rentry;
+                if (++rt < logged) {
+                    const uint32_t pos1 = rt % ILOG_PAGE;
+                    rentry = lg.entries[((uint64_t)(pos1 == 0 ? rpg_next : rpg) * ILOG_PAGE + pos1) * 32 + lane];
+                }
+                __syncwarp();
+            } else {
+                while (n_list[0] < 32 && n_list[1] < 32 && n_list[2] < 32 && n_list[3] < 32) {
+                    if (n_leaf > 0) {
+                        list_leaf();
+                    } else if (sp > 0) {
+                        step();
+                        if (SPLIT > 1 && shared) {
+                            if (part != 0) n_list[0] = n_list[1] = n_leaf = 0;   // the first warp's
+                            if (sp >= SPLIT_AT) {
+                                share_out();
+                                shared = false;
+                            }
+                        }
+                    } else {
+                        break;
+                    }
+                }
+                if (n_list[0] >= 32) kind = 0;
+                else if (n_list[1] >= 32) kind = 1;
+                else if (n_list[2] >= 32) kind = 2;
+                else if (n_list[3] >= 32) kind = 3;
+                else if (n_list[0] > 0) { kind = 0; cnt = n_list[0]; }
+                else if (n_list[1] > 0) { kind = 1; cnt = n_list[1]; }
+                else if (n_list[2] > 0) { kind = 2; cnt = n_list[2]; }
+                else if (n_list[3] > 0) { kind = 3; cnt = n_list[3]; }
+                else break;
+                if (!ADJ && lg.group) {
+                    const uint32_t pos = nt % ILOG_PAGE;
+                    if (pos == 0 && lok) {
+                        uint32_t pg = 0;
+                        if (lane == 0) pg = atomicAdd(&hm->ilog_used, 1u);
+                        pg = __shfl_sync(0xffffffffu, pg, 0);
+                        if (pg >= lg.pages) {
+                            lok = false;
+                        } else {
+                            if (page == ILOG_NONE) first = pg;
+                            else if (lane == 0) lg.next[page] = pg;
+                            page = pg;
+                        }
+                    }
+                    if (lok) {
+                        const uint64_t slot = (uint64_t)page * ILOG_PAGE + pos;
+                        if (lane < cnt) lg.entries[slot * 32 + lane] = T.list[kind][lane];
+                        if (lane == 0) lg.counts[slot] = (uint8_t)(cnt | kind << 6);
+                    }
+                    ++nt;
+                }
+            }
+            // Stage the tile.  An odd last pair repeats its source with no
+            // mass and no lanes.
+            const bool cells = kind < L_BODIES, masked = (kind | cnt) & 1;
+            const int pairs = (cnt + 1) / 2;
+            if (lane < 2 * pairs) {
+                const uint2 en = T.list[kind][lane < cnt ? lane : cnt - 1];
+                const bool pad = lane >= cnt;
+                float *w = reinterpret_cast<float *>(T.pair[lane >> 1]) + (lane & 1);
+                const float4 a = cells ? __ldg(&v.node_a[en.x]) : __ldg(&v.fbody[en.x]);
+                w[0] = -a.x;
+                w[2] = -a.y;
+                w[4] = -a.z;
+                w[6] = pad ? 0.f : -a.w;
+                if (QUAD && cells) {
+                    const float4 q0 = __ldg(&v.node_q[2 * en.x]), q1 = __ldg(&v.node_q[2 * en.x + 1]);
+                    w[8] = pad ? 0.f : q0.x;
+                    w[10] = pad ? 0.f : q0.y;
+                    w[12] = pad ? 0.f : q0.z;
+                    w[14] = pad ? 0.f : q0.w;
+                    w[16] = pad ? 0.f : q1.x;
+                    w[18] = pad ? 0.f : q1.y;
+                }
+                T.mask[lane] = pad ? 0u : en.y;
+            }
+            __syncwarp();
+            if (!ADJ) {
+                if (cells && !masked) {
+#pragma unroll 2
+                    for (int p = 0; p < pairs; ++p) cells_fwd<QUAD>(T.pair[p], px, py, pz, e2, phi, ax, ay, az);
+                } else if (cells) {
+                    for (int p = 0; p < pairs; ++p) {
+                        const bool k0 = T.mask[2 * p] & mine, k1 = T.mask[2 * p + 1] & mine;
+                        f2 dp = pk(0.f), dx = pk(0.f), dy = pk(0.f), dz = pk(0.f);
+                        cells_fwd<QUAD>(T.pair[p], px, py, pz, e2, dp, dx, dy, dz);
+                        phi = add2(phi, keep2(dp, k0, k1));
+                        ax = add2(ax, keep2(dx, k0, k1));
+                        ay = add2(ay, keep2(dy, k0, k1));
+                        az = add2(az, keep2(dz, k0, k1));
+                    }
+                } else {
+#pragma unroll 2
+                    for (int p = 0; p < pairs; ++p) {
+                        const float4 c0 = T.pair[p][0], c1 = T.pair[p][1];
+                        const f2 rx = add2(px, xy(c0)), ry = add2(py, zw(c0)), rz = add2(pz, xy(c1)), nm = zw(c1);
+                        f2 i1 = rsqrt2(fma2(rx, rx, fma2(ry, ry, fma2(rz, rz, e2))));
+                        if (masked) i1 = keep2(i1, T.mask[2 * p] & mine, T.mask[2 * p + 1] & mine);
+                        const f2 mi = mul2(nm, i1), k = mul2(mi, mul2(i1, i1));
+                        phi = add2(phi, mi);
+                        ax = fma2(k, rx, ax);
+                        ay = fma2(k, ry, ay);
+                        az = fma2(k, rz, az);
+                    }
+                }
+            } else {
+                // lane = body, then lane = source (rows past the group's
+                // bodies are spare lanes', which leave zeros)
+#pragma unroll 1
+                for (int p0 = 0; p0 < pairs; p0 += ADJ_SOURCES / 2) {
+                    const int pn = pairs - p0 < ADJ_SOURCES / 2 ? pairs - p0 : ADJ_SOURCES / 2;
+                    auto bodies_side = [&](auto quad, auto msk) {
+#pragma unroll 1
+                        for (int q = 0; q < pn; ++q) {
+                            const int p = p0 + q;
+                            f2 w[5];
+                            sources_adj<quad.value, msk.value>(
+                                T.pair[p], px, py, pz, e2, u, vx, vy, vz, msk.value && T.mask[2 * p] & mine,
+                                msk.value && T.mask[2 * p + 1] & mine, ax, ay, az, w);
+#pragma unroll
+                            for (int k = 0; k < (quad.value ? 5 : 3); ++k)
+                                *reinterpret_cast<f2 *>(&J.coef[k][lane][2 * q]) = w[k];
+                        }
+                    };
+                    if (QUAD && cells) {
+                        if (masked) bodies_side(Flag<QUAD>(), Flag<true>());
+                        else bodies_side(Flag<QUAD>(), Flag<false>());
+                    } else {
+                        bodies_side(Flag<false>(), Flag<true>());
+                    }
+                    __syncwarp();
+                    const int p = p0 + (lane & 7), s0 = 2 * p, s1 = s0 + 1;
+                    const float4 *src = T.pair[p < 16 ? p : 15];
+                    const uint32_t id0 = s0 < cnt ? T.list[kind][s0].x : 0u, id1 = s1 < cnt ? T.list[kind][s1].x : 0u;
+                    if (QUAD && cells)
+                        sources_sum<QUAD>(J, src, gc, s0 < cnt, s1 < cnt, id0, id1, true, G, cell_grad, body_grad);
+                    else
+                        sources_sum<false>(J, src, gc, s0 < cnt, s1 < cnt, id0, id1, cells, G, cell_grad, body_grad);
+                    __syncwarp();
+                }
+            }
+            __syncwarp();
+            if (!replay) {   // the entries past the tile move to the front
+                int left = 0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (q == kind) {
+                        n_list[q] -= cnt;
+                        left = n_list[q];
+                    }
+                if (left > 0) {
+                    const uint2 en = T.list[kind][32 + lane];
+                    if (lane < left) T.list[kind][lane] = en;
+                    __syncwarp();
+                }
             }
         }
-        __syncwarp();
+        if (!ADJ && lg.group && lane == 0) {
+            lg.group[slot_g] = make_uint2(first, lok ? nt : ILOG_NONE);
+            atomicAdd(&hm->ilog_need, (nt + ILOG_PAGE - 1) / ILOG_PAGE);
+        }
+        float4 sum = make_float4(lo(ax) + hi(ax), lo(ay) + hi(ay), lo(az) + hi(az), lo(phi) + hi(phi));
+        if (!ADJ && SPLIT > 1) {   // the first warp adds up the others' sums
+            float4 *sums = T.pair[0];
+            sums[lane] = sum;
+            __syncthreads();
+            if (part == 0)
+                for (int w = 1; w < SPLIT; ++w) {
+                    const float4 o = tiles[w].pair[0][lane];
+                    sum = make_float4(sum.x + o.x, sum.y + o.y, sum.z + o.z, sum.w + o.w);
+                }
+        }
+        if (valid && (ADJ || part == 0)) {
+            if (!ADJ) {
+                const uint32_t o = v.order[i];
+                acc_out[3 * (uint64_t)o] = G * sum.x;
+                acc_out[3 * (uint64_t)o + 1] = G * sum.y;
+                acc_out[3 * (uint64_t)o + 2] = G * sum.z;
+                if (phi_out) phi_out[o] = G * sum.w;
+            } else {
+                atomicAdd(&body_grad[i], make_float4(G * sum.x, G * sum.y, G * sum.z, 0.f));
+            }
+        }
+        if (SPLIT > 1) __syncthreads();
+        else __syncwarp();
     }
     if (lane == 0) atomicMax(&hm->max_stack, max_sp);
 }
@@ -609,17 +791,29 @@ __global__ void __launch_bounds__(128) bh_finish_grad_kernel(const BhView v,
     }
 }
 
-template <bool QUAD, bool ADJ>
+// Whether the warps of a block share a group: only where there are fewer
+// groups than five warps an SM, so that the walk of one group is what the
+// call takes.  Sharing repeats the first steps of the walk and leaves more
+// tiles part empty.  Measured, a warp / a block per group, ms (forward;
+// adjoint): 10,000 bodies 0.45 / 0.34; 0.58 / 0.42, 16,000: 0.51 / 0.33; 0.67
+// / 0.51, 30,000: 0.62 / 0.54; 0.90 / 0.95, 100,000: 0.97 / 1.25; 2.1 / 3.2.
+inline bool split_groups(uint64_t n) { return n <= (uint64_t)NUM_SMS_HINT * 5 * BH_GROUP; }
+
+template <bool QUAD, bool ADJ, int SPLIT>
 rtd_status launch_walk(rtd_bh *b, const rtd_bh_params *p, const float *g_acc, const float *g_phi,
                        float *acc, float *phi, const IlogView &lg, cudaStream_t st) {
     int dev = 0, sms = 148, per_sm = 4;
     RTD_CUDA(cudaGetDevice(&dev));
     RTD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bh_walk_kernel<QUAD, ADJ>,
-                                                           WW * 32, 0));
+    const size_t smem = ADJ ? WW * sizeof(WarpAdj) : 0;
+    if (ADJ)
+        RTD_CUDA(cudaFuncSetAttribute(bh_walk_kernel<QUAD, ADJ, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
+    RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bh_walk_kernel<QUAD, ADJ, SPLIT>,
+                                                           WW * 32, smem));
     if (per_sm < 1) per_sm = 1;
     uint64_t blocks = (uint64_t)sms * (uint64_t)per_sm;
-    const uint64_t need = (b->n + WW - 1) / WW;   // groups <= bodies
+    const uint64_t need = ceil_div(ceil_div(b->n, BH_GROUP) * SPLIT, WW);
     if (blocks > need) blocks = need;
     if (blocks < 1) blocks = 1;
     const uint64_t warps = blocks * WW;
@@ -630,12 +824,19 @@ rtd_status launch_walk(rtd_bh *b, const rtd_bh_params *p, const float *g_acc, co
     BhHeader *h = b->hdr.as<BhHeader>();
     RTD_CUDA(cudaMemsetAsync(&h->group_counter, 0, sizeof(uint32_t), st));
     const BhView v = bh_view(b);
-    bh_walk_kernel<QUAD, ADJ><<<(unsigned)blocks, WW * 32, 0, st>>>(
+    bh_walk_kernel<QUAD, ADJ, SPLIT><<<(unsigned)blocks, WW * 32, smem, st>>>(
         v, p->theta * p->theta, p->eps * p->eps, p->G, g_acc, g_phi, acc, phi,
         b->cell_grad.as<float4>(), b->gpos_flat.as<float4>(), b->stack.as<uint2>(),
         bh_stack_entries(), lg, h);
     RTD_LAUNCH_CHECK();
     return RTD_OK;
+}
+
+template <bool QUAD, bool ADJ>
+rtd_status launch_walk(rtd_bh *b, const rtd_bh_params *p, const float *g_acc, const float *g_phi,
+                       float *acc, float *phi, const IlogView &lg, cudaStream_t st) {
+    return split_groups(b->n) ? launch_walk<QUAD, ADJ, WW>(b, p, g_acc, g_phi, acc, phi, lg, st)
+                              : launch_walk<QUAD, ADJ, 1>(b, p, g_acc, g_phi, acc, phi, lg, st);
 }
 
 }  // namespace
@@ -754,24 +955,24 @@ namespace {
 // Forward walk on a traversal stack supplied by the caller: `stack` holds
 // max_warps slices of BH_STACK_CAP_MAX entries and the launch is capped to that
 // many warps.  Nothing is allocated.
-template <bool QUAD>
+template <bool QUAD, int SPLIT>
 rtd_status launch_walk_on_stack(rtd_bh *b, const rtd_bh_params *p, float *acc, float *phi,
                                 uint2 *stack, uint64_t max_warps, cudaStream_t st) {
     int dev = 0, sms = 148, per_sm = 4;
     RTD_CUDA(cudaGetDevice(&dev));
     RTD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bh_walk_kernel<QUAD, false>,
+    RTD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bh_walk_kernel<QUAD, false, SPLIT>,
                                                            WW * 32, 0));
     if (per_sm < 1) per_sm = 1;
     uint64_t blocks = (uint64_t)sms * (uint64_t)per_sm;
-    const uint64_t need = (b->n + WW - 1) / WW;
+    const uint64_t need = ceil_div(ceil_div(b->n, BH_GROUP) * SPLIT, WW);
     if (blocks > need) blocks = need;
     if (blocks > max_warps / WW) blocks = max_warps / WW;
     if (blocks < 1) return fail(RTD_ERR_INVALID_ARGUMENT, "stack holds less than one block of warps");
     BhHeader *h = b->hdr.as<BhHeader>();
     RTD_CUDA(cudaMemsetAsync(&h->group_counter, 0, sizeof(uint32_t), st));
     const BhView v = bh_view(b);
-    bh_walk_kernel<QUAD, false><<<(unsigned)blocks, WW * 32, 0, st>>>(
+    bh_walk_kernel<QUAD, false, SPLIT><<<(unsigned)blocks, WW * 32, 0, st>>>(
         v, p->theta * p->theta, p->eps * p->eps, p->G, nullptr, nullptr, acc, phi, nullptr,
         nullptr, stack, bh_stack_entries(), IlogView{}, h);
     RTD_LAUNCH_CHECK();
@@ -798,8 +999,11 @@ rtd_status bh_forward_on_stack(rtd_bh *b, const rtd_bh_params *p, float *d_out, 
         return fail(RTD_ERR_INVALID_ARGUMENT, "tree was not built for the Plummer law");
     if (p->quadrupole && !b->has_quad)
         return fail(RTD_ERR_INVALID_ARGUMENT, "tree was built without quadrupoles");
-    if (p->quadrupole) return launch_walk_on_stack<true>(b, p, d_out, d_phi, stack, max_warps, st);
-    return launch_walk_on_stack<false>(b, p, d_out, d_phi, stack, max_warps, st);
+    if (split_groups(b->n))
+        return p->quadrupole ? launch_walk_on_stack<true, WW>(b, p, d_out, d_phi, stack, max_warps, st)
+                             : launch_walk_on_stack<false, WW>(b, p, d_out, d_phi, stack, max_warps, st);
+    return p->quadrupole ? launch_walk_on_stack<true, 1>(b, p, d_out, d_phi, stack, max_warps, st)
+                         : launch_walk_on_stack<false, 1>(b, p, d_out, d_phi, stack, max_warps, st);
 }
 
 }  // namespace rtd
