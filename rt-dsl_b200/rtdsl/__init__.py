@@ -9,7 +9,7 @@ from ._capi import (BH_LAW_PLUMMER, BH_LAW_REFERENCE, EMPTY_ID, RADIUS_FIXED,
                     RtdError, Schedule, default_batch_schedule, default_bh_params,
                     default_schedule, load)
 from .api import (Context, Index, KnnGraph, KnnHostGraph, dbscan, k_nn, k_nn_array, knn_backward, range_query,
-                  spatial_join)
+                  release_kept_index, spatial_join)
 from .batch import Batch
 from .bh import BarnesHut, barnes_hut
 
@@ -18,5 +18,5 @@ __all__ = [
     "RADIUS_SAMPLED_MAX",
     "RADIUS_SAMPLED_NN", "RADIUS_SAMPLED_PERCENTILE", "BhParams", "RtdError", "Schedule",
     "default_batch_schedule", "default_bh_params", "default_schedule", "load", "Context", "Index", "KnnGraph", "KnnHostGraph", "k_nn", "k_nn_array",
-    "knn_backward", "range_query", "spatial_join", "dbscan", "Batch", "BarnesHut", "barnes_hut",
+    "knn_backward", "range_query", "release_kept_index", "spatial_join", "dbscan", "Batch", "BarnesHut", "barnes_hut",
 ]

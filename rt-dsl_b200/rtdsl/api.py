@@ -10,7 +10,9 @@ the current stream).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import threading
 
 import numpy as np
 
@@ -237,6 +239,40 @@ class Index:
                                        C.c_void_p(pairs.data_ptr()), capacity, int(sort_pairs),
                                        C.byref(written), _stream_handle(stream)))
         return pairs[: written.value]
+
+
+# The index a thread keeps between calls that need one only for their own
+# duration: creating an index and its two dozen device buffers, and freeing
+# them, takes 2 to 5 ms of host time, several times the search of a training
+# step.  One per thread, for up to this many points and queries (about 400 MB
+# at the most); release_kept_index() gives it back, as the thread's end does.
+KEPT_INDEX_MAX = 1 << 21
+_kept = threading.local()
+
+
+@contextlib.contextmanager
+def short_lived_index(device, n: int, nq: int):
+    """An Index for work on the current stream that is all enqueued when the
+    block ends.  A kept one was last used by work that an event marks; the
+    current stream, whichever it is, waits for it."""
+    import torch
+    st = torch.cuda.current_stream(device)
+    entry, _kept.entry = getattr(_kept, "entry", None), None   # (a nested call makes its own)
+    if entry is not None and entry[0] == device:
+        _, ix, done = entry
+        st.wait_event(done)
+    else:
+        ix, done = Index(), torch.cuda.Event()
+    yield ix   # an exception drops the index
+    if max(n, nq) <= KEPT_INDEX_MAX:
+        done.record(st)
+        ix.points = None
+        _kept.entry = (device, ix, done)
+
+
+def release_kept_index() -> None:
+    """Frees the index this thread keeps for short calls, if any."""
+    _kept.entry = None
 
 
 class KnnGraph:

@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 
 from ._capi import BH_LAW_PLUMMER, default_bh_params, default_schedule
-from .api import Index, knn_backward
+from .api import knn_backward, short_lived_index
 from .bh import BarnesHut
 
 
@@ -23,8 +23,9 @@ class KnnDistances(torch.autograd.Function):
     @staticmethod
     def forward(ctx, queries, points, k: int, schedule=None):
         s = schedule if schedule is not None else default_schedule()
-        ix = Index().build(points.detach().contiguous(), s)
-        ids, d2 = ix.knn(queries.detach().contiguous(), k, s)
+        p, q = points.detach().contiguous(), queries.detach().contiguous()
+        with short_lived_index(p.device, p.shape[0], q.shape[0]) as ix:
+            ids, d2 = ix.build(p, s).knn(q, k, s)
         ctx.save_for_backward(queries, points, ids)
         ctx.mark_non_differentiable(ids)
         return d2, ids
