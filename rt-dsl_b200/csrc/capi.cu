@@ -79,7 +79,7 @@ rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                        cudaStream_t st);
 rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                       const rtd_schedule *s, uint32_t *d_pairs, uint64_t capacity, int sort_pairs,
-                      uint64_t *h_written, cudaStream_t st);
+                      uint64_t *h_written, cudaStream_t st, bool check = true);
 rtd_status knn_backward(const float *q, uint64_t nq, const float *pts, uint64_t n, uint32_t k,
                         const uint32_t *ids, const float *g, float *gq, float *gp, cudaStream_t st);
 

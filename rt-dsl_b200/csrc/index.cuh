@@ -44,6 +44,8 @@ struct IndexHeader {
     uint64_t total;       // last range-count total
     float nn95_key;       // p95 of the squared 1-NN distance within a 4096-point sample
     uint32_t n_sample;    // points in the radius-seed sample (<= 1000)
+    uint32_t most;        // largest count of the last range count
+    uint32_t heavy;       // some query of its sample has very many hits
     unsigned long long qfp[2];   // query fingerprints of the last range count / fill
 };
 
@@ -110,6 +112,7 @@ struct rtd_index {
         uint64_t nq = 0;
         float radius = 0.f;
         uint64_t total = 0;
+        uint32_t most = 0;     // the largest count
         const uint32_t *perm = nullptr;
         bool spec = false;   // rspec / rrec hold every pair of that count
         uint64_t spec_pairs = 0, spec_recs = 0;
