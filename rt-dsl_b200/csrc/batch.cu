@@ -376,13 +376,16 @@ __global__ void __launch_bounds__(SWARPS * 32, 10) batch_collect_kernel(const Ba
         const uint32_t kk = c.k < c.n_pts ? c.k : (c.n_pts ? c.n_pts : 1u);
         const CollectScratch s = collect_scratch(base, kk, c.n_pts);
         const CollectTree tree{a.pts, a.pyr, s_off, c.pt_begin, c.pt_begin + c.n_pts};
+        // the positions of the part's queries, one a lane
         const uint32_t j0 = it % (32 / COLLECT_PART) * COLLECT_PART;
-        for (uint32_t j = j0; j < w.count && j < j0 + COLLECT_PART; ++j) {
-            const uint32_t qi = a.qperm[w.start + j];
+        const uint32_t have = w.count > j0 ? min(w.count - j0, COLLECT_PART) : 0u;
+        uint32_t my_pos = 0;
+        if ((uint32_t)lane < have) my_pos = cloud_position(a, c, a.qskeys[w.start + j0 + lane]);
+        __syncwarp();
+        for (uint32_t j = 0; j < have; ++j) {
+            const uint32_t qi = a.qperm[w.start + j0 + j], pos = __shfl_sync(0xffffffffu, my_pos, j);
             const float qx = a.q[3 * (uint64_t)qi], qy = a.q[3 * (uint64_t)qi + 1], qz = a.q[3 * (uint64_t)qi + 2];
-            const uint32_t pos = warp_lower_bound<uint64_t>(a.skeys, c.pt_begin, c.pt_begin + c.n_pts,
-                                                            a.qskeys[w.start + j]);
-            const Collected got = collect_query(tree, s, qx, qy, qz, kk, pos);
+            const Collected got = collect_query<false>(tree, s, qx, qy, qz, kk, pos);
             const uint64_t ob = c.out_off + (uint64_t)(qi - c.q_begin) * c.k;
             collect_store(s, got, kk, c.k, a.ids + ob, a.d2 ? a.d2 + ob : nullptr);
         }

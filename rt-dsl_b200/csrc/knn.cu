@@ -173,28 +173,42 @@ __global__ void __launch_bounds__(BLOCK, KC <= 5 ? 1280 / BLOCK : 0) knn_thread_
 }
 
 // One warp per query that collects and selects (knn_collect.cuh); kk =
-// min(k, points) <= COLLECT_MAX_K.
+// min(k, points) <= COLLECT_MAX_K.  A warp takes `part` consecutive queries
+// of the processing order: their positions are found first, a query a lane
+// (part > 1; about 350 instructions a query otherwise), or by the whole warp.
 constexpr int COLLECT_WARPS = 4;
-__global__ void __launch_bounds__(COLLECT_WARPS * 32, 10) knn_collect_kernel(const KnnArgs p, uint32_t kk) {
+constexpr uint32_t COLLECT_PART = 8;
+__global__ void __launch_bounds__(COLLECT_WARPS * 32, 9) knn_collect_kernel(const KnnArgs p, uint32_t kk,
+                                                                             uint32_t part) {
     chain_wait();
     extern __shared__ uint2 s_dyn[];
     __shared__ uint32_t s_off[12];
     const uint32_t n = (uint32_t)p.ix.n;
     if (threadIdx.x == 0) collect_offsets(n, s_off);
     __syncthreads();
-    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const CollectScratch s = collect_scratch(
         reinterpret_cast<char *>(s_dyn) + (size_t)warp * collect_warp_bytes(kk, n), kk, n);
     const CollectTree tree{p.ix.pts, p.pyr, s_off, 0u, n};
-    for (uint64_t t = (uint64_t)blockIdx.x * COLLECT_WARPS + warp; t < p.nq;
-         t += (uint64_t)gridDim.x * COLLECT_WARPS) {
-        const uint64_t qi = p.perm ? p.perm[t] : t;
-        const float qx = p.q[3 * qi], qy = p.q[3 * qi + 1], qz = p.q[3 * qi + 2];
-        const uint32_t pos = p.wpos ? p.wpos[t]
-                                    : morton_position_warp(p.ix.hdr, p.skeys, n, p.key64, p.scale, qx, qy, qz);
-        Collected c = collect_query(tree, s, qx, qy, qz, kk, pos);
-        const uint64_t ob = qi * (uint64_t)p.k;
-        collect_store(s, c, kk, p.k, p.ids + ob, p.d2 ? p.d2 + ob : nullptr);
+    for (uint64_t t0 = ((uint64_t)blockIdx.x * COLLECT_WARPS + warp) * part; t0 < p.nq;
+         t0 += (uint64_t)gridDim.x * COLLECT_WARPS * part) {
+        uint32_t my_pos = 0;   // lane j: query j of the part
+        if (part > 1) {
+            if ((uint32_t)lane < part && t0 + lane < p.nq) {
+                const float *q = p.q + 3 * (p.perm ? (uint64_t)p.perm[t0 + lane] : t0 + lane);
+                my_pos = morton_position(p.ix.hdr, p.skeys, n, p.key64, p.scale, q[0], q[1], q[2]);
+            }
+            __syncwarp();
+        }
+        for (uint32_t j = 0; j < part && t0 + j < p.nq; ++j) {
+            const uint64_t qi = p.perm ? p.perm[t0 + j] : t0 + j;
+            const float qx = p.q[3 * qi], qy = p.q[3 * qi + 1], qz = p.q[3 * qi + 2];
+            const uint32_t pos = part > 1 ? __shfl_sync(0xffffffffu, my_pos, j)
+                                          : morton_position_warp(p.ix.hdr, p.skeys, n, p.key64, p.scale, qx, qy, qz);
+            const Collected c = collect_query<true>(tree, s, qx, qy, qz, kk, pos);
+            const uint64_t ob = qi * (uint64_t)p.k;
+            collect_store(s, c, kk, p.k, p.ids + ob, p.d2 ? p.d2 + ob : nullptr);
+        }
     }
 }
 
@@ -411,8 +425,12 @@ rtd_status launch_collect(rtd_index *idx, const KnnArgs &a, cudaStream_t st) {
     if (smem > 48 * 1024)
         RTD_CUDA(cudaFuncSetAttribute(knn_collect_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(COLLECT_WARPS * collect_warp_bytes(COLLECT_MAX_K, 1ull << 30))));
-    RTD_LAUNCH_CHAINED(knn_collect_kernel, dim3(grid_for(a.nq, COLLECT_WARPS, 1 << 20)), dim3(COLLECT_WARPS * 32),
-                       smem, st, a, kk);
+    // several queries a warp where each of an SM's 36 warps still gets eight
+    // parts: with fewer, the warp whose part is dearest ends too late
+    uint32_t part = 1;
+    while (part < COLLECT_PART && a.nq >= (uint64_t)NUM_SMS_HINT * 36 * 8 * 2 * part) part *= 2;
+    RTD_LAUNCH_CHAINED(knn_collect_kernel, dim3(grid_for(ceil_div(a.nq, part), COLLECT_WARPS, 1 << 20)),
+                       dim3(COLLECT_WARPS * 32), smem, st, a, kk, part);
     return RTD_OK;
 }
 
@@ -461,16 +479,21 @@ rtd_status knn_search(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t k,
 // points around each query in Morton order and need no radius rounds: their
 // result is the same for every starting radius.
 enum class Search { thread_window, collect, rounds };
-// lanes_per_query = 0 (auto): a warp per query for k > 16 and, in exact
-// searches, for few queries.  A thread's search is a serial chain that takes
-// about as long for 1,000 queries as for 100,000, while the warp's grows
-// with their number: measured, 100,000 uniform points, thread / warp, us:
-// k = 5: 10,000 queries 141 / 41, 100,000 156 / 290; k = 16: 331 / 52 and
-// 397 / 373; the two cross near 8,000 k queries.
+// lanes_per_query = 0 (auto).  Exact searches: a warp per query for k > 12
+// and for few queries.  A thread's list of 16 costs as much as the warp's
+// whole search (400,000 queries, k = 16, thread / warp, ms: clustered 1.54 /
+// 1.56, uniform 1.37 / 1.38; 1M on a sheet 4.2 / 3.6 and 7.0 / 4.6; k = 12:
+// 1.25 / 1.43; k = 8: 0.62 / 1.32).  A thread's search is a serial chain that
+// takes about as long for 1,000 queries as for 100,000, while the warp's
+// grows with their number: 100,000 uniform points, us: k = 5: 10,000 queries
+// 141 / 40, 100,000 156 / 265; k = 8: 50,000 180 / 170; the two cross near
+// 8,000 k queries.  Searches with partial_results: a warp for k > 16.
+constexpr uint32_t THREAD_MAX_K = 12;
 constexpr uint64_t WARP_QUERIES_PER_K = 8000;
 static uint32_t search_lanes(const rtd_schedule &s, uint64_t nq, uint32_t k) {
     uint32_t lanes = s.lanes_per_query;
-    if (lanes == 0) lanes = k <= 16 && (s.partial_results || nq > WARP_QUERIES_PER_K * k) ? 1 : 32;
+    if (lanes == 0)
+        lanes = (s.partial_results ? k <= 16 : k <= THREAD_MAX_K && nq > WARP_QUERIES_PER_K * k) ? 1 : 32;
     if (lanes == 1 && k > 32) lanes = 32;
     return lanes;
 }

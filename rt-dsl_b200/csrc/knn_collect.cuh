@@ -26,7 +26,7 @@ namespace rtd {
 struct CollectTree {
     const float4 *pts;
     const float4 *pyr;
-    const uint32_t *off;   // off[j]: first pyramid entry of level j >= 1; off[nlev + 1]: end
+    const uint32_t *off;   // off[j]: first pyramid entry of level j >= 1
     uint32_t begin, end;   // the cloud's sorted points
 };
 
@@ -101,17 +101,38 @@ struct Collected {
 // smallest (exactly kk when keys tie across the cut) and sets the bound.
 // The kk-th smallest key is found bit by bit from the highest bit in which
 // the keys differ (keys are >= +0, so their bits order as they do), stopping
-// at the first threshold that keeps few enough.
-// (Not inlined: its four call sites would not fit the instruction cache.)
-static __device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, Collected c, uint32_t kk, uint32_t slack) {
+// at the first threshold that keeps few enough.  Up to 192 keys (k <= 64)
+// stay in registers meanwhile: a cut of 64 then takes about 150 instructions
+// instead of 450.  (Not inlined: its four call sites would not fit the
+// instruction cache.)
+constexpr int CUT_REGS = 6;
+template <bool small>
+static __device__ __noinline__ Collected collect_cut_sized(float *key, uint32_t *ids, Collected c, uint32_t kk,
+                                                           uint32_t slack) {
+    constexpr int REGS = small ? CUT_REGS : 1;
     const int lane = threadIdx.x & 31;
     const uint32_t *kb = reinterpret_cast<const uint32_t *>(key);
     __syncwarp();
+    uint32_t v[REGS];   // missing ones as the largest value, which is no key
     uint32_t mn = 0xFFFFFFFFu, mx = 0;
-    for (uint32_t j = lane; j < c.cnt; j += 32) {
-        const uint32_t v = kb[j];
-        mn = min(mn, v);
-        mx = max(mx, v);
+    if (small) {
+#pragma unroll
+        for (int u = 0; u < REGS; ++u) {
+            v[u] = 0xFFFFFFFFu;
+            if (u * 32 < c.cnt) {
+                if (u * 32 + lane < c.cnt) {
+                    v[u] = kb[u * 32 + lane];
+                    mx = max(mx, v[u]);
+                }
+                mn = min(mn, v[u]);
+            }
+        }
+    } else {
+        for (uint32_t j = lane; j < c.cnt; j += 32) {
+            const uint32_t x = kb[j];
+            mn = min(mn, x);
+            mx = max(mx, x);
+        }
     }
     mn = __reduce_min_sync(0xffffffffu, mn);
     mx = __reduce_max_sync(0xffffffffu, mx);
@@ -123,7 +144,13 @@ static __device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, 
         for (; b >= 0; --b) {
             const uint32_t test = lo | (1u << b);
             uint32_t n = 0;
-            for (uint32_t j = lane; j < c.cnt; j += 32) n += kb[j] < test;
+            if (small) {
+#pragma unroll
+                for (int u = 0; u < REGS; ++u)
+                    if (u * 32 < c.cnt) n += v[u] < test;
+            } else {
+                for (uint32_t j = lane; j < c.cnt; j += 32) n += kb[j] < test;
+            }
             n = __reduce_add_sync(0xffffffffu, n);
             if (n < kk) {
                 lo = test;
@@ -150,13 +177,10 @@ static __device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, 
         c.ti = id + 1;
     }
     uint32_t out = 0;
-    for (uint32_t base = 0; base < c.cnt; base += 32) {
-        const uint32_t j = base + lane;
-        float k = 0.f;
+    auto chunk = [&](uint32_t j, float k) {
         uint32_t i = 0;
         bool keep = false;
         if (j < c.cnt) {
-            k = key[j];
             i = ids[j];
             keep = key_less(k, i, c.tk, c.ti);
         }
@@ -168,15 +192,31 @@ static __device__ __noinline__ Collected collect_cut(float *key, uint32_t *ids, 
             ids[at] = i;
         }
         out += __popc(m);
+    };
+    if (small) {
+#pragma unroll
+        for (int u = 0; u < REGS; ++u)
+            if (u * 32 < c.cnt) chunk(u * 32 + lane, __uint_as_float(v[u]));
+    } else {
+        for (uint32_t base = 0; base < c.cnt; base += 32) {
+            const uint32_t j = base + lane;
+            chunk(j, j < c.cnt ? key[j] : 0.f);
+        }
     }
     c.cnt = out;
     __syncwarp();
     return c;
 }
+__device__ __forceinline__ Collected collect_cut(float *key, uint32_t *ids, Collected c, uint32_t kk, uint32_t slack) {
+    return c.cnt <= 32 * CUT_REGS ? collect_cut_sized<true>(key, ids, c, kk, slack)
+                                  : collect_cut_sized<false>(key, ids, c, kk, slack);
+}
 
 // The candidates of one query: on return at least min(kk, finite-key points)
 // of them, the kk best among them.  pos: the query's Morton position in
 // [begin, end].  All arguments are warp-uniform.
+// WHOLE: the cloud is the whole index.
+template <bool WHOLE>
 __device__ __forceinline__ Collected collect_query(const CollectTree &t, const CollectScratch &s, float qx, float qy,
                                                    float qz, uint32_t kk, uint32_t pos) {
     const int lane = threadIdx.x & 31;
@@ -254,7 +294,7 @@ __device__ __forceinline__ Collected collect_query(const CollectTree &t, const C
                 if (r < take) {
                     const uint2 e = s.leaf[lq + r];
                     const uint32_t at = (e.x & 0x0FFFFFFFu) * 8 + (lane & 7);
-                    ok[u] = !(__uint_as_float(e.y) > c.tk) && at >= t.begin && at < t.end && at - w0 >= w;
+                    ok[u] = !(__uint_as_float(e.y) > c.tk) && (WHOLE || at >= t.begin) && at < t.end && at - w0 >= w;
                     if (ok[u]) p[u] = __ldg(&t.pts[at]);
                 }
             }
@@ -278,7 +318,7 @@ __device__ __forceinline__ Collected collect_query(const CollectTree &t, const C
             }
             --level;
             // children that hold points of the cloud
-            ok = ok && e <= (t.end - 1) >> (3 * level) && e >= t.begin >> (3 * level);
+            ok = ok && e <= (t.end - 1) >> (3 * level) && (WHOLE || e >= t.begin >> (3 * level));
             __syncwarp();
             visit(ok, level, e);
         }

@@ -63,7 +63,7 @@ def test_collect_non_finite(rtd, orc, cuda, k):
 
 
 @pytest.mark.parametrize("nq,k", [(7_999, 1), (8_000, 1), (8_001, 1), (24_000, 3), (24_001, 3), (49_151, 17),
-                                  (49_152, 17)])
+                                  (49_152, 17), (94_720, 13), (96_001, 12), (189_440, 14), (378_881, 13)])
 def test_search_and_order_rules(rtd, orc, cuda, nq, k):
     pts, q = workloads.clustered(n=6_000, nq=nq, seed=nq, n_clusters=9, box=10.0)
     check(rtd, orc, pts, q, k)
