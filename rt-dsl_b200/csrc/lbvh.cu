@@ -15,8 +15,7 @@ constexpr int BLOCK = 256;
 // Whether a device array can be read as float4.
 inline int aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0 ? 1 : 0; }
 
-__global__ void hdr_init_kernel(IndexHeader *h) {
-    chain_wait();
+__device__ __forceinline__ void hdr_init(IndexHeader *h) {
     h->root = CHILD_NONE;
     h->root_count = 0;
     h->n_internal = 0;
@@ -30,6 +29,11 @@ __global__ void hdr_init_kernel(IndexHeader *h) {
     h->total = 0;
     h->nn95_key = -1.0f;   // "no sample": the seed falls back to radius 1
     h->n_sample = 0;
+}
+
+__global__ void hdr_init_kernel(IndexHeader *h) {
+    chain_wait();
+    hdr_init(h);
 }
 
 // Points 4g .. 4g+3 of a 16-byte aligned xyz array: three float4 loads.
@@ -322,8 +326,12 @@ __global__ void __launch_bounds__(512) pyramid_fold_kernel(const float4 *__restr
 // BATCH entries at a time so that their loads are in flight together.  The
 // last batch repeats entry b - 1 in place of entries past b: a min / max
 // does not change when an entry is added twice.
-template <bool PTS>
-__device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *__restrict__ base,
+// GLOBAL: the entries are global memory that this kernel does not write.
+template <bool GLOBAL>
+__device__ __forceinline__ float4 ld_entry(const float4 *p) { return GLOBAL ? __ldg(p) : *p; }
+
+template <bool PTS, bool GLOBAL>
+__device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *base,
                                         uint32_t a, uint32_t b) {
     constexpr int BATCH = PTS ? 8 : 4;
 #pragma unroll 1
@@ -333,10 +341,10 @@ __device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *__rest
         for (int u = 0; u < BATCH; ++u) {
             const uint32_t e = t + u < b ? t + u : b - 1;
             if (PTS) {
-                lo[u] = __ldg(&base[e]);
+                lo[u] = ld_entry<GLOBAL>(&base[e]);
             } else {
-                lo[u] = __ldg(&base[2 * (uint64_t)e]);
-                hi[u] = __ldg(&base[2 * (uint64_t)e + 1]);
+                lo[u] = ld_entry<GLOBAL>(&base[2 * (uint64_t)e]);
+                hi[u] = ld_entry<GLOBAL>(&base[2 * (uint64_t)e + 1]);
             }
         }
 #pragma unroll
@@ -353,8 +361,8 @@ __device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *__rest
 // The level offsets follow from n as the walk goes up, so the pyramid is
 // passed as scalars (a struct taken by reference would be copied to local
 // memory).
-__device__ __noinline__ Box range_box(const float4 *__restrict__ pts,
-                                      const float4 *__restrict__ pyr, uint32_t n, int nlev,
+template <bool GLOBAL>
+__device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint32_t n, int nlev,
                                       uint32_t first, uint32_t count) {
     Box b;
     box_empty(b);
@@ -366,8 +374,8 @@ __device__ __noinline__ Box range_box(const float4 *__restrict__ pts,
     for (int j = 0; j <= PYR_MAX; ++j) {
         if (l >= r) break;
         if (j == nlev) {
-            if (j == 0) add_run<true>(b, nan, pts, l, r);
-            else add_run<false>(b, nan, lvl, l, r);
+            if (j == 0) add_run<true, GLOBAL>(b, nan, pts, l, r);
+            else add_run<false, GLOBAL>(b, nan, lvl, l, r);
             break;
         }
         uint32_t head = (l + PYR_B - 1) & ~(PYR_B - 1);
@@ -375,11 +383,11 @@ __device__ __noinline__ Box range_box(const float4 *__restrict__ pts,
         uint32_t tail = r & ~(PYR_B - 1);
         if (tail < head) tail = head;
         if (j == 0) {
-            add_run<true>(b, nan, pts, l, head);
-            add_run<true>(b, nan, pts, tail, r);
+            add_run<true, GLOBAL>(b, nan, pts, l, head);
+            add_run<true, GLOBAL>(b, nan, pts, tail, r);
         } else {
-            add_run<false>(b, nan, lvl, l, head);
-            add_run<false>(b, nan, lvl, tail, r);
+            add_run<false, GLOBAL>(b, nan, lvl, l, head);
+            add_run<false, GLOBAL>(b, nan, lvl, tail, r);
             lvl += 2 * (uint64_t)size;
         }
         l = head >> PYR_SH;
@@ -388,6 +396,26 @@ __device__ __noinline__ Box range_box(const float4 *__restrict__ pts,
     }
     if (nan) box_unbounded(b);
     return b;
+}
+
+// The node of the points [f0, last] with children [f0, sp] and [sp + 1, last]:
+// Karras nodes sp and sp + 1 when they keep more than leaf_size points, else
+// leaves.
+template <bool GLOBAL>
+__device__ __forceinline__ BvhNode make_node(const Pyramid &P, const uint32_t *cidx, uint32_t leaf_size, uint32_t f0,
+                                             uint32_t last, uint32_t sp) {
+    const uint32_t c0 = sp - f0 + 1, c1 = last - sp;
+    const uint32_t w0 = c0 > leaf_size ? cidx[sp] : (CHILD_LEAF | f0);
+    const uint32_t w1 = c1 > leaf_size ? cidx[sp + 1] : (CHILD_LEAF | (sp + 1));
+    const Box b0 = range_box<GLOBAL>(P.pts, P.pyr, P.n, P.nlev, f0, c0);
+    const Box b1 = range_box<GLOBAL>(P.pts, P.pyr, P.n, P.nlev, f0 + c0, c1);
+    BvhNode nd;
+    // layout: [lo.x0 lo.y0 lo.z0 hi.x0] [hi.y0 hi.z0 lo.x1 lo.y1] [lo.z1 hi.x1 hi.y1 hi.z1]
+    nd.a = make_float4(b0.lo[0], b0.lo[1], b0.lo[2], b0.hi[0]);
+    nd.b = make_float4(b0.hi[1], b0.hi[2], b1.lo[0], b1.lo[1]);
+    nd.c = make_float4(b1.lo[2], b1.hi[0], b1.hi[1], b1.hi[2]);
+    nd.d = make_uint4(w0, w1, c0, c1);
+    return nd;
 }
 
 // Compact nodes: children become leaves when their subtree has <= leaf_size
@@ -415,34 +443,17 @@ __global__ void __launch_bounds__(BLOCK) node_kernel(
             kfirst[i] = f0;
             klast[i] = last;
         }
-        // children [first, split] and [split + 1, last]: Karras nodes split
-        // and split + 1 when they keep more than leaf_size points, else leaves
-        uint32_t word[2], cnt[2];
-        cnt[0] = sp - f0 + 1;
-        cnt[1] = last - sp;
-        word[0] = cnt[0] > leaf_size ? cidx[sp] : (CHILD_LEAF | f0);
-        word[1] = cnt[1] > leaf_size ? cidx[sp + 1] : (CHILD_LEAF | (sp + 1));
-        const Box b0 = range_box(P.pts, P.pyr, P.n, P.nlev, f0, cnt[0]);
-        const Box b1 = range_box(P.pts, P.pyr, P.n, P.nlev, f0 + cnt[0], cnt[1]);
-        BvhNode nd;
-        // layout: [lo.x0 lo.y0 lo.z0 hi.x0] [hi.y0 hi.z0 lo.x1 lo.y1] [lo.z1 hi.x1 hi.y1 hi.z1]
-        nd.a = make_float4(b0.lo[0], b0.lo[1], b0.lo[2], b0.hi[0]);
-        nd.b = make_float4(b0.hi[1], b0.hi[2], b1.lo[0], b1.lo[1]);
-        nd.c = make_float4(b1.lo[2], b1.hi[0], b1.hi[1], b1.hi[2]);
-        nd.d = make_uint4(word[0], word[1], cnt[0], cnt[1]);
-        nodes[c] = nd;
+        nodes[c] = make_node<true>(P, cidx, leaf_size, f0, last, sp);
     }
 }
 
 // Root word and the breadth-first top levels, copied into `top`.  One warp:
 // each level's nodes are loaded in parallel (level TOP_LEVELS-1 has at most
 // 32 nodes) and their internal children are placed by a warp prefix sum.
-__global__ void __launch_bounds__(32) stage_top_kernel(IndexHeader *h,
-                                                       const BvhNode *__restrict__ nodes,
-                                                       BvhNode *top, uint64_t n,
-                                                       uint32_t leaf_size) {
-    chain_wait();
-    const int lane = threadIdx.x;
+// s_q: TOP_MAX words of shared memory.
+__device__ __forceinline__ void stage_top(IndexHeader *h, const BvhNode *nodes, BvhNode *top, uint64_t n,
+                                          uint32_t leaf_size, uint32_t *s_q) {
+    const int lane = threadIdx.x & 31;
     if (n == 0 || n == 1 || n <= leaf_size) {
         if (lane == 0) {
             h->root = n == 0 ? CHILD_NONE : (CHILD_LEAF | 0u);
@@ -451,7 +462,6 @@ __global__ void __launch_bounds__(32) stage_top_kernel(IndexHeader *h,
         }
         return;
     }
-    __shared__ uint32_t s_q[TOP_MAX];
     if (lane == 0) s_q[0] = 0;
     __syncwarp();
     int begin = 0, end = 1;
@@ -489,18 +499,24 @@ __global__ void __launch_bounds__(32) stage_top_kernel(IndexHeader *h,
     }
 }
 
+__global__ void __launch_bounds__(32) stage_top_kernel(IndexHeader *h, const BvhNode *nodes, BvhNode *top, uint64_t n,
+                                                       uint32_t leaf_size) {
+    chain_wait();
+    __shared__ uint32_t s_q[TOP_MAX];
+    stage_top(h, nodes, top, n, leaf_size, s_q);
+}
+
 // ------------------------------------------------ radius-seed sample data
 // Two stride samples of the points in input order, kept with the index:
 // <= 1000 points (sample[0..n_sample)) for the k_nn! sampled-percentile seed
 // (gprt-macros/src/lib.rs:433-434), and S = min(n, 4096) points, index
 // b*n/S (sample[SEED_PCT_POINTS + b]), for the sampled 1-NN seed, which is
 // computed from them on the first search that needs it (ensure_nn_seed).
-__global__ void seed_sample_kernel(const float *__restrict__ xyz, uint64_t n, float4 *sample,
-                                   IndexHeader *h) {
+__device__ __forceinline__ void seed_sample(const float *__restrict__ xyz, uint64_t n, float4 *sample, IndexHeader *h,
+                                            uint32_t t0, uint32_t stride) {
     uint64_t pstep = n / SEED_PCT_POINTS > 1 ? n / SEED_PCT_POINTS : 1;
     uint64_t cnt = (n + pstep - 1) / pstep;
     if (cnt > SEED_PCT_POINTS) cnt = SEED_PCT_POINTS;
-    const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     for (uint64_t t = t0; t < cnt; t += stride) {
         uint64_t i = t * pstep;
         sample[t] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], 0.0f);
@@ -511,6 +527,10 @@ __global__ void seed_sample_kernel(const float *__restrict__ xyz, uint64_t n, fl
         sample[SEED_PCT_POINTS + b] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], 0.0f);
     }
     if (t0 == 0) h->n_sample = (uint32_t)cnt;
+}
+
+__global__ void seed_sample_kernel(const float *__restrict__ xyz, uint64_t n, float4 *sample, IndexHeader *h) {
+    seed_sample(xyz, n, sample, h, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // Squared 1-NN distance of each of the S sample points p[a] among the other
@@ -618,6 +638,293 @@ rtd_status ensure_nn_seed(rtd_index *idx, cudaStream_t st) {
 }
 
 namespace {
+
+// The smallest clouds: the whole build in one block and one launch.  The
+// chain of two dozen launches that builds larger indexes takes about 75 us
+// for 2,000 points on the GPU and 100 us on the host, almost none of it work;
+// this kernel 38 us.  Same index: keys sorted by (key, input position),
+// the same Karras nodes, boxes and top copy.  Keys, points, pyramid and the
+// kept nodes' indices stay in shared memory (40 B a point).  Bound by
+// barriers and dependent shared-memory loads.
+constexpr uint32_t SMALL_MAX = 4096;
+constexpr int SMALL_THREADS = 1024;
+struct SmallSmem {
+    uint64_t *key;      // P
+    float4 *pts;        // n
+    float4 *pyr;        // 2 per entry
+    uint32_t *idx, *cidx, *sel;   // P each
+};
+__host__ __device__ inline uint32_t small_pow2(uint32_t n) {
+    uint32_t P = SMALL_THREADS;
+    while (P < n) P <<= 1;
+    return P;
+}
+__host__ __device__ inline uint32_t pyramid_entries(uint32_t n) {
+    uint32_t total = 0;
+    while (n > PYR_B) {
+        n = (n + PYR_B - 1) / PYR_B;
+        total += n;
+    }
+    return total ? total : 1;
+}
+__host__ __device__ inline size_t small_smem(uint32_t n) {
+    const size_t P = small_pow2(n);
+    return P * (sizeof(uint64_t) + sizeof(float4) + 3 * sizeof(uint32_t)) + 2 * pyramid_entries(n) * sizeof(float4);
+}
+
+// E elements a thread: element u * 1024 + thread in register u.
+template <typename K, int E>
+__global__ void __launch_bounds__(SMALL_THREADS) small_build_kernel(const float *__restrict__ xyz, uint32_t n,
+                                                                    IndexHeader *h, float scale, uint32_t leaf_size,
+                                                                    K *out_keys, float4 *out_pts, float4 *out_pyr,
+                                                                    BvhNode *nodes, BvhNode *top, float4 *sample) {
+    chain_wait();
+    extern __shared__ float4 s_dyn[];
+    __shared__ float s_box[32][6];
+    __shared__ uint32_t s_cnt[33 * E], s_q[TOP_MAX];
+    constexpr uint32_t P = E * SMALL_THREADS;
+    SmallSmem s;
+    s.pts = s_dyn;
+    s.pyr = s.pts + P;
+    s.key = reinterpret_cast<uint64_t *>(s.pyr + 2 * pyramid_entries(n));
+    s.idx = reinterpret_cast<uint32_t *>(s.key + P);
+    s.cidx = s.idx + P;
+    s.sel = s.cidx + P;
+    const uint32_t tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) hdr_init(h);
+    // scene box, NaN-ignoring
+    float x[E], y[E], z[E], lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const uint32_t i = u * SMALL_THREADS + tid;
+        x[u] = y[u] = z[u] = NAN;
+        if (i < n) {
+            x[u] = xyz[3 * i];
+            y[u] = xyz[3 * i + 1];
+            z[u] = xyz[3 * i + 2];
+        }
+        lo[0] = fminf(lo[0], x[u]); hi[0] = fmaxf(hi[0], x[u]);
+        lo[1] = fminf(lo[1], y[u]); hi[1] = fmaxf(hi[1], y[u]);
+        lo[2] = fminf(lo[2], z[u]); hi[2] = fmaxf(hi[2], z[u]);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+            hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+        }
+        if (lane == 0) {
+            s_box[warp][a] = lo[a];
+            s_box[warp][3 + a] = hi[a];
+        }
+    }
+    __syncthreads();
+    if (warp < 6) {
+        float v = s_box[lane][warp];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = warp < 3 ? fminf(v, w) : fmaxf(v, w);
+        }
+        if (lane == 0) h->box[warp] = float_flip(v);
+        __syncwarp();
+        if (lane == 0) s_box[0][warp] = v;   // (column `warp` is this warp's alone)
+    }
+    __syncthreads();
+    SceneNorm nm;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        nm.lo[a] = s_box[0][a];
+        nm.ext[a] = fmaxf(__fsub_rn(s_box[0][3 + a], nm.lo[a]), 1e-6f);
+    }
+    if (sizeof(K) == 8) nm.ext[0] = nm.ext[1] = nm.ext[2] = fmaxf(nm.ext[0], fmaxf(nm.ext[1], nm.ext[2]));
+    // (key, position) pairs, sorted: runs of 32 by shuffles, merges at
+    // distance 32 and more in shared memory (all-ascending bitonic sort)
+    uint64_t k[E];
+    uint32_t v[E];
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        v[u] = u * SMALL_THREADS + tid;
+        k[u] = v[u] < n ? (uint64_t)morton_key<K>(nm, scale, x[u], y[u], z[u]) : ~0ull;   // padding: last
+    }
+    auto lanes = [&](int mask, bool lower) {
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const uint64_t ok = __shfl_xor_sync(0xffffffffu, k[u], mask);
+            const uint32_t ov = __shfl_xor_sync(0xffffffffu, v[u], mask);
+            if ((ok < k[u] || (ok == k[u] && ov < v[u])) == lower) {
+                k[u] = ok;
+                v[u] = ov;
+            }
+        }
+    };
+#pragma unroll 1
+    for (int kb = 2; kb <= 32; kb <<= 1) {
+        int mask = kb - 1;
+#pragma unroll 1
+        for (int j = kb >> 1; j > 0; j >>= 1) {
+            lanes(mask, (lane & j) == 0);
+            mask = j >> 1;
+        }
+    }
+#pragma unroll 1
+    for (uint32_t kb = 64; kb <= P; kb <<= 1) {
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            s.key[u * SMALL_THREADS + tid] = k[u];
+            s.idx[u * SMALL_THREADS + tid] = v[u];
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (uint32_t j = kb >> 1; j >= 32; j >>= 1) {
+            for (uint32_t t = tid; t < P / 2; t += SMALL_THREADS) {
+                const uint32_t r = t & (j - 1), a = (t - r) * 2 + r, b = j == kb >> 1 ? (t - r) * 2 + 2 * j - 1 - r : a + j;
+                const uint64_t ka = s.key[a], kc = s.key[b];
+                const uint32_t va = s.idx[a], vc = s.idx[b];
+                if (kc < ka || (kc == ka && vc < va)) {
+                    s.key[a] = kc;
+                    s.key[b] = ka;
+                    s.idx[a] = vc;
+                    s.idx[b] = va;
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            k[u] = s.key[u * SMALL_THREADS + tid];
+            v[u] = s.idx[u * SMALL_THREADS + tid];
+        }
+#pragma unroll 1
+        for (int j = 16; j > 0; j >>= 1) lanes(j, (lane & j) == 0);
+    }
+    // sorted keys and points, in shared memory and out
+#pragma unroll
+    for (int u = 0; u < E; ++u) {
+        const uint32_t i = u * SMALL_THREADS + tid;
+        s.key[i] = k[u];   // (each thread's own elements)
+        if (i < n) {
+            const float4 p = make_float4(xyz[3 * v[u]], xyz[3 * v[u] + 1], xyz[3 * v[u] + 2], __uint_as_float(v[u]));
+            s.pts[i] = p;
+            out_pts[i] = p;
+            out_keys[i] = (K)k[u];
+        }
+    }
+    seed_sample(xyz, n, sample, h, tid, SMALL_THREADS);
+    __syncthreads();
+    if (n >= 2 && n > leaf_size) {
+        // box pyramid
+        Pyramid Py;
+        Py.pts = s.pts;
+        Py.pyr = s.pyr;
+        Py.n = n;
+        Py.nlev = 0;
+        uint32_t size = n, off = 0, below = 0;
+        while (size > PYR_B) {
+            const uint32_t up = (size + PYR_B - 1) / PYR_B;
+            for (uint32_t e = tid; e < up; e += SMALL_THREADS) {
+                Box b;
+                bool nan = false;
+                box_empty(b);
+                const uint32_t end = min(size, (e + 1) * PYR_B);
+                for (uint32_t i = e * PYR_B; i < end; ++i) {
+                    if (Py.nlev == 0) box_add_point(b, nan, s.pts[i]);
+                    else box_add(b, s.pyr[2 * (below + i)], s.pyr[2 * (below + i) + 1]);
+                }
+                if (nan) box_unbounded(b);
+                box_store(s.pyr, off + e, b);
+                box_store(out_pyr, off + e, b);
+            }
+            below = off;
+            off += up;
+            size = up;
+            ++Py.nlev;
+            __syncthreads();
+        }
+        // kept nodes (karras_flag_kernel's test), numbered in order
+        bool keep[E];
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const int64_t i = u * SMALL_THREADS + tid;
+            keep[u] = false;
+            if (i + 1 < (int64_t)n) {
+                int dir, dmin;
+                karras_dir<uint64_t>(s.key, n, s.key[i], i, dir, dmin);
+                keep[u] = delta<uint64_t>(s.key, n, s.key[i], i, i + (int64_t)leaf_size * dir) > dmin;
+            }
+            const uint32_t m = __ballot_sync(0xffffffffu, keep[u]);
+            if (lane == 0) s_cnt[u * 32 + warp] = __popc(m);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t run = 0;
+#pragma unroll
+            for (int u = 0; u < E; ++u) {
+                const uint32_t c = s_cnt[u * 32 + lane];
+                uint32_t incl = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t w = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += w;
+                }
+                s_cnt[u * 32 + lane] = run + incl - c;
+                run += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) {
+                s_cnt[32 * E] = run;
+                h->n_internal = run;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < E; ++u) {
+            const uint32_t i = u * SMALL_THREADS + tid, m = __ballot_sync(0xffffffffu, keep[u]);
+            const uint32_t at = s_cnt[u * 32 + warp] + __popc(m & ((1u << lane) - 1u));
+            s.cidx[i] = at;
+            if (keep[u]) s.sel[at] = i;
+        }
+        __syncthreads();
+        for (uint32_t c = tid; c < s_cnt[32 * E]; c += SMALL_THREADS) {
+            uint32_t f0, last, sp;
+            karras_range<uint64_t>(s.key, n, s.sel[c], leaf_size, f0, last, sp);
+            nodes[c] = make_node<false>(Py, s.cidx, leaf_size, f0, last, sp);
+        }
+        __syncthreads();
+    }
+    if (warp == 0) stage_top(h, nodes, top, n, leaf_size, s_q);
+}
+
+template <typename K, int E>
+rtd_status launch_small(rtd_index *idx, const float *d_xyz, uint32_t n, float scale, cudaStream_t st) {
+    RTD_CUDA(cudaFuncSetAttribute(small_build_kernel<K, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)small_smem(E * SMALL_THREADS)));
+    RTD_LAUNCH_CHAINED((small_build_kernel<K, E>), dim3(1), dim3(SMALL_THREADS), small_smem(n), st, d_xyz, n,
+                       idx->hdr.as<IndexHeader>(), scale, idx->leaf_size, idx->keys.as<K>(), idx->pts.as<float4>(),
+                       idx->pyramid.as<float4>(), idx->nodes.as<BvhNode>(), idx->top.as<BvhNode>(),
+                       idx->sample.as<float4>());
+    return RTD_OK;
+}
+
+template <typename K>
+rtd_status build_small(rtd_index *idx, const float *d_xyz, uint32_t n, cudaStream_t st) {
+    const int kbits = sizeof(K) == 4 ? 30 : idx->morton_bits;
+    const float scale = sizeof(K) == 4 ? 1023.0f : (float)((1u << (kbits / 3)) - 1u);
+    RTD_TRY(idx->keys.reserve(n * sizeof(K)));
+    RTD_TRY(idx->pyramid.reserve(2 * pyramid_entries(n) * sizeof(float4)));
+    RTD_TRY(idx->sample.reserve((SEED_PCT_POINTS + SEED_NN_SAMPLE) * sizeof(float4)));
+    RTD_TRY(idx->seed.reserve(SEED_NN_SAMPLE * sizeof(float)));
+    idx->nn_seeded = false;
+    if (n <= SMALL_THREADS) RTD_TRY((launch_small<K, 1>(idx, d_xyz, n, scale, st)));
+    else if (n <= 2 * SMALL_THREADS) RTD_TRY((launch_small<K, 2>(idx, d_xyz, n, scale, st)));
+    else RTD_TRY((launch_small<K, 4>(idx, d_xyz, n, scale, st)));
+    idx->skeys = idx->keys.ptr;
+    idx->mark(EV_BUILD_SORTED, st);
+    if (idx->ev_sorted) RTD_CUDA(cudaEventRecord(idx->ev_sorted, st));
+    idx->mark(EV_BUILD1, st);
+    return RTD_OK;
+}
 
 template <typename K>
 rtd_status build_typed(rtd_index *idx, const float *d_xyz, uint64_t n, cudaStream_t st) {
@@ -781,6 +1088,9 @@ rtd_status index_build(rtd_index *idx, const float *d_xyz, uint64_t n, const rtd
     IndexHeader *h = idx->hdr.as<IndexHeader>();
     for (bool &e : idx->ev_set) e = false;
     idx->mark(EV_BUILD0, st);
+    if (n > 0 && n <= SMALL_MAX)
+        return mb == 30 ? build_small<uint32_t>(idx, d_xyz, (uint32_t)n, st)
+                        : build_small<uint64_t>(idx, d_xyz, (uint32_t)n, st);
     RTD_LAUNCH_CHAINED(hdr_init_kernel, dim3(1), dim3(1), 0, st, h);
     if (n > 0) {
         RTD_LAUNCH_CHAINED(bbox_kernel, dim3(grid_for(n, BLOCK, 148 * 4)), dim3(BLOCK), 0, st, d_xyz,
