@@ -28,8 +28,7 @@ struct BhHeader {
     uint32_t lw;              // first level whose width < min_width
     uint32_t n_nodes, n_leaves;
     uint32_t err;
-    uint32_t level_count[BH_MAX_LEVEL + 2];
-    uint32_t level_off[BH_MAX_LEVEL + 3];
+    uint32_t depth;           // deepest level of a node
     uint32_t max_stack;       // deepest traversal stack seen by a walk
     uint32_t group_counter;   // work queue of the walks (next group to take)
     uint32_t ilog_used;       // interaction-log pages taken by the last logging forward
@@ -72,20 +71,21 @@ struct rtd_bh {
     // build scratch
     rtd::DevBuf mkeys, mkeys_alt, mvals, mvals_alt;   // Morton sort
     rtd::DevBuf pkeys, pkeys_alt, pvals, pvals_alt;   // path-key sort (values: Morton rank)
-    rtd::DevBuf lcp, wmin, lam, nn, base, heads, leaf_head, leaf_of;
+    rtd::DevBuf lcp, wmin, lam, nn, base, heads, leaf_of;
     rtd::DevBuf fkeys, fkeys_alt, fvals, fvals_alt;   // final regroup sort
-    rtd::DevBuf node_start, node_level, level_nodes;
+    rtd::DevBuf node_start, node_level, missing;
     rtd::SortScratch sort;
     rtd::ScanScratch scan;
     // tree
     rtd::DevBuf order;        // flat order: original index of the i-th body
     rtd::DevBuf fbody;        // float4 (pos, mass) in flat order
     rtd::DevBuf node_a, node_b, node_q;
-    // walk structures: child table (8 per node), traversal stacks
-    rtd::DevBuf child8, stack;
+    // child table (8 per node), parents, traversal stacks
+    rtd::DevBuf child8, parent, stack;
+    uint64_t node_cap = 0;        // nodes the node buffers hold
     uint64_t stack_warps = 0;
     // adjoint scratch
-    rtd::DevBuf cell_grad, prefix, gpos_flat, gmass_flat;
+    rtd::DevBuf cell_grad, gpos_flat, gmass_flat;
     // interaction log (Plummer forward -> adjoint), kept once a backward has
     // followed a forward on this handle; its pool is sized from the last
     // logging forward's need (a pinned copy read when it has landed)
@@ -117,12 +117,13 @@ struct BhView {
     const BhHeader *hdr;
     uint64_t n;
     const uint4 *child8;       // 2 uint4 per node: up to 8 children, 0xFFFFFFFF pads
+    const uint32_t *parent;    // 0xFFFFFFFF for the root
 };
 
 inline BhView bh_view(const rtd_bh *b) {
     return BhView{b->node_a.as<float4>(), b->node_b.as<uint4>(), b->node_q.as<float4>(),
                   b->fbody.as<float4>(), b->order.as<uint32_t>(), b->hdr.as<BhHeader>(), b->n,
-                  b->child8.as<uint4>()};
+                  b->child8.as<uint4>(), b->parent.as<uint32_t>()};
 }
 
 rtd_status bh_build(rtd_bh *b, const float *d_pos, const float *d_mass, uint64_t n,

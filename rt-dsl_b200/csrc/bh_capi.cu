@@ -85,10 +85,10 @@ rtd_status rtd_bh_release(rtd_bh *b) {
     if (!b) return fail(RTD_ERR_INVALID_ARGUMENT, "bh handle is NULL");
     for (DevBuf *d : {&b->mkeys, &b->mkeys_alt, &b->mvals, &b->mvals_alt, &b->pkeys, &b->pkeys_alt,
                       &b->pvals, &b->pvals_alt, &b->lcp, &b->wmin, &b->lam, &b->nn, &b->base,
-                      &b->heads, &b->leaf_head, &b->leaf_of, &b->fkeys, &b->fkeys_alt, &b->fvals,
-                      &b->fvals_alt, &b->node_start, &b->node_level, &b->level_nodes, &b->order,
+                      &b->heads, &b->leaf_of, &b->fkeys, &b->fkeys_alt, &b->fvals,
+                      &b->fvals_alt, &b->node_start, &b->node_level, &b->missing, &b->order,
                       &b->fbody, &b->node_a, &b->node_b, &b->node_q, &b->child8,
-                      &b->stack, &b->cell_grad, &b->prefix, &b->gpos_flat,
+                      &b->parent, &b->stack, &b->cell_grad, &b->gpos_flat,
                       &b->gmass_flat})
         d->release();
     for (DevBuf *d : {&b->ilog_entries, &b->ilog_counts, &b->ilog_next, &b->ilog_group})
@@ -126,8 +126,7 @@ rtd_status rtd_bh_info_get(rtd_bh *b, rtd_bh_info *info, rtd_stream stream) {
     RTD_CUDA(cudaStreamSynchronize(st));
     info->n_nodes = h.n_nodes;
     info->n_leaves = h.n_leaves;
-    for (int l = 0; l <= BH_MAX_LEVEL + 1; ++l)
-        if (h.level_count[l]) info->depth = (uint32_t)l;
+    info->depth = h.depth;
     for (int a = 0; a < 3; ++a) {
         info->root_min[a] = h.root_min[a];
         info->root_max[a] = h.root_max[a];

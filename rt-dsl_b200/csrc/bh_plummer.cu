@@ -728,64 +728,50 @@ __device__ __forceinline__ void cell_constants(const float4 a, const float4 *cg,
     out[4] = Bxx; out[5] = Byy; out[6] = Bzz; out[7] = Bxy; out[8] = Bxz; out[9] = Byz;
 }
 
-// Top-down path sums of the per-node constants (one block, level by level).
-__global__ void __launch_bounds__(1024) bh_prefix_kernel(const BhView v,
-                                                         const uint32_t *__restrict__ level_nodes,
-                                                         const float4 *__restrict__ cell_grad,
-                                                         float4 *prefix) {
-    const BhHeader *h = v.hdr;
-    for (int l = 0; l <= BH_MAX_LEVEL + 1; ++l) {
-        const uint32_t off = h->level_off[l], cnt = h->level_count[l];
-        for (uint32_t t = threadIdx.x; t < cnt; t += blockDim.x) {
-            const uint32_t i = level_nodes[off + t];
-            float own[10];
-            cell_constants(v.node_a[i], cell_grad + 3 * i, own);
-            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-            float4 p0 = l == 0 ? z : prefix[3 * i];      // the parent's path sum
-            float4 p1 = l == 0 ? z : prefix[3 * i + 1];
-            float4 p2 = l == 0 ? z : prefix[3 * i + 2];
-            p0 = make_float4(p0.x + own[0], p0.y + own[1], p0.z + own[2], p0.w + own[3]);
-            p1 = make_float4(p1.x + own[4], p1.y + own[5], p1.z + own[6], p1.w + own[7]);
-            p2 = make_float4(p2.x + own[8], p2.y + own[9], 0.f, 0.f);
-            prefix[3 * i] = p0;
-            prefix[3 * i + 1] = p1;
-            prefix[3 * i + 2] = p2;
-            const uint4 b = v.node_b[i];
-            if (!(b.z & BH_LEAF_BIT))
-                for (uint32_t c = i + 1; c < b.x; c = v.node_b[c].x) {
-                    prefix[3 * c] = p0;
-                    prefix[3 * c + 1] = p1;
-                    prefix[3 * c + 2] = p2;
-                }
-        }
-        __syncthreads();
+// Each node's constants in place of its derivatives (10 of 12 words).
+__global__ void __launch_bounds__(256) bh_constants_kernel(const BhView v, float4 *cell_grad) {
+    const uint32_t n_nodes = v.hdr->n_nodes;
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n_nodes; i += gridDim.x * 256) {
+        float own[10];
+        float4 *c = cell_grad + 3 * (uint64_t)i;
+        cell_constants(v.node_a[i], c, own);
+        c[0] = make_float4(own[0], own[1], own[2], own[3]);
+        c[1] = make_float4(own[4], own[5], own[6], own[7]);
+        c[2] = make_float4(own[8], own[9], 0.f, 0.f);
     }
 }
 
-__global__ void __launch_bounds__(128) bh_finish_grad_kernel(const BhView v,
-                                                             const float4 *__restrict__ prefix,
+// The bodies' gradients, a warp per leaf: the constants added up along the
+// path to the root (a word a lane; going through the levels in one block
+// took 0.96 ms at 1M bodies, this 0.05 ms), then applied to the leaf's
+// bodies.
+__global__ void __launch_bounds__(128) bh_finish_grad_kernel(const BhView v, const float *__restrict__ constants,
                                                              const float4 *__restrict__ body_grad,
-                                                             float *__restrict__ g_pos,
-                                                             float *__restrict__ g_mass) {
+                                                             float *__restrict__ g_pos, float *__restrict__ g_mass) {
     const uint32_t n_nodes = v.hdr->n_nodes;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nodes; i += gridDim.x * blockDim.x) {
-        const uint4 b = v.node_b[i];
+    const int lane = threadIdx.x & 31;
+    for (uint32_t leaf = blockIdx.x * 4 + (threadIdx.x >> 5); leaf < n_nodes; leaf += gridDim.x * 4) {
+        const uint4 b = v.node_b[leaf];
         if (!(b.z & BH_LEAF_BIT)) continue;
-        const float4 p0 = prefix[3 * i], p1 = prefix[3 * i + 1], p2 = prefix[3 * i + 2];
-        const float Pxx = p1.x, Pyy = p1.y, Pzz = p1.z, Pxy = p1.w, Pxz = p2.x, Pyz = p2.y;
+        float sum = 0.f;
+        for (uint32_t i = leaf; i != 0xFFFFFFFFu; i = v.parent[i])
+            if (lane < 10) sum += constants[12 * (uint64_t)i + lane];
+        float P[10];
+#pragma unroll
+        for (int k = 0; k < 10; ++k) P[k] = __shfl_sync(0xffffffffu, sum, k);
         const uint32_t s0 = b.y, c = b.z & ~BH_LEAF_BIT;
-        for (uint32_t k = 0; k < c; ++k) {
+        for (uint32_t k = lane; k < c; k += 32) {
             const float4 o = v.fbody[s0 + k];
-            const float Px = Pxx * o.x + Pxy * o.y + Pxz * o.z;
-            const float Py = Pxy * o.x + Pyy * o.y + Pyz * o.z;
-            const float Pz = Pxz * o.x + Pyz * o.y + Pzz * o.z;
+            const float Px = P[4] * o.x + P[7] * o.y + P[8] * o.z;
+            const float Py = P[7] * o.x + P[5] * o.y + P[9] * o.z;
+            const float Pz = P[8] * o.x + P[9] * o.y + P[6] * o.z;
             const float4 bg = body_grad[s0 + k];
             const uint32_t orig = v.order[s0 + k];
-            g_pos[3 * (uint64_t)orig] = bg.x + o.w * (p0.x + 2.f * Px);
-            g_pos[3 * (uint64_t)orig + 1] = bg.y + o.w * (p0.y + 2.f * Py);
-            g_pos[3 * (uint64_t)orig + 2] = bg.z + o.w * (p0.z + 2.f * Pz);
+            g_pos[3 * (uint64_t)orig] = bg.x + o.w * (P[0] + 2.f * Px);
+            g_pos[3 * (uint64_t)orig + 1] = bg.y + o.w * (P[1] + 2.f * Py);
+            g_pos[3 * (uint64_t)orig + 2] = bg.z + o.w * (P[2] + 2.f * Pz);
             if (g_mass)
-                g_mass[orig] = bg.w + p0.w + (p0.x * o.x + p0.y * o.y + p0.z * o.z) +
+                g_mass[orig] = bg.w + P[3] + (P[0] * o.x + P[1] * o.y + P[2] * o.z) +
                                (o.x * Px + o.y * Py + o.z * Pz);
         }
     }
@@ -922,10 +908,10 @@ rtd_status bh_backward(rtd_bh *b, const rtd_bh_params *p, const float *g_acc, co
     if (p->quadrupole && !b->has_quad)
         return fail(RTD_ERR_INVALID_ARGUMENT, "tree was built without quadrupoles");
     const uint64_t n = b->n;
-    RTD_TRY(b->cell_grad.reserve(n * 3 * sizeof(float4) + 64 * sizeof(uint32_t)));
-    RTD_TRY(b->prefix.reserve(n * 3 * sizeof(float4)));
+    const uint64_t cells = b->node_cap;
+    RTD_TRY(b->cell_grad.reserve(cells * 3 * sizeof(float4) + 64 * sizeof(uint32_t)));
     RTD_TRY(b->gpos_flat.reserve(n * sizeof(float4)));
-    RTD_CUDA(cudaMemsetAsync(b->cell_grad.ptr, 0, n * 3 * sizeof(float4), st));
+    RTD_CUDA(cudaMemsetAsync(b->cell_grad.ptr, 0, cells * 3 * sizeof(float4), st));
     RTD_CUDA(cudaMemsetAsync(b->gpos_flat.ptr, 0, n * sizeof(float4), st));
     // replay the last forward's interaction log when it was taken on this
     // tree with these parameters; otherwise walk
@@ -941,11 +927,10 @@ rtd_status bh_backward(rtd_bh *b, const rtd_bh_params *p, const float *g_acc, co
     if (p->quadrupole) RTD_TRY((launch_walk<true, true>(b, p, g_acc, g_phi, nullptr, nullptr, lg, st)));
     else RTD_TRY((launch_walk<false, true>(b, p, g_acc, g_phi, nullptr, nullptr, lg, st)));
     const BhView v = bh_view(b);
-    bh_prefix_kernel<<<1, 1024, 0, st>>>(v, b->level_nodes.as<uint32_t>(), b->cell_grad.as<float4>(),
-                                          b->prefix.as<float4>());
+    bh_constants_kernel<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(v, b->cell_grad.as<float4>());
     RTD_LAUNCH_CHECK();
-    bh_finish_grad_kernel<<<grid_for(n, 128, 1 << 20), 128, 0, st>>>(
-        v, b->prefix.as<float4>(), b->gpos_flat.as<float4>(), g_pos, g_mass);
+    bh_finish_grad_kernel<<<grid_for(cells, 4, 148 * 64), 128, 0, st>>>(
+        v, b->cell_grad.as<float>(), b->gpos_flat.as<float4>(), g_pos, g_mass);
     RTD_LAUNCH_CHECK();
     return RTD_OK;
 }
