@@ -24,7 +24,7 @@
 // each (body, source) pair once, adds the body's derivative up and leaves
 // three to five coefficients in shared memory; then lane = source sums the
 // source's derivative over the bodies from the coefficients (replayed from
-// the log at 1M bodies: 20.2 ms; a table of the derivatives themselves,
+// the log at 1M bodies: 18.8 ms; a table of the derivatives themselves,
 // summed row by row: 33.8 ms) and adds it with one vector atomic per source
 // and part.  Cell derivatives (COM, mass,
 // quadrupole) are then pushed to the bodies by a top-down pass: with Q
@@ -299,7 +299,7 @@ struct Flag {
 // SPLIT_AT of them.
 constexpr int SPLIT_AT = 64;
 template <bool QUAD, bool ADJ, int SPLIT>
-__global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 7) bh_walk_kernel(
+__global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 6) bh_walk_kernel(
     const BhView v, float theta2, float eps2, float G, const float *__restrict__ g_acc,
     const float *__restrict__ g_phi, float *__restrict__ acc_out, float *__restrict__ phi_out,
     float4 *__restrict__ cell_grad, float4 *__restrict__ body_grad, uint2 *__restrict__ stack,
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 7) bh_walk_kernel(
                 for (int p0 = 0; p0 < pairs; p0 += ADJ_SOURCES / 2) {
                     const int pn = pairs - p0 < ADJ_SOURCES / 2 ? pairs - p0 : ADJ_SOURCES / 2;
                     auto bodies_side = [&](auto quad, auto msk) {
-#pragma unroll 1
+#pragma unroll 2
                         for (int q = 0; q < pn; ++q) {
                             const int p = p0 + q;
                             f2 w[5];
