@@ -506,12 +506,18 @@ static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32
     return lanes == 32 && kk <= COLLECT_MAX_K ? Search::collect : Search::rounds;
 }
 // Whether the queries are put in Morton order first.  The warp search gains
-// little from neighbours running together (40,000 queries, k = 300: 1.16 ms
-// without, 1.18 ms with; 100,000: 2.30 and 2.21), so below this many queries
-// it does without the dozen launches of the ordering, about 40 us.
+// from neighbours running together only where the points and their pyramid
+// (about 21 B a point) do not fit the L2 cache, and then only for queries
+// enough to pay for the dozen launches of the ordering (about 40 us).
+// Measured, in order / as they come, ms: 1.8M points, 400,000 queries, k = 16:
+// 1.55 / 1.50, k = 64: 2.73 / 2.54; 3M points, 300,000 queries: uniform 1.12 /
+// 1.13, sheet 1.13 / 1.21; 10M points, 200,000 queries: 1.04 / 1.33,
+// 1M queries: 4.54 / 5.59.
 constexpr uint64_t COLLECT_ORDER_MIN = 49152;
+constexpr uint64_t COLLECT_ORDER_POINTS = 2ull << 20;
 static bool wants_order(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
-    return s.use_morton_lbv && !(nq < COLLECT_ORDER_MIN && search_mode(n, s, nq, k) == Search::collect);
+    return s.use_morton_lbv && !((nq < COLLECT_ORDER_MIN || n < COLLECT_ORDER_POINTS) &&
+                                 search_mode(n, s, nq, k) == Search::collect);
 }
 
 // Launches the search kernel the schedule selects for the queries of a
