@@ -76,7 +76,7 @@ rtd_status knn_search(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t k,
                       const rtd_schedule *sched, uint32_t *d_ids, float *d_d2, cudaStream_t st);
 rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                        const rtd_schedule *s, uint32_t *d_counts, uint64_t *h_total,
-                       cudaStream_t st);
+                       cudaStream_t st, bool own_points = false);
 rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                       const rtd_schedule *s, uint32_t *d_pairs, uint64_t capacity, int sort_pairs,
                       uint64_t *h_written, cudaStream_t st, bool check = true);

@@ -26,7 +26,7 @@ namespace rtd {
 
 rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                        const rtd_schedule *s, uint32_t *d_counts, uint64_t *h_total,
-                       cudaStream_t st);
+                       cudaStream_t st, bool own_points = false);
 rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                       const rtd_schedule *s, uint32_t *d_pairs, uint64_t capacity, int sort_pairs,
                       uint64_t *h_written, cudaStream_t st, bool check = true);
@@ -165,7 +165,7 @@ extern "C" rtd_status rtd_dbscan(rtd_index *idx, const float *d_points, uint64_t
            &ncbuf = idx->db_nc;
     RTD_TRY(counts.reserve(n * 4));
     uint64_t total = 0;
-    RTD_TRY(range_count(idx, d_points, n, eps, nullptr, counts.as<uint32_t>(), &total, st));
+    RTD_TRY(range_count(idx, d_points, n, eps, nullptr, counts.as<uint32_t>(), &total, st, true));
     if (total >= (1ull << 32)) return fail(RTD_ERR_UNSUPPORTED, "more than 2^32 neighbour pairs");
     RTD_TRY(pairs.reserve(total * 8 + 8));
     uint64_t written = 0;

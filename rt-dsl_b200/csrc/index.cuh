@@ -44,9 +44,12 @@ struct IndexHeader {
     uint64_t total;       // last range-count total
     float nn95_key;       // p95 of the squared 1-NN distance within a 4096-point sample
     uint32_t n_sample;    // points in the radius-seed sample (<= 1000)
-    uint32_t most;        // largest count of the last range count
     uint32_t heavy;       // some query of its sample has very many hits
     unsigned long long qfp[2];   // query fingerprints of the last range count / fill
+    // last range count (cleared together): pairs pushed, records, points the
+    // records cover; the largest count.  A pushing fill uses rcur[0].
+    unsigned long long rcur[3];
+    uint32_t most;
 };
 
 constexpr int SEED_NN_SAMPLE = 4096;
@@ -94,7 +97,7 @@ struct rtd_index {
     // search scratch
     rtd::DevBuf qkeys, qkeys_alt, qperm, qperm_alt;
     const void *skeys = nullptr;   // the points' sorted Morton keys (in keys or keys_alt)
-    rtd::DevBuf rcounts, roffsets, rcursor, rpairs_alt, rkeys, rkeys_alt;
+    rtd::DevBuf rcounts, roffsets, rpairs_alt, rkeys, rkeys_alt;
     // the count pass's own (query, id) pairs, kept when a buffer from an
     // earlier count is large enough (rspec_cap pairs), and the fill's
     // per-query cursors

@@ -11,6 +11,7 @@
 // global atomicAdd per flush (warp-aggregated compaction).  Membership:
 // exact FP32 key <= RN(r*r), as the intersection program tests
 // dist_sq <= r_val*r_val (lib.rs:283, 341).
+#include "knn_backward.cuh"
 #include "knn_collect.cuh"
 
 namespace rtd {
@@ -756,12 +757,19 @@ __global__ void keys_from_pairs_kernel(const uint2 *__restrict__ pairs, uint64_t
     }
 }
 
-constexpr uint64_t RANGE_ORDER_MIN = 49152;
+// The points' ids in Morton order.
+__global__ void own_order_kernel(const float4 *__restrict__ pts, uint64_t n, uint32_t *__restrict__ perm) {
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        perm[i] = __float_as_uint(__ldg(&pts[i].w));
+}
+
+constexpr uint64_t RANGE_ORDER_MIN = 49152, RANGE_ORDER_POINTS = 2ull << 20;
 constexpr uint64_t THREAD_QUERIES = 131072;   // see launch_count
 rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r, cudaStream_t st);
 
 rtd_status range_args(rtd_index *idx, const float *d_q, uint64_t nq, float r,
-                      const rtd_schedule *sched, RangeArgs &a, cudaStream_t st, bool count) {
+                      const rtd_schedule *sched, RangeArgs &a, cudaStream_t st, bool count,
+                      bool own_points = false) {
     if (!idx || !idx->hdr.ptr) return fail(RTD_ERR_INVALID_ARGUMENT, "index not built");
     if (nq && !d_q) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL queries");
     if (!(r >= 0.0f)) return fail(RTD_ERR_INVALID_ARGUMENT, "radius must be >= 0");
@@ -773,11 +781,26 @@ rtd_status range_args(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     for (int e = EV_SEARCH0; e <= EV_SEARCH1; ++e) idx->ev_set[e] = false;
     idx->mark(EV_SEARCH0, st);
     idx->mark(EV_SEEDED, st);
-    // (as for the k-NN warp search: few queries gain less from the order than
-    // its launches cost)
+    // A thread's walk needs its warp's queries to be neighbours; a warp's
+    // gains from the order only as the k-NN warp search does (knn.cu).
     const bool sample = count && nq >= THREAD_QUERIES;
+    const bool wants_order = nq >= THREAD_QUERIES || (nq >= RANGE_ORDER_MIN && idx->n >= RANGE_ORDER_POINTS);
     if (sample) RTD_TRY(launch_sample(idx, d_q, nq, r, st));
-    const rtd_status os = order_queries(idx, d_q, nq, s.use_morton_lbv && nq >= RANGE_ORDER_MIN, &perm, st);
+    rtd_status os;
+    if (own_points) {   // the queries are the index's points: its own order
+        os = order_queries(idx, d_q, nq, false, &perm, st);
+        if (os == RTD_OK && wants_order) os = idx->qperm.reserve(nq * sizeof(uint32_t));
+        if (os == RTD_OK && wants_order) {
+            own_order_kernel<<<grid_for(nq, 256, 148 * 8), 256, 0, st>>>(idx->pts.as<float4>(), nq,
+                                                                        idx->qperm.as<uint32_t>());
+            note_launch();
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) os = cuda_fail(e, "own_order_kernel launch");
+            perm = idx->qperm.as<uint32_t>();
+        }
+    } else {
+        os = order_queries(idx, d_q, nq, s.use_morton_lbv && wants_order, &perm, st);
+    }
     if (sample) RTD_CUDA(cudaStreamWaitEvent(st, idx->ev_join, 0));   // also on the error path
     RTD_TRY(os);
     idx->mark(EV_ORDERED, st);
@@ -872,26 +895,25 @@ rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r,
 
 rtd_status check_index_errors(rtd_index *idx, cudaStream_t st);
 
+// own_points: the queries are the points the index was built over.
 rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                        const rtd_schedule *s, uint32_t *d_counts, uint64_t *h_total,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool own_points) {
     if (!d_counts && nq) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL counts");
     RangeArgs a = {};
-    RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, true));
+    RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, true, own_points));
     a.counts = d_counts;
     IndexHeader *h = idx->hdr.as<IndexHeader>();
     // With a buffer left by an earlier count, this count also pushes its
     // pairs there (and fingerprints the queries), so that a fill of the same
     // queries only scatters them into their segments.
     const bool spec = nq > 0 && idx->rspec_cap > 0;
-    RTD_CUDA(cudaMemsetAsync(&h->most, 0, sizeof(uint32_t), st));
+    RTD_CUDA(cudaMemsetAsync(h->rcur, 0, offsetof(IndexHeader, most) + sizeof(uint32_t) - offsetof(IndexHeader, rcur), st));
     if (nq) {
         if (spec) {
-            RTD_TRY(idx->rcursor.reserve(3 * sizeof(unsigned long long)));
-            RTD_CUDA(cudaMemsetAsync(idx->rcursor.ptr, 0, 3 * sizeof(unsigned long long), st));
             a.pairs = idx->rspec.as<uint2>();
             a.capacity = idx->rspec_cap;
-            a.cursor = idx->rcursor.as<unsigned long long>();
+            a.cursor = h->rcur;
             a.recs = idx->rrec.as<uint4>();
             a.rec_cap = idx->rrec_cap;
             RTD_TRY(query_fingerprint(d_q, nq, &h->qfp[0], st));
@@ -906,14 +928,17 @@ rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     } else {
         RTD_CUDA(cudaMemsetAsync(&h->total, 0, sizeof(uint64_t), st));
     }
-    uint64_t total = 0;
-    unsigned long long cur[3] = {0, 0, 0};   // pairs pushed, records, points the records cover
-    uint32_t most = 0;
-    RTD_CUDA(cudaMemcpyAsync(&total, &h->total, sizeof(total), cudaMemcpyDeviceToHost, st));
-    RTD_CUDA(cudaMemcpyAsync(&most, &h->most, sizeof(most), cudaMemcpyDeviceToHost, st));
-    if (spec)
-        RTD_CUDA(cudaMemcpyAsync(cur, idx->rcursor.ptr, sizeof(cur), cudaMemcpyDeviceToHost, st));
-    RTD_TRY(check_index_errors(idx, st));   // synchronises
+    // everything the host needs in one copy: total, cursors, largest count, errors
+    IndexHeader now;
+    RTD_CUDA(cudaMemcpyAsync(&now, h, sizeof(now), cudaMemcpyDeviceToHost, st));
+    RTD_CUDA(cudaStreamSynchronize(st));
+    if (now.err) {
+        RTD_CUDA(cudaMemsetAsync(&h->err, 0, sizeof(uint32_t), st));
+        return status_from_deverr(now.err);
+    }
+    const uint64_t total = now.total;
+    const unsigned long long *cur = now.rcur;
+    const uint32_t most = now.most;
     if (h_total) *h_total = total;
     const bool spec_ok = spec && cur[0] + cur[2] == total && cur[0] <= idx->rspec_cap &&
                          cur[1] <= idx->rrec_cap;
@@ -980,9 +1005,9 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
         a.err = &idx->hdr.as<IndexHeader>()->err;
     } else {
         RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, false));
-        RTD_TRY(idx->rcursor.reserve(sizeof(unsigned long long)));
-        RTD_CUDA(cudaMemsetAsync(idx->rcursor.ptr, 0, sizeof(unsigned long long), st));
-        a.cursor = idx->rcursor.as<unsigned long long>();
+        IndexHeader *h = idx->hdr.as<IndexHeader>();
+        RTD_CUDA(cudaMemsetAsync(h->rcur, 0, sizeof(unsigned long long), st));
+        a.cursor = h->rcur;
     }
     a.pairs = reinterpret_cast<uint2 *>(d_pairs);
     a.capacity = capacity;
@@ -1018,7 +1043,7 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     if (seg) {
         total = tk.total;
     } else {
-        RTD_CUDA(cudaMemcpyAsync(&total, idx->rcursor.ptr, sizeof(total), cudaMemcpyDeviceToHost, st));
+        RTD_CUDA(cudaMemcpyAsync(&total, a.cursor, sizeof(total), cudaMemcpyDeviceToHost, st));
         RTD_CUDA(cudaStreamSynchronize(st));
     }
     if (h_written) *h_written = total;
@@ -1074,28 +1099,19 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
 
 // ------------------------------------------------------- kNN backward
 namespace {
-__global__ void knn_backward_kernel(const float *__restrict__ q, uint64_t nq,
-                                    const float *__restrict__ pts, uint64_t n, uint32_t k,
-                                    const uint32_t *__restrict__ ids, const float *__restrict__ g,
-                                    float *__restrict__ gq, float *__restrict__ gp) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nq;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        float qx = q[3 * i], qy = q[3 * i + 1], qz = q[3 * i + 2];
-        float ax = 0.f, ay = 0.f, az = 0.f;
-        for (uint32_t j = 0; j < k; ++j) {
-            uint32_t id = ids[i * k + j];
-            if (id == EMPTY_ID || id >= n) continue;
-            float w = 2.0f * g[i * k + j];
-            float dx = qx - pts[3 * (uint64_t)id], dy = qy - pts[3 * (uint64_t)id + 1],
-                  dz = qz - pts[3 * (uint64_t)id + 2];
-            ax += w * dx; ay += w * dy; az += w * dz;
-            if (gp) {
-                atomicAdd(&gp[3 * (uint64_t)id], -w * dx);
-                atomicAdd(&gp[3 * (uint64_t)id + 1], -w * dy);
-                atomicAdd(&gp[3 * (uint64_t)id + 2], -w * dz);
-            }
-        }
-        if (gq) { gq[3 * i] = ax; gq[3 * i + 1] = ay; gq[3 * i + 2] = az; }
+__global__ void __launch_bounds__(256) knn_backward_kernel(const float *__restrict__ q, uint64_t nq,
+                                                           const float *__restrict__ pts, uint64_t n, uint32_t k,
+                                                           const uint32_t *__restrict__ ids,
+                                                           const float *__restrict__ g, float *__restrict__ gq,
+                                                           float *__restrict__ gp) {
+    const uint32_t T = backward_lanes(k);
+    const int lane = threadIdx.x & 31;
+    const bool pairs = backward_pairs(gp);
+    const uint64_t per = 32 / T;
+    for (uint64_t i0 = (((uint64_t)blockIdx.x * 256 + threadIdx.x) >> 5) * per; i0 < nq;
+         i0 += (((uint64_t)gridDim.x * 256) >> 5) * per) {
+        const uint64_t i = i0 + lane / T;
+        backward_query(i < nq, q, pts, n, k, ids + i * k, g + i * k, gq, gp, i, T, pairs);
     }
 }
 }  // namespace
@@ -1104,7 +1120,8 @@ rtd_status knn_backward(const float *q, uint64_t nq, const float *pts, uint64_t 
                         const uint32_t *ids, const float *g, float *gq, float *gp, cudaStream_t st) {
     if (nq == 0 || k == 0) return RTD_OK;
     if (!q || !pts || !ids || !g) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL input");
-    knn_backward_kernel<<<grid_for(nq, 256, 148 * 16), 256, 0, st>>>(q, nq, pts, n, k, ids, g, gq, gp);
+    knn_backward_kernel<<<grid_for(nq * backward_lanes(k), 256, 148 * 16), 256, 0, st>>>(q, nq, pts, n, k, ids, g, gq,
+                                                                                        gp);
     RTD_LAUNCH_CHECK();
     return RTD_OK;
 }
