@@ -50,6 +50,7 @@ struct IndexHeader {
     // records cover; the largest count.  A pushing fill uses rcur[0].
     unsigned long long rcur[3];
     uint32_t most;
+    uint32_t n_cross;     // tree nodes whose points lie in more than one tile
 };
 
 constexpr int SEED_NN_SAMPLE = 4096;
@@ -82,9 +83,10 @@ struct rtd_index {
     rtd::DevBuf keys, keys_alt, vals, vals_alt;
     rtd::DevBuf k32a, k32b;   // 32-bit top keys of the split sort
     // Karras node flags (1: the node keeps more than leaf_size points),
-    // compact indices, the list of kept nodes, and (forest builds) the kept
-    // nodes' first and last points by Karras index
-    rtd::DevBuf flags, cidx, csel, kfirst, klast;
+    // compact indices, the list of kept nodes, those whose points lie in more
+    // than one tile, and (forest builds) the kept nodes' first and last points
+    // by Karras index
+    rtd::DevBuf flags, cidx, csel, cross, kfirst, klast;
     rtd::DevBuf pyramid;    // run boxes over the sorted points (2 float4 per run)
     rtd::SortScratch sort;
     rtd::ScanScratch scan;
@@ -121,12 +123,10 @@ struct rtd_index {
         uint64_t spec_pairs = 0, spec_recs = 0;
     } rtoken;
     // Side stream for work that overlaps the build: the radius-seed sample
-    // (every build) and rtd_k_nn's query ordering; tree stream: the box
-    // pyramid, beside the Karras flags and their scan
-    cudaStream_t side_stream = nullptr, tree_stream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_seed_fork = nullptr,
-                ev_seed_join = nullptr, ev_sorted = nullptr, ev_tree_fork = nullptr,
-                ev_tree_join = nullptr;
+    // (every build) and rtd_k_nn's query ordering
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_seed_fork = nullptr, ev_seed_join = nullptr,
+                ev_sorted = nullptr;
     rtd::DevBuf wpos;       // queries' Morton positions for the window seed
     rtd::DevBuf wide;       // per-warp list slabs of the k > 2048 search
     rtd::QueryOrderScratch qorder;
@@ -142,11 +142,9 @@ struct rtd_index {
     ~rtd_index() {
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {ev_fork, ev_join, ev_seed_fork, ev_seed_join, ev_sorted,
-                              ev_tree_fork, ev_tree_join})
+        for (cudaEvent_t e : {ev_fork, ev_join, ev_seed_fork, ev_seed_join, ev_sorted})
             if (e) cudaEventDestroy(e);
         if (side_stream) cudaStreamDestroy(side_stream);
-        if (tree_stream) cudaStreamDestroy(tree_stream);
     }
 };
 

@@ -157,7 +157,7 @@ __device__ __forceinline__ void karras_dir(const K *__restrict__ keys, int64_t n
 // of the (key, position) pairs, which are strictly increasing, cannot grow
 // with distance.  This kernel makes that one test per node; the range and
 // split searches run afterwards for the kept nodes alone, packed densely by
-// the scan of these flags (node_kernel), so no warp carries idle lanes of
+// the scan of these flags (tile_nodes_kernel), so no warp carries idle lanes of
 // collapsed nodes through them.
 // A block takes FLAG_TILE consecutive nodes and first stages their keys
 // with a halo of leaf_size + 1 on each side in shared memory (one
@@ -166,8 +166,9 @@ constexpr int FLAG_TILE = 2048;
 constexpr int FLAG_HALO = 65;   // leaf_size (<= 64) + 1
 template <typename K>
 __global__ void __launch_bounds__(BLOCK) karras_flag_kernel(const K *__restrict__ keys, int64_t n,
-                                                            uint32_t leaf_size, uint32_t *flags) {
+                                                            uint32_t leaf_size, uint32_t *flags, IndexHeader *h) {
     chain_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) h->n_cross = 0;   // (tile_nodes_kernel counts)
     __shared__ K s_k[FLAG_TILE + 2 * FLAG_HALO];
     const int64_t b0 = (int64_t)blockIdx.x * FLAG_TILE, base = b0 - FLAG_HALO;
     for (int t = threadIdx.x; t < FLAG_TILE + 2 * FLAG_HALO; t += BLOCK) {
@@ -192,31 +193,28 @@ __global__ void __launch_bounds__(BLOCK) karras_flag_kernel(const K *__restrict_
     }
 }
 
-// Point range [first, last] and split of kept Karras node i: the children
-// hold [first, split] and [split + 1, last].
-template <typename K>
-__device__ __forceinline__ void karras_range(const K *__restrict__ keys, int64_t n, int64_t i,
-                                             uint32_t leaf_size, uint32_t &first, uint32_t &last,
-                                             uint32_t &split) {
-    const K ki = keys[i];
-    int dir, dmin;
-    karras_dir(keys, n, ki, i, dir, dmin);
-    int64_t lmax = 2;
-    while (lmax <= (int64_t)leaf_size) lmax <<= 1;
-    while (delta(keys, n, ki, i, i + lmax * dir) > dmin) lmax <<= 1;
-    int64_t l = 0;
-    for (int64_t t = lmax >> 1; t >= 1; t >>= 1)
-        if (delta(keys, n, ki, i, i + (l + t) * dir) > dmin) l += t;
-    const int64_t j = i + l * dir;
-    const int dnode = delta(keys, n, ki, i, j);
-    int64_t s = 0, t = l;
+// Point range [first, last] and split of the kept Karras node at local
+// position i, whose range holds at most `room` points after i in direction
+// dir: the children hold [first, split] and [split + 1, last].  dl(j): the
+// common prefix with the key at local position j.  REACH: a power of two
+// above the longest range.
+template <int REACH, typename Delta>
+__device__ __forceinline__ void karras_range(const Delta &dl, int i, int dir, int dmin, int room, uint32_t &first,
+                                             uint32_t &last, uint32_t &split) {
+    int l = 0;
+#pragma unroll 1
+    for (int t = REACH / 2; t >= 1; t >>= 1)
+        if (l + t <= room && dl(i + (l + t) * dir) > dmin) l += t;
+    const int dnode = dl(i + l * dir);
+    int s = 0, t = l;
+#pragma unroll 1
     do {
         t = (t + 1) >> 1;
-        if (delta(keys, n, ki, i, i + (s + t) * dir) > dnode) s += t;
+        if (s + t < l && dl(i + (s + t) * dir) > dnode) s += t;
     } while (t > 1);
     split = (uint32_t)(i + s * dir + (dir < 0 ? -1 : 0));
-    first = (uint32_t)(i < j ? i : j);
-    last = (uint32_t)(i < j ? j : i);
+    first = (uint32_t)(dir > 0 ? i : i - l);
+    last = (uint32_t)(dir > 0 ? i + l : i);
 }
 
 // ---------------------------------------------------- box pyramid
@@ -273,30 +271,22 @@ __device__ __forceinline__ void box_store(float4 *out, uint64_t e, const Box &b)
     out[2 * e + 1] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
 }
 
-// Three levels of the pyramid from `count` inputs (the sorted points when
-// PTS, else the boxes of the level below o1): a 512-thread block per 512
+// Three levels of the pyramid from the `count` boxes of the level below o1
+// (levels 1 to 3 come from tile_nodes_kernel): a 512-thread block per 512
 // inputs, one input a thread.  Lanes fold 8 inputs into an o1 entry and a
 // warp's 32 into half an o2 entry; warp 0 folds the block's 16 warp boxes
 // into its 8 o2 entries and its o3 entry.  Inputs past count hold the empty
 // box; a null output is a level above the top and is not written.
-template <bool PTS>
 __global__ void __launch_bounds__(512) pyramid_fold_kernel(const float4 *__restrict__ in,
                                                            uint64_t count, float4 *o1, float4 *o2,
                                                            float4 *o3) {
+    chain_wait();
     __shared__ float4 s_lo[16], s_hi[16];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t i = (uint64_t)blockIdx.x * 512 + threadIdx.x;
     Box b;
     box_empty(b);
-    if (i < count) {
-        if (PTS) {
-            bool nan = false;
-            box_add_point(b, nan, __ldg(&in[i]));
-            if (nan) box_unbounded(b);
-        } else {
-            box_add(b, __ldg(&in[2 * i]), __ldg(&in[2 * i + 1]));
-        }
-    }
+    if (i < count) box_add(b, in[2 * i], in[2 * i + 1]);
     box_xor(b, 1);
     box_xor(b, 2);
     box_xor(b, 4);
@@ -326,14 +316,10 @@ __global__ void __launch_bounds__(512) pyramid_fold_kernel(const float4 *__restr
 // BATCH entries at a time so that their loads are in flight together.  The
 // last batch repeats entry b - 1 in place of entries past b: a min / max
 // does not change when an entry is added twice.
-// GLOBAL: the entries are global memory that this kernel does not write.
-template <bool GLOBAL>
-__device__ __forceinline__ float4 ld_entry(const float4 *p) { return GLOBAL ? __ldg(p) : *p; }
-
-template <bool PTS, bool GLOBAL>
+template <bool PTS>
 __device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *base,
                                         uint32_t a, uint32_t b) {
-    constexpr int BATCH = PTS ? 8 : 4;
+    constexpr int BATCH = PTS ? 4 : 2;
 #pragma unroll 1
     for (uint32_t t = a; t < b; t += BATCH) {
         float4 lo[BATCH], hi[BATCH];
@@ -341,10 +327,10 @@ __device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *base,
         for (int u = 0; u < BATCH; ++u) {
             const uint32_t e = t + u < b ? t + u : b - 1;
             if (PTS) {
-                lo[u] = ld_entry<GLOBAL>(&base[e]);
+                lo[u] = base[e];
             } else {
-                lo[u] = ld_entry<GLOBAL>(&base[2 * (uint64_t)e]);
-                hi[u] = ld_entry<GLOBAL>(&base[2 * (uint64_t)e + 1]);
+                lo[u] = base[2 * (uint64_t)e];
+                hi[u] = base[2 * (uint64_t)e + 1];
             }
         }
 #pragma unroll
@@ -361,7 +347,6 @@ __device__ __forceinline__ void add_run(Box &bx, bool &nan, const float4 *base,
 // The level offsets follow from n as the walk goes up, so the pyramid is
 // passed as scalars (a struct taken by reference would be copied to local
 // memory).
-template <bool GLOBAL>
 __device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint32_t n, int nlev,
                                       uint32_t first, uint32_t count) {
     Box b;
@@ -374,8 +359,8 @@ __device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint
     for (int j = 0; j <= PYR_MAX; ++j) {
         if (l >= r) break;
         if (j == nlev) {
-            if (j == 0) add_run<true, GLOBAL>(b, nan, pts, l, r);
-            else add_run<false, GLOBAL>(b, nan, lvl, l, r);
+            if (j == 0) add_run<true>(b, nan, pts, l, r);
+            else add_run<false>(b, nan, lvl, l, r);
             break;
         }
         uint32_t head = (l + PYR_B - 1) & ~(PYR_B - 1);
@@ -383,11 +368,11 @@ __device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint
         uint32_t tail = r & ~(PYR_B - 1);
         if (tail < head) tail = head;
         if (j == 0) {
-            add_run<true, GLOBAL>(b, nan, pts, l, head);
-            add_run<true, GLOBAL>(b, nan, pts, tail, r);
+            add_run<true>(b, nan, pts, l, head);
+            add_run<true>(b, nan, pts, tail, r);
         } else {
-            add_run<false, GLOBAL>(b, nan, lvl, l, head);
-            add_run<false, GLOBAL>(b, nan, lvl, tail, r);
+            add_run<false>(b, nan, lvl, l, head);
+            add_run<false>(b, nan, lvl, tail, r);
             lvl += 2 * (uint64_t)size;
         }
         l = head >> PYR_SH;
@@ -400,50 +385,215 @@ __device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint
 
 // The node of the points [f0, last] with children [f0, sp] and [sp + 1, last]:
 // Karras nodes sp and sp + 1 when they keep more than leaf_size points, else
-// leaves.
-template <bool GLOBAL>
-__device__ __forceinline__ BvhNode make_node(const Pyramid &P, const uint32_t *cidx, uint32_t leaf_size, uint32_t f0,
-                                             uint32_t last, uint32_t sp) {
+// leaves.  The positions count from base.
+__device__ __forceinline__ BvhNode pack_node(const uint32_t *cidx, uint32_t leaf_size, uint32_t f0, uint32_t last,
+                                             uint32_t sp, uint32_t base, const Box &b0, const Box &b1) {
     const uint32_t c0 = sp - f0 + 1, c1 = last - sp;
-    const uint32_t w0 = c0 > leaf_size ? cidx[sp] : (CHILD_LEAF | f0);
-    const uint32_t w1 = c1 > leaf_size ? cidx[sp + 1] : (CHILD_LEAF | (sp + 1));
-    const Box b0 = range_box<GLOBAL>(P.pts, P.pyr, P.n, P.nlev, f0, c0);
-    const Box b1 = range_box<GLOBAL>(P.pts, P.pyr, P.n, P.nlev, f0 + c0, c1);
     BvhNode nd;
     // layout: [lo.x0 lo.y0 lo.z0 hi.x0] [hi.y0 hi.z0 lo.x1 lo.y1] [lo.z1 hi.x1 hi.y1 hi.z1]
     nd.a = make_float4(b0.lo[0], b0.lo[1], b0.lo[2], b0.hi[0]);
     nd.b = make_float4(b0.hi[1], b0.hi[2], b1.lo[0], b1.lo[1]);
     nd.c = make_float4(b1.lo[2], b1.hi[0], b1.hi[1], b1.hi[2]);
-    nd.d = make_uint4(w0, w1, c0, c1);
+    nd.d = make_uint4(c0 > leaf_size ? cidx[base + sp] : (CHILD_LEAF | (base + f0)),
+                      c1 > leaf_size ? cidx[base + sp + 1] : (CHILD_LEAF | (base + sp + 1)), c0, c1);
     return nd;
+}
+__device__ __forceinline__ BvhNode make_node(const Pyramid &P, const uint32_t *cidx, uint32_t leaf_size, uint32_t f0,
+                                             uint32_t last, uint32_t sp, uint32_t base) {
+    const Box b0 = range_box(P.pts, P.pyr, P.n, P.nlev, f0, sp - f0 + 1);
+    const Box b1 = range_box(P.pts, P.pyr, P.n, P.nlev, sp + 1, last - sp);
+    return pack_node(cidx, leaf_size, f0, last, sp, base, b0, b1);
 }
 
 // Compact nodes: children become leaves when their subtree has <= leaf_size
-// points.  A thread per kept node (sel[c] = its Karras index) finds the
-// node's range and split, then writes it.  Every child carries the number
-// of points below it (a subtree's points are contiguous in sorted order,
-// starting at the parent's first point for the left child and after the
-// left child's points for the right one), and its box: the box of its
-// contiguous points, from the pyramid.  Every node's boxes are computed
-// independently, so no bottom-up pass over the tree follows.  With kfirst
-// non-null the range is also stored by Karras index.
+// points.  Every child carries the number of points below it (a subtree's
+// points are contiguous in sorted order, starting at the parent's first point
+// for the left child and after the left child's points for the right one),
+// and its box: the box of its contiguous points, from the pyramid.  Every
+// node is computed independently, so no bottom-up pass over the tree follows.
+// With kfirst non-null the range is also stored by Karras index.
+//
+// tile_nodes_kernel: a block takes NODE_TILE sorted points.  It stages their
+// keys and points in shared memory, folds levels 1 to 3 of the pyramid there
+// (and writes them out), and makes the nodes whose points all lie in the
+// tile, a thread a node: all but about one in ten.  The searches for a node's
+// range and split and the walk of its boxes are chains of dependent reads,
+// which is why they run on shared memory.  A node's prefix with the keys of
+// its direction cannot grow with distance, so its range ends inside the tile
+// exactly when the first key past the tile no longer exceeds its lower bound;
+// the others are listed in `cross` for cross_nodes_kernel.  Bound by the
+// issue slots of the searches and box walks (half of them used; ~12,000 warp
+// instructions a tile).  With global searches a thread a node the nodes of
+// 100 K points took 34 us (51 dependent reads at the root), now 18 + 11;
+// those of 10 M 454 us, with the pyramid's own 79, now 330 + 84.
+constexpr int NODE_TILE = 1024;
+constexpr int NODE_DEPTH = 96;   // prefix lengths of (key, position) pairs: nodes that share a tile boundary are nested
 template <typename K>
-__global__ void __launch_bounds__(BLOCK) node_kernel(
-    const K *__restrict__ keys, uint64_t n, const IndexHeader *h, const uint32_t *__restrict__ sel,
-    const uint32_t *__restrict__ cidx, uint32_t leaf_size, const Pyramid P, BvhNode *nodes,
-    uint32_t *kfirst, uint32_t *klast) {
+__global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
+    const K *__restrict__ keys, uint64_t n, IndexHeader *h, const uint32_t *__restrict__ sel,
+    const uint32_t *__restrict__ cidx, uint32_t leaf_size, const float4 *__restrict__ pts, float4 *lv1, float4 *lv2,
+    float4 *lv3, BvhNode *nodes, uint32_t *kfirst, uint32_t *klast, uint32_t *cross, uint32_t cross_cap) {
     chain_wait();
-    const uint32_t n_int = h->n_internal;
-    for (uint32_t c = blockIdx.x * BLOCK + threadIdx.x; c < n_int && c + 1 < n;
-         c += gridDim.x * BLOCK) {
-        const uint32_t i = sel[c];
-        uint32_t f0, last, sp;
-        karras_range<K>(keys, (int64_t)n, i, leaf_size, f0, last, sp);
-        if (kfirst) {
-            kfirst[i] = f0;
-            klast[i] = last;
+    __shared__ K s_k[NODE_TILE + 2];
+    __shared__ float4 s_p[NODE_TILE];
+    __shared__ float4 s_pyr[2 * (NODE_TILE / 8 + NODE_TILE / 64 + NODE_TILE / 512)];
+    const int64_t b0 = (int64_t)blockIdx.x * NODE_TILE;
+    const uint32_t m = (uint32_t)(n - b0 < NODE_TILE ? n - b0 : NODE_TILE);
+    const uint32_t n1 = (m + 7) / 8, n2 = (n1 + 7) / 8, n3 = (n2 + 7) / 8;
+    for (uint32_t t = threadIdx.x; t < NODE_TILE + 2; t += BLOCK) {
+        const int64_t j = b0 + (int64_t)t - 1;
+        if (j >= 0 && j < (int64_t)n) s_k[t] = keys[j];
+    }
+    // level 1: the 8 lanes of an entry
+    for (uint32_t t = threadIdx.x; t < NODE_TILE; t += BLOCK) {
+        Box b;
+        box_empty(b);
+        if (t < m) {
+            const float4 p = pts[b0 + t];
+            s_p[t] = p;
+            bool nan = false;
+            box_add_point(b, nan, p);
+            if (nan) box_unbounded(b);
         }
-        nodes[c] = make_node<true>(P, cidx, leaf_size, f0, last, sp);
+        box_xor(b, 1);
+        box_xor(b, 2);
+        box_xor(b, 4);
+        if ((t & 7) == 0 && t < m) {
+            box_store(s_pyr, t / 8, b);
+            if (lv1) box_store(lv1, b0 / 8 + t / 8, b);
+        }
+    }
+    __syncthreads();
+    // levels 2 and 3
+    for (int lev = 2; lev <= 3; ++lev) {
+        const float4 *in = lev == 2 ? s_pyr : s_pyr + 2 * n1;
+        float4 *out = lev == 2 ? s_pyr + 2 * n1 : s_pyr + 2 * (n1 + n2), *g = lev == 2 ? lv2 : lv3;
+        const uint32_t cnt_in = lev == 2 ? n1 : n2, cnt = lev == 2 ? n2 : n3;
+        for (uint32_t e = threadIdx.x; e < cnt; e += BLOCK) {
+            Box b;
+            box_empty(b);
+            for (uint32_t u = 8 * e; u < 8 * e + 8 && u < cnt_in; ++u) box_add(b, in[2 * u], in[2 * u + 1]);
+            box_store(out, e, b);
+            if (g) box_store(g, (uint64_t)(lev == 2 ? b0 / 64 : b0 / 512) + e, b);
+        }
+        __syncthreads();
+    }
+    Pyramid P;
+    P.pts = s_p;
+    P.pyr = s_pyr;
+    P.n = m;
+    P.nlev = 3;
+    const uint32_t n_int = h->n_internal;
+    const uint32_t c0 = b0 < (int64_t)n - 1 ? cidx[b0] : n_int;
+    const uint32_t c1 = b0 + NODE_TILE < (int64_t)n - 1 ? cidx[b0 + NODE_TILE] : n_int;
+    for (uint32_t c = c0 + threadIdx.x; c < c1; c += BLOCK) {
+        const uint32_t i = sel[c];
+        const int li = (int)(i - (uint32_t)b0);
+        const K ki = s_k[li + 1];
+        auto dl = [&](int lj) -> int {   // lj in [-1, NODE_TILE]
+            const int64_t j = b0 + lj;
+            if (j < 0 || j >= (int64_t)n) return -1;
+            const K b = s_k[lj + 1];
+            if (ki == b) return (int)(8 * sizeof(K)) + __clz(i ^ (uint32_t)j);
+            return sizeof(K) == 8 ? __clzll((unsigned long long)(ki ^ b)) : __clz((uint32_t)(ki ^ b));
+        };
+        const int dp = dl(li + 1), dm = dl(li - 1), dir = (dp - dm) >= 0 ? 1 : -1, dmin = dir > 0 ? dm : dp;
+        if (dl(dir > 0 ? NODE_TILE : -1) > dmin) {
+            const uint32_t at = atomicAdd(&h->n_cross, 1u);
+            if (at < cross_cap) cross[at] = c;
+            else atomicOr(&h->err, DEVERR_OVERFLOW);
+            continue;
+        }
+        uint32_t f0, last, sp;
+        karras_range<NODE_TILE>(dl, li, dir, dmin, dir > 0 ? NODE_TILE - 1 - li : li, f0, last, sp);
+        const uint32_t base = (uint32_t)b0;
+        if (kfirst) {
+            kfirst[i] = base + f0;
+            klast[i] = base + last;
+        }
+        nodes[c] = make_node(P, cidx, leaf_size, f0, last, sp, base);
+    }
+}
+
+// The nodes whose points lie in more than one tile, a warp a node: the range
+// and the split are found 32 probes at a time (an end among n keys takes
+// log32 n dependent reads), and the lanes of a half warp read the entries of
+// one child's box at each level of the pyramid together.
+template <typename K>
+__global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
+    const K *__restrict__ keys, uint64_t n, const IndexHeader *h, const uint32_t *__restrict__ sel,
+    const uint32_t *__restrict__ cidx, uint32_t leaf_size, const Pyramid P, BvhNode *nodes, uint32_t *kfirst,
+    uint32_t *klast, const uint32_t *__restrict__ cross, uint32_t cross_cap) {
+    chain_wait();
+    const uint32_t count = h->n_cross < cross_cap ? h->n_cross : cross_cap;
+    const int lane = threadIdx.x & 31;
+    for (uint32_t w = (blockIdx.x * BLOCK + threadIdx.x) >> 5; w < count; w += (gridDim.x * BLOCK) >> 5) {
+        const uint32_t c = cross[w];
+        const int64_t i = sel[c];
+        const K ki = keys[i];
+        int dir, dmin;
+        karras_dir(keys, (int64_t)n, ki, i, dir, dmin);
+        // 2^up <= length < 2^(up + 1)
+        const int up =
+            __popc(__ballot_sync(0xffffffffu, lane < 31 && delta(keys, (int64_t)n, ki, i, i + ((int64_t)1 << lane) * dir) > dmin)) - 1;
+        // largest x of [lo, lo + width) whose key still shares more than d
+        auto furthest = [&](int64_t lo, int64_t width, int d) {
+            while (width > 1) {
+                const int64_t step = width > 32 ? width >> 5 : 1, x = lo + lane * step;
+                const bool ok = lane == 0 || (lane * step < width && delta(keys, (int64_t)n, ki, i, i + x * dir) > d);
+                lo += (__popc(__ballot_sync(0xffffffffu, ok)) - 1) * step;
+                width = step;
+            }
+            return lo;
+        };
+        const int64_t l = furthest((int64_t)1 << up, (int64_t)1 << up, dmin);
+        const int64_t s = furthest(0, (int64_t)2 << up, delta(keys, (int64_t)n, ki, i, i + l * dir));
+        const uint32_t f0 = (uint32_t)(dir > 0 ? i : i - l), last = (uint32_t)(dir > 0 ? i + l : i);
+        const uint32_t sp = (uint32_t)(i + s * dir + (dir < 0 ? -1 : 0));
+        // boxes: lanes 0-15 the left child, 16-31 the right one; of 16 lanes
+        // 8 take the partial run at the start of a level, 8 that at its end
+        Box b;
+        box_empty(b);
+        const uint32_t e = lane & 7;
+        const bool tail_lane = lane & 8;
+        uint32_t a = lane < 16 ? f0 : sp + 1, r = lane < 16 ? sp + 1 : last + 1, size = P.n;
+        const float4 *lvl = P.pyr;
+#pragma unroll 1
+        for (int j = 0; j <= P.nlev && a < r; ++j) {
+            uint32_t head = (a + PYR_B - 1) & ~(PYR_B - 1);
+            if (head > r) head = r;
+            uint32_t tail = r & ~(PYR_B - 1);
+            if (tail < head) tail = head;
+            if (j == P.nlev) head = tail = r;   // (at most 8 entries: whole)
+            const uint32_t x = tail_lane ? tail + e : a + e;
+            if (x < (tail_lane ? r : head)) {
+                if (j == 0) {
+                    bool nan = false;
+                    box_add_point(b, nan, P.pts[x]);
+                    if (nan) box_unbounded(b);
+                } else {
+                    box_add(b, lvl[2 * (uint64_t)x], lvl[2 * (uint64_t)x + 1]);
+                }
+            }
+            if (j) lvl += 2 * (uint64_t)size;
+            size = (size + PYR_B - 1) >> PYR_SH;
+            a = head >> PYR_SH;
+            r = tail >> PYR_SH;
+        }
+        __syncwarp();
+        for (int o = 1; o < 16; o <<= 1) box_xor(b, o);
+        Box b1;
+        for (int x = 0; x < 3; ++x) {
+            b1.lo[x] = __shfl_sync(0xffffffffu, b.lo[x], 16);
+            b1.hi[x] = __shfl_sync(0xffffffffu, b.hi[x], 16);
+        }
+        if (lane == 0) {
+            nodes[c] = pack_node(cidx, leaf_size, f0, last, sp, 0u, b, b1);
+            if (kfirst) {
+                kfirst[i] = f0;
+                klast[i] = last;
+            }
+        }
     }
 }
 
@@ -888,8 +1038,13 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_build_kernel(const float 
         __syncthreads();
         for (uint32_t c = tid; c < s_cnt[32 * E]; c += SMALL_THREADS) {
             uint32_t f0, last, sp;
-            karras_range<uint64_t>(s.key, n, s.sel[c], leaf_size, f0, last, sp);
-            nodes[c] = make_node<false>(Py, s.cidx, leaf_size, f0, last, sp);
+            const int i = (int)s.sel[c];
+            const uint64_t ki = s.key[i];
+            auto dl = [&](int j) -> int { return delta(s.key, (int64_t)n, ki, i, j); };
+            int dir, dmin;
+            karras_dir(s.key, (int64_t)n, ki, i, dir, dmin);
+            karras_range<SMALL_MAX>(dl, i, dir, dmin, dir > 0 ? (int)n - 1 - i : i, f0, last, sp);
+            nodes[c] = make_node(Py, s.cidx, leaf_size, f0, last, sp, 0u);
         }
         __syncthreads();
     }
@@ -1000,46 +1155,27 @@ rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStr
     P.pyr = pyr;
     float4 *lv[PYR_MAX + 1] = {};
     for (int j = 1; j <= nlev; ++j) lv[j] = pyr + 2 * offs[j];
-    // The pyramid (from the points) runs on the tree stream while the flags
-    // and their scan (from the keys) run on st; the node kernel needs both.
-    RTD_TRY(ensure_side_stream(idx));
-    cudaStream_t ts = idx->tree_stream;
-    RTD_CUDA(cudaEventRecord(idx->ev_tree_fork, st));
-    RTD_CUDA(cudaStreamWaitEvent(ts, idx->ev_tree_fork, 0));
-    // three levels per launch: 1-3 from the points, 4-6 from level 3, ...
-    cudaError_t pe = cudaSuccess;
-    for (int j = 1; j <= nlev && pe == cudaSuccess; j += 3) {
-        float4 *o2 = j + 1 <= nlev ? lv[j + 1] : nullptr;
-        float4 *o3 = j + 2 <= nlev ? lv[j + 2] : nullptr;
-        const unsigned g = (unsigned)ceil_div(sizes[j - 1], 512);
-        if (j == 1) pyramid_fold_kernel<true><<<g, 512, 0, ts>>>(P.pts, n, lv[1], o2, o3);
-        else pyramid_fold_kernel<false><<<g, 512, 0, ts>>>(lv[j - 1], sizes[j - 1], lv[j], o2, o3);
-        note_launch();
-        pe = cudaGetLastError();
-    }
-    RTD_CUDA(cudaEventRecord(idx->ev_tree_join, ts));
-    const unsigned gi = (unsigned)ceil_div(ni, (uint64_t)FLAG_TILE);
-    note_launch();
-    cudaError_t fe = launch_chained(karras_flag_kernel<K>, dim3(gi), dim3(BLOCK), 0, st, skeys,
-                                    (int64_t)n, idx->leaf_size, idx->flags.as<uint32_t>());
-    const rtd_status sr =
-        fe != cudaSuccess ? RTD_OK
-                          : exclusive_scan_select_u32(idx->flags.as<uint32_t>(), idx->cidx.as<uint32_t>(),
-                                                      idx->csel.as<uint32_t>(), ni, &h->n_internal,
-                                                      idx->scan, d_err, st);
-    RTD_CUDA(cudaStreamWaitEvent(st, idx->ev_tree_join, 0));   // also on the error paths
-    if (pe != cudaSuccess) return cuda_fail(pe, "pyramid_fold_kernel launch");
-    if (fe != cudaSuccess) return cuda_fail(fe, "karras_flag_kernel launch");
-    RTD_TRY(sr);
-    // grid for about (n - 1) / leaf_size kept nodes, the count of a balanced
-    // tree; the kernel strides over however many there are (up to
-    // n - 1 - leaf_size in a chain-shaped tree)
-    const uint64_t kept_max = ni / idx->leaf_size + 1 < ni ? ni / idx->leaf_size + 1 : ni;
-    RTD_LAUNCH_CHAINED(node_kernel<K>, dim3(grid_for(kept_max, BLOCK, 148 * 8)), dim3(BLOCK), 0, st,
-                       skeys, n, (const IndexHeader *)h, (const uint32_t *)idx->csel.as<uint32_t>(),
-                       (const uint32_t *)idx->cidx.as<uint32_t>(), idx->leaf_size, P,
-                       idx->nodes.as<BvhNode>(), ranges ? idx->kfirst.as<uint32_t>() : nullptr,
-                       ranges ? idx->klast.as<uint32_t>() : nullptr);
+    const uint64_t tiles = ceil_div(n, (uint64_t)NODE_TILE);
+    const uint32_t cross_cap = (uint32_t)(ni < NODE_DEPTH * tiles ? ni : NODE_DEPTH * tiles);
+    RTD_TRY(idx->cross.reserve(cross_cap * sizeof(uint32_t)));
+    RTD_LAUNCH_CHAINED(karras_flag_kernel<K>, dim3((unsigned)ceil_div(ni, (uint64_t)FLAG_TILE)), dim3(BLOCK), 0, st,
+                       skeys, (int64_t)n, idx->leaf_size, idx->flags.as<uint32_t>(), h);
+    RTD_TRY(exclusive_scan_select_u32(idx->flags.as<uint32_t>(), idx->cidx.as<uint32_t>(), idx->csel.as<uint32_t>(),
+                                      ni, &h->n_internal, idx->scan, d_err, st));
+    uint32_t *kf = ranges ? idx->kfirst.as<uint32_t>() : nullptr, *kl = ranges ? idx->klast.as<uint32_t>() : nullptr;
+    const uint32_t *sel = idx->csel.as<uint32_t>(), *cidx = idx->cidx.as<uint32_t>();
+    RTD_LAUNCH_CHAINED(tile_nodes_kernel<K>, dim3((unsigned)tiles), dim3(BLOCK), 0, st, skeys, n, h, sel, cidx,
+                       idx->leaf_size, (const float4 *)P.pts, lv[1], lv[2], lv[3], idx->nodes.as<BvhNode>(), kf, kl,
+                       idx->cross.as<uint32_t>(), cross_cap);
+    // three levels of the pyramid per launch: 4-6 from level 3, ...
+    for (int j = 4; j <= nlev; j += 3)
+        RTD_LAUNCH_CHAINED(pyramid_fold_kernel, dim3((unsigned)ceil_div(sizes[j - 1], 512)), dim3(512), 0, st,
+                           (const float4 *)lv[j - 1], sizes[j - 1], lv[j], j + 1 <= nlev ? lv[j + 1] : nullptr,
+                           j + 2 <= nlev ? lv[j + 2] : nullptr);
+    // (a warp a node, for about 8 nodes a tile)
+    RTD_LAUNCH_CHAINED(cross_nodes_kernel<K>, dim3((unsigned)(tiles < 148 * 8 ? tiles : 148 * 8)), dim3(BLOCK), 0, st,
+                       skeys, n, (const IndexHeader *)h, sel, cidx, idx->leaf_size, P, idx->nodes.as<BvhNode>(), kf,
+                       kl, (const uint32_t *)idx->cross.as<uint32_t>(), cross_cap);
     return RTD_OK;
 }
 
@@ -1050,9 +1186,8 @@ template rtd_status build_tree_sorted<uint64_t>(rtd_index *, const uint64_t *, u
 
 rtd_status ensure_side_stream(rtd_index *idx) {
     if (idx->side_stream) return RTD_OK;
-    RTD_CUDA(cudaStreamCreateWithFlags(&idx->tree_stream, cudaStreamNonBlocking));
     for (cudaEvent_t *e : {&idx->ev_fork, &idx->ev_join, &idx->ev_seed_fork, &idx->ev_seed_join,
-                           &idx->ev_sorted, &idx->ev_tree_fork, &idx->ev_tree_join})
+                           &idx->ev_sorted})
         RTD_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     // created last: its presence means every stream and event exists
     RTD_CUDA(cudaStreamCreateWithFlags(&idx->side_stream, cudaStreamNonBlocking));
