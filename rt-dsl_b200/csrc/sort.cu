@@ -9,8 +9,12 @@ namespace {
 
 constexpr int RS_BLOCK = 256;
 constexpr int RS_WARPS = RS_BLOCK / 32;
-constexpr int RS_ITEMS = 12;
-constexpr int RS_TILE = RS_BLOCK * RS_ITEMS;
+// Keys a thread of a tile: 12, or 4 while such tiles of 1,024 keys fit two
+// blocks an SM, where a pass takes as long as one block takes for its tile:
+// the build over 100 K points 113 us with 12 and 95 with 4, 300 K 115 and
+// 116, 1.8 M 243 and 310 (more count rows to read for every tile).
+constexpr int RS_ITEMS = 12, RS_ITEMS_FEW = 4;
+constexpr uint64_t RS_FEW_MAX = 148 * 2 * RS_BLOCK * RS_ITEMS_FEW;
 
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
@@ -95,32 +99,33 @@ __device__ __forceinline__ void digit_counts(const uint32_t *tcount, const uint3
     *total = t;
 }
 
-// Counts of one pass: the digit histogram of each tile of RS_TILE keys in
+// Counts of one pass: the digit histogram of each tile of keys in
 // tcount[tile][d], added into its group's row of gsum and, when there is
 // more than one super group, into its super group's row of ssum.  Each
 // warp counts its keys in a private shared row with shared-memory atomics
 // (measured faster here than ballot-matched counting).
-template <typename K>
+template <typename K, int ITEMS>
 __global__ void __launch_bounds__(RS_BLOCK) rs_count_kernel(const K *__restrict__ kin, uint64_t n,
                                                             int shift, uint32_t *__restrict__ tcount,
                                                             uint32_t *gsum, uint32_t *ssum,
                                                             int supers) {
     chain_wait();
+    constexpr int TILE = RS_BLOCK * ITEMS;
     __shared__ uint32_t s_wh[RS_WARPS][256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < RS_WARPS * 256; i += RS_BLOCK) (&s_wh[0][0])[i] = 0;
     const uint64_t tile = blockIdx.x;
-    const uint64_t wbase = tile * RS_TILE + (uint64_t)warp * RS_ITEMS * 32;
-    K key[RS_ITEMS];
+    const uint64_t wbase = tile * TILE + (uint64_t)warp * ITEMS * 32;
+    K key[ITEMS];
 #pragma unroll
-    for (int i = 0; i < RS_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint64_t idx = wbase + (uint64_t)i * 32 + lane;
         key[i] = idx < n ? kin[idx] : K(0);
     }
     __syncthreads();
     uint32_t *wh = s_wh[warp];
 #pragma unroll
-    for (int i = 0; i < RS_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const bool ok = wbase + (uint64_t)i * 32 + lane < n;
         const uint32_t dig = (uint32_t)(key[i] >> shift) & 255u;
         if (ok) atomicAdd(&wh[dig], 1u);
@@ -165,7 +170,7 @@ struct ValuePack {
 // shift32 up (a 64-bit key becoming the 32-bit key of later passes); with
 // gk_out, gk_out[dst] = gk_in[v] for the key's value v; and vout[dst] = v,
 // or with gout (the last pass) the point gxyz[v] with v in w instead.
-template <typename K>
+template <typename K, int ITEMS>
 __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     const K *__restrict__ kin, K *__restrict__ kout, const uint32_t *__restrict__ vin,
     uint32_t *__restrict__ vout, uint64_t n, int shift, const uint32_t *__restrict__ tcount,
@@ -174,10 +179,11 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     uint32_t *__restrict__ kout32, int shift32, const uint64_t *__restrict__ gk_in,
     uint64_t *__restrict__ gk_out, const ValuePack pk) {
     chain_wait();
+    constexpr int TILE = RS_BLOCK * ITEMS;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     K *s_keys = reinterpret_cast<K *>(rs_smem);
-    uint32_t *s_vals = reinterpret_cast<uint32_t *>(s_keys + RS_TILE);
-    uint32_t *s_wh = s_vals + RS_TILE;            // [RS_WARPS][256]
+    uint32_t *s_vals = reinterpret_cast<uint32_t *>(s_keys + TILE);
+    uint32_t *s_wh = s_vals + TILE;            // [RS_WARPS][256]
     uint32_t *s_excl = s_wh + RS_WARPS * 256;     // [256] tile-local digit start
     uint32_t *s_base = s_excl + 256;              // [256] global dest of local pos 0 (mod 2^32)
     uint32_t *s_misc = s_base + 256;              // [RS_WARPS + 1]
@@ -185,13 +191,13 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < RS_WARPS * 256; i += RS_BLOCK) s_wh[i] = 0;
     const uint64_t tile = blockIdx.x;
-    const uint64_t base = tile * RS_TILE;
+    const uint64_t base = tile * TILE;
 
-    K key[RS_ITEMS];
-    uint32_t val[RS_ITEMS], rank[RS_ITEMS];
-    const uint64_t wbase = base + (uint64_t)warp * RS_ITEMS * 32;
+    K key[ITEMS];
+    uint32_t val[ITEMS], rank[ITEMS];
+    const uint64_t wbase = base + (uint64_t)warp * ITEMS * 32;
 #pragma unroll
-    for (int i = 0; i < RS_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint64_t idx = wbase + (uint64_t)i * 32 + lane;
         const bool ok = idx < n;
         key[i] = ok ? kin[idx] : ~K(0);
@@ -205,7 +211,7 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     const uint32_t lt = lanemask_lt();
     uint32_t *wh = s_wh + warp * 256;
 #pragma unroll
-    for (int i = 0; i < RS_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint32_t dig = (uint32_t)(key[i] >> shift) & 255u;
         const uint32_t peers = digit_peers(dig);
         const uint32_t below = __popc(peers & lt);
@@ -230,7 +236,7 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     s_base[d] = digit_start + before - excl_local;
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < RS_ITEMS; ++i) {
+    for (int i = 0; i < ITEMS; ++i) {
         const uint32_t dig = (uint32_t)(key[i] >> shift) & 255u;
         const uint32_t lp = s_excl[dig] + s_wh[warp * 256 + dig] + rank[i];
         s_keys[lp] = key[i];
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     }
     __syncthreads();
     const uint64_t rem = n - base;
-    const uint32_t valid = rem < (uint64_t)RS_TILE ? (uint32_t)rem : (uint32_t)RS_TILE;
+    const uint32_t valid = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
     if (gout) {
         // Last pass with a gather: the points (and keys) are read at random,
         // so GATHER slots' loads are issued together before their stores.
@@ -292,17 +298,19 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     }
 }
 
-size_t rs_scatter_smem(size_t key_bytes) {
-    return RS_TILE * (key_bytes + 4) + (RS_WARPS * 256 + 512 + RS_WARPS + 1) * 4;
+size_t rs_scatter_smem(size_t key_bytes, int items) {
+    return RS_BLOCK * items * (key_bytes + 4) + (RS_WARPS * 256 + 512 + RS_WARPS + 1) * 4;
 }
 
 // Count rows for `passes` passes over n keys: every pass's tile rows, then
 // every pass's group and super rows (zeroed together: the count kernels add
 // into them).
 struct PassRows {
+    int items;   // keys a thread
     Levels L;
     uint32_t *tc = nullptr, *sc = nullptr;
-    explicit PassRows(uint64_t n) : L(ceil_div(n, RS_TILE)) {}
+    explicit PassRows(uint64_t n)
+        : items(n <= RS_FEW_MAX ? RS_ITEMS_FEW : RS_ITEMS), L(ceil_div(n, (uint64_t)RS_BLOCK * items)) {}
     rtd_status reserve(SortScratch &scr, int passes, cudaStream_t stream) {
         const size_t trows = (size_t)passes * L.tiles, srows = (size_t)passes * (L.groups + L.supers);
         RTD_TRY(scr.counts.reserve((trows + srows) * 256 * sizeof(uint32_t)));
@@ -326,23 +334,29 @@ template <typename K> struct PassOut {
 };
 
 // Count + scatter of pass p (its count rows) over bits [shift, shift + 8).
-template <typename K>
-rtd_status run_pass(const PassRows &R, int p, const K *kin, const uint32_t *vin, uint32_t *vout,
+template <typename K, int ITEMS>
+rtd_status run_pass_items(const PassRows &R, int p, const K *kin, const uint32_t *vin, uint32_t *vout,
                     uint64_t n, int shift, const PassOut<K> &o, cudaStream_t stream) {
     const Levels &L = R.L;
     uint32_t *tcount = R.tc + (size_t)p * L.tiles * 256;
     uint32_t *gsum = R.sc + (size_t)p * (L.groups + L.supers) * 256;
     uint32_t *ssum = gsum + L.groups * 256;
-    RTD_LAUNCH_CHAINED(rs_count_kernel<K>, dim3((unsigned)L.tiles), dim3(RS_BLOCK), 0, stream, kin,
-                       n, shift, tcount, gsum, ssum, (int)L.supers);
-    const size_t smem = rs_scatter_smem(sizeof(K));
-    RTD_CUDA(cudaFuncSetAttribute(rs_scatter_kernel<K>,
+    RTD_LAUNCH_CHAINED((rs_count_kernel<K, ITEMS>), dim3((unsigned)L.tiles), dim3(RS_BLOCK), 0, stream, kin, n,
+                       shift, tcount, gsum, ssum, (int)L.supers);
+    const size_t smem = rs_scatter_smem(sizeof(K), ITEMS);
+    RTD_CUDA(cudaFuncSetAttribute(rs_scatter_kernel<K, ITEMS>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    RTD_LAUNCH_CHAINED(rs_scatter_kernel<K>, dim3((unsigned)L.tiles), dim3(RS_BLOCK), smem, stream,
+    RTD_LAUNCH_CHAINED((rs_scatter_kernel<K, ITEMS>), dim3((unsigned)L.tiles), dim3(RS_BLOCK), smem, stream,
                        kin, o.kout, vin, vout, n, shift, tcount, gsum, ssum, (uint32_t)L.groups,
                        (uint32_t)L.supers, o.gxyz, o.gout, o.kout32, o.shift32, o.gk_in, o.gk_out,
                        o.pk);
     return RTD_OK;
+}
+template <typename K>
+rtd_status run_pass(const PassRows &R, int p, const K *kin, const uint32_t *vin, uint32_t *vout, uint64_t n,
+                    int shift, const PassOut<K> &o, cudaStream_t stream) {
+    return R.items == RS_ITEMS ? run_pass_items<K, RS_ITEMS>(R, p, kin, vin, vout, n, shift, o, stream)
+                               : run_pass_items<K, RS_ITEMS_FEW>(R, p, kin, vin, vout, n, shift, o, stream);
 }
 
 }  // namespace
