@@ -168,18 +168,17 @@ __global__ void __launch_bounds__(BLOCK) batch_gather_kernel(const float *__rest
 // cloud's root.
 __global__ void __launch_bounds__(BLOCK) batch_roots_kernel(
     const uint64_t *__restrict__ skeys, uint64_t n, int shift, const uint32_t *__restrict__ kfirst,
-    const uint32_t *__restrict__ klast, const uint32_t *__restrict__ flags,
-    const uint32_t *__restrict__ cidx, CloudDesc *cd) {
+    const uint32_t *__restrict__ klast, const KeptNodes kept, CloudDesc *cd) {
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i + 1 < n;
          i += (uint64_t)gridDim.x * BLOCK) {
         // only kept nodes carry their range; a cloud of <= leaf_size points
         // keeps the leaf root batch_reset_kernel gave it
-        if (!flags[i]) continue;
+        if (!kept.has((uint32_t)i)) continue;
         const uint32_t f = kfirst[i], l = klast[i];
         const uint32_t c = (uint32_t)(skeys[f] >> shift);
         const CloudDesc d = cd[c];
         if (f == d.pt_begin && l + 1 == d.pt_begin + d.n_pts) {
-            cd[c].root = cidx[i];
+            cd[c].root = kept.number((uint32_t)i);
             cd[c].root_count = d.n_pts;
         }
     }
@@ -497,7 +496,7 @@ static rtd_status batch_pass(rtd_batch *b, const float *d_pts, const float *d_q,
         if (n >= 2 && n > f.leaf_size) {
             batch_roots_kernel<<<grid_for(n, BLOCK, 148 * 8), BLOCK, 0, st>>>(
                 sk, n, 3 * b->bpa, f.kfirst.as<uint32_t>(), f.klast.as<uint32_t>(),
-                f.flags.as<uint32_t>(), f.cidx.as<uint32_t>(), cd);
+                KeptNodes{f.kept_bits.as<uint32_t>(), f.kept_before.as<uint32_t>()}, cd);
             RTD_LAUNCH_CHECK();
         }
     }

@@ -50,7 +50,17 @@ struct IndexHeader {
     // records cover; the largest count.  A pushing fill uses rcur[0].
     unsigned long long rcur[3];
     uint32_t most;
-    uint32_t n_cross;     // tree nodes whose points lie in more than one tile
+};
+
+// The Karras nodes kept in the tree, a bit each, and the kept nodes before
+// every word of 32.
+struct KeptNodes {
+    const uint32_t *bits, *before;
+    __device__ __forceinline__ bool has(uint32_t i) const { return bits[i >> 5] >> (i & 31) & 1u; }
+    // index of kept node i in the node array
+    __device__ __forceinline__ uint32_t number(uint32_t i) const {
+        return before[i >> 5] + __popc(bits[i >> 5] & ((1u << (i & 31)) - 1u));
+    }
 };
 
 constexpr int SEED_NN_SAMPLE = 4096;
@@ -82,11 +92,10 @@ struct rtd_index {
     // build scratch
     rtd::DevBuf keys, keys_alt, vals, vals_alt;
     rtd::DevBuf k32a, k32b;   // 32-bit top keys of the split sort
-    // Karras node flags (1: the node keeps more than leaf_size points),
-    // compact indices, the list of kept nodes, those whose points lie in more
-    // than one tile, and (forest builds) the kept nodes' first and last points
-    // by Karras index
-    rtd::DevBuf flags, cidx, csel, cross, kfirst, klast;
+    // kept Karras nodes (KeptNodes), their counts by tile, the list of those
+    // whose points lie in more than one tile, and (forest builds) the kept
+    // nodes' first and last points by Karras index
+    rtd::DevBuf kept_bits, kept_before, kept_counts, cross, kfirst, klast;
     rtd::DevBuf pyramid;    // run boxes over the sorted points (2 float4 per run)
     rtd::SortScratch sort;
     rtd::ScanScratch scan;
@@ -201,10 +210,11 @@ inline IndexView view_of(const rtd_index *idx) {
 // Karras tree, leaf collapse and child boxes over n keys already sorted
 // (idx->pts holds the points in key order; idx->leaf_size set).  With
 // ranges, every kept Karras node i also leaves its point range in
-// kfirst[i], klast[i] (flags[i] says which nodes are kept).
+// kfirst[i], klast[i] (KeptNodes says which are kept).  With top, the top
+// levels are staged as well and the counts are zero already (index_build).
 template <typename K>
 rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStream_t st,
-                             bool ranges = false);
+                             bool ranges = false, bool top = false);
 
 // Query ordering: Morton codes of the queries against the scene box, sorted;
 // perm[i] is the i-th query to process.  Returns perm (device) or nullptr

@@ -6,6 +6,7 @@
 // gprt-optix/host/kernels.cu:3-16: the tree holds point boxes only and the
 // search radius is applied inside the search kernels.
 #include "index.cuh"
+#include "scan.cuh"
 
 namespace rtd {
 namespace {
@@ -31,9 +32,15 @@ __device__ __forceinline__ void hdr_init(IndexHeader *h) {
     h->n_sample = 0;
 }
 
-__global__ void hdr_init_kernel(IndexHeader *h) {
+// Also zeroes the words that the kernels of a build add into: the sort's
+// count rows and the tree's counts.
+__global__ void __launch_bounds__(256) hdr_init_kernel(IndexHeader *h, uint32_t *rows, uint64_t n_rows, uint32_t *counts,
+                                                       uint32_t n_counts) {
     chain_wait();
-    hdr_init(h);
+    const uint64_t t = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    if (t == 0) hdr_init(h);
+    for (uint64_t i = t; i < n_rows; i += (uint64_t)gridDim.x * 256) rows[i] = 0u;
+    for (uint64_t i = t; i < n_counts; i += (uint64_t)gridDim.x * 256) counts[i] = 0u;
 }
 
 // Points 4g .. 4g+3 of a 16-byte aligned xyz array: three float4 loads.
@@ -155,62 +162,115 @@ __device__ __forceinline__ void karras_dir(const K *__restrict__ keys, int64_t n
 // exactly when the key leaf_size steps away in its direction still shares
 // more than the node's lower bound on the common prefix: the prefix length
 // of the (key, position) pairs, which are strictly increasing, cannot grow
-// with distance.  This kernel makes that one test per node; the range and
-// split searches run afterwards for the kept nodes alone, packed densely by
-// the scan of these flags (tile_nodes_kernel), so no warp carries idle lanes of
-// collapsed nodes through them.
-// A block takes FLAG_TILE consecutive nodes and first stages their keys
-// with a halo of leaf_size + 1 on each side in shared memory (one
-// coalesced read), so that the four keys of each test come from there.
-constexpr int FLAG_TILE = 2048;
-constexpr int FLAG_HALO = 65;   // leaf_size (<= 64) + 1
+// with distance.  keeps_node makes that one test on keys staged in shared
+// memory with a halo of leaf_size + 1 on each side (s_k[0] is the key of
+// position base).
+constexpr int NODE_TILE = 1024;   // sorted points (and Karras nodes) of a tile
+constexpr int FLAG_HALO = 65;     // leaf_size (<= 64) + 1
+// Prefixes are compared without counting zeros: of two differences from the
+// node's key the one with the lower top bit shares the longer prefix.  Equal
+// keys (ties by position) take the counts.
 template <typename K>
-__global__ void __launch_bounds__(BLOCK) karras_flag_kernel(const K *__restrict__ keys, int64_t n,
-                                                            uint32_t leaf_size, uint32_t *flags, IndexHeader *h) {
+__device__ __forceinline__ bool shares_more(K x, K y) { return x < y && x < (x ^ y); }
+
+template <typename K>
+__device__ __forceinline__ bool keeps_node(const K *s_k, int64_t base, int64_t n, int64_t i, uint32_t leaf_size) {
+    if (i == 0) return leaf_size < n;   // the root
+    const K *k = s_k + (i - base);
+    const K ki = *k, xp = ki ^ k[1], xm = ki ^ k[-1];   // (i < n - 1)
+    if (xp == 0 || xm == 0) {
+        auto dl = [&](int64_t j) -> int { return delta(s_k - base, n, ki, i, j); };
+        const int dp = dl(i + 1), dm = dl(i - 1), dir = (dp - dm) >= 0 ? 1 : -1;
+        return dl(i + (int64_t)leaf_size * dir) > (dir > 0 ? dm : dp);
+    }
+    const bool up = !shares_more(xm, xp);
+    const int64_t j = up ? i + leaf_size : i - leaf_size;
+    if (j < 0 || j >= n) return false;
+    return shares_more<K>(ki ^ k[up ? (int)leaf_size : -(int)leaf_size], up ? xm : xp);
+}
+
+// Whether the keys of a node's direction share more than its lower bound:
+// their differences from its key then have no bit of the bound's prefix or
+// the one after it.  A bound inside the ties (dmin >= the key's width) takes
+// the counts.
+template <typename K>
+struct PrefixTest {
+    K lim;
+    int dmin;
+    __device__ __forceinline__ explicit PrefixTest(int d)
+        : lim(d < 0 ? ~K(0) : d + 1 < (int)(8 * sizeof(K)) ? ~K(0) >> (d + 1) : K(0)), dmin(d) {}
+    // x: the difference of the keys at positions i and j
+    __device__ __forceinline__ bool operator()(K x, uint32_t i, uint32_t j) const {
+        if (dmin < (int)(8 * sizeof(K))) return x <= lim;
+        return x == 0 && (int)(8 * sizeof(K)) + __clz(i ^ j) > dmin;
+    }
+};
+
+// Kept nodes of every tile, added into the sums of its group (32 tiles) and
+// super group (32 groups), from which tile_nodes_kernel numbers them: the
+// numbers follow the Karras index.  A block takes COUNT_TILES tiles.
+constexpr int COUNT_TILES = 2;
+struct TreeCounts {
+    uint32_t *tiles, *groups, *supers;
+    uint32_t *cross, *done;   // nodes listed for cross_nodes_kernel; its finished blocks
+};
+template <typename K>
+__global__ void __launch_bounds__(BLOCK) karras_count_kernel(const K *__restrict__ keys, int64_t n, uint32_t leaf_size,
+                                                             uint32_t tiles, const TreeCounts tc) {
     chain_wait();
-    if (blockIdx.x == 0 && threadIdx.x == 0) h->n_cross = 0;   // (tile_nodes_kernel counts)
-    __shared__ K s_k[FLAG_TILE + 2 * FLAG_HALO];
-    const int64_t b0 = (int64_t)blockIdx.x * FLAG_TILE, base = b0 - FLAG_HALO;
-    for (int t = threadIdx.x; t < FLAG_TILE + 2 * FLAG_HALO; t += BLOCK) {
+    constexpr int SPAN = COUNT_TILES * NODE_TILE;
+    __shared__ K s_k[SPAN + 2 * FLAG_HALO];
+    __shared__ uint32_t s_cnt[COUNT_TILES];
+    const int64_t b0 = (int64_t)blockIdx.x * SPAN, base = b0 - FLAG_HALO;
+    for (int t = threadIdx.x; t < SPAN + 2 * FLAG_HALO; t += BLOCK) {
         const int64_t j = base + t;
         if (j >= 0 && j < n) s_k[t] = keys[j];
     }
+    if (threadIdx.x < COUNT_TILES) s_cnt[threadIdx.x] = 0;
     __syncthreads();
-    // delta on the staged keys (j within the halo whenever j is in [0, n))
-    auto dl = [&](K ki, int64_t i, int64_t j) -> int {
-        if (j < 0 || j >= n) return -1;
-        const K b = s_k[j - base];
-        if (ki == b) return (int)(8 * sizeof(K)) + __clz((uint32_t)(i ^ j));
-        return sizeof(K) == 8 ? __clzll((unsigned long long)(ki ^ b)) : __clz((uint32_t)(ki ^ b));
-    };
-    for (int t = threadIdx.x; t < FLAG_TILE; t += BLOCK) {
-        const int64_t i = b0 + t;
-        if (i >= n - 1) break;
-        const K ki = s_k[i - base];
-        const int dir = (dl(ki, i, i + 1) - dl(ki, i, i - 1)) >= 0 ? 1 : -1;
-        const int dmin = dl(ki, i, i - dir);
-        flags[i] = dl(ki, i, i + (int64_t)leaf_size * dir) > dmin ? 1u : 0u;
+    for (int u = 0; u < COUNT_TILES; ++u) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int t = 0; t < NODE_TILE; t += BLOCK) {
+            const int64_t i = b0 + u * NODE_TILE + t + (int)threadIdx.x;
+            c += __popc(__ballot_sync(0xffffffffu, i < n - 1 && keeps_node<K>(s_k, base, n, i, leaf_size)));
+        }
+        if ((threadIdx.x & 31) == 0) atomicAdd(&s_cnt[u], c);
+    }
+    __syncthreads();
+    const uint32_t tile = blockIdx.x * COUNT_TILES + threadIdx.x;
+    if (threadIdx.x < COUNT_TILES && tile < tiles) {
+        const uint32_t c = s_cnt[threadIdx.x];
+        tc.tiles[tile] = c;
+        if (c) {
+            atomicAdd(&tc.groups[tile / GROUP_TILES], c);
+            atomicAdd(&tc.supers[tile / SUPER_TILES], c);
+        }
     }
 }
 
-// Point range [first, last] and split of the kept Karras node at local
-// position i, whose range holds at most `room` points after i in direction
-// dir: the children hold [first, split] and [split + 1, last].  dl(j): the
-// common prefix with the key at local position j.  REACH: a power of two
-// above the longest range.
-template <int REACH, typename Delta>
-__device__ __forceinline__ void karras_range(const Delta &dl, int i, int dir, int dmin, int room, uint32_t &first,
-                                             uint32_t &last, uint32_t &split) {
+// Point range [first, last] and split of the kept Karras node at position i,
+// whose range holds at most `room` points after i in direction dir: the
+// children hold [first, split] and [split + 1, last].  k: the keys, at
+// positions base and up.  REACH: a power of two above the longest range.
+template <int REACH, typename K>
+__device__ __forceinline__ void karras_range(const K *k, uint32_t base, int i, int dir, int dmin, int room,
+                                             uint32_t &first, uint32_t &last, uint32_t &split) {
+    const K ki = k[i];
+    auto more = [&](int j, const PrefixTest<K> &t) { return t(ki ^ k[j], base + i, base + j); };
+    const PrefixTest<K> in(dmin);
     int l = 0;
 #pragma unroll 1
     for (int t = REACH / 2; t >= 1; t >>= 1)
-        if (l + t <= room && dl(i + (l + t) * dir) > dmin) l += t;
-    const int dnode = dl(i + l * dir);
+        if (l + t <= room && more(i + (l + t) * dir, in)) l += t;
+    const K x = ki ^ k[i + l * dir];
+    const PrefixTest<K> left(x == 0 ? (int)(8 * sizeof(K)) + __clz((base + i) ^ (base + i + l * dir))
+                                    : sizeof(K) == 8 ? __clzll((unsigned long long)x) : __clz((uint32_t)x));
     int s = 0, t = l;
 #pragma unroll 1
     do {
         t = (t + 1) >> 1;
-        if (s + t < l && dl(i + (s + t) * dir) > dnode) s += t;
+        if (s + t < l && more(i + (s + t) * dir, left)) s += t;
     } while (t > 1);
     split = (uint32_t)(i + s * dir + (dir < 0 ? -1 : 0));
     first = (uint32_t)(dir > 0 ? i : i - l);
@@ -385,8 +445,10 @@ __device__ __noinline__ Box range_box(const float4 *pts, const float4 *pyr, uint
 
 // The node of the points [f0, last] with children [f0, sp] and [sp + 1, last]:
 // Karras nodes sp and sp + 1 when they keep more than leaf_size points, else
-// leaves.  The positions count from base.
-__device__ __forceinline__ BvhNode pack_node(const uint32_t *cidx, uint32_t leaf_size, uint32_t f0, uint32_t last,
+// leaves.  The positions count from base; number(i) is the index of kept
+// Karras node i.
+template <typename Number>
+__device__ __forceinline__ BvhNode pack_node(const Number &number, uint32_t leaf_size, uint32_t f0, uint32_t last,
                                              uint32_t sp, uint32_t base, const Box &b0, const Box &b1) {
     const uint32_t c0 = sp - f0 + 1, c1 = last - sp;
     BvhNode nd;
@@ -394,15 +456,16 @@ __device__ __forceinline__ BvhNode pack_node(const uint32_t *cidx, uint32_t leaf
     nd.a = make_float4(b0.lo[0], b0.lo[1], b0.lo[2], b0.hi[0]);
     nd.b = make_float4(b0.hi[1], b0.hi[2], b1.lo[0], b1.lo[1]);
     nd.c = make_float4(b1.lo[2], b1.hi[0], b1.hi[1], b1.hi[2]);
-    nd.d = make_uint4(c0 > leaf_size ? cidx[base + sp] : (CHILD_LEAF | (base + f0)),
-                      c1 > leaf_size ? cidx[base + sp + 1] : (CHILD_LEAF | (base + sp + 1)), c0, c1);
+    nd.d = make_uint4(c0 > leaf_size ? number(base + sp) : (CHILD_LEAF | (base + f0)),
+                      c1 > leaf_size ? number(base + sp + 1) : (CHILD_LEAF | (base + sp + 1)), c0, c1);
     return nd;
 }
-__device__ __forceinline__ BvhNode make_node(const Pyramid &P, const uint32_t *cidx, uint32_t leaf_size, uint32_t f0,
+template <typename Number>
+__device__ __forceinline__ BvhNode make_node(const Pyramid &P, const Number &number, uint32_t leaf_size, uint32_t f0,
                                              uint32_t last, uint32_t sp, uint32_t base) {
     const Box b0 = range_box(P.pts, P.pyr, P.n, P.nlev, f0, sp - f0 + 1);
     const Box b1 = range_box(P.pts, P.pyr, P.n, P.nlev, sp + 1, last - sp);
-    return pack_node(cidx, leaf_size, f0, last, sp, base, b0, b1);
+    return pack_node(number, leaf_size, f0, last, sp, base, b0, b1);
 }
 
 // Compact nodes: children become leaves when their subtree has <= leaf_size
@@ -415,33 +478,37 @@ __device__ __forceinline__ BvhNode make_node(const Pyramid &P, const uint32_t *c
 //
 // tile_nodes_kernel: a block takes NODE_TILE sorted points.  It stages their
 // keys and points in shared memory, folds levels 1 to 3 of the pyramid there
-// (and writes them out), and makes the nodes whose points all lie in the
-// tile, a thread a node: all but about one in ten.  The searches for a node's
-// range and split and the walk of its boxes are chains of dependent reads,
-// which is why they run on shared memory.  A node's prefix with the keys of
-// its direction cannot grow with distance, so its range ends inside the tile
-// exactly when the first key past the tile no longer exceeds its lower bound;
-// the others are listed in `cross` for cross_nodes_kernel.  Bound by the
-// issue slots of the searches and box walks (half of them used; ~12,000 warp
-// instructions a tile).  With global searches a thread a node the nodes of
-// 100 K points took 34 us (51 dependent reads at the root), now 18 + 11;
-// those of 10 M 454 us, with the pyramid's own 79, now 330 + 84.
-constexpr int NODE_TILE = 1024;
+// (and writes them out), numbers its kept nodes, and makes those whose points
+// all lie in the tile, a thread a node: all but about one in ten.  The
+// searches for a node's range and split and the walk of its boxes are chains
+// of dependent reads, which is why they run on shared memory.  A node's prefix
+// with the keys of its direction cannot grow with distance, so its range ends
+// inside the tile exactly when the first key past the tile no longer exceeds
+// its lower bound; the others are listed in `cross` for cross_nodes_kernel.
+// Bound by the issue slots of the searches and box walks.  With flags, their
+// scan, a list of the kept nodes and global searches a thread a node, the tree
+// of 100 K points took 50 us (51 dependent reads at the root), now 40; that of
+// 10 M 575 us besides the pyramid's 79, now 535 with it.
 constexpr int NODE_DEPTH = 96;   // prefix lengths of (key, position) pairs: nodes that share a tile boundary are nested
 template <typename K>
 __global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
-    const K *__restrict__ keys, uint64_t n, IndexHeader *h, const uint32_t *__restrict__ sel,
-    const uint32_t *__restrict__ cidx, uint32_t leaf_size, const float4 *__restrict__ pts, float4 *lv1, float4 *lv2,
-    float4 *lv3, BvhNode *nodes, uint32_t *kfirst, uint32_t *klast, uint32_t *cross, uint32_t cross_cap) {
+    const K *__restrict__ keys, uint64_t n, IndexHeader *h, const TreeCounts tc, uint32_t *bits, uint32_t *before,
+    uint32_t leaf_size, const float4 *__restrict__ pts, float4 *lv1, float4 *lv2, float4 *lv3, BvhNode *nodes,
+    uint32_t *kfirst, uint32_t *klast, uint32_t *cross, uint32_t cross_cap) {
     chain_wait();
-    __shared__ K s_k[NODE_TILE + 2];
+    __shared__ K s_k[NODE_TILE + 2 * FLAG_HALO];
     __shared__ float4 s_p[NODE_TILE];
     __shared__ float4 s_pyr[2 * (NODE_TILE / 8 + NODE_TILE / 64 + NODE_TILE / 512)];
-    const int64_t b0 = (int64_t)blockIdx.x * NODE_TILE;
+    __shared__ uint32_t s_bits[NODE_TILE / 32], s_before[NODE_TILE / 32], s_kept, s_prefix;
+    __shared__ uint16_t s_list[NODE_TILE];
+    static_assert(NODE_TILE == 32 * 32, "a warp numbers the words of a tile");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t tile = blockIdx.x;
+    const int64_t b0 = (int64_t)tile * NODE_TILE, base_k = b0 - FLAG_HALO;
     const uint32_t m = (uint32_t)(n - b0 < NODE_TILE ? n - b0 : NODE_TILE);
     const uint32_t n1 = (m + 7) / 8, n2 = (n1 + 7) / 8, n3 = (n2 + 7) / 8;
-    for (uint32_t t = threadIdx.x; t < NODE_TILE + 2; t += BLOCK) {
-        const int64_t j = b0 + (int64_t)t - 1;
+    for (uint32_t t = threadIdx.x; t < NODE_TILE + 2 * FLAG_HALO; t += BLOCK) {
+        const int64_t j = base_k + (int64_t)t;
         if (j >= 0 && j < (int64_t)n) s_k[t] = keys[j];
     }
     // level 1: the 8 lanes of an entry
@@ -464,6 +531,14 @@ __global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
         }
     }
     __syncthreads();
+    // which nodes are kept
+#pragma unroll
+    for (int t = 0; t < NODE_TILE; t += BLOCK) {
+        const int li = t + (int)threadIdx.x;
+        const uint32_t w = __ballot_sync(
+            0xffffffffu, b0 + li < (int64_t)n - 1 && keeps_node<K>(s_k, base_k, (int64_t)n, b0 + li, leaf_size));
+        if (lane == 0) s_bits[li >> 5] = w;
+    }
     // levels 2 and 3
     for (int lev = 2; lev <= 3; ++lev) {
         const float4 *in = lev == 2 ? s_pyr : s_pyr + 2 * n1;
@@ -483,53 +558,144 @@ __global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
     P.pyr = s_pyr;
     P.n = m;
     P.nlev = 3;
-    const uint32_t n_int = h->n_internal;
-    const uint32_t c0 = b0 < (int64_t)n - 1 ? cidx[b0] : n_int;
-    const uint32_t c1 = b0 + NODE_TILE < (int64_t)n - 1 ? cidx[b0 + NODE_TILE] : n_int;
-    for (uint32_t c = c0 + threadIdx.x; c < c1; c += BLOCK) {
-        const uint32_t i = sel[c];
-        const int li = (int)(i - (uint32_t)b0);
-        const K ki = s_k[li + 1];
+    // their numbers: those of the earlier tiles, then a scan over the words
+    if (warp == 0) {
+        const uint32_t c = __popc(s_bits[lane]);
+        uint32_t x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_before[lane] = x - c;
+        if (lane == 31) s_kept = x;
+    } else if (warp == 1) {
+        const uint32_t g = tile / GROUP_TILES, sg = tile / SUPER_TILES;
+        uint32_t v = 0;
+        if ((uint32_t)lane < tile % GROUP_TILES) v += tc.tiles[g * GROUP_TILES + lane];
+        if ((uint32_t)lane < g % 32) v += tc.groups[sg * 32 + lane];
+        for (uint32_t j = lane; j < sg; j += 32) v += tc.supers[j];
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0) s_prefix = v;
+    }
+    __syncthreads();
+    const uint32_t prefix = s_prefix, kept = s_kept;
+    if (warp == 0) {
+        const uint64_t w = (uint64_t)b0 / 32 + lane;
+        if (w * 32 < n) {
+            bits[w] = s_bits[lane];
+            before[w] = prefix + s_before[lane];
+        }
+        if (lane == 0 && (uint64_t)b0 + NODE_TILE >= n) h->n_internal = prefix + kept;
+    }
+#pragma unroll
+    for (int t = 0; t < NODE_TILE; t += BLOCK) {
+        const uint32_t li = t + threadIdx.x, w = s_bits[li >> 5];
+        if (w >> lane & 1u) s_list[s_before[li >> 5] + __popc(w & ((1u << lane) - 1u))] = (uint16_t)li;
+    }
+    __syncthreads();
+    const uint32_t base = (uint32_t)b0;
+    auto number = [&](uint32_t i) {   // (a node of the tile)
+        const uint32_t w = (i - base) >> 5;
+        return prefix + s_before[w] + __popc(s_bits[w] & ((1u << (i & 31)) - 1u));
+    };
+    for (uint32_t c = threadIdx.x; c < kept; c += BLOCK) {
+        const int li = s_list[c];
+        const uint32_t i = base + li;
+        const K ki = s_k[li + FLAG_HALO];
         auto dl = [&](int lj) -> int {   // lj in [-1, NODE_TILE]
             const int64_t j = b0 + lj;
             if (j < 0 || j >= (int64_t)n) return -1;
-            const K b = s_k[lj + 1];
+            const K b = s_k[lj + FLAG_HALO];
             if (ki == b) return (int)(8 * sizeof(K)) + __clz(i ^ (uint32_t)j);
             return sizeof(K) == 8 ? __clzll((unsigned long long)(ki ^ b)) : __clz((uint32_t)(ki ^ b));
         };
         const int dp = dl(li + 1), dm = dl(li - 1), dir = (dp - dm) >= 0 ? 1 : -1, dmin = dir > 0 ? dm : dp;
         if (dl(dir > 0 ? NODE_TILE : -1) > dmin) {
-            const uint32_t at = atomicAdd(&h->n_cross, 1u);
-            if (at < cross_cap) cross[at] = c;
+            const uint32_t at = atomicAdd(tc.cross, 1u);
+            if (at < cross_cap) cross[at] = i;
             else atomicOr(&h->err, DEVERR_OVERFLOW);
             continue;
         }
         uint32_t f0, last, sp;
-        karras_range<NODE_TILE>(dl, li, dir, dmin, dir > 0 ? NODE_TILE - 1 - li : li, f0, last, sp);
-        const uint32_t base = (uint32_t)b0;
+        karras_range<NODE_TILE>(s_k + FLAG_HALO, base, li, dir, dmin,
+                                dir > 0 ? (int)m - 1 - li : li, f0, last, sp);
         if (kfirst) {
             kfirst[i] = base + f0;
             klast[i] = base + last;
         }
-        nodes[c] = make_node(P, cidx, leaf_size, f0, last, sp, base);
+        nodes[prefix + c] = make_node(P, number, leaf_size, f0, last, sp, base);
+    }
+}
+
+// Root word and the breadth-first top levels, copied into `top`.  One warp:
+// each level's nodes are loaded in parallel (level TOP_LEVELS-1 has at most
+// 32 nodes) and their internal children are placed by a warp prefix sum.
+// s_q: TOP_MAX words of shared memory.
+__device__ __forceinline__ void stage_top(IndexHeader *h, const BvhNode *nodes, BvhNode *top, uint64_t n,
+                                          uint32_t leaf_size, uint32_t *s_q) {
+    const int lane = threadIdx.x & 31;
+    if (n == 0 || n == 1 || n <= leaf_size) {
+        if (lane == 0) {
+            h->root = n == 0 ? CHILD_NONE : (CHILD_LEAF | 0u);
+            h->root_count = (uint32_t)n;
+            h->n_top = 0;
+        }
+        return;
+    }
+    if (lane == 0) s_q[0] = 0;
+    __syncwarp();
+    int begin = 0, end = 1;
+    for (int depth = 0; depth < TOP_LEVELS; ++depth) {
+        const int i = begin + lane;
+        const bool has = i < end;
+        BvhNode nd;
+        if (has) nd = nodes[s_q[i]];
+        const bool deeper = depth + 1 < TOP_LEVELS;
+        const bool c0 = has && deeper && !(nd.d.x & CHILD_LEAF);
+        const bool c1 = has && deeper && !(nd.d.y & CHILD_LEAF);
+        const uint32_t cnt = (uint32_t)c0 + (uint32_t)c1;
+        uint32_t incl = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        const uint32_t pos = (uint32_t)end + incl - cnt;
+        if (c0) s_q[pos] = nd.d.x;
+        if (c1) s_q[pos + (c0 ? 1u : 0u)] = nd.d.y;
+        if (has) {
+            if (c0) nd.d.x = CHILD_TOP | pos;
+            if (c1) nd.d.y = CHILD_TOP | (pos + (c0 ? 1u : 0u));
+            top[i] = nd;
+        }
+        __syncwarp();
+        begin = end;
+        end += (int)total;
+        if (total == 0) break;
+    }
+    if (lane == 0) {
+        h->root = CHILD_TOP | 0u;
+        h->n_top = (uint32_t)end;
     }
 }
 
 // The nodes whose points lie in more than one tile, a warp a node: the range
 // and the split are found 32 probes at a time (an end among n keys takes
 // log32 n dependent reads), and the lanes of a half warp read the entries of
-// one child's box at each level of the pyramid together.
+// one child's box at each level of the pyramid together.  The last block
+// stages the top levels (with top non-null).
 template <typename K>
 __global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
-    const K *__restrict__ keys, uint64_t n, const IndexHeader *h, const uint32_t *__restrict__ sel,
-    const uint32_t *__restrict__ cidx, uint32_t leaf_size, const Pyramid P, BvhNode *nodes, uint32_t *kfirst,
-    uint32_t *klast, const uint32_t *__restrict__ cross, uint32_t cross_cap) {
+    const K *__restrict__ keys, uint64_t n, IndexHeader *h, const TreeCounts tc, const KeptNodes kept,
+    uint32_t leaf_size, const Pyramid P, BvhNode *nodes, uint32_t *kfirst, uint32_t *klast,
+    const uint32_t *__restrict__ cross, uint32_t cross_cap, BvhNode *top) {
     chain_wait();
-    const uint32_t count = h->n_cross < cross_cap ? h->n_cross : cross_cap;
+    const uint32_t count = *tc.cross < cross_cap ? *tc.cross : cross_cap;
     const int lane = threadIdx.x & 31;
+    auto number = [&](uint32_t i) { return kept.number(i); };
     for (uint32_t w = (blockIdx.x * BLOCK + threadIdx.x) >> 5; w < count; w += (gridDim.x * BLOCK) >> 5) {
-        const uint32_t c = cross[w];
-        const int64_t i = sel[c];
+        const int64_t i = cross[w];
         const K ki = keys[i];
         int dir, dmin;
         karras_dir(keys, (int64_t)n, ki, i, dir, dmin);
@@ -588,72 +754,24 @@ __global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
             b1.hi[x] = __shfl_sync(0xffffffffu, b.hi[x], 16);
         }
         if (lane == 0) {
-            nodes[c] = pack_node(cidx, leaf_size, f0, last, sp, 0u, b, b1);
+            nodes[number((uint32_t)i)] = pack_node(number, leaf_size, f0, last, sp, 0u, b, b1);
             if (kfirst) {
                 kfirst[i] = f0;
                 klast[i] = last;
             }
         }
     }
-}
-
-// Root word and the breadth-first top levels, copied into `top`.  One warp:
-// each level's nodes are loaded in parallel (level TOP_LEVELS-1 has at most
-// 32 nodes) and their internal children are placed by a warp prefix sum.
-// s_q: TOP_MAX words of shared memory.
-__device__ __forceinline__ void stage_top(IndexHeader *h, const BvhNode *nodes, BvhNode *top, uint64_t n,
-                                          uint32_t leaf_size, uint32_t *s_q) {
-    const int lane = threadIdx.x & 31;
-    if (n == 0 || n == 1 || n <= leaf_size) {
-        if (lane == 0) {
-            h->root = n == 0 ? CHILD_NONE : (CHILD_LEAF | 0u);
-            h->root_count = (uint32_t)n;
-            h->n_top = 0;
-        }
-        return;
-    }
-    if (lane == 0) s_q[0] = 0;
-    __syncwarp();
-    int begin = 0, end = 1;
-    for (int depth = 0; depth < TOP_LEVELS; ++depth) {
-        const int i = begin + lane;
-        const bool has = i < end;
-        BvhNode nd;
-        if (has) nd = nodes[s_q[i]];
-        const bool deeper = depth + 1 < TOP_LEVELS;
-        const bool c0 = has && deeper && !(nd.d.x & CHILD_LEAF);
-        const bool c1 = has && deeper && !(nd.d.y & CHILD_LEAF);
-        const uint32_t cnt = (uint32_t)c0 + (uint32_t)c1;
-        uint32_t incl = cnt;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        const uint32_t pos = (uint32_t)end + incl - cnt;
-        if (c0) s_q[pos] = nd.d.x;
-        if (c1) s_q[pos + (c0 ? 1u : 0u)] = nd.d.y;
-        if (has) {
-            if (c0) nd.d.x = CHILD_TOP | pos;
-            if (c1) nd.d.y = CHILD_TOP | (pos + (c0 ? 1u : 0u));
-            top[i] = nd;
-        }
-        __syncwarp();
-        begin = end;
-        end += (int)total;
-        if (total == 0) break;
-    }
-    if (lane == 0) {
-        h->root = CHILD_TOP | 0u;
-        h->n_top = (uint32_t)end;
-    }
-}
-
-__global__ void __launch_bounds__(32) stage_top_kernel(IndexHeader *h, const BvhNode *nodes, BvhNode *top, uint64_t n,
-                                                       uint32_t leaf_size) {
-    chain_wait();
+    if (!top) return;
+    __shared__ bool s_last;
     __shared__ uint32_t s_q[TOP_MAX];
-    stage_top(h, nodes, top, n, leaf_size, s_q);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();   // (cumulative over the block's stores, ordered by the barrier)
+        s_last = atomicAdd(tc.done, 1u) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last && threadIdx.x < 32) stage_top(h, nodes, top, n, leaf_size, s_q);
 }
 
 // ------------------------------------------------ radius-seed sample data
@@ -993,7 +1111,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_build_kernel(const float 
             ++Py.nlev;
             __syncthreads();
         }
-        // kept nodes (karras_flag_kernel's test), numbered in order
+        // kept nodes (keeps_node's test), numbered in order
         bool keep[E];
 #pragma unroll
         for (int u = 0; u < E; ++u) {
@@ -1040,11 +1158,10 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_build_kernel(const float 
             uint32_t f0, last, sp;
             const int i = (int)s.sel[c];
             const uint64_t ki = s.key[i];
-            auto dl = [&](int j) -> int { return delta(s.key, (int64_t)n, ki, i, j); };
             int dir, dmin;
             karras_dir(s.key, (int64_t)n, ki, i, dir, dmin);
-            karras_range<SMALL_MAX>(dl, i, dir, dmin, dir > 0 ? (int)n - 1 - i : i, f0, last, sp);
-            nodes[c] = make_node(Py, s.cidx, leaf_size, f0, last, sp, 0u);
+            karras_range<SMALL_MAX>(s.key, 0u, i, dir, dmin, dir > 0 ? (int)n - 1 - i : i, f0, last, sp);
+            nodes[c] = make_node(Py, [&](uint32_t j) { return s.cidx[j]; }, leaf_size, f0, last, sp, 0u);
         }
         __syncthreads();
     }
@@ -1105,36 +1222,53 @@ rtd_status build_typed(rtd_index *idx, const float *d_xyz, uint64_t n, cudaStrea
                                    idx->keys_alt.as<uint64_t>(), idx->k32a.as<uint32_t>(),
                                    idx->k32b.as<uint32_t>(), idx->vals.as<uint32_t>(),
                                    idx->vals_alt.as<uint32_t>(), n, kbits, idx->sort, st, d_xyz,
-                                   idx->pts.as<float4>(), idx->keys_alt.as<uint64_t>()));
+                                   idx->pts.as<float4>(), idx->keys_alt.as<uint64_t>(), nullptr, true));
         skeys = idx->keys_alt.as<K>();
     } else {
         bool in_alt = false;
         RTD_TRY(radix_sort_pairs<K>(idx->keys.as<K>(), idx->keys_alt.as<K>(),
                                     idx->vals.as<uint32_t>(), idx->vals_alt.as<uint32_t>(), true, n,
                                     0, kbits, idx->sort, d_err, st, &in_alt, d_xyz,
-                                    idx->pts.as<float4>()));
+                                    idx->pts.as<float4>(), true));
         skeys = in_alt ? idx->keys_alt.as<K>() : idx->keys.as<K>();
     }
     idx->skeys = skeys;
     idx->mark(EV_BUILD_SORTED, st);
     // the sorted keys are ready: side-stream work may wait on this
     if (idx->ev_sorted) RTD_CUDA(cudaEventRecord(idx->ev_sorted, st));
-    return build_tree_sorted<K>(idx, skeys, n, st);
+    return build_tree_sorted<K>(idx, skeys, n, st, false, true);
 }
 
 }  // namespace
 
+// The counts of the kept nodes: the words before the tiles' are added into
+// and must be zero when the build of the tree starts.
+static rtd_status tree_counts(rtd_index *idx, uint64_t n, TreeCounts &tc, uint32_t &n_zero) {
+    const Levels L(ceil_div(n, (uint64_t)NODE_TILE));
+    RTD_TRY(idx->kept_counts.reserve((2 + L.groups + L.supers + L.tiles) * sizeof(uint32_t)));
+    tc.cross = idx->kept_counts.as<uint32_t>();
+    tc.done = tc.cross + 1;
+    tc.groups = tc.cross + 2;
+    tc.supers = tc.groups + L.groups;
+    tc.tiles = tc.supers + L.supers;
+    n_zero = (uint32_t)(2 + L.groups + L.supers);
+    return RTD_OK;
+}
+
 // Karras tree, leaf collapse and child boxes over keys already sorted, with
-// idx->pts holding the points in key order.
+// idx->pts holding the points in key order.  top: stages the top levels too,
+// and the counts are zero already (index_build).
 template <typename K>
 rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStream_t st,
-                             bool ranges) {
+                             bool ranges, bool top) {
     IndexHeader *h = idx->hdr.as<IndexHeader>();
-    uint32_t *d_err = &h->err;
     if (n < 2 || n <= idx->leaf_size) return RTD_OK;
     const uint64_t ni = n - 1;
-    for (rtd::DevBuf *b : {&idx->flags, &idx->cidx, &idx->csel})
-        RTD_TRY(b->reserve(ni * sizeof(uint32_t)));
+    TreeCounts tc;
+    uint32_t n_zero;
+    RTD_TRY(tree_counts(idx, n, tc, n_zero));
+    if (!top) RTD_TRY(zero_words(tc.cross, n_zero, st));
+    for (rtd::DevBuf *b : {&idx->kept_bits, &idx->kept_before}) RTD_TRY(b->reserve(ceil_div(n, 32) * sizeof(uint32_t)));
     if (ranges)
         for (rtd::DevBuf *b : {&idx->kfirst, &idx->klast}) RTD_TRY(b->reserve(ni * sizeof(uint32_t)));
     // box pyramid over the sorted points (levels until one has <= 8 entries)
@@ -1158,13 +1292,11 @@ rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStr
     const uint64_t tiles = ceil_div(n, (uint64_t)NODE_TILE);
     const uint32_t cross_cap = (uint32_t)(ni < NODE_DEPTH * tiles ? ni : NODE_DEPTH * tiles);
     RTD_TRY(idx->cross.reserve(cross_cap * sizeof(uint32_t)));
-    RTD_LAUNCH_CHAINED(karras_flag_kernel<K>, dim3((unsigned)ceil_div(ni, (uint64_t)FLAG_TILE)), dim3(BLOCK), 0, st,
-                       skeys, (int64_t)n, idx->leaf_size, idx->flags.as<uint32_t>(), h);
-    RTD_TRY(exclusive_scan_select_u32(idx->flags.as<uint32_t>(), idx->cidx.as<uint32_t>(), idx->csel.as<uint32_t>(),
-                                      ni, &h->n_internal, idx->scan, d_err, st));
+    RTD_LAUNCH_CHAINED(karras_count_kernel<K>, dim3((unsigned)ceil_div(tiles, (uint64_t)COUNT_TILES)), dim3(BLOCK), 0,
+                       st, skeys, (int64_t)n, idx->leaf_size, (uint32_t)tiles, tc);
     uint32_t *kf = ranges ? idx->kfirst.as<uint32_t>() : nullptr, *kl = ranges ? idx->klast.as<uint32_t>() : nullptr;
-    const uint32_t *sel = idx->csel.as<uint32_t>(), *cidx = idx->cidx.as<uint32_t>();
-    RTD_LAUNCH_CHAINED(tile_nodes_kernel<K>, dim3((unsigned)tiles), dim3(BLOCK), 0, st, skeys, n, h, sel, cidx,
+    uint32_t *bits = idx->kept_bits.as<uint32_t>(), *before = idx->kept_before.as<uint32_t>();
+    RTD_LAUNCH_CHAINED(tile_nodes_kernel<K>, dim3((unsigned)tiles), dim3(BLOCK), 0, st, skeys, n, h, tc, bits, before,
                        idx->leaf_size, (const float4 *)P.pts, lv[1], lv[2], lv[3], idx->nodes.as<BvhNode>(), kf, kl,
                        idx->cross.as<uint32_t>(), cross_cap);
     // three levels of the pyramid per launch: 4-6 from level 3, ...
@@ -1174,15 +1306,16 @@ rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStr
                            j + 2 <= nlev ? lv[j + 2] : nullptr);
     // (a warp a node, for about 8 nodes a tile)
     RTD_LAUNCH_CHAINED(cross_nodes_kernel<K>, dim3((unsigned)(tiles < 148 * 8 ? tiles : 148 * 8)), dim3(BLOCK), 0, st,
-                       skeys, n, (const IndexHeader *)h, sel, cidx, idx->leaf_size, P, idx->nodes.as<BvhNode>(), kf,
-                       kl, (const uint32_t *)idx->cross.as<uint32_t>(), cross_cap);
+                       skeys, n, h, tc, KeptNodes{bits, before}, idx->leaf_size, P, idx->nodes.as<BvhNode>(), kf, kl,
+                       (const uint32_t *)idx->cross.as<uint32_t>(), cross_cap,
+                       top ? idx->top.as<BvhNode>() : nullptr);
     return RTD_OK;
 }
 
 template rtd_status build_tree_sorted<uint32_t>(rtd_index *, const uint32_t *, uint64_t,
-                                                cudaStream_t, bool);
+                                                cudaStream_t, bool, bool);
 template rtd_status build_tree_sorted<uint64_t>(rtd_index *, const uint64_t *, uint64_t,
-                                                cudaStream_t, bool);
+                                                cudaStream_t, bool, bool);
 
 rtd_status ensure_side_stream(rtd_index *idx) {
     if (idx->side_stream) return RTD_OK;
@@ -1226,7 +1359,15 @@ rtd_status index_build(rtd_index *idx, const float *d_xyz, uint64_t n, const rtd
     if (n > 0 && n <= SMALL_MAX)
         return mb == 30 ? build_small<uint32_t>(idx, d_xyz, (uint32_t)n, st)
                         : build_small<uint64_t>(idx, d_xyz, (uint32_t)n, st);
-    RTD_LAUNCH_CHAINED(hdr_init_kernel, dim3(1), dim3(1), 0, st, h);
+    uint32_t *rows = nullptr, n_counts = 0;
+    uint64_t n_rows = 0;
+    TreeCounts tc{};
+    if (n > 0) {
+        RTD_TRY(radix_sort_sums(n, mb, idx->sort, &rows, &n_rows));
+        RTD_TRY(tree_counts(idx, n, tc, n_counts));
+    }
+    RTD_LAUNCH_CHAINED(hdr_init_kernel, dim3(n_rows ? grid_for(n_rows, 256, 148 * 4) : 1), dim3(256), 0, st, h, rows,
+                       n_rows, tc.cross, n_counts);
     if (n > 0) {
         RTD_LAUNCH_CHAINED(bbox_kernel, dim3(grid_for(n, BLOCK, 148 * 4)), dim3(BLOCK), 0, st, d_xyz,
                            n, h, aligned16(d_xyz));
@@ -1243,9 +1384,6 @@ rtd_status index_build(rtd_index *idx, const float *d_xyz, uint64_t n, const rtd
         RTD_TRY(rs);
         RTD_TRY(rb);
     }
-    RTD_LAUNCH_CHAINED(stage_top_kernel, dim3(1), dim3(32), 0, st, h,
-                       (const BvhNode *)idx->nodes.as<BvhNode>(), idx->top.as<BvhNode>(), n,
-                       idx->leaf_size);
     idx->mark(EV_BUILD1, st);
     return RTD_OK;
 }
@@ -1305,7 +1443,7 @@ rtd_status order_queries_own(QueryOrderScratch &qs, const float *d_q, uint64_t n
     RTD_TRY(qs.perm.reserve(nq * 4));
     RTD_TRY(qs.perm_alt.reserve(nq * 4));
     IndexHeader *h = qs.hdr.as<IndexHeader>();
-    hdr_init_kernel<<<1, 1, 0, st>>>(h);
+    hdr_init_kernel<<<1, 256, 0, st>>>(h, nullptr, 0, nullptr, 0);
     RTD_LAUNCH_CHECK();
     bbox_kernel<<<grid_for(nq, BLOCK, 148 * 4), BLOCK, 0, st>>>(d_q, nq, h, aligned16(d_q));
     RTD_LAUNCH_CHECK();

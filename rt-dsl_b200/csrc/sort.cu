@@ -311,13 +311,18 @@ struct PassRows {
     uint32_t *tc = nullptr, *sc = nullptr;
     explicit PassRows(uint64_t n)
         : items(n <= RS_FEW_MAX ? RS_ITEMS_FEW : RS_ITEMS), L(ceil_div(n, (uint64_t)RS_BLOCK * items)) {}
-    rtd_status reserve(SortScratch &scr, int passes, cudaStream_t stream) {
+    uint64_t sums = 0;   // words at sc
+    rtd_status reserve(SortScratch &scr, int passes) {
         const size_t trows = (size_t)passes * L.tiles, srows = (size_t)passes * (L.groups + L.supers);
         RTD_TRY(scr.counts.reserve((trows + srows) * 256 * sizeof(uint32_t)));
         tc = scr.counts.as<uint32_t>();
         sc = tc + trows * 256;
-        RTD_TRY(zero_words(sc, srows * 256, stream));
+        sums = srows * 256;
         return RTD_OK;
+    }
+    rtd_status reserve(SortScratch &scr, int passes, bool zeroed, cudaStream_t stream) {
+        RTD_TRY(reserve(scr, passes));
+        return zeroed ? RTD_OK : zero_words(sc, sums, stream);
     }
 };
 
@@ -361,11 +366,19 @@ rtd_status run_pass(const PassRows &R, int p, const K *kin, const uint32_t *vin,
 
 }  // namespace
 
+rtd_status radix_sort_sums(uint64_t n, int key_bits, SortScratch &scr, uint32_t **words, uint64_t *count) {
+    PassRows R(n);
+    RTD_TRY(R.reserve(scr, (key_bits + 7) / 8));
+    *words = R.sc;
+    *count = R.sums;
+    return RTD_OK;
+}
+
 template <typename K>
 rtd_status radix_sort_pairs(K *keys, K *keys_alt, uint32_t *vals, uint32_t *vals_alt,
                             bool vals_iota, uint64_t n, int begin_bit, int end_bit,
                             SortScratch &scr, uint32_t *d_err, cudaStream_t stream, bool *in_alt,
-                            const float *gather_xyz, float4 *gather_out) {
+                            const float *gather_xyz, float4 *gather_out, bool sums_zeroed) {
     (void)d_err;   // no pass waits on another tile: nothing can time out
     *in_alt = false;
     if (n == 0) return RTD_OK;
@@ -374,7 +387,7 @@ rtd_status radix_sort_pairs(K *keys, K *keys_alt, uint32_t *vals, uint32_t *vals
     if (passes <= 0 || passes > 8 || end_bit > (int)(8 * sizeof(K)))
         return fail(RTD_ERR_INVALID_ARGUMENT, "radix sort: bad bit range");
     PassRows R(n);
-    RTD_TRY(R.reserve(scr, passes, stream));
+    RTD_TRY(R.reserve(scr, passes, sums_zeroed, stream));
     K *kin = keys, *kout = keys_alt;
     uint32_t *vin = vals, *vout = vals_alt;
     for (int p = 0; p < passes; ++p) {
@@ -398,7 +411,7 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
                               uint32_t *k32b, uint32_t *vals, uint32_t *vals_alt, uint64_t n,
                               int key_bits, SortScratch &scr, cudaStream_t stream,
                               const float *gather_xyz, float4 *gather_out,
-                              uint64_t *sorted_keys, uint32_t **sorted_vals) {
+                              uint64_t *sorted_keys, uint32_t **sorted_vals, bool sums_zeroed) {
     if (n == 0) return RTD_OK;
     if (n >= (1ull << 30)) return fail(RTD_ERR_INVALID_ARGUMENT, "radix sort: n must be < 2^30");
     if (key_bits <= 32 || key_bits > 48)
@@ -415,7 +428,7 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
         pk.low_mask = (1ull << low) - 1ull;
     }
     PassRows R(n);
-    RTD_TRY(R.reserve(scr, lp + 4, stream));
+    RTD_TRY(R.reserve(scr, lp + 4, sums_zeroed, stream));
     const uint32_t *vin = nullptr;          // pass 0: values 0..n-1 on the fly
     uint32_t *vout = vals;
     // low passes; the last writes the top 32 bits as the next passes' keys
@@ -459,11 +472,11 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
 template rtd_status radix_sort_pairs<uint32_t>(uint32_t *, uint32_t *, uint32_t *, uint32_t *,
                                                bool, uint64_t, int, int, SortScratch &,
                                                uint32_t *, cudaStream_t, bool *, const float *,
-                                               float4 *);
+                                               float4 *, bool);
 template rtd_status radix_sort_pairs<uint64_t>(uint64_t *, uint64_t *, uint32_t *, uint32_t *,
                                                bool, uint64_t, int, int, SortScratch &,
                                                uint32_t *, cudaStream_t, bool *, const float *,
-                                               float4 *);
+                                               float4 *, bool);
 
 rtd_status exclusive_scan_u32(const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *d_total,
                               ScanScratch &scr, uint32_t *d_err, cudaStream_t stream) {

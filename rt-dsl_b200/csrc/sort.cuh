@@ -34,7 +34,13 @@ template <typename K>
 rtd_status radix_sort_pairs(K *keys, K *keys_alt, uint32_t *vals, uint32_t *vals_alt,
                             bool vals_iota, uint64_t n, int begin_bit, int end_bit,
                             SortScratch &scr, uint32_t *d_err, cudaStream_t stream, bool *in_alt,
-                            const float *gather_xyz = nullptr, float4 *gather_out = nullptr);
+                            const float *gather_xyz = nullptr, float4 *gather_out = nullptr,
+                            bool sums_zeroed = false);
+
+// The words that the count kernels of a sort of n keys by key_bits bits add
+// into, for a caller that zeroes them with words of its own and then sorts
+// with sums_zeroed (a launch fewer).
+rtd_status radix_sort_sums(uint64_t n, int key_bits, SortScratch &scr, uint32_t **words, uint64_t *count);
 
 // Sorts n 64-bit keys of key_bits bits, 32 < key_bits <= 48, with their
 // indices as values (stable): one or two passes over the low key_bits - 32
@@ -49,7 +55,8 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
                               uint32_t *k32b, uint32_t *vals, uint32_t *vals_alt, uint64_t n,
                               int key_bits, SortScratch &scr, cudaStream_t stream,
                               const float *gather_xyz, float4 *gather_out,
-                              uint64_t *sorted_keys, uint32_t **sorted_vals = nullptr);
+                              uint64_t *sorted_keys, uint32_t **sorted_vals = nullptr,
+                              bool sums_zeroed = false);
 
 // out[i] = sum(in[0..i)), out has n entries; *d_total (device) = sum(in).
 // As for the sort, d_err is not written.
