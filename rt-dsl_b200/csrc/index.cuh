@@ -194,6 +194,19 @@ __device__ __forceinline__ SceneNorm scene_norm_cubic(const IndexHeader *h) {
     return s;
 }
 
+// 30-bit codes follow compute_morton_codes (gprt-core/src/morton.rs:19-48),
+// extent per axis; wider codes (B = bits / 3 per axis, scale = 2^B - 1,
+// B <= 21, interleaved in the low 3B bits of a u64) use one cubic extent.
+template <typename K>
+__device__ __forceinline__ K morton_key(const SceneNorm &s, float scale, float x, float y, float z) {
+    if (sizeof(K) == 4)
+        return (K)morton30(quantize(x, s.lo[0], s.ext[0], 1023.0f),
+                           quantize(y, s.lo[1], s.ext[1], 1023.0f),
+                           quantize(z, s.lo[2], s.ext[2], 1023.0f));
+    return (K)morton63(quantize(x, s.lo[0], s.ext[0], scale), quantize(y, s.lo[1], s.ext[1], scale),
+                       quantize(z, s.lo[2], s.ext[2], scale));
+}
+
 // Arguments the search kernels need from an index.
 struct IndexView {
     const float4 *pts;

@@ -102,19 +102,6 @@ __global__ void __launch_bounds__(BLOCK) bbox_kernel(const float *__restrict__ x
     }
 }
 
-// 30-bit codes follow compute_morton_codes (gprt-core/src/morton.rs:19-48),
-// extent per axis; wider codes (B = bits / 3 per axis, scale = 2^B - 1,
-// B <= 21, interleaved in the low 3B bits of a u64) use one cubic extent.
-template <typename K>
-__device__ __forceinline__ K morton_key(const SceneNorm &s, float scale, float x, float y, float z) {
-    if (sizeof(K) == 4)
-        return (K)morton30(quantize(x, s.lo[0], s.ext[0], 1023.0f),
-                           quantize(y, s.lo[1], s.ext[1], 1023.0f),
-                           quantize(z, s.lo[2], s.ext[2], 1023.0f));
-    return (K)morton63(quantize(x, s.lo[0], s.ext[0], scale), quantize(y, s.lo[1], s.ext[1], scale),
-                       quantize(z, s.lo[2], s.ext[2], scale));
-}
-
 // Keys of the points; with vec4 (as bbox_kernel) whole groups of 4 points
 // are read as three float4 each.
 template <typename K>
@@ -1222,7 +1209,8 @@ rtd_status build_typed(rtd_index *idx, const float *d_xyz, uint64_t n, cudaStrea
                                    idx->keys_alt.as<uint64_t>(), idx->k32a.as<uint32_t>(),
                                    idx->k32b.as<uint32_t>(), idx->vals.as<uint32_t>(),
                                    idx->vals_alt.as<uint32_t>(), n, kbits, idx->sort, st, d_xyz,
-                                   idx->pts.as<float4>(), idx->keys_alt.as<uint64_t>(), nullptr, true));
+                                   idx->pts.as<float4>(), idx->keys_alt.as<uint64_t>(), nullptr, true,
+                                   SceneKeys{h, scale}));
         skeys = idx->keys_alt.as<K>();
     } else {
         bool in_alt = false;

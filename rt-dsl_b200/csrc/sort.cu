@@ -1,5 +1,6 @@
 // sort.cu -- LSD radix sort of (key, u32 value) pairs and exclusive scan,
 // both as a count kernel and a scatter kernel over fixed tiles (sort.cuh).
+#include "index.cuh"
 #include "sort.cuh"
 #include "scan.cuh"
 
@@ -161,6 +162,27 @@ struct ValuePack {
     }
 };
 
+// Point o of n: with vec4 (a 16-byte aligned array) the aligned float4 that
+// holds its first coordinate and, where it ends there, the two floats after,
+// 1.5 scattered requests a point instead of 3; the last point by coordinate.
+__device__ __forceinline__ void load_point(const float *__restrict__ xyz, uint64_t o, uint64_t n, int vec4, float &x,
+                                           float &y, float &z) {
+    const uint64_t f = 3 * o;
+    if (!vec4 || o + 1 >= n) {
+        x = xyz[f];
+        y = xyz[f + 1];
+        z = xyz[f + 2];
+        return;
+    }
+    const uint32_t r = (uint32_t)f & 3u;
+    const float4 a = *reinterpret_cast<const float4 *>(xyz + (f - r));
+    float2 b = make_float2(0.f, 0.f);
+    if (r >= 2) b = *reinterpret_cast<const float2 *>(xyz + (f - r) + 4);
+    x = r == 0 ? a.x : r == 1 ? a.y : r == 2 ? a.z : a.w;
+    y = r == 0 ? a.y : r == 1 ? a.z : r == 2 ? a.w : b.x;
+    z = r == 0 ? a.z : r == 1 ? a.w : r == 2 ? b.x : b.y;
+}
+
 // Scatter of one pass over 8 bits at `shift`: the tile's keys are ranked
 // in registers (stable: warp, item, lane order), staged in shared memory
 // grouped by digit, and each digit run is written contiguously from the
@@ -177,7 +199,7 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     const uint32_t *__restrict__ gsum, const uint32_t *__restrict__ ssum, uint32_t groups,
     uint32_t supers, const float *__restrict__ gxyz, float4 *__restrict__ gout,
     uint32_t *__restrict__ kout32, int shift32, const uint64_t *__restrict__ gk_in,
-    uint64_t *__restrict__ gk_out, const ValuePack pk) {
+    uint64_t *__restrict__ gk_out, const ValuePack pk, const SceneKeys scene, int vec4) {
     chain_wait();
     constexpr int TILE = RS_BLOCK * ITEMS;
     extern __shared__ __align__(16) unsigned char rs_smem[];
@@ -246,9 +268,15 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
     const uint64_t rem = n - base;
     const uint32_t valid = rem < (uint64_t)TILE ? (uint32_t)rem : (uint32_t)TILE;
     if (gout) {
-        // Last pass with a gather: the points (and keys) are read at random,
-        // so GATHER slots' loads are issued together before their stores.
+        // Last pass with a gather: the points are read at random, so GATHER
+        // slots' loads are issued together before their stores.  Bound by
+        // those reads; a key that is not carried along is made again from its
+        // point rather than read at random too (10 M points: 338 us with
+        // scalar loads and the keys read, now 221).
         constexpr int GATHER = 4;
+        const bool remake = scene.hdr && !pk.bits;
+        SceneNorm norm{};
+        if (remake) norm = scene_norm_cubic(scene.hdr);
         for (uint32_t j0 = tid; j0 < valid; j0 += GATHER * RS_BLOCK) {
             uint32_t v[GATHER], dst[GATHER];
             float x[GATHER], y[GATHER], z[GATHER];
@@ -262,10 +290,8 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
                 const uint32_t w = s_vals[jj];
                 v[u] = pk.index(w);
                 const uint64_t o = v[u];
-                x[u] = gxyz[3 * o];
-                y[u] = gxyz[3 * o + 1];
-                z[u] = gxyz[3 * o + 2];
-                gk[u] = !gk_out ? 0ull : pk.bits ? pk.key((uint64_t)k, w) : gk_in[o];
+                load_point(gxyz, o, n, vec4, x[u], y[u], z[u]);
+                gk[u] = !gk_out || remake ? 0ull : pk.bits ? pk.key((uint64_t)k, w) : gk_in[o];
                 if (j < valid) {
                     if (kout) kout[dst[u]] = k;
                     if (kout32) kout32[dst[u]] = (uint32_t)((uint64_t)k >> shift32);
@@ -275,7 +301,7 @@ __global__ void __launch_bounds__(RS_BLOCK) rs_scatter_kernel(
             for (int u = 0; u < GATHER; ++u) {
                 if (j0 + u * RS_BLOCK < valid) {
                     gout[dst[u]] = make_float4(x[u], y[u], z[u], __uint_as_float(v[u]));
-                    if (gk_out) gk_out[dst[u]] = gk[u];
+                    if (gk_out) gk_out[dst[u]] = remake ? morton_key<uint64_t>(norm, scene.scale, x[u], y[u], z[u]) : gk[u];
                 }
             }
         }
@@ -336,6 +362,7 @@ template <typename K> struct PassOut {
     const uint64_t *gk_in = nullptr;
     uint64_t *gk_out = nullptr;
     ValuePack pk;
+    SceneKeys scene;
 };
 
 // Count + scatter of pass p (its count rows) over bits [shift, shift + 8).
@@ -354,7 +381,7 @@ rtd_status run_pass_items(const PassRows &R, int p, const K *kin, const uint32_t
     RTD_LAUNCH_CHAINED((rs_scatter_kernel<K, ITEMS>), dim3((unsigned)L.tiles), dim3(RS_BLOCK), smem, stream,
                        kin, o.kout, vin, vout, n, shift, tcount, gsum, ssum, (uint32_t)L.groups,
                        (uint32_t)L.supers, o.gxyz, o.gout, o.kout32, o.shift32, o.gk_in, o.gk_out,
-                       o.pk);
+                       o.pk, o.scene, ((uintptr_t)o.gxyz & 15u) == 0 ? 1 : 0);
     return RTD_OK;
 }
 template <typename K>
@@ -411,7 +438,8 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
                               uint32_t *k32b, uint32_t *vals, uint32_t *vals_alt, uint64_t n,
                               int key_bits, SortScratch &scr, cudaStream_t stream,
                               const float *gather_xyz, float4 *gather_out,
-                              uint64_t *sorted_keys, uint32_t **sorted_vals, bool sums_zeroed) {
+                              uint64_t *sorted_keys, uint32_t **sorted_vals, bool sums_zeroed,
+                              const SceneKeys &scene) {
     if (n == 0) return RTD_OK;
     if (n >= (1ull << 30)) return fail(RTD_ERR_INVALID_ARGUMENT, "radix sort: n must be < 2^30");
     if (key_bits <= 32 || key_bits > 48)
@@ -456,6 +484,7 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
             o.gout = gather_out;
             o.gk_in = keys;
             o.gk_out = sorted_keys;
+            if (gather_out) o.scene = scene;
             o.pk = pk;   // unpacks the values, rebuilds the keys
         } else {
             o.kout = k32out;

@@ -17,6 +17,13 @@
 
 namespace rtd {
 
+struct IndexHeader;
+// What makes a point's key: the scene of the index and the quantisation.
+struct SceneKeys {
+    const IndexHeader *hdr = nullptr;
+    float scale = 0.f;
+};
+
 struct SortScratch {
     DevBuf counts;    // passes * (tiles + groups + super groups) * 256 u32
 };
@@ -49,6 +56,7 @@ rtd_status radix_sort_sums(uint64_t n, int key_bits, SortScratch &scr, uint32_t 
 // last pass writes sorted_keys[i] = keys[v] for the i-th sorted index v,
 // and the index itself to *sorted_vals (one of vals / vals_alt) or, with
 // gather_out, the point gather_xyz[v] with v in w (as radix_sort_pairs).
+// With scene, keys[v] is made again from the point (the same bits).
 // keys is not modified; keys_alt is scratch for two low passes; all
 // buffers hold n entries.
 rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t *k32a,
@@ -56,7 +64,7 @@ rtd_status radix_sort_split64(const uint64_t *keys, uint64_t *keys_alt, uint32_t
                               int key_bits, SortScratch &scr, cudaStream_t stream,
                               const float *gather_xyz, float4 *gather_out,
                               uint64_t *sorted_keys, uint32_t **sorted_vals = nullptr,
-                              bool sums_zeroed = false);
+                              bool sums_zeroed = false, const SceneKeys &scene = SceneKeys());
 
 // out[i] = sum(in[0..i)), out has n entries; *d_total (device) = sum(in).
 // As for the sort, d_err is not written.
