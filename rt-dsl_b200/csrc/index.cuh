@@ -207,6 +207,27 @@ __device__ __forceinline__ K morton_key(const SceneNorm &s, float scale, float x
                        quantize(z, s.lo[2], s.ext[2], scale));
 }
 
+// Point o of n: with vec4 (a 16-byte aligned array) the aligned float4 that
+// holds its first coordinate and, where it ends there, the two floats after,
+// 1.5 scattered requests a point instead of 3; the last point by coordinate.
+__device__ __forceinline__ void load_point(const float *__restrict__ xyz, uint64_t o, uint64_t n, int vec4, float &x,
+                                           float &y, float &z) {
+    const uint64_t f = 3 * o;
+    if (!vec4 || o + 1 >= n) {
+        x = xyz[f];
+        y = xyz[f + 1];
+        z = xyz[f + 2];
+        return;
+    }
+    const uint32_t r = (uint32_t)f & 3u;
+    const float4 a = *reinterpret_cast<const float4 *>(xyz + (f - r));
+    float2 b = make_float2(0.f, 0.f);
+    if (r >= 2) b = *reinterpret_cast<const float2 *>(xyz + (f - r) + 4);
+    x = r == 0 ? a.x : r == 1 ? a.y : r == 2 ? a.z : a.w;
+    y = r == 0 ? a.y : r == 1 ? a.z : r == 2 ? a.w : b.x;
+    z = r == 0 ? a.z : r == 1 ? a.w : r == 2 ? b.x : b.y;
+}
+
 // Arguments the search kernels need from an index.
 struct IndexView {
     const float4 *pts;
