@@ -193,41 +193,54 @@ struct PrefixTest {
     }
 };
 
+// The keys at positions base .. base + COUNT - 1 that exist, all loads in
+// flight together.
+template <int COUNT, typename K>
+__device__ __forceinline__ void stage_keys(const K *__restrict__ keys, int64_t n, int64_t base, K *s_k) {
+    constexpr int U = (COUNT + BLOCK - 1) / BLOCK;
+    K k[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int t = u * BLOCK + (int)threadIdx.x;
+        const int64_t j = base + t;
+        if (t < COUNT && j >= 0 && j < n) k[u] = keys[j];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int t = u * BLOCK + (int)threadIdx.x;
+        const int64_t j = base + t;
+        if (t < COUNT && j >= 0 && j < n) s_k[t] = k[u];
+    }
+}
+
 // Kept nodes of every tile, added into the sums of its group (32 tiles) and
 // super group (32 groups), from which tile_nodes_kernel numbers them: the
-// numbers follow the Karras index.  A block takes COUNT_TILES tiles.
-constexpr int COUNT_TILES = 2;
+// numbers follow the Karras index.
 struct TreeCounts {
     uint32_t *tiles, *groups, *supers;
     uint32_t *cross, *done;   // nodes listed for cross_nodes_kernel; its finished blocks
 };
 template <typename K>
 __global__ void __launch_bounds__(BLOCK) karras_count_kernel(const K *__restrict__ keys, int64_t n, uint32_t leaf_size,
-                                                             uint32_t tiles, const TreeCounts tc) {
+                                                             const TreeCounts tc) {
     chain_wait();
-    constexpr int SPAN = COUNT_TILES * NODE_TILE;
-    __shared__ K s_k[SPAN + 2 * FLAG_HALO];
-    __shared__ uint32_t s_cnt[COUNT_TILES];
-    const int64_t b0 = (int64_t)blockIdx.x * SPAN, base = b0 - FLAG_HALO;
-    for (int t = threadIdx.x; t < SPAN + 2 * FLAG_HALO; t += BLOCK) {
-        const int64_t j = base + t;
-        if (j >= 0 && j < n) s_k[t] = keys[j];
-    }
-    if (threadIdx.x < COUNT_TILES) s_cnt[threadIdx.x] = 0;
+    __shared__ K s_k[NODE_TILE + 2 * FLAG_HALO];
+    __shared__ uint32_t s_cnt[BLOCK / 32];
+    const uint32_t tile = blockIdx.x;
+    const int64_t b0 = (int64_t)tile * NODE_TILE, base = b0 - FLAG_HALO;
+    stage_keys<NODE_TILE + 2 * FLAG_HALO>(keys, n, base, s_k);
     __syncthreads();
-    for (int u = 0; u < COUNT_TILES; ++u) {
-        uint32_t c = 0;
+    uint32_t c = 0;
 #pragma unroll
-        for (int t = 0; t < NODE_TILE; t += BLOCK) {
-            const int64_t i = b0 + u * NODE_TILE + t + (int)threadIdx.x;
-            c += __popc(__ballot_sync(0xffffffffu, i < n - 1 && keeps_node<K>(s_k, base, n, i, leaf_size)));
-        }
-        if ((threadIdx.x & 31) == 0) atomicAdd(&s_cnt[u], c);
+    for (int t = 0; t < NODE_TILE; t += BLOCK) {
+        const int64_t i = b0 + t + (int)threadIdx.x;
+        c += __popc(__ballot_sync(0xffffffffu, i < n - 1 && keeps_node<K>(s_k, base, n, i, leaf_size)));
     }
+    if ((threadIdx.x & 31) == 0) s_cnt[threadIdx.x >> 5] = c;
     __syncthreads();
-    const uint32_t tile = blockIdx.x * COUNT_TILES + threadIdx.x;
-    if (threadIdx.x < COUNT_TILES && tile < tiles) {
-        const uint32_t c = s_cnt[threadIdx.x];
+    if (threadIdx.x == 0) {
+        c = 0;
+        for (int w = 0; w < BLOCK / 32; ++w) c += s_cnt[w];
         tc.tiles[tile] = c;
         if (c) {
             atomicAdd(&tc.groups[tile / GROUP_TILES], c);
@@ -474,8 +487,9 @@ __device__ __forceinline__ BvhNode make_node(const Pyramid &P, const Number &num
 // its lower bound; the others are listed in `cross` for cross_nodes_kernel.
 // Bound by the issue slots of the searches and box walks.  With flags, their
 // scan, a list of the kept nodes and global searches a thread a node, the tree
-// of 100 K points took 50 us (51 dependent reads at the root), now 40; that of
-// 10 M 575 us besides the pyramid's 79, now 535 with it.
+// of 100 K points took 50 us (51 dependent reads at the root), now 37; that of
+// 10 M 575 us besides the pyramid's 79, now 495 with it (counts 50, tiles 347,
+// crossing nodes 95).
 constexpr int NODE_DEPTH = 96;   // prefix lengths of (key, position) pairs: nodes that share a tile boundary are nested
 template <typename K>
 __global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
@@ -494,16 +508,21 @@ __global__ void __launch_bounds__(BLOCK, 6) tile_nodes_kernel(
     const int64_t b0 = (int64_t)tile * NODE_TILE, base_k = b0 - FLAG_HALO;
     const uint32_t m = (uint32_t)(n - b0 < NODE_TILE ? n - b0 : NODE_TILE);
     const uint32_t n1 = (m + 7) / 8, n2 = (n1 + 7) / 8, n3 = (n2 + 7) / 8;
-    for (uint32_t t = threadIdx.x; t < NODE_TILE + 2 * FLAG_HALO; t += BLOCK) {
-        const int64_t j = base_k + (int64_t)t;
-        if (j >= 0 && j < (int64_t)n) s_k[t] = keys[j];
+    float4 pt[NODE_TILE / BLOCK];   // (in flight with the keys)
+#pragma unroll
+    for (int u = 0; u < NODE_TILE / BLOCK; ++u) {
+        const uint32_t t = u * BLOCK + threadIdx.x;
+        if (t < m) pt[u] = pts[b0 + t];
     }
+    stage_keys<NODE_TILE + 2 * FLAG_HALO>(keys, (int64_t)n, base_k, s_k);
     // level 1: the 8 lanes of an entry
-    for (uint32_t t = threadIdx.x; t < NODE_TILE; t += BLOCK) {
+#pragma unroll
+    for (int u = 0; u < NODE_TILE / BLOCK; ++u) {
+        const uint32_t t = u * BLOCK + threadIdx.x;
         Box b;
         box_empty(b);
         if (t < m) {
-            const float4 p = pts[b0 + t];
+            const float4 p = pt[u];
             s_p[t] = p;
             bool nan = false;
             box_add_point(b, nan, p);
@@ -680,7 +699,6 @@ __global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
     chain_wait();
     const uint32_t count = *tc.cross < cross_cap ? *tc.cross : cross_cap;
     const int lane = threadIdx.x & 31;
-    auto number = [&](uint32_t i) { return kept.number(i); };
     for (uint32_t w = (blockIdx.x * BLOCK + threadIdx.x) >> 5; w < count; w += (gridDim.x * BLOCK) >> 5) {
         const int64_t i = cross[w];
         const K ki = keys[i];
@@ -703,6 +721,8 @@ __global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
         const int64_t s = furthest(0, (int64_t)2 << up, delta(keys, (int64_t)n, ki, i, i + l * dir));
         const uint32_t f0 = (uint32_t)(dir > 0 ? i : i - l), last = (uint32_t)(dir > 0 ? i + l : i);
         const uint32_t sp = (uint32_t)(i + s * dir + (dir < 0 ? -1 : 0));
+        // numbers of the node and its children (read beside the boxes)
+        const uint32_t num = lane < 3 ? kept.number(lane == 0 ? (uint32_t)i : sp + lane - 1) : 0u;
         // boxes: lanes 0-15 the left child, 16-31 the right one; of 16 lanes
         // 8 take the partial run at the start of a level, 8 that at its end
         Box b;
@@ -740,8 +760,10 @@ __global__ void __launch_bounds__(BLOCK) cross_nodes_kernel(
             b1.lo[x] = __shfl_sync(0xffffffffu, b.lo[x], 16);
             b1.hi[x] = __shfl_sync(0xffffffffu, b.hi[x], 16);
         }
+        const uint32_t left = __shfl_sync(0xffffffffu, num, 1), right = __shfl_sync(0xffffffffu, num, 2);
         if (lane == 0) {
-            nodes[number((uint32_t)i)] = pack_node(number, leaf_size, f0, last, sp, 0u, b, b1);
+            nodes[num] = pack_node([&](uint32_t j) { return j == sp ? left : right; }, leaf_size, f0, last, sp, 0u, b,
+                                   b1);
             if (kfirst) {
                 kfirst[i] = f0;
                 klast[i] = last;
@@ -1280,8 +1302,8 @@ rtd_status build_tree_sorted(rtd_index *idx, const K *skeys, uint64_t n, cudaStr
     const uint64_t tiles = ceil_div(n, (uint64_t)NODE_TILE);
     const uint32_t cross_cap = (uint32_t)(ni < NODE_DEPTH * tiles ? ni : NODE_DEPTH * tiles);
     RTD_TRY(idx->cross.reserve(cross_cap * sizeof(uint32_t)));
-    RTD_LAUNCH_CHAINED(karras_count_kernel<K>, dim3((unsigned)ceil_div(tiles, (uint64_t)COUNT_TILES)), dim3(BLOCK), 0,
-                       st, skeys, (int64_t)n, idx->leaf_size, (uint32_t)tiles, tc);
+    RTD_LAUNCH_CHAINED(karras_count_kernel<K>, dim3((unsigned)tiles), dim3(BLOCK), 0, st, skeys, (int64_t)n,
+                       idx->leaf_size, tc);
     uint32_t *kf = ranges ? idx->kfirst.as<uint32_t>() : nullptr, *kl = ranges ? idx->klast.as<uint32_t>() : nullptr;
     uint32_t *bits = idx->kept_bits.as<uint32_t>(), *before = idx->kept_before.as<uint32_t>();
     RTD_LAUNCH_CHAINED(tile_nodes_kernel<K>, dim3((unsigned)tiles), dim3(BLOCK), 0, st, skeys, n, h, tc, bits, before,
