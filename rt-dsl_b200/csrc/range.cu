@@ -25,7 +25,7 @@ constexpr uint32_t WRECS = 64;     // staged records per warp (1 KB)
 // Kernel modes: count hits, push pairs through warp staging and a global
 // cursor, write pairs into per-query segments at known offsets, or count
 // hits and push them at once (a count whose pairs the next fill scatters).
-// MODE_SAMPLE counts a sample of the queries for use_threads.
+// MODE_SAMPLE counts a sample of the queries for launch_count.
 enum : int { MODE_COUNT = 0, MODE_PUSH = 1, MODE_SEG = 2, MODE_CPUSH = 3, MODE_SAMPLE = 4 };
 
 struct RangeArgs {
@@ -37,8 +37,9 @@ struct RangeArgs {
     float r2;
     uint32_t *counts;
     uint32_t *most;            // counts: the largest count
-    int if_heavy;              // counts: do nothing unless the header's heavy is set
+    int if_heavy;              // counts: do nothing unless the header's heavy says so
     uint64_t sample_step;      // MODE_SAMPLE: every sample_step-th query
+    uint32_t heavy_at;         // MODE_SAMPLE: hits that alone make the count heavy
     uint2 *pairs;
     uint64_t capacity;
     unsigned long long *cursor;
@@ -54,9 +55,10 @@ struct RangeArgs {
     uint32_t *err;
 };
 
-// Queries with this many hits among a sample make a count heavy (use_threads).
-constexpr uint32_t HEAVY_COUNT = 256;
+// IndexHeader::heavy sums the hits of a sample of the queries, in which one of
+// heavy_at hits counts for all of HEAVY_SUM (launch_count).
 constexpr uint64_t HEAVY_SAMPLE = 1024;
+constexpr uint32_t HEAVY_SUM = 64 * HEAVY_SAMPLE;
 
 // Shared memory of one warp: the boxes to visit (level << 28 | entry), runs
 // of 8 points to test, staged pairs and records.
@@ -89,7 +91,7 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
     constexpr bool SEG = MODE == MODE_SEG;
     constexpr bool COUNTS = MODE == MODE_COUNT || MODE == MODE_CPUSH;
     if (SEG && p.skip_if_same && p.ix.hdr->qfp[0] == p.ix.hdr->qfp[1]) return;
-    if (COUNTS && p.if_heavy && p.ix.hdr->heavy == 0) return;
+    if (COUNTS && p.if_heavy && p.ix.hdr->heavy < HEAVY_SUM) return;
     extern __shared__ uint4 s_dyn[];
     __shared__ uint32_t s_off[12];
     const uint32_t n = (uint32_t)p.ix.n;
@@ -262,7 +264,8 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
             }
         }
         if (COUNTS && lane == 0) p.counts[qi] = cnt;
-        if (COUNTS || MODE == MODE_SAMPLE) most = cnt > most ? cnt : most;
+        if (COUNTS) most = cnt > most ? cnt : most;
+        if (MODE == MODE_SAMPLE && lane == 0) atomicAdd(p.most, cnt < p.heavy_at ? (cnt < HEAVY_SUM ? cnt : HEAVY_SUM) : HEAVY_SUM);
         // a segment left short or overrun: the queries changed since the count
         if (SEG && (seg_bad || cnt != wlen)) atomicOr(p.err, DEVERR_MISMATCH);
     }
@@ -272,7 +275,6 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
         if (lane == 0 && covered) atomicAdd(&p.cursor[2], covered);
     }
     if (COUNTS && lane == 0 && most) atomicMax(p.most, most);
-    if (MODE == MODE_SAMPLE && lane == 0 && most >= HEAVY_COUNT) *p.most = 1;
 }
 
 constexpr int SHORT_DEPTH = 12;  // stack entries per thread in shared memory
@@ -298,7 +300,7 @@ enum : int { F_QX = 0, F_QY, F_QZ, F_QI, F_F0, F_C0, F_F1, F_DONE, F_COUNT };
 // The counting passes (MODE_COUNT, MODE_CPUSH) a thread per query over the
 // binary tree: where many queries have few hits each, its tighter boxes and
 // 32 walks a warp need less than half the instructions of range_kernel
-// (use_threads says when).  Threads of a warp advance their own traversals
+// (launch_count says when).  Threads of a warp advance their own traversals
 // one node per iteration of a warp-converged loop; a stack entry carries the
 // node and the first sorted point below it.  A child whose whole box lies
 // inside the ball counts without a test (pushed as a record).  After each
@@ -309,7 +311,7 @@ enum : int { F_QX = 0, F_QY, F_QZ, F_QI, F_F0, F_C0, F_F1, F_DONE, F_COUNT };
 template <int MODE>
 __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thread_kernel(const RangeArgs p) {
     constexpr bool PUSH = MODE == MODE_CPUSH;
-    if (p.ix.hdr->heavy != 0) return;
+    if (p.ix.hdr->heavy >= HEAVY_SUM) return;
     __shared__ BvhNode s_top[TOP_MAX];
     __shared__ uint2 s_stack[SHORT_DEPTH][RBLOCK];
     __shared__ uint2 s_buf[PUSH ? RWARPS : 1][PUSH ? WBUF : 1];
@@ -844,17 +846,21 @@ rtd_status launch_range(RangeArgs &a, cudaStream_t st) {
     return RTD_OK;
 }
 
-// Which kernel counts.  A thread per query is the better one for many
-// queries of few hits; a warp per query for few queries (it runs them side
-// by side) and where some have very many hits (a thread's walk holds the
-// other 31 of its warp).  Measured, counting with pushes, thread / warp, ms:
+// Which kernel counts.  A thread per query takes about 0.8 ns + 0.03 ns a hit
+// for each, a warp per query 2.2 ns + 0.01 ns a hit: the thread is ahead below
+// some 60 hits on average.  But a warp of 32 threads takes as long as its
+// longest walk, some 1.1 us for each of that query's hits, and the last such
+// warp ends the launch: with fewer than about 500 queries for every hit of the
+// largest query (1,000 for the largest of a sample, which misses the top) the
+// warp kernel is ahead.  Measured, counting with pushes, thread / warp, ms:
 // 1.8M points, 400,000 queries, clustered: 1 hit on average 0.35 / 0.88, 8
-// hits (230 at the most) 0.64 / 0.93, 50 hits (1,456) 1.54 / 1.10; uniform,
-// 50 hits (87) 0.99 / 1.11; 200,000 of each, 20 hits (513) 0.61 / 0.44; 20,000
-// queries on 50,000 points, 10 hits 0.20 / 0.12.  From THREAD_QUERIES on, a
-// sample of the queries says on the device (IndexHeader::heavy) which of the
-// two launches does the work; it runs on the side stream beside the query
-// ordering.
+// hits (230 at the most) 0.64 / 0.93, 50 hits (1,456) 1.54 / 1.10; uniform, 50
+// hits (87) 0.99 / 1.11; 200,000 of each, 20 hits (513) 0.61 / 0.44; clustered
+// points as their own queries, 1.8M with 20 hits 1.8 / 3.9, 600,000 with 8
+// hits 0.54 / 1.03; 20,000 queries on 50,000 points, 10 hits 0.20 / 0.12.  From
+// THREAD_QUERIES on, a sample of the queries says on the device
+// (IndexHeader::heavy) which of the two launches does the work; it runs on the
+// side stream beside the query ordering.
 template <int MODE>
 rtd_status launch_count(RangeArgs &a, cudaStream_t st) {
     a.if_heavy = a.nq >= THREAD_QUERIES;
@@ -878,6 +884,7 @@ rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     a.q = d_q;
     a.nq = HEAVY_SAMPLE;
     a.sample_step = nq / HEAVY_SAMPLE;
+    a.heavy_at = (uint32_t)(nq / HEAVY_SAMPLE);
     a.r2 = r * r;
     a.most = &h->heavy;
     a.err = &h->err;
