@@ -193,13 +193,13 @@ void rtd_limits_get(rtd_limits *l);
 /* ---------------------------------------------------------------------
  * Exact k-NN.  Replaces the k_nn! round loop (gprt-macros/src/lib.rs:
  * 408-604) and its per-round gprt_execute + gprt_retrieve_array_* calls
- * (main.cpp:313-365): all rounds run inside one kernel launch.
+ * (main.cpp:313-365): every query finishes inside one kernel launch.
  * Output per query: the k smallest (FP32 squared distance, point id)
  * pairs, ascending, ties to the lower id; ids[q*k+j] (and d2[q*k+j] when
  * d2 != NULL).  Slots beyond the number of points hold 0xFFFFFFFF / +inf.
  * Any k >= 1, as the reference's 2K-slot per-query slab
- * (gprt-macros/src/lib.rs:300-310): k <= 16 keeps a thread's list in
- * registers, larger k (and small calls) collect a warp's candidates in
+ * (gprt-macros/src/lib.rs:300-310): k <= 12 (32 with lanes_per_query 1) keeps
+ * a thread's list in registers, larger k (and small calls) collect a warp's candidates in
  * shared memory (min(k, n) <= 2048), and the largest k keep a warp's sorted
  * list in a device slab of the index (grown on demand, at most 1 GiB).
  * ------------------------------------------------------------------- */
@@ -330,9 +330,9 @@ rtd_status rtd_knn_backward(const float *d_queries, uint64_t nq, const float *d_
  * queries and k (no reference counterpart: the reference searches one scene
  * per k_nn! call).  One pass builds every cloud's LBVH as one forest (a
  * single sort over (cloud, Morton) keys) and searches every query of every
- * cloud, whatever its k, in one persistent launch fed from one device work
- * queue; with use_graph the pass is captured once as a CUDA graph and
- * replayed.
+ * cloud in two persistent launches fed from device work queues (lists up to 8
+ * and longer ones); with use_graph the pass is captured once as a CUDA graph
+ * and replayed.
  * ------------------------------------------------------------------- */
 typedef struct rtd_cloud {
     uint64_t point_offset;  /* first point of the cloud in the packed point array */
@@ -340,7 +340,7 @@ typedef struct rtd_cloud {
     uint64_t out_offset;    /* results of the cloud's query j at out_offset + j*k */
     uint32_t n_points;
     uint32_t n_queries;
-    uint32_t k;             /* >= 1, any size (k above 256 keeps its list in a device slab) */
+    uint32_t k;             /* >= 1, any size (k above 512 keeps its list in a device slab) */
     uint32_t pad;
 } rtd_cloud;
 

@@ -2,7 +2,9 @@
 // kernel.  Replaces the k_nn! round loop (gprt-macros/src/lib.rs:462-595)
 // and its OptiX register-heap programs (lib.rs:305-377): where the
 // reference relaunches per round, copies a Q x 2k slab back to the host and
-// filters there, every query here runs all its rounds inside one launch
+// filters there, every query here finishes inside one launch: exact searches
+// without rounds (from the query's Morton neighbours, or collecting over the
+// box pyramid, knn_collect.cuh), partial_results with them
 // (knn_traverse.cuh).
 #include <atomic>
 

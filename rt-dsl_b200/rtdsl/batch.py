@@ -3,8 +3,8 @@
 The reference searches one scene per ``k_nn!`` call (gprt-macros/src/lib.rs:
 316-476); a workload of many small clouds there pays one BVH build and one
 launch per cloud.  ``Batch`` plans the packed layout once, then each call
-builds every cloud's LBVH as one forest and searches all queries in one
-persistent launch per k class, optionally replayed as a CUDA graph.
+builds every cloud's LBVH as one forest and searches all queries in two
+persistent launches, optionally replayed as a CUDA graph.
 """
 from __future__ import annotations
 
