@@ -414,8 +414,6 @@ __global__ void __launch_bounds__(SWARPS * 32, 10) batch_collect_kernel(const Ba
     }
 }
 
-// A warp takes 32 consecutive queries, T lanes each at a time (T for the
-// longest list among them).
 __global__ void __launch_bounds__(256) batch_backward_kernel(const float *__restrict__ q, uint64_t nq,
                                                              const float *__restrict__ pts,
                                                              const uint32_t *__restrict__ qcloud,
@@ -423,20 +421,13 @@ __global__ void __launch_bounds__(256) batch_backward_kernel(const float *__rest
                                                              const uint32_t *__restrict__ ids,
                                                              const float *__restrict__ g, float *__restrict__ gq,
                                                              float *__restrict__ gp) {
-    const int lane = threadIdx.x & 31;
-    for (uint64_t i0 = ((uint64_t)blockIdx.x * 256 + threadIdx.x) & ~31ull; i0 < nq; i0 += (uint64_t)gridDim.x * 256) {
-        const uint32_t mine = i0 + lane < nq ? cd[qcloud[i0 + lane]].k : 0u;
-        const uint32_t T = backward_lanes(__reduce_max_sync(0xffffffffu, mine));
-        for (uint32_t r = 0; r < T; ++r) {
-            const uint64_t i = i0 + r * (32 / T) + lane / T;
-            const bool have = i < nq;
-            const CloudDesc &c = cd[have ? qcloud[i] : 0u];
-            const uint64_t ob = c.out_off + (uint64_t)(i - c.q_begin) * c.k;
-            // (a cloud's rows may start at an odd point, 4 bytes off)
-            float *const cgp = gp ? gp + 3 * (uint64_t)c.pt_begin : nullptr;
-            backward_query(have, q, pts + 3 * (uint64_t)c.pt_begin, c.n_pts, c.k, ids + ob, g + ob, gq, cgp, i, T,
-                           backward_pairs(cgp));
-        }
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < nq; i += (uint64_t)gridDim.x * 256) {
+        const CloudDesc &c = cd[qcloud[i]];
+        const uint64_t ob = c.out_off + (uint64_t)(i - c.q_begin) * c.k;
+        // (a cloud's rows may start at an odd point, 4 bytes off)
+        float *const cgp = gp ? gp + 3 * (uint64_t)c.pt_begin : nullptr;
+        backward_query(q, pts + 3 * (uint64_t)c.pt_begin, c.n_pts, c.k, ids + ob, g + ob, gq, cgp, i,
+                       backward_pairs(cgp));
     }
 }
 

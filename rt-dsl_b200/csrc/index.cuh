@@ -279,7 +279,7 @@ inline uint64_t chunk_begin(uint64_t nq, uint32_t chunks, uint32_t c) {
     return (c * nq + chunks - 1) / chunks;
 }
 
-// Creates the index's side and tree streams and their events on first use.
+// Creates the index's side stream and its events on first use.
 rtd_status ensure_side_stream(rtd_index *idx);
 
 // The sampled 1-NN seed of the last build (IndexHeader::nn95_key), computed

@@ -1111,15 +1111,9 @@ __global__ void __launch_bounds__(256) knn_backward_kernel(const float *__restri
                                                            const uint32_t *__restrict__ ids,
                                                            const float *__restrict__ g, float *__restrict__ gq,
                                                            float *__restrict__ gp) {
-    const uint32_t T = backward_lanes(k);
-    const int lane = threadIdx.x & 31;
     const bool pairs = backward_pairs(gp);
-    const uint64_t per = 32 / T;
-    for (uint64_t i0 = (((uint64_t)blockIdx.x * 256 + threadIdx.x) >> 5) * per; i0 < nq;
-         i0 += (((uint64_t)gridDim.x * 256) >> 5) * per) {
-        const uint64_t i = i0 + lane / T;
-        backward_query(i < nq, q, pts, n, k, ids + i * k, g + i * k, gq, gp, i, T, pairs);
-    }
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < nq; i += (uint64_t)gridDim.x * 256)
+        backward_query(q, pts, n, k, ids + i * k, g + i * k, gq, gp, i, pairs);
 }
 }  // namespace
 
@@ -1127,8 +1121,7 @@ rtd_status knn_backward(const float *q, uint64_t nq, const float *pts, uint64_t 
                         const uint32_t *ids, const float *g, float *gq, float *gp, cudaStream_t st) {
     if (nq == 0 || k == 0) return RTD_OK;
     if (!q || !pts || !ids || !g) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL input");
-    knn_backward_kernel<<<grid_for(nq * backward_lanes(k), 256, 148 * 16), 256, 0, st>>>(q, nq, pts, n, k, ids, g, gq,
-                                                                                        gp);
+    knn_backward_kernel<<<grid_for(nq, 256, 148 * 16), 256, 0, st>>>(q, nq, pts, n, k, ids, g, gq, gp);
     RTD_LAUNCH_CHECK();
     return RTD_OK;
 }
