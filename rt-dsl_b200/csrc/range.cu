@@ -385,10 +385,13 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
                     const uint32_t fl = first, fr = first + d.z;
                     bool v0 = !(box_min_key(qx, qy, qz, a.x, a.y, a.z, a.w, b.x, b.y) > r2);
                     bool v1 = !(box_min_key(qx, qy, qz, b.z, b.w, c.x, c.y, c.z, c.w) > r2);
-                    if (v0 && !(box_max_key(qx, qy, qz, a.x, a.y, a.z, a.w, b.x, b.y) > r2)) {
+                    const float far0 = box_max_key(qx, qy, qz, a.x, a.y, a.z, a.w, b.x, b.y);
+                    const float far1 = box_max_key(qx, qy, qz, b.z, b.w, c.x, c.y, c.z, c.w);
+                    // (an unbounded box holds a NaN point, as in range_kernel)
+                    if (v0 && far0 <= r2 && far0 < INFINITY) {
                         g0 = fl; n0 = d.z; v0 = false;
                     }
-                    if (v1 && !(box_max_key(qx, qy, qz, b.z, b.w, c.x, c.y, c.z, c.w) > r2)) {
+                    if (v1 && far1 <= r2 && far1 < INFINITY) {
                         g1 = fr; n1 = d.w; v1 = false;
                     }
                     if (v0 && (d.x & CHILD_LEAF)) { f0 = fl; c0 = d.z; v0 = false; }
