@@ -414,8 +414,11 @@ __global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 6) bh_walk_kernel(
                 }
                 const bool far = w2 < __fmul_rn(theta2, dot3_rn(dn[0], dn[1], dn[2]));
                 const bool near = !(w2 < __fmul_rn(theta2, dot3_rn(df[0], df[1], df[2])));
+                // (A centre with a NaN, from products that overflowed to inf -
+                // inf, is accepted by no body: then near holds, and far may
+                // too, since fmaxf drops the NaN.)
                 if (boxed && (far || near)) {
-                    if (far) A = e.y;
+                    if (!near) A = e.y;
                     open = false;
                 }
             }
