@@ -573,6 +573,8 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
     if (s.reserved != 0) return fail(RTD_ERR_INVALID_ARGUMENT, "schedule.reserved must be 0");
     if (s.radius_heuristic == RTD_RADIUS_FIXED && !(s.radius_param > 0.0f))
         return fail(RTD_ERR_INVALID_ARGUMENT, "fixed radius must be > 0");
+    if (s.radius_heuristic < 0 || s.radius_heuristic > RTD_RADIUS_MORTON_WINDOW)   // (also where no round uses it)
+        return fail(RTD_ERR_INVALID_ARGUMENT, "unknown radius heuristic");
     for (int e = EV_SEARCH0; e <= EV_SEARCH1; ++e) idx->ev_set[e] = false;
     idx->mark(EV_SEARCH0, st);
     // (only the radius rounds need an initial radius)
