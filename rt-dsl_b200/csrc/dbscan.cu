@@ -61,9 +61,15 @@ __global__ void dbscan_init_kernel(const uint32_t *__restrict__ counts, uint64_t
     }
 }
 
+// The fill's errors reach the host at the end of the call only.  After one,
+// slots of the pair buffer may never have been written (the points changed
+// since the count): the kernels that read pairs, and those that write labels,
+// return at once.
+
 // Core points under their smallest core neighbour.
 __global__ void dbscan_hook_kernel(const uint2 *__restrict__ pairs, uint64_t n_pairs,
-                                   const uint8_t *__restrict__ core, uint32_t *parent) {
+                                   const uint8_t *__restrict__ core, uint32_t *parent, const uint32_t *err) {
+    if (*err) return;
     for (uint64_t t = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; t < n_pairs;
          t += (uint64_t)gridDim.x * BLOCK) {
         const uint2 pr = pairs[t];
@@ -82,6 +88,7 @@ __global__ void dbscan_compress_kernel(uint64_t n, uint32_t *parent, uint32_t *e
 __global__ void dbscan_union_kernel(const uint2 *__restrict__ pairs, uint64_t n_pairs,
                                     const uint8_t *__restrict__ core, uint32_t *parent,
                                     uint32_t *err) {
+    if (*(volatile uint32_t *)err) return;
     for (uint64_t t = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; t < n_pairs;
          t += (uint64_t)gridDim.x * BLOCK) {
         const uint2 pr = pairs[t];
@@ -122,14 +129,16 @@ __global__ void dbscan_roots_kernel(uint64_t n, const uint8_t *__restrict__ core
 __global__ void dbscan_core_labels_kernel(uint64_t n, const uint8_t *__restrict__ core,
                                           const uint32_t *__restrict__ parent,
                                           const uint32_t *__restrict__ rank,
-                                          int32_t *__restrict__ labels) {
+                                          int32_t *__restrict__ labels, const uint32_t *err) {
+    if (*err) return;
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * BLOCK)
         labels[i] = core[i] ? (int32_t)rank[parent[i]] : INT_MAX;
 }
 
 __global__ void dbscan_border_kernel(const uint2 *__restrict__ pairs, uint64_t n_pairs,
-                                     const uint8_t *__restrict__ core, int32_t *labels) {
+                                     const uint8_t *__restrict__ core, int32_t *labels, const uint32_t *err) {
+    if (*err) return;
     for (uint64_t t = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; t < n_pairs;
          t += (uint64_t)gridDim.x * BLOCK) {
         const uint2 pr = pairs[t];
@@ -137,7 +146,8 @@ __global__ void dbscan_border_kernel(const uint2 *__restrict__ pairs, uint64_t n
     }
 }
 
-__global__ void dbscan_noise_kernel(uint64_t n, int32_t *labels) {
+__global__ void dbscan_noise_kernel(uint64_t n, int32_t *labels, const uint32_t *err) {
+    if (*err) return;
     for (uint64_t i = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * BLOCK)
         if (labels[i] == INT_MAX) labels[i] = -1;
@@ -170,7 +180,7 @@ extern "C" rtd_status rtd_dbscan(rtd_index *idx, const float *d_points, uint64_t
     RTD_TRY(pairs.reserve(total * 8 + 8));
     uint64_t written = 0;
     RTD_TRY(range_fill(idx, d_points, n, eps, nullptr, pairs.as<uint32_t>(), total, 0, &written, st,
-                       false));   // (errors are read at the end)
+                       false));   // (errors are read at the end, and by the kernels)
     RTD_TRY(core.reserve(n));
     RTD_TRY(parent.reserve(n * 4));
     RTD_TRY(flag.reserve(n * 4));
@@ -182,7 +192,7 @@ extern "C" rtd_status rtd_dbscan(rtd_index *idx, const float *d_points, uint64_t
     RTD_LAUNCH_CHECK();
     if (total) {
         dbscan_hook_kernel<<<gp, BLOCK, 0, st>>>(pairs.as<uint2>(), total, core.as<uint8_t>(),
-                                                 parent.as<uint32_t>());
+                                                 parent.as<uint32_t>(), err);
         RTD_LAUNCH_CHECK();
         dbscan_compress_kernel<<<g, BLOCK, 0, st>>>(n, parent.as<uint32_t>(), err);
         RTD_LAUNCH_CHECK();
@@ -198,14 +208,14 @@ extern "C" rtd_status rtd_dbscan(rtd_index *idx, const float *d_points, uint64_t
     uint32_t *d_nc = ncbuf.as<uint32_t>();
     RTD_TRY(exclusive_scan_u32_32(flag.as<uint32_t>(), rank.as<uint32_t>(), n, d_nc, scan, err, st));
     dbscan_core_labels_kernel<<<g, BLOCK, 0, st>>>(n, core.as<uint8_t>(), parent.as<uint32_t>(),
-                                                   rank.as<uint32_t>(), d_labels);
+                                                   rank.as<uint32_t>(), d_labels, err);
     RTD_LAUNCH_CHECK();
     if (total) {
         dbscan_border_kernel<<<gp, BLOCK, 0, st>>>(pairs.as<uint2>(), total, core.as<uint8_t>(),
-                                                   d_labels);
+                                                   d_labels, err);
         RTD_LAUNCH_CHECK();
     }
-    dbscan_noise_kernel<<<g, BLOCK, 0, st>>>(n, d_labels);
+    dbscan_noise_kernel<<<g, BLOCK, 0, st>>>(n, d_labels, err);
     RTD_LAUNCH_CHECK();
     uint32_t nc = 0;
     RTD_CUDA(cudaMemcpyAsync(&nc, d_nc, sizeof(nc), cudaMemcpyDeviceToHost, st));
