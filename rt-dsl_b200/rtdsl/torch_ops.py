@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 
 from ._capi import BH_LAW_PLUMMER, default_bh_params, default_schedule
-from .api import knn_backward, short_lived_index
+from .api import _check_points_tensor, knn_backward, short_lived_index
 from .bh import BarnesHut
 
 
@@ -24,6 +24,8 @@ class KnnDistances(torch.autograd.Function):
     def forward(ctx, queries, points, k: int, schedule=None):
         s = schedule if schedule is not None else default_schedule()
         p, q = points.detach().contiguous(), queries.detach().contiguous()
+        _check_points_tensor(p, "points")
+        _check_points_tensor(q, "queries")
         with short_lived_index(p.device, p.shape[0], q.shape[0]) as ix:
             ids, d2 = ix.build(p, s).knn(q, k, s)
         ctx.save_for_backward(queries, points, ids)
