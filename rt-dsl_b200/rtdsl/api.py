@@ -252,22 +252,25 @@ _kept = threading.local()
 
 @contextlib.contextmanager
 def short_lived_index(device, n: int, nq: int):
-    """An Index for work on the current stream that is all enqueued when the
-    block ends.  A kept one was last used by work that an event marks; the
-    current stream, whichever it is, waits for it."""
+    """An Index for work on `device`'s current stream that is all enqueued when
+    the block ends; the block runs with that device current, on which the
+    index's buffers and launches therefore are.  A kept one was last used by
+    work that an event marks; the current stream, whichever it is, waits for
+    it."""
     import torch
-    st = torch.cuda.current_stream(device)
     entry, _kept.entry = getattr(_kept, "entry", None), None   # (a nested call makes its own)
-    if entry is not None and entry[0] == device:
-        _, ix, done = entry
-        st.wait_event(done)
-    else:
-        ix, done = Index(), torch.cuda.Event()
-    yield ix   # an exception drops the index
-    if max(n, nq) <= KEPT_INDEX_MAX:
-        done.record(st)
-        ix.points = None
-        _kept.entry = (device, ix, done)
+    with torch.cuda.device(device):
+        st = torch.cuda.current_stream()
+        if entry is not None and entry[0] == device:
+            _, ix, done = entry
+            st.wait_event(done)
+        else:
+            ix, done = Index(), torch.cuda.Event()
+        yield ix   # an exception drops the index
+        if max(n, nq) <= KEPT_INDEX_MAX:
+            done.record(st)
+            ix.points = None
+            _kept.entry = (device, ix, done)
 
 
 def release_kept_index() -> None:
