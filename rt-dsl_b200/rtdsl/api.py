@@ -244,14 +244,17 @@ class Index:
 # The index a thread keeps between calls that need one only for their own
 # duration: creating an index and its two dozen device buffers, and freeing
 # them, takes 2 to 5 ms of host time, several times the search of a training
-# step.  One per thread, for up to this many points and queries (about 400 MB
-# at the most); release_kept_index() gives it back, as the thread's end does.
+# step.  One per thread, for up to this many points and queries (287 MB at the
+# most) and for lists that need no slab on the index (up to 1 GiB above this
+# many neighbours, whatever the sizes); release_kept_index() gives it back, as
+# the thread's end does.
 KEPT_INDEX_MAX = 1 << 21
+KEPT_LIST_MAX = 2048
 _kept = threading.local()
 
 
 @contextlib.contextmanager
-def short_lived_index(device, n: int, nq: int):
+def short_lived_index(device, n: int, nq: int, k: int):
     """An Index for work on `device`'s current stream that is all enqueued when
     the block ends; the block runs with that device current, on which the
     index's buffers and launches therefore are.  A kept one was last used by
@@ -267,7 +270,7 @@ def short_lived_index(device, n: int, nq: int):
         else:
             ix, done = Index(), torch.cuda.Event()
         yield ix   # an exception drops the index
-        if max(n, nq) <= KEPT_INDEX_MAX:
+        if max(n, nq) <= KEPT_INDEX_MAX and min(k, n) <= KEPT_LIST_MAX:
             done.record(st)
             ix.points = None
             _kept.entry = (device, ix, done)

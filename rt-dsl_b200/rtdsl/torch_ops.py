@@ -26,7 +26,7 @@ class KnnDistances(torch.autograd.Function):
         p, q = points.detach().contiguous(), queries.detach().contiguous()
         _check_points_tensor(p, "points")
         _check_points_tensor(q, "queries")
-        with short_lived_index(p.device, p.shape[0], q.shape[0]) as ix:
+        with short_lived_index(p.device, p.shape[0], q.shape[0], k) as ix:
             ids, d2 = ix.build(p, s).knn(q, k, s)
         ctx.save_for_backward(queries, points, ids)
         ctx.mark_non_differentiable(ids)

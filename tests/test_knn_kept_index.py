@@ -81,15 +81,26 @@ def test_kept_index_lives_on_the_device_of_its_points(fake):
     from rtdsl.api import short_lived_index
     one = torch.device("cuda", 1)
     for _ in range(2):   # the current device is 0
-        with short_lived_index(one, 10, 10) as ix:
+        with short_lived_index(one, 10, 10, 5) as ix:
             ix.use()
     assert fake.now == 0
     fake.now = 1
-    with short_lived_index(one, 10, 10) as ix:
+    with short_lived_index(one, 10, 10, 5) as ix:
         ix.use()
     fake.now = 0
-    with short_lived_index(torch.device("cuda", 0), 10, 10) as ix:
+    with short_lived_index(torch.device("cuda", 0), 10, 10, 5) as ix:
         ix.use()
     # made, used, awaited and marked on one and the same device
     assert fake.log == [("use", 1, 1), ("record", 1), ("wait", 1, 1), ("use", 1, 1), ("record", 1),
                         ("wait", 1, 1), ("use", 1, 1), ("record", 1), ("use", 0, 0), ("record", 0)]
+
+
+@pytest.mark.parametrize("n,nq,k,kept", [(5_000, 10, 2048, True), (5_000, 10, 2049, False), (2_048, 10, 9_000, True),
+                                         (1 << 21, 1 << 21, 1, True), ((1 << 21) + 1, 1, 1, False),
+                                         (1, (1 << 21) + 1, 1, False)])
+def test_kept_index_is_bounded(fake, n, nq, k, kept):
+    """Lists above 2,048 entries take a slab of up to 1 GiB on the index."""
+    from rtdsl import api
+    with api.short_lived_index(torch.device("cuda", 0), n, nq, k) as ix:
+        ix.use()
+    assert (api._kept.entry is not None) == kept
