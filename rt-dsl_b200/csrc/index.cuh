@@ -47,9 +47,12 @@ struct IndexHeader {
     uint32_t heavy;       // hits of a sample of the queries (range.cu, launch_count)
     unsigned long long qfp[2];   // query fingerprints of the last range count / fill
     // last range count (cleared together): pairs pushed, records, points the
-    // records cover; the largest count.  A pushing fill uses rcur[0].
-    unsigned long long rcur[3];
-    uint32_t most;
+    // records cover; the largest count.  A pushing fill uses rcur[0].  Each in
+    // a cache line of its own: the pushes are atomics on one address, and the
+    // blocks that start meanwhile read the fields above (1.8M uniform points,
+    // 400,000 queries, 25 hits, pushing count: 1.56 ms in one line, now 1.51).
+    alignas(128) unsigned long long rcur[3];
+    alignas(128) uint32_t most;
 };
 
 // The Karras nodes kept in the tree, a bit each, and the kept nodes before
