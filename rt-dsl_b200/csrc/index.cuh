@@ -44,7 +44,8 @@ struct IndexHeader {
     uint64_t total;       // last range-count total
     float nn95_key;       // p95 of the squared 1-NN distance within a 4096-point sample
     uint32_t n_sample;    // points in the radius-seed sample (<= 1000)
-    uint32_t heavy;       // hits of a sample of the queries (range.cu, launch_count)
+    uint32_t sample_sum, sample_most;   // hits of a sample of the queries, and the
+                                        // largest of them (range.cu, launch_pass)
     unsigned long long qfp[2];   // query fingerprints of the last range count / fill
     // last range count (cleared together): pairs pushed, records, points the
     // records cover; the largest count.  A pushing fill uses rcur[0].  Each in

@@ -25,7 +25,7 @@ constexpr uint32_t WRECS = 64;     // staged records per warp (1 KB)
 // Kernel modes: count hits, push pairs through warp staging and a global
 // cursor, write pairs into per-query segments at known offsets, or count
 // hits and push them at once (a count whose pairs the next fill scatters).
-// MODE_SAMPLE counts a sample of the queries for launch_count.
+// MODE_SAMPLE counts a sample of the queries for launch_pass.
 enum : int { MODE_COUNT = 0, MODE_PUSH = 1, MODE_SEG = 2, MODE_CPUSH = 3, MODE_SAMPLE = 4 };
 
 struct RangeArgs {
@@ -36,10 +36,10 @@ struct RangeArgs {
     const uint32_t *perm;
     float r2;
     uint32_t *counts;
-    uint32_t *most;            // counts: the largest count
-    int if_heavy;              // counts: do nothing unless the header's heavy says so
+    uint32_t *most;            // counts and MODE_SAMPLE: the largest count
+    int by_sample;             // the sample of the queries says which kernel runs (warp_walks)
     uint64_t sample_step;      // MODE_SAMPLE: every sample_step-th query
-    uint32_t heavy_at;         // MODE_SAMPLE: hits that alone make the count heavy
+    uint32_t *sample_sum;      // MODE_SAMPLE: the sum of the counts
     uint2 *pairs;
     uint64_t capacity;
     unsigned long long *cursor;
@@ -55,10 +55,15 @@ struct RangeArgs {
     uint32_t *err;
 };
 
-// IndexHeader::heavy sums the hits of a sample of the queries, in which one of
-// heavy_at hits counts for all of HEAVY_SUM (launch_count).
-constexpr uint64_t HEAVY_SAMPLE = 1024;
-constexpr uint32_t HEAVY_SUM = 64 * HEAVY_SAMPLE;
+// Whether a warp per query is ahead of a thread per query, by the hits of
+// SAMPLE of the nq queries (launch_pass says why the lines lie here).
+constexpr uint64_t SAMPLE = 1024;
+template <int MODE>
+__device__ __forceinline__ bool warp_walks(const IndexHeader *h, uint64_t nq) {
+    const uint64_t sum = h->sample_sum, most = h->sample_most;
+    if (sum >= 64 * SAMPLE || most * SAMPLE >= nq) return true;
+    return sum * sum * (MODE == MODE_CPUSH ? 2800 : 100) >= nq * SAMPLE * SAMPLE;
+}
 
 // Shared memory of one warp: the boxes to visit (level << 28 | entry), runs
 // of 8 points to test, staged pairs and records.
@@ -91,7 +96,7 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
     constexpr bool SEG = MODE == MODE_SEG;
     constexpr bool COUNTS = MODE == MODE_COUNT || MODE == MODE_CPUSH;
     if (SEG && p.skip_if_same && p.ix.hdr->qfp[0] == p.ix.hdr->qfp[1]) return;
-    if (COUNTS && p.if_heavy && p.ix.hdr->heavy < HEAVY_SUM) return;
+    if (MODE != MODE_SAMPLE && p.by_sample && !warp_walks<MODE>(p.ix.hdr, p.nq)) return;
     extern __shared__ uint4 s_dyn[];
     __shared__ uint32_t s_off[12];
     const uint32_t n = (uint32_t)p.ix.n;
@@ -265,7 +270,10 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
         }
         if (COUNTS && lane == 0) p.counts[qi] = cnt;
         if (COUNTS) most = cnt > most ? cnt : most;
-        if (MODE == MODE_SAMPLE && lane == 0) atomicAdd(p.most, cnt < p.heavy_at ? (cnt < HEAVY_SUM ? cnt : HEAVY_SUM) : HEAVY_SUM);
+        if (MODE == MODE_SAMPLE) {
+            most = cnt > most ? cnt : most;
+            if (lane == 0) atomicAdd(p.sample_sum, cnt < 64 * SAMPLE ? cnt : (uint32_t)(64 * SAMPLE));
+        }
         // a segment left short or overrun: the queries changed since the count
         if (SEG && (seg_bad || cnt != wlen)) atomicOr(p.err, DEVERR_MISMATCH);
     }
@@ -274,7 +282,7 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
         flush_recs();
         if (lane == 0 && covered) atomicAdd(&p.cursor[2], covered);
     }
-    if (COUNTS && lane == 0 && most) atomicMax(p.most, most);
+    if ((COUNTS || MODE == MODE_SAMPLE) && lane == 0 && most) atomicMax(p.most, most);
 }
 
 constexpr int SHORT_DEPTH = 12;  // stack entries per thread in shared memory
@@ -294,28 +302,37 @@ __device__ __forceinline__ void load_node_r(const BvhNode *__restrict__ s_top,
 
 // Fields of the per-lane work a traversal step stages for the warp (one
 // 32-word row per field, so lanes reading different owners hit different
-// banks).
-enum : int { F_QX = 0, F_QY, F_QZ, F_QI, F_F0, F_C0, F_F1, F_DONE, F_COUNT };
+// banks): the counts need the first, the fills the others too.
+enum : int { F_QX = 0, F_QY, F_QZ, F_QI, F_F0, F_C0, F_F1, F_DONE, F_COUNT,
+             F_T = F_COUNT, F_G0, F_N0, F_G1, F_PUSH, F_WLEN = F_PUSH, F_WBLO, F_WBHI, F_SEG };
+constexpr uint32_t BIG_SUB = 32;  // contained subtrees of this size or more: copied by the warp
 
-// The counting passes (MODE_COUNT, MODE_CPUSH) a thread per query over the
-// binary tree: where many queries have few hits each, its tighter boxes and
-// 32 walks a warp need less than half the instructions of range_kernel
-// (launch_count says when).  Threads of a warp advance their own traversals
-// one node per iteration of a warp-converged loop; a stack entry carries the
-// node and the first sorted point below it.  A child whose whole box lies
-// inside the ball counts without a test (pushed as a record).  After each
-// step the points of the leaves that straddle the sphere are flattened over
-// the warp by a prefix sum and tested 32 at a time: a lane finds its
-// candidate's owner by a binary search over the prefix (shuffles) and reads
-// the owner's query and ranges from shared memory.
+// A thread per query over the binary tree: where many queries have few hits
+// each, its tighter boxes and 32 walks a warp need less than half the
+// instructions of range_kernel (launch_pass says when).  Threads of a warp
+// advance their own traversals one node per iteration of a warp-converged
+// loop; a stack entry carries the node and the first sorted point below it.  A
+// child whose whole box lies inside the ball contributes its points without a
+// test: their number in the counts (MODE_CPUSH: a record), their ids in the
+// fills, by the whole warp for BIG_SUB points and more.  After each step the
+// lanes' other work, points of the leaves that straddle the sphere and (fills)
+// of small contained subtrees, is flattened over the warp by a prefix sum and
+// handled 32 points at a time: a lane finds its candidate's owner by a binary
+// search over the prefix (shuffles) and reads the owner's query and ranges
+// from shared memory.  MODE_SEG writes an owner's hits at the next slots of
+// its segment and checks that the query fills it exactly; the pushing modes
+// compact them into the warp's staging buffer.
 template <int MODE>
 __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thread_kernel(const RangeArgs p) {
-    constexpr bool PUSH = MODE == MODE_CPUSH;
-    if (p.ix.hdr->heavy >= HEAVY_SUM) return;
+    constexpr bool PUSH = MODE == MODE_PUSH || MODE == MODE_CPUSH;   // through warp staging
+    constexpr bool COUNTS = MODE == MODE_COUNT || MODE == MODE_CPUSH;
+    constexpr bool SEG = MODE == MODE_SEG, FILL = !COUNTS;
+    constexpr int NF = SEG ? F_SEG : FILL ? F_PUSH : F_COUNT;
+    if (warp_walks<MODE>(p.ix.hdr, p.nq)) return;
     __shared__ BvhNode s_top[TOP_MAX];
     __shared__ uint2 s_stack[SHORT_DEPTH][RBLOCK];
     __shared__ uint2 s_buf[PUSH ? RWARPS : 1][PUSH ? WBUF : 1];
-    __shared__ uint32_t s_work[RWARPS][F_COUNT][32];
+    __shared__ uint32_t s_work[RWARPS][NF][32];
     const IndexHeader *h = p.ix.hdr;
     const uint32_t ntop = h->n_top;
     for (uint32_t i = threadIdx.x; i < ntop; i += RBLOCK) s_top[i] = p.ix.top[i];
@@ -339,6 +356,7 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
         __syncwarp();
         for (uint32_t j = lane; j < fill; j += 32)
             if (base + j < p.capacity) p.pairs[base + j] = buf[j];
+        if (MODE == MODE_PUSH && lane == 0 && base + fill > p.capacity) atomicOr(p.err, DEVERR_OVERFLOW);
         __syncwarp();
         fill = 0;
     };
@@ -358,6 +376,17 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
         W[F_QZ][lane] = __float_as_uint(qz);
         W[F_QI][lane] = (uint32_t)qi;
         W[F_DONE][lane] = 0;
+        if (SEG) {   // this query's segment of the pair buffer
+            uint64_t wb = 0, wend = 0;
+            if (have) {
+                wb = p.offsets[qi];
+                wend = qi + 1 < p.nq ? p.offsets[qi + 1] : p.total;
+            }
+            W[F_WLEN][lane] = (uint32_t)(wend - wb);
+            W[F_WBLO][lane] = (uint32_t)wb;
+            W[F_WBHI][lane] = (uint32_t)(wb >> 32);
+        }
+        bool seg_bad = false;
         // a query with a NaN coordinate has no neighbours (its keys are NaN)
         const bool live = have && !isnan(qx) && !isnan(qy) && !isnan(qz);
         uint32_t node = (live && root != CHILD_NONE) ? root : CHILD_NONE;
@@ -424,8 +453,8 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
                 node = next;
                 first = next_first;
             }
-            cnt += n0 + n1;
-            if (PUSH) {
+            if (COUNTS) cnt += n0 + n1;
+            if (MODE == MODE_CPUSH) {
                 const uint32_t rm0 = __ballot_sync(0xffffffffu, n0 != 0);
                 const uint32_t rm1 = __ballot_sync(0xffffffffu, n1 != 0);
                 const uint32_t nr = __popc(rm0) + __popc(rm1);
@@ -446,8 +475,46 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
                     if (n1 && r < p.rec_cap) p.recs[r] = make_uint4((uint32_t)qi, g1, n1, 0u);
                 }
             }
+            if (FILL) {
+                // contained subtrees of BIG_SUB points or more: their
+                // contiguous ids, one pair per lane
+                const uint32_t b0 = n0 >= BIG_SUB ? n0 : 0u, b1 = n1 >= BIG_SUB ? n1 : 0u;
+                if (b0) n0 = 0;
+                if (b1) n1 = 0;
+                for (uint32_t m = __ballot_sync(0xffffffffu, (b0 | b1) != 0); m; m &= m - 1) {
+                    const int src = __ffs(m) - 1;
+                    const uint32_t sq = W[F_QI][src];
+                    for (int r = 0; r < 2; ++r) {
+                        const uint32_t gs = __shfl_sync(0xffffffffu, r ? g1 : g0, src);
+                        const uint32_t ns = __shfl_sync(0xffffffffu, r ? b1 : b0, src);
+                        if (ns == 0) continue;
+                        if (SEG) {
+                            const uint32_t done = W[F_DONE][src];
+                            if ((uint64_t)done + ns <= W[F_WLEN][src]) {
+                                const uint64_t dst = ((uint64_t)W[F_WBHI][src] << 32 | W[F_WBLO][src]) + done;
+                                for (uint32_t k = lane; k < ns; k += 32)
+                                    p.pairs[dst + k] = make_uint2(sq, __float_as_uint(__ldg(&pts[gs + k].w)));
+                            } else {
+                                seg_bad = true;
+                            }
+                            __syncwarp();
+                            if (lane == src) W[F_DONE][src] = done + ns;
+                            __syncwarp();
+                        } else {
+                            for (uint32_t k = 0; k < ns; k += 32) {
+                                const uint32_t take = ns - k < 32u ? ns - k : 32u;
+                                if ((uint32_t)lane < take)
+                                    buf[fill + lane] = make_uint2(sq, __float_as_uint(__ldg(&pts[gs + k + lane].w)));
+                                fill += take;
+                                __syncwarp();
+                                if (fill > WBUF - 32) flush();
+                            }
+                        }
+                    }
+                }
+            }
             // flatten this step's candidates over the warp
-            const uint32_t items = c0 + c1;
+            const uint32_t tl = c0 + c1, items = tl + (FILL ? n0 + n1 : 0u);
             uint32_t incl = items;
 #pragma unroll
             for (int dlt = 1; dlt < 32; dlt <<= 1) {
@@ -460,6 +527,12 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
             W[F_F0][lane] = f0;
             W[F_C0][lane] = c0;
             W[F_F1][lane] = f1;
+            if (FILL) {
+                W[F_T][lane] = tl;
+                W[F_G0][lane] = g0;
+                W[F_N0][lane] = n0;
+                W[F_G1][lane] = g1;
+            }
             __syncwarp();
             for (uint32_t base = 0; base < total; base += 32) {
                 const uint32_t ci = base + lane;
@@ -475,7 +548,11 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
                 const uint32_t oitems = __shfl_sync(0xffffffffu, items, o);
                 bool hit = false;
                 uint32_t id = 0;
-                if (valid) {
+                if (FILL && valid && ci - oexcl >= W[F_T][o]) {   // a point of a contained subtree
+                    const uint32_t j = ci - oexcl - W[F_T][o], on0 = W[F_N0][o];
+                    id = __float_as_uint(__ldg(&pts[j < on0 ? W[F_G0][o] + j : W[F_G1][o] + (j - on0)].w));
+                    hit = true;
+                } else if (valid) {
                     const uint32_t j = ci - oexcl, oc0 = W[F_C0][o];
                     const uint32_t pi = j < oc0 ? W[F_F0][o] + j : W[F_F1][o] + (j - oc0);
                     const float4 pt = __ldg(&pts[pi]);
@@ -495,20 +572,33 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
                     fill += __popc(hm);
                     if (fill > WBUF - 32) flush();
                 }
-                if (valid && lane == re) W[F_DONE][o] += __popc(hm & upto_re & ~below_rs);
+                const uint32_t done = SEG ? W[F_DONE][o] : 0u;
+                if (SEG) {
+                    const uint32_t at = done + __popc(hm & lt & ~below_rs);
+                    if (hit && at < W[F_WLEN][o])
+                        p.pairs[((uint64_t)W[F_WBHI][o] << 32 | W[F_WBLO][o]) + at] = make_uint2(W[F_QI][o], id);
+                    seg_bad |= hit && at >= W[F_WLEN][o];
+                    __syncwarp();
+                }
+                if (valid && lane == re)
+                    W[F_DONE][o] = (SEG ? done : W[F_DONE][o]) + __popc(hm & upto_re & ~below_rs);
                 __syncwarp();
             }
         }
         __syncwarp();
-        if (have) {
+        // a segment left short or overrun: the queries changed since the count
+        if (SEG && (seg_bad || (have && W[F_DONE][lane] != W[F_WLEN][lane]))) atomicOr(p.err, DEVERR_MISMATCH);
+        if (COUNTS && have) {
             const uint32_t c = cnt + W[F_DONE][lane];
             p.counts[qi] = c;
             most = c > most ? c : most;
         }
     }
     flush();
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (lane == 0 && most) atomicMax(p.most, most);
+    if (COUNTS) {
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0 && most) atomicMax(p.most, most);
+    }
 }
 
 // Order-free 64-bit fingerprint of a query array (wrapping sum of mixed
@@ -778,12 +868,11 @@ __global__ void own_order_kernel(const float4 *__restrict__ pts, uint64_t n, uin
 }
 
 constexpr uint64_t RANGE_ORDER_MIN = 49152, RANGE_ORDER_POINTS = 2ull << 20;
-constexpr uint64_t THREAD_QUERIES = 131072;   // see launch_count
+constexpr uint64_t THREAD_QUERIES = 131072;   // see launch_pass
 rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r, cudaStream_t st);
 
 rtd_status range_args(rtd_index *idx, const float *d_q, uint64_t nq, float r,
-                      const rtd_schedule *sched, RangeArgs &a, cudaStream_t st, bool count,
-                      bool own_points = false) {
+                      const rtd_schedule *sched, RangeArgs &a, cudaStream_t st, bool own_points = false) {
     if (!idx || !idx->hdr.ptr) return fail(RTD_ERR_INVALID_ARGUMENT, "index not built");
     if (nq && !d_q) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL queries");
     if (!(r >= 0.0f)) return fail(RTD_ERR_INVALID_ARGUMENT, "radius must be >= 0");
@@ -797,7 +886,7 @@ rtd_status range_args(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     idx->mark(EV_SEEDED, st);
     // A thread's walk needs its warp's queries to be neighbours; a warp's
     // gains from the order only as the k-NN warp search does (knn.cu).
-    const bool sample = count && nq >= THREAD_QUERIES;
+    const bool sample = nq >= THREAD_QUERIES;
     const bool wants_order = nq >= THREAD_QUERIES || (nq >= RANGE_ORDER_MIN && idx->n >= RANGE_ORDER_POINTS);
     if (sample) RTD_TRY(launch_sample(idx, d_q, nq, r, st));
     rtd_status os;
@@ -858,32 +947,50 @@ rtd_status launch_range(RangeArgs &a, cudaStream_t st) {
     return RTD_OK;
 }
 
-// Which kernel counts.  A thread per query takes about 0.8 ns + 0.03 ns a hit
-// for each, a warp per query 2.2 ns + 0.01 ns a hit: the thread is ahead below
-// some 60 hits on average.  But a warp of 32 threads takes as long as its
-// longest walk, some 1.1 us for each of that query's hits, and the last such
-// warp ends the launch: with fewer than about 500 queries for every hit of the
-// largest query (1,000 for the largest of a sample, which misses the top) the
-// warp kernel is ahead.  Measured, counting with pushes, thread / warp, ms:
-// 1.8M points, 400,000 queries, clustered: 1 hit on average 0.35 / 0.88, 8
-// hits (230 at the most) 0.64 / 0.93, 50 hits (1,456) 1.54 / 1.10; uniform, 50
-// hits (87) 0.99 / 1.11; 200,000 of each, 20 hits (513) 0.61 / 0.44; clustered
-// points as their own queries, 1.8M with 20 hits 1.8 / 3.9, 600,000 with 8
-// hits 0.54 / 1.03; 20,000 queries on 50,000 points, 10 hits 0.20 / 0.12.  From
-// THREAD_QUERIES on, a sample of the queries says on the device
-// (IndexHeader::heavy) which of the two launches does the work; it runs on the
-// side stream beside the query ordering.
+// Which kernel counts or fills.  A thread per query costs less where the hits
+// are few: the warp kernel takes about 1.8 ns a query besides the hits.  But a
+// warp of 32 threads takes as long as its longest walk, some 1.1 us for each
+// of that query's hits, and the last such warp ends the launch: the warp
+// kernel is ahead with fewer than 500 to 1,000 queries for every hit of the
+// largest query (1,024 for the largest of a sample, which misses the top).
+// And it is ahead from some mean number of hits on, which grows as the root of
+// the number of queries:
+// 400,000 queries fill the SMs with threads, 100,000 do not, and the threads'
+// pushes (one reservation for every step of a warp) queue up on the cursors.
+// Measured, thread / warp, us; 1.8M points:
+//                       400,000 queries: count  segment fill  pushing count
+//   uniform     1 hit              152 / 491     170 / 526     184 / 529
+//               8                  363 / 645     396 / 701     610 / 690
+//               12                 427 / 680     471 / 744     834 / 731
+//               50                 774 / 905    902 / 1016   2240 / 1002
+//   clustered   8, 308 at most     408 / 773     537 / 830     620 / 819
+//               20, 802            663 / 830     998 / 903    1157 / 893
+//               50, 1849          1109 / 921   1845 / 1011   2079 / 1014
+//                       100,000 queries:
+//   uniform     1 hit               75 / 133      72 / 144      82 / 150
+//               8                  142 / 173     141 / 189     223 / 194
+//               32                 221 / 216     248 / 240     524 / 246
+//   clustered   1, 32 at most      145 / 189     143 / 202     168 / 209
+//               4, 145             234 / 201     282 / 210     320 / 216
+//   1.8M clustered points as their own queries, 20 hits, 813 at most:
+//                                1431 / 3611   1867 / 3955   3469 / 3910
+// The queries have to be in order for the threads' walks (50 us), before the
+// sample can say which kernel runs, which decides below THREAD_QUERIES: count
+// and first fill of 100,000 queries on 1.8M uniform points with it, 1 hit 200
+// / 280 us, 8 hits 330 / 370, and count and fill with pushes, 8 hits 330 (in
+// order, then a warp a query) / 270; 50,000 queries, 1 hit 180 / 163, 8 hits
+// 289 / 205.  The sample runs on the side stream beside the ordering.
 template <int MODE>
-rtd_status launch_count(RangeArgs &a, cudaStream_t st) {
-    a.if_heavy = a.nq >= THREAD_QUERIES;
-    if (a.if_heavy) {
+rtd_status launch_pass(RangeArgs &a, cudaStream_t st) {
+    a.by_sample = a.nq >= THREAD_QUERIES;
+    if (a.by_sample) {
         range_thread_kernel<MODE><<<grid_for(a.nq, RBLOCK, 1 << 20), RBLOCK, 0, st>>>(a);
         RTD_LAUNCH_CHECK();
     }
     return launch_range<MODE>(a, st);
 }
 
-// Starts the sample of launch_count on the side stream.
+// Starts the sample of launch_pass on the side stream.
 rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r, cudaStream_t st) {
     RTD_TRY(ensure_side_stream(idx));
     cudaStream_t side = idx->side_stream;
@@ -894,13 +1001,13 @@ rtd_status launch_sample(rtd_index *idx, const float *d_q, uint64_t nq, float r,
     a.ix = view_of(idx);
     a.pyr = idx->pyramid.as<float4>();
     a.q = d_q;
-    a.nq = HEAVY_SAMPLE;
-    a.sample_step = nq / HEAVY_SAMPLE;
-    a.heavy_at = (uint32_t)(nq / HEAVY_SAMPLE);
+    a.nq = SAMPLE;
+    a.sample_step = nq / SAMPLE;
     a.r2 = r * r;
-    a.most = &h->heavy;
+    a.sample_sum = &h->sample_sum;
+    a.most = &h->sample_most;
     a.err = &h->err;
-    const cudaError_t me = cudaMemsetAsync(&h->heavy, 0, sizeof(uint32_t), side);
+    const cudaError_t me = cudaMemsetAsync(&h->sample_sum, 0, 2 * sizeof(uint32_t), side);
     const rtd_status s = launch_range<MODE_SAMPLE>(a, side);
     RTD_CUDA(cudaEventRecord(idx->ev_join, side));
     if (me != cudaSuccess || s != RTD_OK) {
@@ -920,7 +1027,7 @@ rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
                        cudaStream_t st, bool own_points) {
     if (!d_counts && nq) return fail(RTD_ERR_INVALID_ARGUMENT, "NULL counts");
     RangeArgs a = {};
-    RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, true, own_points));
+    RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, own_points));
     a.counts = d_counts;
     IndexHeader *h = idx->hdr.as<IndexHeader>();
     // With a buffer left by an earlier count, this count also pushes its
@@ -936,9 +1043,9 @@ rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
             a.recs = idx->rrec.as<uint4>();
             a.rec_cap = idx->rrec_cap;
             RTD_TRY(query_fingerprint(d_q, nq, &h->qfp[0], st));
-            RTD_TRY(launch_count<MODE_CPUSH>(a, st));
+            RTD_TRY(launch_pass<MODE_CPUSH>(a, st));
         } else {
-            RTD_TRY(launch_count<MODE_COUNT>(a, st));
+            RTD_TRY(launch_pass<MODE_COUNT>(a, st));
         }
         idx->mark(EV_SEARCH1, st);
         RTD_TRY(idx->roffsets.reserve(nq * sizeof(uint64_t)));
@@ -1023,7 +1130,7 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
         a.skip_if_same = 0;
         a.err = &idx->hdr.as<IndexHeader>()->err;
     } else {
-        RTD_TRY(range_args(idx, d_q, nq, r, s, a, st, false));
+        RTD_TRY(range_args(idx, d_q, nq, r, s, a, st));
         IndexHeader *h = idx->hdr.as<IndexHeader>();
         RTD_CUDA(cudaMemsetAsync(h->rcur, 0, sizeof(unsigned long long), st));
         a.cursor = h->rcur;
@@ -1054,11 +1161,11 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
         a.skip_if_same = 1;
         RTD_TRY(launch_range<MODE_SEG>(a, st));
         idx->mark(EV_SEARCH1, st);
-    } else if (seg) {
-        RTD_TRY(launch_range<MODE_SEG>(a, st));
+    } else if (seg) {   // (the count's sample of the queries still stands)
+        RTD_TRY(launch_pass<MODE_SEG>(a, st));
         idx->mark(EV_SEARCH1, st);
     } else if (nq) {
-        RTD_TRY(launch_range<MODE_PUSH>(a, st));
+        RTD_TRY(launch_pass<MODE_PUSH>(a, st));
         idx->mark(EV_SEARCH1, st);
     }
     unsigned long long total = 0;
