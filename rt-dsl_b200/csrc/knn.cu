@@ -481,28 +481,35 @@ rtd_status knn_search(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t k,
 // points around each query in Morton order and need no radius rounds: their
 // result is the same for every starting radius.
 enum class Search { thread_window, collect, rounds };
-// lanes_per_query = 0 (auto).  Exact searches: a warp per query for k > 12
-// and for few queries.  A thread's list of 16 costs as much as the warp's
-// whole search (400,000 queries, k = 16, thread / warp, ms: clustered 1.54 /
-// 1.56, uniform 1.37 / 1.38; 1M on a sheet 4.2 / 3.6 and 7.0 / 4.6; k = 12:
-// 1.25 / 1.43; k = 8: 0.62 / 1.32).  A thread's search is a serial chain that
-// takes about as long for 1,000 queries as for 100,000, while the warp's
-// grows with their number: 100,000 uniform points, us: k = 5: 10,000 queries
-// 141 / 40, 100,000 156 / 265; k = 8: 50,000 180 / 170; the two cross near
-// 8,000 k queries.  Searches with partial_results: a warp for k > 16.
-constexpr uint32_t THREAD_MAX_K = 12;
-constexpr uint64_t WARP_QUERIES_PER_K = 8000;
-static uint32_t search_lanes(const rtd_schedule &s, uint64_t nq, uint32_t k) {
+// lanes_per_query = 0 (auto).  Exact searches: a warp per query for long lists
+// and for few queries.  A thread's search is a serial chain that takes about
+// as long for 1,000 queries as for 100,000, while the warp's grows with their
+// number; measured with the ordering of the queries that the thread needs, the
+// two cross at 27,000 queries for k = 1, 38,000 for 3, 44,000 for 5, 56,000
+// for 8 (3,000 to 1.8M points, within 15 % of it; k = 5 on 100,000 uniform
+// points, us: 20,000 queries 139 / 73, 90,000 151 / 243).  A thread's list of
+// 16 costs as much as the warp's whole search where the points are many
+// (400,000 queries, k = 16, thread / warp, ms: 1.8M clustered 1.54 / 1.56,
+// uniform 1.37 / 1.38; 1M on a sheet 4.2 / 3.6 and 7.0 / 4.6; k = 12: 1.25 /
+// 1.43; k = 8: 0.62 / 1.32), and less where they are few and hundreds of
+// thousands of queries share the L1 caches' lines: the lines cross at 110,000
+// queries for k = 16 on 10,000 points, at 200,000 on 80,000 points.  Searches
+// with partial_results: a warp for k > 16.
+static bool thread_search(uint64_t n, uint64_t nq, uint32_t k) {
+    if (k <= 8) return nq > 22000 + 4500 * (uint64_t)k;
+    if (k <= 12) return nq > 8000 * (uint64_t)k;
+    return k <= 16 && n <= 131072 && nq > 12000 * (uint64_t)k;
+}
+static uint32_t search_lanes(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
     uint32_t lanes = s.lanes_per_query;
-    if (lanes == 0)
-        lanes = (s.partial_results ? k <= 16 : k <= THREAD_MAX_K && nq > WARP_QUERIES_PER_K * k) ? 1 : 32;
+    if (lanes == 0) lanes = (s.partial_results ? k <= 16 : thread_search(n, nq, k)) ? 1 : 32;
     if (lanes == 1 && k > 32) lanes = 32;
     return lanes;
 }
 // (n: points of the index, whose sorted keys every build of n > 0 keeps)
 static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
     if (s.partial_results || n < 2) return Search::rounds;
-    const uint32_t lanes = search_lanes(s, nq, k);
+    const uint32_t lanes = search_lanes(n, s, nq, k);
     if (lanes == 1) return Search::thread_window;
     const uint64_t kk = k < n ? k : n;
     return lanes == 32 && kk <= COLLECT_MAX_K ? Search::collect : Search::rounds;
@@ -526,7 +533,7 @@ static bool wants_order(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t
 // (nq: of the whole search, of which a may hold a chunk).
 static rtd_status launch_search(rtd_index *idx, const rtd_schedule &s, uint64_t nq, uint32_t k, KnnArgs a,
                                 cudaStream_t st) {
-    const uint32_t lanes = search_lanes(s, nq, k);
+    const uint32_t lanes = search_lanes(idx->n, s, nq, k);
     const uint32_t block = s.block_size;
     const Search mode = search_mode(idx->n, s, nq, k);
     rtd_status r;
