@@ -4,13 +4,13 @@ cache keyed by workload features.
 The reference tunes its Schedule offline and stores one gprt_wisdom.json per
 dataset (gprt-sandbox/src/main.rs:53-77; grid + subsample funnel in
 gprt-profiler/src/main.rs:40-126; hill-climb in gprt-macros/src/lib.rs:
-120-214).  Here the knobs are the LBVH leaf size and key width, the
-initial-radius heuristic (sampled 1-NN radius with its multiplier and growth
-factor, or the Morton-window seed), the block size and the traversal mode
-(thread or warp per query) for the k-NN and range searches, the batched
-schedule, and the Barnes-Hut leaf bucket.  Every candidate returns identical
-results (exact search), so the tuner only times them; it still checks each
-candidate's ids against the first candidate's and refuses one that differs.
+120-214).  Here the knobs are the LBVH leaf size and key width, the block size
+and the traversal mode (thread or warp per query) for the k-NN and range
+searches, the initial-radius heuristic where a search still runs radius rounds
+(lists of more than 2,048 entries), the batched schedule, and the Barnes-Hut
+leaf bucket.  Every candidate returns identical results (exact search), so the
+tuner only times them; it still checks each candidate's ids against the first
+candidate's and refuses one that differs.
 
 Cache key (WorkloadKey): kind (knn / range / batch / bh), the point and query
 counts as powers of two, the k class (1, <=8, <=16, <=32, <=64, <=256, >256)
@@ -215,27 +215,51 @@ def save(key: WorkloadKey, schedule: _capi.Schedule | None, meta: dict,
 
 
 # ------------------------------------------------------------------ tuners
-def _candidates(grid: dict, k: int) -> list[dict]:
-    keys = list(grid)
-    cands, seen = [], set()
-    for combo in itertools.product(*(grid[k_] for k_ in keys)):
-        kw = dict(zip(keys, combo))
+# the longest lists that exact searches collect without radius rounds: of one
+# index, of a batch (and of its lists a thread per query)
+COLLECT_MAX_K = 2048
+BATCH_COLLECT_MAX_K = 512
+
+
+def _first(grid: dict, kw: dict, *names: str) -> None:
+    """Knobs that a candidate's kernels do not read take the grid's first value."""
+    for name in names:
+        if name in kw:
+            kw[name] = grid[name][0]
+
+
+def _unique(cands: list[dict]) -> list[dict]:
+    return [dict(c) for c in dict.fromkeys(tuple(sorted(c.items())) for c in cands)]
+
+
+def _candidates(grid: dict, k: int, n: int) -> list[dict]:
+    cands = []
+    for combo in itertools.product(*grid.values()):
+        kw = dict(zip(grid, combo))
         mode = kw.pop("mode", "thread")
         if mode != "warp" and k > 16:
             continue
-        if kw.get("radius_heuristic") == _capi.RADIUS_MORTON_WINDOW:
-            if mode != "thread":
-                continue   # the window seed runs in the thread-per-query kernel only
-            # one unbounded round: the radius knobs do not apply
-            kw["radius_param"] = grid.get("radius_param", [0.5])[0]
-            kw["radius_increment_mult"] = grid.get("radius_increment_mult", [2.0])[0]
+        if min(k, n) <= COLLECT_MAX_K:
+            # exact searches start from the Morton order: no radius rounds
+            _first(grid, kw, "radius_heuristic", "radius_param", "radius_increment_mult")
+            if mode == "warp":
+                _first(grid, kw, "block_size")
+        elif kw.get("radius_heuristic") == _capi.RADIUS_MORTON_WINDOW:
+            continue   # (rounds treat it as RADIUS_SAMPLED_NN)
         kw.update(_MODES[mode])
-        key = tuple(sorted(kw.items()))
-        if key in seen:
-            continue
-        seen.add(key)
         cands.append(kw)
-    return cands
+    return _unique(cands)
+
+
+def _batch_candidates(grid: dict, sizes) -> list[dict]:
+    """sizes: (points, queries, k) of every cloud."""
+    cands = []
+    for combo in itertools.product(*grid.values()):
+        kw = dict(zip(grid, combo))
+        if all(min(k, n) <= BATCH_COLLECT_MAX_K for n, nq, k in sizes if nq):
+            _first(grid, kw, "radius_param", "radius_increment_mult")
+        cands.append(kw)
+    return _unique(cands)
 
 
 def _funnel(cands: list[dict], nq: int, time_fn, funnel=FUNNEL, log=None):
@@ -296,7 +320,7 @@ def tune_knn(P, Q, k: int, grid: dict | None = None, reps: int = 3, funnel=FUNNE
     def time_fn(kw, m):
         return _time_knn(P, Q[perm[:m]].contiguous(), k, _capi.default_schedule(**kw), reps)
 
-    table = _funnel(_candidates(grid, k), nq, time_fn, funnel, log)
+    table = _funnel(_candidates(grid, k, int(P.shape[0])), nq, time_fn, funnel, log)
     best_ms, best_kw = table[0]
     best = _capi.default_schedule(**best_kw)
     key = knn_key(P.shape[0], nq, k, dist or describe(P))
@@ -309,7 +333,6 @@ def tune_knn(P, Q, k: int, grid: dict | None = None, reps: int = 3, funnel=FUNNE
 RANGE_GRID = {
     "leaf_size": [8, 12, 16],
     "morton_bits": [42, 48],
-    "block_size": [128, 256],
 }
 
 
@@ -369,11 +392,9 @@ def tune_batch(P, Q, sizes, grid: dict | None = None, reps: int = 3, save_result
     import torch
     from .batch import Batch
     grid = grid or BATCH_GRID
-    keys = list(grid)
     table = []
     ref_ids = None
-    for combo in itertools.product(*(grid[k_] for k_ in keys)):
-        kw = dict(zip(keys, combo))
+    for kw in _batch_candidates(grid, sizes):
         s = _capi.default_batch_schedule(**kw)
         b = Batch(sizes, s)
         ids = torch.empty(max(b.n_out, 1), dtype=torch.int32, device=Q.device)
