@@ -20,10 +20,12 @@ name.  A lookup takes the exact key, else the entry of the same kind, k
 class, distribution and GPU whose sizes are nearest (at most a factor 4 in
 points and in queries), else the defaults.
 
-Funnel (tune_knn / tune_range), after the profiler's: every candidate on a
+Funnel (tune_knn), after the profiler's: every candidate on a
 5,000-query subsample, the best 20 on 25,000 queries, the best 5 on 100,000
-(or all) queries, the fastest of those wins.  The points stay at full size
-(the build is part of every step here).
+(or all) queries, the fastest of those wins; thread- and warp-per-query
+candidates each for themselves, their winners then on all queries.  The points
+stay at full size (the build is part of every step here).  tune_range has few
+candidates and times each on all queries, whose number says which kernels run.
 """
 from __future__ import annotations
 
@@ -264,27 +266,44 @@ def _batch_candidates(grid: dict, sizes) -> list[dict]:
 
 def _funnel(cands: list[dict], nq: int, time_fn, funnel=FUNNEL, log=None):
     """Runs the funnel: time_fn(kw, n_queries) -> (ms, ids); returns the
-    final stage's [(ms, kw)] sorted, fastest first."""
+    final stage's [(ms, kw)] sorted, fastest first.
+
+    Candidates with different lanes_per_query go through it by themselves,
+    and what is left of each is timed on all queries: a warp per query is
+    several times faster than a thread per query for a few thousand queries
+    and slower for a few hundred thousand, so a small stage says nothing about
+    the choice between them."""
     import torch
-    stage = [(None, kw) for kw in cands]
     ref = {}
-    for target, keep in funnel:
-        m = min(target, nq)
-        timed = []
+
+    def timed(stage, m):
+        out = []
         for _, kw in stage:
             ms, ids = time_fn(kw, m)
             if m not in ref:
                 ref[m] = ids.clone()
             elif not bool(torch.equal(ids, ref[m])):
                 raise RuntimeError(f"autotune: candidate {kw} returned different neighbours")
-            timed.append((ms, kw))
+            out.append((ms, kw))
             if log:
                 log(f"stage {m} queries: {ms:.4f} ms {kw}")
-        timed.sort(key=lambda x: x[0])
-        stage = timed[:keep] if keep else timed
-        if m == nq:
-            break
-    return stage
+        return sorted(out, key=lambda x: x[0])
+
+    left = []
+    lanes = list(dict.fromkeys(kw.get("lanes_per_query") for kw in cands))
+    for of in lanes:
+        stage = [(None, kw) for kw in cands if kw.get("lanes_per_query") == of]
+        for target, keep in funnel:
+            m = min(target, nq)
+            stage = timed(stage, m)
+            stage = stage[:keep] if keep else stage
+            if m == nq:
+                break
+        left += stage
+    if len(lanes) > 1:
+        keep = funnel[-1][1]
+        left = (timed(left, nq) if m < nq else sorted(left, key=lambda x: x[0]))[:keep or None]
+    return left
 
 
 def _time_knn(P, Q, k, s, reps: int):
@@ -330,6 +349,8 @@ def tune_knn(P, Q, k: int, grid: dict | None = None, reps: int = 3, funnel=FUNNE
     return best, table, key
 
 
+RANGE_FUNNEL = ((1 << 30, 1),)   # one stage, of all queries
+
 RANGE_GRID = {
     "leaf_size": [8, 12, 16],
     "morton_bits": [42, 48],
@@ -337,7 +358,7 @@ RANGE_GRID = {
 
 
 def tune_range(P, Q, radius: float, mean_neighbours: float, grid: dict | None = None,
-               reps: int = 3, funnel=FUNNEL, save_result: bool = True, path: str | None = None,
+               reps: int = 3, funnel=RANGE_FUNNEL, save_result: bool = True, path: str | None = None,
                dist: str | None = None, log=None):
     """Times build + count + fill for every grid point through the funnel
     (pairs compared as sorted (query, id) lists); caches the winner."""

@@ -1,4 +1,6 @@
-"""Which schedules the autotuner times: no two that run the same kernels."""
+"""Which schedules the autotuner times, and on how many queries: no two that
+run the same kernels, and a thread against a warp per query on all queries."""
+import torch
 
 
 def grid(rtd):
@@ -32,3 +34,33 @@ def test_batches_sweep_the_radius_for_long_lists_only(rtd):
          "lanes_per_query": [0, 32]}
     assert len(autotune._batch_candidates(g, [(1_000, 10, 5), (9_000, 10, 512), (100, 10, 900), (9_000, 0, 900)])) == 4
     assert len(autotune._batch_candidates(g, [(1_000, 10, 5), (9_000, 10, 513)])) == 24
+
+
+def test_modes_are_compared_on_all_queries(rtd):
+    """A warp per query is ahead up to 50,000 queries, a thread per query
+    beyond, as the searches are."""
+    from rtdsl import autotune
+    asked = []
+
+    def time_fn(kw, m):
+        asked.append((kw["lanes_per_query"], m))
+        ms = 0.15 + kw["leaf_size"] * 1e-3 if kw["lanes_per_query"] == 1 else m * 2.5e-6 + kw["leaf_size"] * 1e-3
+        return ms, torch.zeros(m, dtype=torch.int32)
+
+    cands = autotune._candidates(grid(rtd), 5, 1_000_000)
+    for nq, lanes in ((400_000, 1), (100_000, 1), (20_000, 32), (3_000, 32)):
+        asked.clear()
+        table = autotune._funnel(cands, nq, time_fn)
+        assert len(table) == 1 and table[0][1]["lanes_per_query"] == lanes and table[0][1]["leaf_size"] == 2
+        assert {x for x, m in asked if m == nq} == {1, 32}
+
+
+def test_different_neighbours_are_refused_across_modes(rtd):
+    import pytest
+    from rtdsl import autotune
+
+    def time_fn(kw, m):
+        return 1.0, torch.full((m,), kw["lanes_per_query"], dtype=torch.int32)
+
+    with pytest.raises(RuntimeError, match="different neighbours"):
+        autotune._funnel(autotune._candidates(grid(rtd), 5, 1_000), 100, time_fn)
