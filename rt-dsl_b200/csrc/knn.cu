@@ -398,10 +398,11 @@ rtd_status launch_wide(rtd_index *idx, const KnnArgs &a, cudaStream_t st) {
     const uint64_t warps = a.nq;
     if (kk <= WIDE_SMEM_MAX_K) {
         const size_t smem = (size_t)WIDE_WARPS * kk * sizeof(uint2);
-        // the opt-in above 48 KB is per device, set once on each (an eager
-        // search always comes before a captured one)
+        // the opt-in above 48 KB (which the kernel's own arrays count towards) is
+        // per device, set once on each (an eager search always comes before a
+        // captured one)
         static std::atomic<uint64_t> opted{0};
-        if (smem > 48 * 1024 && (idx->device >= 64 || !(opted.load() >> idx->device & 1u))) {
+        if (idx->device >= 64 || !(opted.load() >> idx->device & 1u)) {
             RTD_CUDA(cudaFuncSetAttribute(knn_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)(WIDE_WARPS * WIDE_SMEM_MAX_K * sizeof(uint2))));
             if (idx->device < 64) opted.fetch_or(1ull << idx->device);
