@@ -786,6 +786,10 @@ __global__ void __launch_bounds__(128) bh_finish_grad_kernel(const BhView v, con
 // tiles part empty.  Measured, a warp / a block per group, ms (forward;
 // adjoint): 10,000 bodies 0.45 / 0.34; 0.58 / 0.42, 16,000: 0.51 / 0.33; 0.67
 // / 0.51, 30,000: 0.62 / 0.54; 0.90 / 0.95, 100,000: 0.97 / 1.25; 2.1 / 3.2.
+// rtd_bh_forward_noalloc, whose results are the same bits, follows the same
+// rule, although its 148 blocks then take several groups in turn (whole call
+// 4,000: 0.32 / 0.14, 10,000: 0.44 / 0.42, 16,000: 0.49 / 0.63, 23,600: 0.68 /
+// 1.03; 1.5 ms before groups were shared or walked by their box).
 inline bool split_groups(uint64_t n) { return n <= (uint64_t)NUM_SMS_HINT * 5 * BH_GROUP; }
 
 template <bool QUAD, bool ADJ, int SPLIT>
