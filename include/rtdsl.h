@@ -137,9 +137,11 @@ rtd_status rtd_index_info_get(rtd_index *idx, rtd_index_info *info, rtd_stream s
  * 314-340): when enabled, the index records CUDA events around its phases
  * on the caller's stream; rtd_index_profile_get waits for them. */
 typedef struct rtd_profile {
-    float build_sort_ms;   /* scene box + Morton codes + radix sort + point gather */
-    float build_tree_ms;   /* Karras tree + leaf collapse + child boxes + top staging */
-    float seed_ms;         /* initial-radius seed */
+    float build_sort_ms;   /* scene box + Morton codes + radix sort + point gather; up to
+                              4,096 points, which build in one launch, the whole build */
+    float build_tree_ms;   /* Karras tree + leaf collapse + child boxes + top staging
+                              (about 0 up to 4,096 points) */
+    float seed_ms;         /* initial-radius seed (about 0 where no radius rounds run) */
     float order_ms;        /* query Morton ordering */
     float search_ms;       /* the search kernel (kNN or range count + fill) */
 } rtd_profile;

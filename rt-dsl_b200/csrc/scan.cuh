@@ -1,6 +1,6 @@
 // scan.cuh -- exclusive scan as a count kernel and an apply kernel over
-// fixed tiles, for any input read through a functor (sort.cu scans arrays;
-// lbvh.cu scans the Karras keep flags computed from the sorted keys).
+// fixed tiles, and the prefix levels and zeroing that the sort and the tree
+// build share with it.
 //
 // The count kernel writes each tile's sum and adds it into the sums of its
 // group (32 tiles) and super group (32 groups); the apply kernel takes the
@@ -41,20 +41,13 @@ inline rtd_status zero_words(uint32_t *p, uint64_t count, cudaStream_t stream) {
     return RTD_OK;
 }
 
-// Scan input: an array.
-struct ArrayIn {
-    const uint32_t *in;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return in[i]; }
-};
-
 constexpr int SC_BLOCK = 256;
 constexpr int SC_ITEMS = 8;
 constexpr int SC_TILE = SC_BLOCK * SC_ITEMS;
 
 // Scan counts: each tile's sum in tsum[tile], added into its group's sum
 // and, with more than one super group, its super group's.
-template <typename In>
-__global__ void __launch_bounds__(SC_BLOCK) scan_count_kernel(const In in, uint64_t n,
+__global__ void __launch_bounds__(SC_BLOCK) scan_count_kernel(const uint32_t *__restrict__ in, uint64_t n,
                                                               uint64_t *__restrict__ tsum,
                                                               unsigned long long *gsum,
                                                               unsigned long long *ssum, int supers) {
@@ -66,7 +59,7 @@ __global__ void __launch_bounds__(SC_BLOCK) scan_count_kernel(const In in, uint6
 #pragma unroll
     for (int i = 0; i < SC_ITEMS; ++i) {
         const uint64_t idx = base + (uint64_t)i * SC_BLOCK + tid;
-        if (idx < n) sum += in(idx);
+        if (idx < n) sum += in[idx];
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -87,11 +80,11 @@ __global__ void __launch_bounds__(SC_BLOCK) scan_count_kernel(const In in, uint6
 // Scan output: out[i] = prefix of the tile (the sums of the earlier tiles
 // of its group, earlier groups of its super group and earlier super groups)
 // + the block's exclusive scan within the tile.  With select != nullptr,
-// also select[out[i]] = i for every i with in(i) != 0 (stream compaction
+// also select[out[i]] = i for every i with in[i] != 0 (stream compaction
 // of the indices of flagged entries).
-template <typename In, typename OutT>
+template <typename OutT>
 __global__ void __launch_bounds__(SC_BLOCK) scan_apply_kernel(
-    const In in, OutT *__restrict__ out, uint64_t n, OutT *d_total,
+    const uint32_t *in, OutT *__restrict__ out, uint64_t n, OutT *d_total,
     const uint64_t *__restrict__ tsum, const uint64_t *__restrict__ gsum,
     const uint64_t *__restrict__ ssum, uint64_t ntiles, uint32_t *select) {
     chain_wait();
@@ -115,7 +108,7 @@ __global__ void __launch_bounds__(SC_BLOCK) scan_apply_kernel(
     }
     for (int i = tid; i < SC_TILE; i += SC_BLOCK) {
         uint64_t idx = base + i;
-        s_io[i] = idx < n ? (uint64_t)in(idx) : 0ull;
+        s_io[i] = idx < n ? (uint64_t)in[idx] : 0ull;
     }
     __syncthreads();
     uint64_t v[SC_ITEMS];
@@ -162,10 +155,10 @@ __global__ void __launch_bounds__(SC_BLOCK) scan_apply_kernel(
     }
 }
 
-// Exclusive scan of in(0 .. n) into out (and *d_total, device), with the
+// Exclusive scan of in[0 .. n) into out (and *d_total, device), with the
 // stream compaction above when select != nullptr.
-template <typename In, typename OutT>
-rtd_status scan_impl(const In in, OutT *out, uint64_t n, OutT *d_total, ScanScratch &scr,
+template <typename OutT>
+rtd_status scan_impl(const uint32_t *in, OutT *out, uint64_t n, OutT *d_total, ScanScratch &scr,
                      cudaStream_t stream, uint32_t *select = nullptr) {
     if (n == 0) {
         if (d_total) RTD_CUDA(cudaMemsetAsync(d_total, 0, sizeof(OutT), stream));
@@ -177,10 +170,10 @@ rtd_status scan_impl(const In in, OutT *out, uint64_t n, OutT *d_total, ScanScra
     uint64_t *tsum = scr.sums.as<uint64_t>();
     uint64_t *gsum = tsum + L.tiles, *ssum = gsum + L.groups;
     RTD_TRY(zero_words(reinterpret_cast<uint32_t *>(gsum), 2 * (L.groups + L.supers), stream));
-    RTD_LAUNCH_CHAINED(scan_count_kernel<In>, dim3((unsigned)L.tiles), dim3(SC_BLOCK), 0, stream, in,
+    RTD_LAUNCH_CHAINED(scan_count_kernel, dim3((unsigned)L.tiles), dim3(SC_BLOCK), 0, stream, in,
                        n, tsum, reinterpret_cast<unsigned long long *>(gsum),
                        reinterpret_cast<unsigned long long *>(ssum), (int)L.supers);
-    RTD_LAUNCH_CHAINED((scan_apply_kernel<In, OutT>), dim3((unsigned)L.tiles), dim3(SC_BLOCK), 0,
+    RTD_LAUNCH_CHAINED(scan_apply_kernel<OutT>, dim3((unsigned)L.tiles), dim3(SC_BLOCK), 0,
                        stream, in, out, n, d_total, (const uint64_t *)tsum, (const uint64_t *)gsum,
                        (const uint64_t *)ssum, L.tiles, select);
     return RTD_OK;

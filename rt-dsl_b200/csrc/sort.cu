@@ -492,18 +492,18 @@ template rtd_status radix_sort_pairs<uint64_t>(uint64_t *, uint64_t *, uint32_t 
 rtd_status exclusive_scan_u32(const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *d_total,
                               ScanScratch &scr, uint32_t *d_err, cudaStream_t stream) {
     (void)d_err;
-    return scan_impl<ArrayIn, uint64_t>(ArrayIn{in}, out, n, d_total, scr, stream);
+    return scan_impl<uint64_t>(in, out, n, d_total, scr, stream);
 }
 rtd_status exclusive_scan_u32_32(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *d_total,
                                  ScanScratch &scr, uint32_t *d_err, cudaStream_t stream) {
     (void)d_err;
-    return scan_impl<ArrayIn, uint32_t>(ArrayIn{in}, out, n, d_total, scr, stream);
+    return scan_impl<uint32_t>(in, out, n, d_total, scr, stream);
 }
 rtd_status exclusive_scan_select_u32(const uint32_t *in, uint32_t *out, uint32_t *select,
                                      uint64_t n, uint32_t *d_total, ScanScratch &scr,
                                      uint32_t *d_err, cudaStream_t stream) {
     (void)d_err;
-    return scan_impl<ArrayIn, uint32_t>(ArrayIn{in}, out, n, d_total, scr, stream, select);
+    return scan_impl<uint32_t>(in, out, n, d_total, scr, stream, select);
 }
 
 }  // namespace rtd
