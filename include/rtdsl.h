@@ -200,10 +200,11 @@ void rtd_limits_get(rtd_limits *l);
  * pairs, ascending, ties to the lower id; ids[q*k+j] (and d2[q*k+j] when
  * d2 != NULL).  Slots beyond the number of points hold 0xFFFFFFFF / +inf.
  * Any k >= 1, as the reference's 2K-slot per-query slab
- * (gprt-macros/src/lib.rs:300-310): k <= 12 (32 with lanes_per_query 1) keeps
- * a thread's list in registers, larger k (and small calls) collect a warp's candidates in
- * shared memory (min(k, n) <= 2048), and the largest k keep a warp's sorted
- * list in a device slab of the index (grown on demand, at most 1 GiB).
+ * (gprt-macros/src/lib.rs:300-310): k <= 12 (16 on up to 131,072 points, 32
+ * with lanes_per_query 1) keeps a thread's list in registers, larger k (and
+ * small calls) collect a warp's candidates in shared memory (min(k, n) <=
+ * 2048), and the largest k keep a warp's sorted list in a device slab of the
+ * index (grown on demand, at most 1 GiB).
  * ------------------------------------------------------------------- */
 rtd_status rtd_knn(rtd_index *idx, const float *d_queries, uint64_t nq, uint32_t k,
                    const rtd_schedule *sched, uint32_t *d_ids, float *d_d2, rtd_stream stream);

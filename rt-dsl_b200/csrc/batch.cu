@@ -14,8 +14,9 @@
 // holds the warp-per-query lists of passes with partial_results and the
 // memory lists of more than 512 entries.  256 clouds, 9M points, 2.2M
 // queries, k from {1, 5, 16, 64}: 25.0 ms with radius rounds and merged
-// warp lists, now 7.1 ms; bound by instruction issue (0.85 of the slots).  The whole pass is launch-only (no host
-// synchronisation), so it can be captured as one CUDA graph and replayed.
+// warp lists, now 6.4 ms; bound by instruction issue (0.85 of the slots).
+// The whole pass is launch-only (no host synchronisation), so it can be
+// captured as one CUDA graph and replayed.
 #include <algorithm>
 #include <new>
 #include <vector>
