@@ -52,6 +52,7 @@ struct WarpTile {
     uint32_t mask[32];
     uint2 list[4][64];    // (cell or body, lane mask)
     uint4 leaf[32];       // rejected leaves not yet listed: first body, bodies, lane mask
+    uint32_t lost;        // the lanes that take a body without a place (forward)
 };
 
 // Adjoint: what the bodies' side of an interaction leaves for the source's
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 6) bh_walk_kernel(
             }
         const bool boxed = !__any_sync(0xffffffffu, isnan(me.x) || isnan(me.y) || isnan(me.z));
         int n_list[4] = {0, 0, 0, 0};   // (constant indices only)
+        if (!ADJ && lane == 0) T.lost = 0;
         int n_leaf = 0, sp = 0;
         // The adjoint replays the group's tiles from the forward's log when
         // the log holds them all; otherwise it walks the tree.
@@ -580,9 +582,16 @@ __global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 6) bh_walk_kernel(
             const int pairs = (cnt + 1) / 2;
             if (lane < 2 * pairs) {
                 const uint2 en = T.list[kind][lane < cnt ? lane : cnt - 1];
-                const bool pad = lane >= cnt;
+                bool pad = lane >= cnt;
                 float *w = reinterpret_cast<float *>(T.pair[lane >> 1]) + (lane & 1);
-                const float4 a = cells ? __ldg(&v.node_a[en.x]) : __ldg(&v.fbody[en.x]);
+                float4 a = cells ? __ldg(&v.node_a[en.x]) : __ldg(&v.fbody[en.x]);
+                if (!ADJ && masked && !cells && (isnan(a.x) || isnan(a.y) || isnan(a.z))) {
+                    // 1 / r masked to 0 times an r that is no number would be
+                    // no number: such a body reaches its lanes at the end
+                    if (!pad) atomicOr(&T.lost, en.y);
+                    pad = true;
+                    a = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
                 w[0] = -a.x;
                 w[2] = -a.y;
                 w[4] = -a.z;
@@ -684,6 +693,7 @@ __global__ void __launch_bounds__(WW * 32, ADJ ? 3 : 6) bh_walk_kernel(
             atomicAdd(&hm->ilog_need, (nt + ILOG_PAGE - 1) / ILOG_PAGE);
         }
         float4 sum = make_float4(lo(ax) + hi(ax), lo(ay) + hi(ay), lo(az) + hi(az), lo(phi) + hi(phi));
+        if (!ADJ && (T.lost & mine)) sum = make_float4(NAN, NAN, NAN, NAN);
         if (!ADJ && SPLIT > 1) {   // the first warp adds up the others' sums
             float4 *sums = T.pair[0];
             sums[lane] = sum;
