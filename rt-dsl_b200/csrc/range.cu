@@ -38,6 +38,7 @@ struct RangeArgs {
     uint32_t *counts;
     uint32_t *most;            // counts and MODE_SAMPLE: the largest count
     int by_sample;             // the sample of the queries says which kernel runs (warp_walks)
+    int small_leaves;          // the tree's leaves hold fewer than 6 points
     uint64_t sample_step;      // MODE_SAMPLE: every sample_step-th query
     uint32_t *sample_sum;      // MODE_SAMPLE: the sum of the counts
     uint2 *pairs;
@@ -59,10 +60,10 @@ struct RangeArgs {
 // SAMPLE of the nq queries (launch_pass says why the lines lie here).
 constexpr uint64_t SAMPLE = 1024;
 template <int MODE>
-__device__ __forceinline__ bool warp_walks(const IndexHeader *h, uint64_t nq) {
+__device__ __forceinline__ bool warp_walks(const IndexHeader *h, uint64_t nq, int small_leaves) {
     const uint64_t sum = h->sample_sum, most = h->sample_most;
     if (sum >= 64 * SAMPLE || most * SAMPLE >= nq) return true;
-    return sum * sum * (MODE == MODE_CPUSH ? 2800 : 100) >= nq * SAMPLE * SAMPLE;
+    return MODE == MODE_CPUSH && small_leaves && sum * sum * 2800 >= nq * SAMPLE * SAMPLE;
 }
 
 // Shared memory of one warp: the boxes to visit (level << 28 | entry), runs
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(RBLOCK, 10) range_kernel(const RangeArgs p) {
     constexpr bool SEG = MODE == MODE_SEG;
     constexpr bool COUNTS = MODE == MODE_COUNT || MODE == MODE_CPUSH;
     if (SEG && p.skip_if_same && p.ix.hdr->qfp[0] == p.ix.hdr->qfp[1]) return;
-    if (MODE != MODE_SAMPLE && p.by_sample && !warp_walks<MODE>(p.ix.hdr, p.nq)) return;
+    if (MODE != MODE_SAMPLE && p.by_sample && !warp_walks<MODE>(p.ix.hdr, p.nq, p.small_leaves)) return;
     extern __shared__ uint4 s_dyn[];
     __shared__ uint32_t s_off[12];
     const uint32_t n = (uint32_t)p.ix.n;
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(RBLOCK, MODE == MODE_COUNT ? 10 : 8) range_thr
     constexpr bool COUNTS = MODE == MODE_COUNT || MODE == MODE_CPUSH;
     constexpr bool SEG = MODE == MODE_SEG, FILL = !COUNTS;
     constexpr int NF = SEG ? F_SEG : FILL ? F_PUSH : F_COUNT;
-    if (warp_walks<MODE>(p.ix.hdr, p.nq)) return;
+    if (warp_walks<MODE>(p.ix.hdr, p.nq, p.small_leaves)) return;
     __shared__ BvhNode s_top[TOP_MAX];
     __shared__ uint2 s_stack[SHORT_DEPTH][RBLOCK];
     __shared__ uint2 s_buf[PUSH ? RWARPS : 1][PUSH ? WBUF : 1];
@@ -948,32 +949,31 @@ rtd_status launch_range(RangeArgs &a, cudaStream_t st) {
 }
 
 // Which kernel counts or fills.  A thread per query costs less where the hits
-// are few: the warp kernel takes about 1.8 ns a query besides the hits.  But a
-// warp of 32 threads takes as long as its longest walk, some 1.1 us for each
-// of that query's hits, and the last such warp ends the launch: the warp
-// kernel is ahead with fewer than 500 to 1,000 queries for every hit of the
-// largest query (1,024 for the largest of a sample, which misses the top).
-// And it is ahead from some mean number of hits on, which grows as the root of
-// the number of queries:
-// 400,000 queries fill the SMs with threads, 100,000 do not, and the threads'
-// pushes (one reservation for every step of a warp) queue up on the cursors.
-// Measured, thread / warp, us; 1.8M points:
-//                       400,000 queries: count  segment fill  pushing count
-//   uniform     1 hit              152 / 491     170 / 526     184 / 529
-//               8                  363 / 645     396 / 701     610 / 690
-//               12                 427 / 680     471 / 744     834 / 731
-//               50                 774 / 905    902 / 1016   2240 / 1002
-//   clustered   8, 308 at most     408 / 773     537 / 830     620 / 819
-//               20, 802            663 / 830     998 / 903    1157 / 893
-//               50, 1849          1109 / 921   1845 / 1011   2079 / 1014
-//                       100,000 queries:
-//   uniform     1 hit               75 / 133      72 / 144      82 / 150
-//               8                  142 / 173     141 / 189     223 / 194
-//               32                 221 / 216     248 / 240     524 / 246
-//   clustered   1, 32 at most      145 / 189     143 / 202     168 / 209
-//               4, 145             234 / 201     282 / 210     320 / 216
-//   1.8M clustered points as their own queries, 20 hits, 813 at most:
-//                                1431 / 3611   1867 / 3955   3469 / 3910
+// are few: the warp kernel takes about 1.8 ns a query besides the hits.  The
+// warp kernel is ahead from some 64 hits a query on, and earlier where a few
+// queries find most: a warp of 32 threads takes as long as its longest walk,
+// some 1.1 us for each of that query's hits, and the last such warp ends the
+// launch, which shows with fewer than 500 to 1,000 queries for every hit of
+// the largest query (1,024 for the largest of a sample, which misses the top).
+// Pushing counts over leaves of 4 points change over earlier: a record for
+// every such leaf inside the ball takes two reservations a step of a warp, and
+// these queue up on the cursors; the line grows as the root of the number of
+// queries.  Measured, thread / warp, us; 1.5M points, 400,000 queries:
+//                             count  segment fill  pushing count, leaves of 4 / 12
+//   uniform     4 hits    267 / 596     297 / 646     373 / 633     317 / 637
+//               16        424 / 725     490 / 796    1016 / 787     518 / 784
+//               50        677 / 905    794 / 1013   2213 / 1008    860 / 1000
+//               62        750 / 960    893 / 1079   2554 / 1074    996 / 1071
+//   clustered   8         395 / 750     512 / 802     625 / 803     512 / 797
+//               24        724 / 813    1072 / 884    1302 / 884     995 / 879
+//               50       1036 / 891    1672 / 975    2064 / 985    1429 / 973
+//   the points as queries, 24 hits:
+//   uniform             1416 / 2787   1757 / 3106   4556 / 3048   1855 / 3037
+//   clustered           1208 / 2930   1621 / 3213   3411 / 3181   1572 / 3170
+//   140,000 queries:
+//   uniform     8         157 / 237     165 / 260     297 / 262     217 / 264
+//               50        269 / 335     313 / 375     876 / 379     450 / 377
+//   clustered   4         254 / 260     303 / 276     350 / 282     315 / 281
 // The queries have to be in order for the threads' walks (50 us), before the
 // sample can say which kernel runs, which decides below THREAD_QUERIES: count
 // and first fill of 100,000 queries on 1.8M uniform points with it, 1 hit 200
@@ -981,7 +981,8 @@ rtd_status launch_range(RangeArgs &a, cudaStream_t st) {
 // order, then a warp a query) / 270; 50,000 queries, 1 hit 180 / 163, 8 hits
 // 289 / 205.  The sample runs on the side stream beside the ordering.
 template <int MODE>
-rtd_status launch_pass(RangeArgs &a, cudaStream_t st) {
+rtd_status launch_pass(const rtd_index *idx, RangeArgs &a, cudaStream_t st) {
+    a.small_leaves = idx->leaf_size < 6;
     a.by_sample = a.nq >= THREAD_QUERIES;
     if (a.by_sample) {
         range_thread_kernel<MODE><<<grid_for(a.nq, RBLOCK, 1 << 20), RBLOCK, 0, st>>>(a);
@@ -1043,9 +1044,9 @@ rtd_status range_count(rtd_index *idx, const float *d_q, uint64_t nq, float r,
             a.recs = idx->rrec.as<uint4>();
             a.rec_cap = idx->rrec_cap;
             RTD_TRY(query_fingerprint(d_q, nq, &h->qfp[0], st));
-            RTD_TRY(launch_pass<MODE_CPUSH>(a, st));
+            RTD_TRY(launch_pass<MODE_CPUSH>(idx, a, st));
         } else {
-            RTD_TRY(launch_pass<MODE_COUNT>(a, st));
+            RTD_TRY(launch_pass<MODE_COUNT>(idx, a, st));
         }
         idx->mark(EV_SEARCH1, st);
         RTD_TRY(idx->roffsets.reserve(nq * sizeof(uint64_t)));
@@ -1162,10 +1163,10 @@ rtd_status range_fill(rtd_index *idx, const float *d_q, uint64_t nq, float r,
         RTD_TRY(launch_range<MODE_SEG>(a, st));
         idx->mark(EV_SEARCH1, st);
     } else if (seg) {   // (the count's sample of the queries still stands)
-        RTD_TRY(launch_pass<MODE_SEG>(a, st));
+        RTD_TRY(launch_pass<MODE_SEG>(idx, a, st));
         idx->mark(EV_SEARCH1, st);
     } else if (nq) {
-        RTD_TRY(launch_pass<MODE_PUSH>(a, st));
+        RTD_TRY(launch_pass<MODE_PUSH>(idx, a, st));
         idx->mark(EV_SEARCH1, st);
     }
     unsigned long long total = 0;
