@@ -10,8 +10,7 @@
 //      core point.  Every core point starts under its smallest core
 //      neighbour, and the paths are compressed before the pairs are united:
 //      most pairs then share a parent and need two loads (200,000 clustered
-//      points, 3.9M pairs: 204 -> 116 us; uniform points in one component see
-//      dbscan_hook_kernel's launches);
+//      points, 3.9M pairs: 204 -> 116 us);
 //   4. clusters numbered by a scan over roots in point order (the order of
 //      their smallest core point), core points take their root's number;
 //   5. a non-core point takes the smallest number among its core neighbours
@@ -67,17 +66,19 @@ __global__ void dbscan_init_kernel(const uint32_t *__restrict__ counts, uint64_t
 // since the count): the kernels that read pairs, and those that write labels,
 // return at once.
 
-// Every core point's parent under the smallest parent of its core neighbours,
-// at first the neighbours themselves.  A parent linked twice loses its first
-// link; the union visits every pair again.
+// Core points under their smallest core neighbour, or (PARENTS) every core
+// point's parent under the smallest parent of its core neighbours, at first
+// the neighbours themselves.  A parent linked twice loses its first link; the
+// union visits every pair again.
+template <bool PARENTS>
 __global__ void dbscan_hook_kernel(const uint2 *__restrict__ pairs, uint64_t n_pairs,
                                    const uint8_t *__restrict__ core, uint32_t *parent, const uint32_t *err) {
     if (*err) return;
     for (uint64_t t = (uint64_t)blockIdx.x * BLOCK + threadIdx.x; t < n_pairs;
          t += (uint64_t)gridDim.x * BLOCK) {
         const uint2 pr = pairs[t];
-        if (!core[pr.x] || !core[pr.y]) continue;
-        const uint32_t a = parent[pr.x], b = parent[pr.y];
+        if ((!PARENTS && pr.y >= pr.x) || !core[pr.x] || !core[pr.y]) continue;
+        const uint32_t a = PARENTS ? parent[pr.x] : pr.x, b = PARENTS ? parent[pr.y] : pr.y;
         // (a stale parent only means an atomic that changes nothing)
         if (b < a && b < parent[a]) atomicMin(&parent[a], b);
     }
@@ -196,16 +197,18 @@ extern "C" rtd_status rtd_dbscan(rtd_index *idx, const float *d_points, uint64_t
                                             parent.as<uint32_t>());
     RTD_LAUNCH_CHECK();
     if (total) {
-        // A second round where the points have few neighbours: one then leaves
-        // many roots, and the union of a component that spans the cloud meets
-        // all of them (uniform points, one / two rounds, ms: 1.5M with 5
-        // neighbours 2.26 / 2.04, 500,000 with 8 1.49 / 1.39, with 40 3.25 /
-        // 3.36; clustered, 500,000 with 8 1.05 / 1.06, with 20 1.32 / 1.40).
-        // Below 131,072 points its two launches cost more than it saves.
-        const int rounds = n >= 131072 && total < 16 * n ? 2 : 1;
+        // By parents from 131,072 points on (500,000 uniform points with 22
+        // neighbours, leaves of 12: 1.76 ms by neighbours, 1.60 by parents;
+        // 30,000: 0.49 / 0.56), and in two rounds where the points have few
+        // neighbours: one then leaves many roots, and the union of a component
+        // that spans the cloud meets all of them (1.5M uniform points with 5
+        // neighbours, one / two rounds, 2.26 / 2.04 ms; with 8 3.51 / 3.38;
+        // clustered, 5: 1.70 / 1.73, 8: 2.28 / 2.36).
+        const bool many = n >= 131072;
+        const int rounds = many && total < 7 * n ? 2 : 1;
         for (int round = 0; round < rounds; ++round) {
-            dbscan_hook_kernel<<<gp, BLOCK, 0, st>>>(pairs.as<uint2>(), total, core.as<uint8_t>(),
-                                                     parent.as<uint32_t>(), err);
+            auto *hook = many ? dbscan_hook_kernel<true> : dbscan_hook_kernel<false>;
+            hook<<<gp, BLOCK, 0, st>>>(pairs.as<uint2>(), total, core.as<uint8_t>(), parent.as<uint32_t>(), err);
             RTD_LAUNCH_CHECK();
             dbscan_compress_kernel<<<g, BLOCK, 0, st>>>(n, parent.as<uint32_t>(), err);
             RTD_LAUNCH_CHECK();

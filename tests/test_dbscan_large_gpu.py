@@ -1,6 +1,6 @@
 """DBSCAN from 131,072 points on, where the queries run in the index's own order
 and a sample of them chooses the counting kernel, and on both sides of the rule
-for a second hooking round (16 neighbours a point): against labels made from
+for a second hooking round (7 neighbours a point): against labels made from
 the oracle's neighbour pairs."""
 import numpy as np
 import pytest
