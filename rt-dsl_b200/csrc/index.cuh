@@ -295,9 +295,9 @@ rtd_status index_build(rtd_index *idx, const float *d_xyz, uint64_t n, const rtd
                        cudaStream_t st);
 
 // k-NN search (knn.cu); with have_perm the query order is given (perm, or
-// nullptr for caller order) instead of computed on the index; wpos, when
-// not nullptr, holds the Morton-window positions of the queries in that
-// order.
+// nullptr for caller order) instead of computed on the index: the caller has
+// ordered them beside the build.  wpos, when not nullptr, holds the
+// Morton-window positions of the queries in that order.
 rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t k,
                          const rtd_schedule *sched, uint32_t *d_ids, float *d_d2,
                          cudaStream_t st, bool have_perm, const uint32_t *perm,

@@ -488,7 +488,12 @@ enum class Search { thread_window, collect, rounds };
 // number; measured with the ordering of the queries that the thread needs, the
 // two cross at 27,000 queries for k = 1, 38,000 for 3, 44,000 for 5, 56,000
 // for 8 (3,000 to 1.8M points, within 15 % of it; k = 5 on 100,000 uniform
-// points, us: 20,000 queries 139 / 73, 90,000 151 / 243).  A thread's list of
+// points, us: 20,000 queries 139 / 73, 90,000 151 / 243).  Where the points
+// are built in the same call (beside), the ordering runs beside the build and
+// the thread's line lies lower: at 9,000 to 16,000 queries for k = 1, 15,000
+// to 21,000 for 2, 24,000 to 34,000 for 4, 40,000 to 55,000 for 8 (3,000 to
+// 100,000 points; build and search of 27,703 clustered points, 20,000 queries,
+// k = 1: 113 / 131 us, k = 8, 34,000: 233 / 184).  A thread's list of
 // 16 costs as much as the warp's whole search where the points are many
 // (400,000 queries, k = 16, thread / warp, ms: 1.8M clustered 1.54 / 1.56,
 // uniform 1.37 / 1.38; 1M on a sheet 4.2 / 3.6 and 7.0 / 4.6; k = 12: 1.25 /
@@ -496,21 +501,21 @@ enum class Search { thread_window, collect, rounds };
 // thousands of queries share the L1 caches' lines: the lines cross at 110,000
 // queries for k = 16 on 10,000 points, at 200,000 on 80,000 points.  Searches
 // with partial_results: a warp for k > 16.
-static bool thread_search(uint64_t n, uint64_t nq, uint32_t k) {
-    if (k <= 8) return nq > 22000 + 4500 * (uint64_t)k;
+static bool thread_search(uint64_t n, uint64_t nq, uint32_t k, bool beside) {
+    if (k <= 8) return nq > (beside ? 4000 + 6500 * (uint64_t)k : 22000 + 4500 * (uint64_t)k);
     if (k <= 12) return nq > 8000 * (uint64_t)k;
     return k <= 16 && n <= 131072 && nq > 12000 * (uint64_t)k;
 }
-static uint32_t search_lanes(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
+static uint32_t search_lanes(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k, bool beside) {
     uint32_t lanes = s.lanes_per_query;
-    if (lanes == 0) lanes = (s.partial_results ? k <= 16 : thread_search(n, nq, k)) ? 1 : 32;
+    if (lanes == 0) lanes = (s.partial_results ? k <= 16 : thread_search(n, nq, k, beside)) ? 1 : 32;
     if (lanes == 1 && k > 32) lanes = 32;
     return lanes;
 }
 // (n: points of the index, whose sorted keys every build of n > 0 keeps)
-static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
+static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k, bool beside) {
     if (s.partial_results || n < 2) return Search::rounds;
-    const uint32_t lanes = search_lanes(n, s, nq, k);
+    const uint32_t lanes = search_lanes(n, s, nq, k, beside);
     if (lanes == 1) return Search::thread_window;
     const uint64_t kk = k < n ? k : n;
     return lanes == 32 && kk <= COLLECT_MAX_K ? Search::collect : Search::rounds;
@@ -525,18 +530,18 @@ static Search search_mode(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32
 // 1M queries: 4.54 / 5.59.
 constexpr uint64_t COLLECT_ORDER_MIN = 49152;
 constexpr uint64_t COLLECT_ORDER_POINTS = 2ull << 20;
-static bool wants_order(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k) {
+static bool wants_order(uint64_t n, const rtd_schedule &s, uint64_t nq, uint32_t k, bool beside) {
     return s.use_morton_lbv && !((nq < COLLECT_ORDER_MIN || n < COLLECT_ORDER_POINTS) &&
-                                 search_mode(n, s, nq, k) == Search::collect);
+                                 search_mode(n, s, nq, k, beside) == Search::collect);
 }
 
 // Launches the search kernel the schedule selects for the queries of a
 // (nq: of the whole search, of which a may hold a chunk).
-static rtd_status launch_search(rtd_index *idx, const rtd_schedule &s, uint64_t nq, uint32_t k, KnnArgs a,
-                                cudaStream_t st) {
-    const uint32_t lanes = search_lanes(idx->n, s, nq, k);
+static rtd_status launch_search(rtd_index *idx, const rtd_schedule &s, uint64_t nq, uint32_t k, bool beside,
+                                KnnArgs a, cudaStream_t st) {
+    const uint32_t lanes = search_lanes(idx->n, s, nq, k, beside);
     const uint32_t block = s.block_size;
-    const Search mode = search_mode(idx->n, s, nq, k);
+    const Search mode = search_mode(idx->n, s, nq, k, beside);
     rtd_status r;
     if (mode != Search::rounds) a.skeys = idx->skeys;
     else a.wpos = nullptr;
@@ -586,10 +591,10 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
     for (int e = EV_SEARCH0; e <= EV_SEARCH1; ++e) idx->ev_set[e] = false;
     idx->mark(EV_SEARCH0, st);
     // (only the radius rounds need an initial radius)
-    if (search_mode(idx->n, s, nq, k) == Search::rounds) RTD_TRY(seed_radius(idx, d_q, nq, k, s, st));
+    if (search_mode(idx->n, s, nq, k, have_perm) == Search::rounds) RTD_TRY(seed_radius(idx, d_q, nq, k, s, st));
     idx->mark(EV_SEEDED, st);
     const uint32_t *perm = given_perm;
-    if (!have_perm) RTD_TRY(order_queries(idx, d_q, nq, wants_order(idx->n, s, nq, k), &perm, st));
+    if (!have_perm) RTD_TRY(order_queries(idx, d_q, nq, wants_order(idx->n, s, nq, k, false), &perm, st));
     idx->mark(EV_ORDERED, st);
     KnnArgs a;
     a.ix = view_of(idx);
@@ -611,7 +616,7 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
     a.scale = idx->morton_bits == 30 ? 1023.0f : (float)((1u << (idx->morton_bits / 3)) - 1u);
     rtd_status r = RTD_OK;
     if (!hc || hc->chunks <= 1) {
-        r = launch_search(idx, s, nq, k, a, st);
+        r = launch_search(idx, s, nq, k, have_perm, a, st);
         if (r == RTD_OK && hc) {   // one chunk: copy every row out
             RTD_CUDA(cudaMemcpyAsync(hc->h_ids, d_ids, nq * (uint64_t)k * 4, cudaMemcpyDeviceToHost, st));
             if (d_d2 && hc->h_d2)
@@ -638,7 +643,7 @@ rtd_status knn_search_ex(rtd_index *idx, const float *d_q, uint64_t nq, uint32_t
                     if (a.d2) ac.d2 = a.d2 + b * k;
                 }
                 if (a.wpos) ac.wpos = a.wpos + b;
-                r = launch_search(idx, s, nq, k, ac, cs);
+                r = launch_search(idx, s, nq, k, have_perm, ac, cs);
                 if (r == RTD_OK) {
                     RTD_CUDA(cudaMemcpyAsync(hc->h_ids + b * k, d_ids + b * k, (e - b) * k * 4,
                                              cudaMemcpyDeviceToHost, cs));
@@ -668,11 +673,11 @@ rtd_status k_nn_device(rtd_index *idx, const float *d_points, uint64_t n, const 
     rtd_schedule_default(&def);
     const rtd_schedule &s = sched ? *sched : def;
     const uint32_t chunks = hc ? hc->chunks : 1u;
-    const bool order = nq >= 2 && k > 0 && wants_order(n, s, nq, k);
+    const bool order = nq >= 2 && k > 0 && wants_order(n, s, nq, k, true);
     // With the thread-per-query window search, the queries' positions among
     // the sorted keys are found on the side stream as soon as the keys are
     // sorted, while the tree is built (a warp finds its own).
-    const bool window = nq && k > 0 && search_mode(n, s, nq, k) == Search::thread_window;
+    const bool window = nq && k > 0 && search_mode(n, s, nq, k, true) == Search::thread_window;
     const bool fork = order || window || hc;   // (a host call copies its queries in on the side stream)
     RTD_TRY(ensure_side_stream(idx));
     cudaStream_t side = idx->side_stream;

@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("n,k,line", [(3_000, 1, 26_500), (3_000, 8, 58_000), (70_000, 5, 44_500), (3_000, 9, 72_000),
                                       (40_000, 12, 96_000), (700, 13, 156_000), (131_072, 16, 192_000),
-                                      (131_073, 16, 192_000), (15, 16, 192_000)])
+                                      (131_073, 16, 192_000), (15, 16, 192_000), (900, 1, 10_500), (30_000, 5, 36_500)])
 @pytest.mark.parametrize("over", [0, 1])
 def test_knn_both_sides_of_the_line(rtd, orc, cuda, n, k, line, over):
     import torch
